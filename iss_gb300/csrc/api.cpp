@@ -449,7 +449,9 @@ iss_status prepare(iss_handle* h) {
         // at this sampler's acceptance the cap shapes which cells are sampled
         if (!h->params.has("gpu_max_tries")) c.max_tries = 4999;
     }
-    c.item_size = h->tune.item_size;
+    // the lab-frame sampler gives a whole warp to each hadron: small work
+    // items keep its long chains of proposals spread over the warps
+    c.item_size = mc == 2 ? kEfaItem : h->tune.item_size;
     c.yield_groups = h->tune.yield_groups;
     c.sampler_ctas = h->tune.sampler_ctas;
     c.assign_bps = h->tune.assign_blocks;

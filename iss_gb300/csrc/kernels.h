@@ -45,6 +45,9 @@ cudaError_t launch_cdf_scan(const float* yields, int64_t N, const SurfSeg* surf,
 cudaError_t launch_counts(const DevConfig& cfg, const SpeciesDev* species, const double* totals,
                           double* pois, int32_t* counts, int32_t* items, int* error,
                           cudaStream_t stream);
+// draws per work item of the lab-frame sampler (even: the cell assignment
+// pairs draws)
+constexpr int kEfaItem = 4;
 int offsets_num_tiles(int64_t n);
 cudaError_t launch_offsets_scan(const int32_t* counts, int64_t n, int64_t* tile_sum,
                                 int64_t* offsets, cudaStream_t stream);

@@ -967,12 +967,20 @@ __device__ bool setup_efa(const DevConfig& cfg, const CellArrays& cells, const S
     return true;
 }
 
-// one lab-frame proposal (sample_momemtum_from_a_fluid_cell): pl = (pT, phi,
-// y - eta_s, -) on acceptance, u_rap the uniform of the rapidity draw
-__device__ __forceinline__ bool try_efa(const DevConfig& cfg, const PropEfa& p, const Unit& u,
-                                        float4& pl, float& u_rap, unsigned& violations) {
-    const uint32_t c3 = static_cast<uint32_t>(u.s) | (kTagEfa << 16);
-    const uint4 A = block(u.t, u.i, u.eg, c3, cfg.key0, cfg.key1);
+// one lab-frame proposal (sample_momemtum_from_a_fluid_cell) with counter t:
+// pl = (pT, phi, y - eta_s, -) on acceptance, u_rap the uniform of the
+// rapidity draw.  Of the about 1,900 proposals per hadron all but a few in a
+// thousand fail f0 p.dsigma tau (1 + df_max) / maximum > u already, where
+// df_max bounds |delta f| (restrict_deltaf); those leave before the delta f
+// terms, and a warp whose 32 proposals all fail it skips them.  The margin is
+// far above the rounding of the terms left out, so the outcome is that of
+// the full expression; a NaN or an infinity fails the comparison and takes the
+// full path.
+constexpr float kEfaMargin = 1.0001f;
+__device__ __forceinline__ bool try_efa(const DevConfig& cfg, const PropEfa& p, uint32_t t, uint32_t i,
+                                        uint32_t eg, int s, float4& pl, float& u_rap, bool& violation) {
+    const uint32_t c3 = static_cast<uint32_t>(s) | (kTagEfa << 16);
+    const uint4 A = block(t, i, eg, c3, cfg.key0, cfg.key1);
     const float pT = sqrtf(cfg.pt_max * cfg.pt_max * u01f(A.x));
     const float phi = 2.0f * 3.14159265f * u01f(A.y);
     const float yme = (1.0f - 2.0f * u01f(A.z)) * cfg.yme_range;
@@ -984,6 +992,9 @@ __device__ __forceinline__ bool try_efa(const DevConfig& cfg, const PropEfa& p, 
     const float pdotu = p0 * p.u0 - px * p.u1 - py * p.u2 - p3 * p.u3;
     const float f0 = 1.0f / (expf((pdotu - p.mu) / p.T) + p.sign);
     const float pdsig = p0 * p.da0 + px * p.da1 + py * p.da2 + p3 * p.da3 / p.tau;
+    if (cfg.restrict_df &&
+        fabsf(f0 * pdsig * p.tau) * ((1.0f + fabsf(cfg.df_max_ratio)) * kEfaMargin) <= u01f(A.w) * p.bmax)
+        return false;
     const float one_m = 1.0f - p.sign * f0;
     float df = 0.0f;
     if (cfg.include_shear) {
@@ -1005,13 +1016,12 @@ __device__ __forceinline__ bool try_efa(const DevConfig& cfg, const PropEfa& p, 
     if (cfg.restrict_df) resize = fminf(1.0f, cfg.df_max_ratio / (fabsf(df) + 1e-10f));
     const float result = f0 * pdsig * p.tau * (1.0f + df * resize);
     const float acc = result / p.bmax;
-    if (acc > 1.0f) violations++;
+    violation = acc > 1.0f;
     if (!(u01f(A.w) < acc)) return false;
     pl = make_float4(pT, phi, yme, 0.0f);
     u_rap = 0.0f;
     if (cfg.hydro_mode != 2) {
-        const uint4 B = block(u.t, u.i, u.eg, static_cast<uint32_t>(u.s) | (kTagEfaRap << 16),
-                              cfg.key0, cfg.key1);
+        const uint4 B = block(t, i, eg, static_cast<uint32_t>(s) | (kTagEfaRap << 16), cfg.key0, cfg.key1);
         u_rap = u01f(B.x);
     }
     return true;
@@ -1313,46 +1323,14 @@ __device__ void emit_efa(const DevConfig& cfg, const CellArrays& cells, const Pr
                  pos.x * coshf(eta_s), pos.y, pos.z, pos.x * sinhf(eta_s));
 }
 
-// the two samplers behind one work loop: FSSW (Prop) and the lab-frame
-// EmissionFunctionArray sampler (PropEfa)
-template <int kAlg> struct PropOf { using type = Prop; };
-template <> struct PropOf<2> { using type = PropEfa; };
-
 // bose2: the hadron takes the plain proposal (prop_bose2); false for those
 // of the learned proposal, whose densities assume the one-term proposal
 template <int kMode>
-__device__ __forceinline__ bool setup_any(const DevConfig& cfg, const CellArrays& cells,
-                                          const SpeciesDev& sp, int l, Prop& p, bool, bool bose2) {
+__device__ __forceinline__ bool setup_hadron(const DevConfig& cfg, const CellArrays& cells,
+                                             const SpeciesDev& sp, int l, Prop& p, bool bose2) {
     const bool ok = setup_prop<kMode>(cfg, cells, sp, l, p);
     if (bose2) prop_bose2(p);
     return ok;
-}
-template <int kMode>
-__device__ __forceinline__ bool setup_any(const DevConfig& cfg, const CellArrays& cells,
-                                          const SpeciesDev& sp, int l, PropEfa& p, bool keep_max, bool) {
-    return setup_efa(cfg, cells, sp, l, p, keep_max);
-}
-template <int kMode, bool kBose2>
-__device__ __forceinline__ bool try_any(const DevConfig& cfg, const Prop& p, const Unit& u, float4& pl,
-                                        float& u_rap, unsigned& viol) {
-    return try_once<kMode, kBose2>(cfg, p, u, pl, u_rap, viol);
-}
-template <int kMode, bool kBose2>
-__device__ __forceinline__ bool try_any(const DevConfig& cfg, const PropEfa& p, const Unit& u,
-                                        float4& pl, float& u_rap, unsigned& viol) {
-    return try_efa(cfg, p, u, pl, u_rap, viol);
-}
-template <int kMode>
-__device__ __forceinline__ void emit_any(const DevConfig& cfg, const CellArrays& cells, const Prop& p,
-                                         int l, int pid, float4 pl, float u_rap, HadronRec* out,
-                                         int64_t slot) {
-    emit<kMode>(cfg, cells, p, l, pid, pl, u_rap, out, slot);
-}
-template <int kMode>
-__device__ __forceinline__ void emit_any(const DevConfig& cfg, const CellArrays& cells,
-                                         const PropEfa& p, int l, int pid, float4 pl, float u_rap,
-                                         HadronRec* out, int64_t slot) {
-    emit_efa(cfg, cells, p, l, pid, pl, u_rap, out, slot);
 }
 
 // Cell of every hadron's first draw (redraw 0), one warp per work item in
@@ -1473,7 +1451,7 @@ constexpr int kSampleThreads = 256;
 // correction (both compile out, which frees registers), 2 the same with
 // diffusion; 1 and 2 read the prologue's lean cell records (the learned
 // proposal's plain component uses the same Prop fields)
-template <bool kLcc, bool kLearned, int kAlg, int kMode>
+template <bool kLcc, bool kLearned, int kMode>
 __global__ void __launch_bounds__(kSampleThreads, 3)
 sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict__ species,
                const int32_t* __restrict__ pids, const unsigned long long* __restrict__ cdf,
@@ -1492,7 +1470,7 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
     // diffusion; the other modes keep the one-term proposal, whose fewer
     // registers spill less there (finite density: sample phase 30.3 ms with
     // the Bose terms, 28.3 ms without)
-    constexpr bool kBose = kAlg == 4 && kMode == 1;
+    constexpr bool kBose = kMode == 1;
     // the warp's current work item: units [next, end) of species cur_s in event cur_e
     // draws [next, end), records from seg_base; a segment's draws are
     // counted by an int32, so draw indices fit in an int
@@ -1502,7 +1480,7 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
     bool exhausted = false;
     bool active = false;
     Unit u;
-    typename PropOf<kAlg>::type p;
+    Prop p;
     // per-thread counts (a thread makes far fewer than 2^32 tries in a launch)
     unsigned n_tries = 0, n_redraws = 0, n_fail = 0;
     unsigned n_viol = 0;
@@ -1600,7 +1578,7 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
                     u.lp = sl >= 0 ? cfg.lpairs + (static_cast<int64_t>(sl) * cfg.n_cells + l) * kPairFloats
                                    : nullptr;
                 }
-                if (!setup_any<kMode>(cfg, cells, species[u.s], l, p, false, kBose && (!kLearned || !u.lp))) {
+                if (!setup_hadron<kMode>(cfg, cells, species[u.s], l, p, kBose && (!kLearned || !u.lp))) {
                     atomicCAS(&ctrs->error_code, 0, 1);
                     ctrs->error_species = u.s;
                     for (int q = 0; q < (kLcc ? u.mult : 1); q++)
@@ -1622,7 +1600,7 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
                     ok = try_once<kMode, kBose>(cfg, p, u, pl, u_rap, n_viol);
                 }
             } else {
-                ok = try_any<kMode, kBose>(cfg, p, u, pl, u_rap, n_viol);
+                ok = try_once<kMode, kBose>(cfg, p, u, pl, u_rap, n_viol);
             }
             u.t++;
             u.tries_cell++;
@@ -1633,10 +1611,10 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
                 // hadron's cell: the training rows of the learned proposal)
                 if (u.redraw > 0 && u.phase == 0) cell_of[u.slot] = u.cell;
                 if (kLcc)
-                    emit_any<kMode>(cfg, cells, p, u.cell, u.phase ? -pid : pid, pl, u_rap, out,
-                                    u.slot + u.phase);
+                    emit<kMode>(cfg, cells, p, u.cell, u.phase ? -pid : pid, pl, u_rap, out,
+                                u.slot + u.phase);
                 else
-                    emit_any<kMode>(cfg, cells, p, u.cell, pid, pl, u_rap, out, u.slot);
+                    emit<kMode>(cfg, cells, p, u.cell, pid, pl, u_rap, out, u.slot);
                 if (kLcc && u.mult == 2 && u.phase == 0) {
                     // the partner: same cell and mass, opposite B, S, Q
                     SpeciesDev sp2 = species[u.s];
@@ -1646,9 +1624,7 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
                     u.phase = 1;
                     u.tries_cell = 0;
                     u.lp = nullptr;   // the pair's envelope is the hadron's, not the partner's
-                    // (the lab-frame sampler keeps the hadron's maximum for
-                    // its partner, src/emissionfunction.cpp:3503-3509)
-                    if (!setup_any<kMode>(cfg, cells, sp2, u.cell, p, true, kBose)) {
+                    if (!setup_hadron<kMode>(cfg, cells, sp2, u.cell, p, kBose)) {
                         atomicCAS(&ctrs->error_code, 0, 1);
                         ctrs->error_species = u.s;
                         write_hadron(out, u.slot + 1, 0, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f);
@@ -1695,6 +1671,138 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
                 atomicAdd(&ctrs->learned_over_one, static_cast<unsigned long long>(lts.over_one));
             if (n_lhad) atomicAdd(&ctrs->learned_hadrons, static_cast<unsigned long long>(n_lhad));
         }
+    }
+}
+
+// The lab-frame sampler (MC_sampling = 2).  A hadron takes about 1,900
+// proposals on average and up to max_tries x (max_redraws + 1), so one hadron
+// belongs to a whole warp: the 32 lanes make proposals t .. t + 31 and the
+// first accepted one (lowest counter) is the hadron, which is the draw a single
+// lane would have made one by one.  A lane per hadron, as the FSSW kernel has
+// it, left the chip waiting for the few lanes with the longest chains: 50,000
+// cells, 40 events, 213,000 hadrons took 194 ms and now take 8.2 ms.  The
+// kernel is bound by instruction issue (Philox, the hyperbolic functions and
+// the exponential of every proposal).
+template <bool kLcc>
+__global__ void __launch_bounds__(kSampleThreads, 4)
+efa_sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict__ species,
+                   const int32_t* __restrict__ pids, const unsigned long long* __restrict__ cdf,
+                   const int32_t* __restrict__ guide, const unsigned long long* __restrict__ qtot,
+                   const int64_t* __restrict__ offsets, const int64_t* __restrict__ item_off,
+                   const int32_t* __restrict__ item_seg, int64_t k_begin, int64_t k_end,
+                   int32_t* __restrict__ cell_of, HadronRec* __restrict__ out,
+                   unsigned long long* __restrict__ work_counter, SampleCounters* __restrict__ ctrs,
+                   const int64_t* __restrict__ k_end_dev) {
+    const DevConfig cfg = with_run_keys(cfg_in);
+    if (k_end_dev) k_end = *k_end_dev;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    unsigned long long n_tries = 0;
+    unsigned n_redraws = 0, n_fail = 0, n_viol = 0;   // warp-uniform
+    for (;;) {
+        long long k = 0;
+        if (lane == 0) k = k_begin + static_cast<long long>(atomicAdd(work_counter, 1ull));
+        k = __shfl_sync(FULL, k, 0);
+        if (k >= k_end) break;
+        const int q = item_seg[k];
+        const int64_t j = k - item_off[q];
+        int e, s;
+        item_decode(cfg, q, e, s);
+        const int64_t seg = static_cast<int64_t>(e) * cfg.n_species + s;
+        const int64_t seg_base = offsets[seg];
+        const SpeciesDev sp = species[s];
+        const int mult = kLcc ? records_per_draw(cfg, sp) : 1;
+        const int64_t first = j * cfg.item_size;
+        const int64_t end = min(first + cfg.item_size, (offsets[seg + 1] - seg_base) / mult);
+        const uint32_t eg = cfg.event_offset + static_cast<uint32_t>(e);
+        const int pid = pids[s];
+        for (int64_t d = first; d < end; d++) {
+            const int64_t slot = seg_base - cfg.slot_base + d * mult;
+            const uint32_t i = static_cast<uint32_t>(d);
+            uint32_t t = 0;               // proposals of this hadron so far (counter)
+            int redraw = 0, tries_cell = 0;
+            // up to `limit` proposals from counter t; the accepted one is emitted
+            const auto propose = [&](const PropEfa& p, int l, int limit, int phase) {
+                for (int b0 = 0; b0 < limit; b0 += 32) {
+                    float4 pl;
+                    float u_rap;
+                    bool viol = false;
+                    const bool ok = b0 + lane < limit &&
+                                    try_efa(cfg, p, t + static_cast<uint32_t>(b0 + lane), i, eg, s, pl, u_rap, viol);
+                    const unsigned hit = __ballot_sync(FULL, ok);
+                    const int made = hit ? __ffs(hit) : min(32, limit - b0);
+                    n_viol += __popc(__ballot_sync(FULL, viol && lane < made));
+                    n_tries += made;
+                    if (hit) {
+                        if (lane == made - 1)
+                            emit_efa(cfg, cells, p, l, phase ? -pid : pid, pl, u_rap, out, slot + phase);
+                        t += static_cast<uint32_t>(b0 + made);
+                        return true;
+                    }
+                }
+                t += static_cast<uint32_t>(limit);
+                return false;
+            };
+            PropEfa p;
+            int l = cell_of[slot];
+            bool done = false;
+            for (;;) {
+                setup_efa(cfg, cells, sp, l, p, false);
+                done = propose(p, l, max(cfg.max_tries, 1), 0);
+                if (done) break;
+                redraw++;
+                n_redraws++;
+                if (redraw > cfg.max_redraws) break;
+                const uint4 w = block(static_cast<uint32_t>(redraw), i, eg,
+                                      static_cast<uint32_t>(s) | (kTagCell << 16), cfg.key0, cfg.key1);
+                const unsigned long long r =
+                    (static_cast<unsigned long long>(w.x) << 32) | static_cast<unsigned long long>(w.y);
+                const int b = cfg.ev_surf[e];
+                const SurfSeg sg = cfg.surf[b];
+                l = static_cast<int>(sg.c0) +
+                    cell_search(cdf + sg.cdf_base + static_cast<int64_t>(s) * (sg.n + 1), sg.n,
+                                guide + sg.guide_base + static_cast<int64_t>(s) * ((int64_t(1) << sg.g) + 1),
+                                sg.g, qtot[b * cfg.n_species + s], r);
+            }
+            if (!done) {
+                if (lane < mult)
+                    write_hadron(out, slot + lane, 0, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f);
+                n_fail += mult;
+                continue;
+            }
+            // the final cell of a redrawn hadron
+            if (redraw > 0 && lane == 0) cell_of[slot] = l;
+            if (kLcc && mult == 2) {
+                // the partner: same cell and mass, opposite B, S, Q; it keeps
+                // the hadron's maximum (src/emissionfunction.cpp:3503-3509) and
+                // its cell (the reference retries there)
+                SpeciesDev sp2 = sp;
+                sp2.baryon = -sp2.baryon;
+                sp2.strange = -sp2.strange;
+                sp2.charge = -sp2.charge;
+                setup_efa(cfg, cells, sp2, l, p, true);
+                for (;;) {
+                    if (tries_cell >= cfg.max_tries) {
+                        redraw++;
+                        n_redraws++;
+                        if (redraw > cfg.max_redraws) {
+                            if (lane == 0)
+                                write_hadron(out, slot + 1, 0, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f);
+                            n_fail++;
+                            break;
+                        }
+                    }
+                    tries_cell = max(cfg.max_tries, 1);
+                    if (propose(p, l, tries_cell, 1)) break;
+                }
+            }
+        }
+    }
+    if (lane == 0) {
+        atomicAdd(&ctrs->tries, n_tries);
+        if (n_redraws) atomicAdd(&ctrs->redraws, static_cast<unsigned long long>(n_redraws));
+        if (n_fail) atomicAdd(&ctrs->failures, static_cast<unsigned long long>(n_fail));
+        if (n_viol) atomicAdd(&ctrs->bound_violations, static_cast<unsigned long long>(n_viol));
     }
 }
 
@@ -1949,6 +2057,18 @@ cudaError_t launch_sampler(const DevConfig& cfg, const CellArrays& cells, const 
             cfg, cdf, guide, qtot, offsets, item_off, item_seg, k_begin, k_end, sp, cell_of,
             k_end_dev);
     }
+    if (cfg.mc_sampling == 2) {
+        // 4 blocks of 256 per SM (64 registers); the work item is a few
+        // hadrons (kEfaItem), a warp each
+        int64_t blocks = static_cast<int64_t>(num_sms) * 4;
+        const int64_t need = (n_items + (kSampleThreads / 32) - 1) / (kSampleThreads / 32);
+        if (blocks > need) blocks = need;
+        auto efa = cfg.lcc ? efa_sampler_kernel<true> : efa_sampler_kernel<false>;
+        efa<<<static_cast<unsigned>(blocks), kSampleThreads, 0, stream>>>(
+            cfg, cells, sp, pids, cdf, guide, qtot, offsets, item_off, item_seg, k_begin, k_end, cell_of, out,
+            work_counter, counters, k_end_dev);
+        return cudaGetLastError();
+    }
     const int per_sm = std::min(3, std::max(1, cfg.sampler_ctas));
     int64_t blocks = static_cast<int64_t>(num_sms) * per_sm;
     const int64_t max_blocks = (n_items + (kSampleThreads / 32) - 1) / (kSampleThreads / 32);
@@ -1956,15 +2076,13 @@ cudaError_t launch_sampler(const DevConfig& cfg, const CellArrays& cells, const 
     if (blocks < 1) blocks = 1;
     const int mode = cfg.compat_fermion ? 0 : (cfg.include_diff ? 2 : 1);
     auto kernel =
-        cfg.mc_sampling == 2
-            ? (cfg.lcc ? sampler_kernel<true, false, 2, 0> : sampler_kernel<false, false, 2, 0>)
-        : cfg.lpairs
-            ? (mode == 1 ? (cfg.lcc ? sampler_kernel<true, true, 4, 1> : sampler_kernel<false, true, 4, 1>)
-             : mode == 2 ? (cfg.lcc ? sampler_kernel<true, true, 4, 2> : sampler_kernel<false, true, 4, 2>)
-                         : (cfg.lcc ? sampler_kernel<true, true, 4, 0> : sampler_kernel<false, true, 4, 0>))
-        : mode == 1 ? (cfg.lcc ? sampler_kernel<true, false, 4, 1> : sampler_kernel<false, false, 4, 1>)
-        : mode == 2 ? (cfg.lcc ? sampler_kernel<true, false, 4, 2> : sampler_kernel<false, false, 4, 2>)
-                    : (cfg.lcc ? sampler_kernel<true, false, 4, 0> : sampler_kernel<false, false, 4, 0>);
+        cfg.lpairs
+            ? (mode == 1 ? (cfg.lcc ? sampler_kernel<true, true, 1> : sampler_kernel<false, true, 1>)
+             : mode == 2 ? (cfg.lcc ? sampler_kernel<true, true, 2> : sampler_kernel<false, true, 2>)
+                         : (cfg.lcc ? sampler_kernel<true, true, 0> : sampler_kernel<false, true, 0>))
+        : mode == 1 ? (cfg.lcc ? sampler_kernel<true, false, 1> : sampler_kernel<false, false, 1>)
+        : mode == 2 ? (cfg.lcc ? sampler_kernel<true, false, 2> : sampler_kernel<false, false, 2>)
+                    : (cfg.lcc ? sampler_kernel<true, false, 0> : sampler_kernel<false, false, 0>);
     kernel<<<static_cast<unsigned>(blocks), kSampleThreads, 0, stream>>>(
         cfg, cells, sp, pids, cdf, guide, qtot, offsets, item_off, item_seg, k_begin,
         k_end, cell_of, out, work_counter, counters, k_end_dev);
