@@ -132,7 +132,8 @@ struct iss_handle {
     DevBuf<int32_t> d_pids;
     DevBuf<int32_t> d_yorder;        // yields kernel: species grouped by identical series
     DevBuf<float> d_yields;
-    DevBuf<unsigned long long> d_cdf, d_tile_sum, d_tile_off, d_qtot;
+    DevBuf<unsigned long long> d_cdf, d_tile_sum, d_tile_off, d_sub, d_qtot;
+    DevBuf<int32_t> d_sparse;        // rows whose CDF is not written (CellRows)
     DevBuf<double> d_totals;
     DevBuf<uint32_t> d_ymax;
     DevBuf<int32_t> d_counts, d_items, d_item_seg, d_guide, d_cell_of, d_ev_surf;
@@ -193,9 +194,10 @@ struct iss_handle {
             DevBuf<double>* db[] = {&d_totals, &d_b14c0, &d_b14c1, &d_b14c2, &d_ce, &d_qmu,
                                     &d_logfact, &d_pois};
             for (auto* b : db) b->release();
-            DevBuf<unsigned long long>* ub[] = {&d_cdf, &d_tile_sum, &d_tile_off, &d_qtot};
+            DevBuf<unsigned long long>* ub[] = {&d_cdf, &d_tile_sum, &d_tile_off, &d_sub, &d_qtot};
             for (auto* b : ub) b->release();
             d_ymax.release();
+            d_sparse.release();
             d_counts.release();
             d_items.release();
             d_item_seg.release();
@@ -638,6 +640,17 @@ CellArrays cell_arrays(iss_handle* h) {
     return a;
 }
 
+CdfBuffers cdf_buffers(iss_handle* h) {
+    return CdfBuffers{h->d_tile_sum.ptr, h->d_tile_off.ptr, h->d_sub.ptr,   h->d_qtot.ptr,
+                      h->d_sparse.ptr,   h->d_totals.ptr,   h->d_cdf.ptr,   h->d_guide.ptr};
+}
+
+CellRows cell_rows(iss_handle* h) {
+    return CellRows{h->d_cdf.ptr, h->d_guide.ptr, h->d_qtot.ptr, h->d_sparse.ptr, h->d_tile_off.ptr,
+                    h->d_sub.ptr, h->d_ymax.ptr, h->d_yields.ptr, h->n_cells,
+                    static_cast<int>(h->species.size())};
+}
+
 // surface upload + prologue + yields + CDF (the per-cell half of generate)
 iss_status run_cells(iss_handle* h) {
     const int64_t n = h->n_cells;
@@ -654,12 +667,15 @@ iss_status run_cells(iss_handle* h) {
     // 8 SoA arrays, the records and the lean sampler's records
     CUDA_TRY(h, h->d_cells.reserve(static_cast<size_t>(n) * 24));
     if (c.mc_sampling == 2) CUDA_TRY(h, h->d_milne.reserve(static_cast<size_t>(n) * 6));
-    CUDA_TRY(h, h->d_yields.reserve(static_cast<size_t>(n) * S));
+    // (sparse_cell reads the yields 16 bytes at a time)
+    CUDA_TRY(h, h->d_yields.reserve(static_cast<size_t>(n) * S + 4));
     const size_t rows = static_cast<size_t>(c.n_surfaces) * S;
     CUDA_TRY(h, h->d_cdf.reserve(static_cast<size_t>(std::max<int64_t>(h->cdf_len, 1))));
     CUDA_TRY(h, h->d_tile_sum.reserve(static_cast<size_t>(std::max<int64_t>(h->n_tiles, 1))));
     CUDA_TRY(h, h->d_tile_off.reserve(static_cast<size_t>(std::max<int64_t>(h->n_tiles, 1))));
+    CUDA_TRY(h, h->d_sub.reserve(static_cast<size_t>(std::max<int64_t>(h->n_tiles, 1)) * kCdfSubs));
     CUDA_TRY(h, h->d_totals.reserve(rows));
+    CUDA_TRY(h, h->d_sparse.reserve(rows));
     CUDA_TRY(h, h->d_qtot.reserve(rows));
     CUDA_TRY(h, h->d_ymax.reserve(rows));
     CUDA_TRY(h, h->d_guide.reserve(static_cast<size_t>(std::max<int64_t>(h->guide_len, 1))));
@@ -669,9 +685,13 @@ iss_status run_cells(iss_handle* h) {
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvPrologue], st));
     CUDA_TRY(h, launch_yields(c, cells, h->d_species.ptr, h->d_yields.ptr, h->d_ymax.ptr, st));
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvYields], st));
-    CUDA_TRY(h, launch_cdf(h->d_yields.ptr, n, h->d_surf.ptr, c.n_surfaces, h->n_tiles, S,
-                           h->d_ymax.ptr, h->d_tile_sum.ptr, h->d_tile_off.ptr, h->d_qtot.ptr,
-                           h->d_totals.ptr, h->d_cdf.ptr, h->d_guide.ptr, st));
+    // the number of events is not known yet when it follows from the yields
+    const bool allow_sparse = h->params.get_or("sample_upto_desired_particle_number", 0) != 1;
+    const CdfBuffers cb = cdf_buffers(h);
+    CUDA_TRY(h, launch_cdf_head(h->d_yields.ptr, n, h->d_surf.ptr, c.n_surfaces, h->n_tiles, S, h->d_ymax.ptr,
+                                c.ymult, allow_sparse, cb, st));
+    CUDA_TRY(h, launch_cdf_scan(h->d_yields.ptr, n, h->d_surf.ptr, c.n_surfaces, h->n_tiles, S, h->d_ymax.ptr,
+                                cb, st));
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvCdf], st));
     h->yields_valid = true;
     return ISS_OK;
@@ -1006,7 +1026,8 @@ std::vector<unsigned char> graph_key_of(iss_handle* h) {
                           h->d_offsets.ptr,  h->d_off_tiles.ptr, h->d_item_off.ptr, h->d_item_seg.ptr,
                           h->d_hadrons.ptr,  h->d_cell_of.ptr,  h->d_work.ptr,     h->d_counters.ptr,
                           h->d_error.ptr,    h->d_pois.ptr,     h->d_species.ptr,  h->d_pids.ptr,
-                          h->d_surf.ptr,     h->d_limits.ptr,   h->gh,            h->d_milne.ptr};
+                          h->d_surf.ptr,     h->d_limits.ptr,   h->gh,            h->d_milne.ptr,
+                          h->d_sub.ptr,      h->d_sparse.ptr};
     const unsigned char* pb = reinterpret_cast<const unsigned char*>(ptrs);
     k.insert(k.end(), pb, pb + sizeof(ptrs));
     const int64_t nums[] = {h->n_cells, h->n_tiles, h->cdf_len, h->guide_len, h->graph_cap_units,
@@ -1047,9 +1068,9 @@ cudaError_t enqueue_generate(iss_handle* h, const DevConfig& c) {
     record(h, kEvPrologue, true);
     GTRY(launch_yields(c, cells, h->d_species.ptr, h->d_yields.ptr, h->d_ymax.ptr, s));
     record(h, kEvYields, true);
+    const CdfBuffers cb = cdf_buffers(h);
     GTRY(launch_cdf_head(h->d_yields.ptr, n, h->d_surf.ptr, c.n_surfaces, h->n_tiles, S, h->d_ymax.ptr,
-                         h->d_tile_sum.ptr, h->d_tile_off.ptr, h->d_qtot.ptr, h->d_totals.ptr, h->d_cdf.ptr,
-                         h->d_guide.ptr, s));
+                         c.ymult, true, cb, s));
     GTRY(cudaEventRecord(h->ev_fork, s));
     GTRY(cudaStreamWaitEvent(a, h->ev_fork, 0));
     GTRY(cudaMemsetAsync(h->d_error.ptr, 0, sizeof(int), a));
@@ -1061,16 +1082,15 @@ cudaError_t enqueue_generate(iss_handle* h, const DevConfig& c) {
                              h->graph_cap_items, h->d_limits.ptr, a));
     GTRY(launch_item_map(h->d_items.ptr, h->d_item_off.ptr, nseg, h->d_item_seg.ptr, a, h->d_limits.ptr));
     GTRY(cudaEventRecord(h->ev_join, a));
-    GTRY(launch_cdf_scan(h->d_yields.ptr, n, h->d_surf.ptr, c.n_surfaces, h->n_tiles, S, h->d_ymax.ptr,
-                         h->d_tile_off.ptr, h->d_qtot.ptr, h->d_cdf.ptr, h->d_guide.ptr, s));
+    GTRY(launch_cdf_scan(h->d_yields.ptr, n, h->d_surf.ptr, c.n_surfaces, h->n_tiles, S, h->d_ymax.ptr, cb, s));
     record(h, kEvCdf, true);
     GTRY(cudaStreamWaitEvent(s, h->ev_join, 0));
     record(h, kEvCounts, true);
     GTRY(cudaMemsetAsync(h->d_work.ptr, 0, sizeof(unsigned long long), s));
     GTRY(cudaMemsetAsync(h->d_counters.ptr, 0, sizeof(SampleCounters), s));
     record(h, kEvSampleStart, true);
-    GTRY(launch_sampler(c, cells, h->d_species.ptr, h->d_pids.ptr, h->d_cdf.ptr, h->d_guide.ptr,
-                        h->d_qtot.ptr, h->d_offsets.ptr, h->d_item_off.ptr, h->d_item_seg.ptr, 0,
+    GTRY(launch_sampler(c, cells, h->d_species.ptr, h->d_pids.ptr, cell_rows(h), h->d_offsets.ptr,
+                        h->d_item_off.ptr, h->d_item_seg.ptr, 0,
                         h->graph_cap_items, h->d_cell_of.ptr, h->d_hadrons.ptr, h->d_work.ptr,
                         h->d_counters.ptr, h->num_sms, s, h->d_limits.ptr));
     record(h, kEvSample, true);
@@ -1429,8 +1449,8 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
         if (ch >= 2) CUDA_TRY(h, cudaStreamWaitEvent(s, h->copy_ev[ch - 2], 0));
         DevConfig cc = c;
         cc.slot_base = b;
-        CUDA_TRY(h, launch_sampler(cc, cell_arrays(h), h->d_species.ptr, h->d_pids.ptr, h->d_cdf.ptr,
-                                   h->d_guide.ptr, h->d_qtot.ptr, h->d_offsets.ptr, h->d_item_off.ptr,
+        CUDA_TRY(h, launch_sampler(cc, cell_arrays(h), h->d_species.ptr, h->d_pids.ptr, cell_rows(h),
+                                   h->d_offsets.ptr, h->d_item_off.ptr,
                                    h->d_item_seg.ptr, chunk_item[ch], chunk_item[ch + 1],
                                    h->d_cell_of.ptr + slot * ring, h->d_hadrons.ptr + slot * ring,
                                    h->d_work.ptr + ch, h->d_counters.ptr, h->num_sms, s));
@@ -1479,8 +1499,7 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
             e1 = std::min(E, ch * c.chunk_events);
         } while (ch < n_chunks && (!to_host || h->event_offsets[e1] - h->event_offsets[e0] < group_records));
         cudaStream_t gs = (n_groups & 1) ? h->sample_stream : s;
-        CUDA_TRY(h, launch_sampler(c, cell_arrays(h), h->d_species.ptr, h->d_pids.ptr, h->d_cdf.ptr,
-                                   h->d_guide.ptr, h->d_qtot.ptr,
+        CUDA_TRY(h, launch_sampler(c, cell_arrays(h), h->d_species.ptr, h->d_pids.ptr, cell_rows(h),
                                    h->d_offsets.ptr, h->d_item_off.ptr, h->d_item_seg.ptr,
                                    chunk_item[ch0], chunk_item[ch], h->d_cell_of.ptr,
                                    h->d_hadrons.ptr, h->d_work.ptr + n_groups, h->d_counters.ptr,

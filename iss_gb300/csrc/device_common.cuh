@@ -107,6 +107,26 @@ struct SpeciesDev {
     int baryon, strange, charge, sign;
 };
 
+// What a cell draw reads of the (surface, species) rows r = b S + k: the full
+// prefix sums and guide table of dense rows, and for the others (sparse[r])
+// the tile offsets, the prefix sums of each tile's runs of kCdfSub cells and
+// the yields themselves (cell_search).
+struct CellRows {
+    const unsigned long long* cdf;       // rows of n + 1 entries (SurfSeg::cdf_base)
+    const int32_t* guide;                // rows of 2^g + 1 entries (SurfSeg::guide_base)
+    const unsigned long long* qtot;      // [rows] Q
+    const int32_t* sparse;               // [rows] 1: cdf and guide are not written
+    const unsigned long long* tile_off;  // [tiles] Q of the row's tiles before this one
+    const unsigned long long* sub;       // [tiles][kCdfSubs] Q of the tile's runs before this one
+    const uint32_t* ymax;                // [rows] largest yield (float bits)
+    const float* yields;                 // [species][n_cells]
+    int64_t n_cells;
+    int n_species;
+};
+constexpr int kCdfTile = 2048;                   // cells per tile of the scan
+constexpr int kCdfSub = 32;                      // cells per run
+constexpr int kCdfSubs = kCdfTile / kCdfSub;
+
 // Local-rest-frame cells, structure of arrays of float4.
 struct CellArrays {
     float4* pos;    // tau, x, y, eta

@@ -16,26 +16,38 @@ cudaError_t launch_cell_prologue(const DevConfig& cfg, const float* fo34, int64_
 cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, const SpeciesDev* sp,
                           float* yields, uint32_t* ymax, cudaStream_t stream);
 int cdf_num_tiles(int64_t n);
-// Fixed-point cell CDF (cdf_quantize) of every (surface, species) row of a
-// batch from the yields and their row maxima (launch_yields); three launches
-// over n_tiles = sum over surfaces of S * nt tiles (tile sums, tile offsets,
-// scan).  Row (b, k) of the CDF holds
-// n_b + 1 entries C[0..n_b] at surf[b].cdf_base + k (n_b + 1); its guide
-// table 2^g_b + 1 entries at surf[b].guide_base + k (2^g_b + 1).  ymax,
-// qtot and totals hold n_surf * S rows.  surf is a device array.
-cudaError_t launch_cdf(const float* yields, int64_t N, const SurfSeg* surf, int n_surf,
-                       int64_t n_tiles, int S, uint32_t* ymax, unsigned long long* tile_sum,
-                       unsigned long long* tile_off, unsigned long long* qtot, double* totals,
-                       unsigned long long* cdf, int32_t* guide, cudaStream_t stream);
-// the same in two parts: tile sums and tile offsets (which also give qtot and
-// totals), then the scan that writes the CDF rows and guide tables
+// Buffers of the fixed-point cell CDF (cdf_quantize) of every (surface,
+// species) row of a batch, n_tiles = sum over surfaces of S * nt tiles
+struct CdfBuffers {
+    unsigned long long* tile_sum;   // [n_tiles]
+    unsigned long long* tile_off;   // [n_tiles]
+    unsigned long long* sub;        // [n_tiles][kCdfSubs]
+    unsigned long long* qtot;       // [n_surf * S]
+    int32_t* sparse;                // [n_surf * S]
+    double* totals;                 // [n_surf * S]
+    unsigned long long* cdf;        // dense row (b, k): n_b + 1 entries C[0..n_b] at
+                                    // surf[b].cdf_base + k (n_b + 1)
+    int32_t* guide;                 // 2^g_b + 1 entries at surf[b].guide_base + k (2^g_b + 1)
+};
+// From the yields and their row maxima (launch_yields), in two parts: the
+// head gives the tile sums and offsets, qtot, totals and which rows are sparse
+// (fewer than n_b / kSparseDraws draws expected in all events; none unless
+// allow_sparse and n_tiles >= kSparseTiles), the scan writes the CDF rows and
+// guide tables of the dense rows.  surf is a device array.
+//
+// A CDF row costs about 4.5 ps per cell to write, a draw on a sparse row some
+// 30 ps more than on a dense one: at 8 cells per draw both calls with few and
+// with many events gain (200,000 cells: 1 event CDF 365 -> 119 us, 300 events
+// 371 -> 185 us; 4, 16 and 32 cells per draw were no better).  Below 2048
+// tiles (13,000 cells of 319 species) the rows are written in a wave or two
+// of blocks, less than the longer search takes.
+constexpr int kSparseDraws = 8;
+constexpr int64_t kSparseTiles = 2048;
 cudaError_t launch_cdf_head(const float* yields, int64_t N, const SurfSeg* surf, int n_surf,
-                            int64_t n_tiles, int S, uint32_t* ymax, unsigned long long* tile_sum,
-                            unsigned long long* tile_off, unsigned long long* qtot, double* totals,
-                            unsigned long long* cdf, int32_t* guide, cudaStream_t stream);
+                            int64_t n_tiles, int S, const uint32_t* ymax, double ymult, bool allow_sparse,
+                            const CdfBuffers& b, cudaStream_t stream);
 cudaError_t launch_cdf_scan(const float* yields, int64_t N, const SurfSeg* surf, int n_surf,
-                            int64_t n_tiles, int S, const uint32_t* ymax, const unsigned long long* tile_off,
-                            const unsigned long long* qtot, unsigned long long* cdf, int32_t* guide,
+                            int64_t n_tiles, int S, const uint32_t* ymax, const CdfBuffers& b,
                             cudaStream_t stream);
 
 // kernels_sample.cu
@@ -63,9 +75,7 @@ cudaError_t launch_graph_limits(const int64_t* offsets, const int64_t* item_off,
 // hadron (cell_of, one int32 per slot), then the sampler; work_counter must
 // be zero
 cudaError_t launch_sampler(const DevConfig& cfg, const CellArrays& cells, const SpeciesDev* sp,
-                           const int32_t* pids, const unsigned long long* cdf,
-                           const int32_t* guide, const unsigned long long* qtot,
-                           const int64_t* offsets,
+                           const int32_t* pids, const CellRows& rows, const int64_t* offsets,
                            const int64_t* item_off, const int32_t* item_seg, int64_t k_begin,
                            int64_t k_end, int32_t* cell_of, HadronRec* out,
                            unsigned long long* work_counter, SampleCounters* counters, int num_sms,

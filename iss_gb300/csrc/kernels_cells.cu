@@ -403,6 +403,12 @@ yields_kernel(DevConfig cfg, CellArrays cells, const SpeciesDev* __restrict__ sp
 constexpr int kScanThreads = 256;
 constexpr int kScanPer = 8;
 constexpr int kScanTile = kScanThreads * kScanPer;
+static_assert(kScanTile == kCdfTile && kCdfSub % kScanPer == 0, "runs are whole threads of the scan");
+// tiles per block of the scan, whose blocks leave at once where the row is
+// sparse: 4 (31,262 tiles, all rows but a few sparse: 18 us), 1 where the
+// blocks fit the chip in a wave or two anyway (319 tiles: 8 us, 16 us with 4)
+constexpr int kScanTilesPerBlock = 4;
+constexpr int64_t kScanFewTiles = 4096;
 
 __device__ __forceinline__ unsigned long long warp_incl_scan_u64(unsigned long long v) {
     const int lane = threadIdx.x & 31;
@@ -461,46 +467,61 @@ __device__ __forceinline__ TileRef tile_ref(const SurfSeg* __restrict__ surf, in
     return r;
 }
 
-__global__ void __launch_bounds__(kScanThreads)
-cdf_tile_sum_kernel(const float* __restrict__ yields, int64_t N, const SurfSeg* __restrict__ surf,
-                    int n_surf, int S, const uint32_t* __restrict__ ymax,
-                    unsigned long long* __restrict__ tile_sum) {
-    __shared__ unsigned long long s_warp[kScanThreads / 32];
-    const TileRef tr = tile_ref(surf, n_surf, S, blockIdx.x);
-    const int64_t n = tr.sg->n;
-    const int64_t t0 = tr.tile * kScanTile;
-    const uint32_t* row =
-        reinterpret_cast<const uint32_t*>(yields + static_cast<int64_t>(tr.k) * N + tr.sg->c0);
-    const int base = cdf_quant_base(ymax[tr.b * S + tr.k], tr.sg->L);
+// The yields of a tile, read coalesced, to a thread's kScanPer consecutive
+// cells (padded: element e of the tile sits at (e / 8) * 9 + e % 8)
+__device__ __forceinline__ void load_tile(const uint32_t* __restrict__ row, int64_t t0, int64_t n,
+                                          uint32_t* s_in) {
     uint32_t v[kScanPer];
 #pragma unroll
     for (int k = 0; k < kScanPer; k++) {
         const int64_t i = t0 + k * kScanThreads + threadIdx.x;
         v[k] = i < n ? __ldg(row + i) : 0u;
     }
-    unsigned long long acc = 0;
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) acc += cdf_quantize(v[k], base);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long t = 0;
-#pragma unroll
-        for (int w = 0; w < kScanThreads / 32; w++) t += s_warp[w];
-        tile_sum[blockIdx.x] = t;
+    for (int k = 0; k < kScanPer; k++) {
+        const int e = k * kScanThreads + threadIdx.x;
+        s_in[(e / kScanPer) * (kScanPer + 1) + e % kScanPer] = v[k];
     }
 }
 
+// Sum of every tile, and inside it the prefix sums of its runs of kCdfSub
+// cells, which are what the cell draws of sparse rows search.
+__global__ void __launch_bounds__(kScanThreads)
+cdf_tile_sum_kernel(const float* __restrict__ yields, int64_t N, const SurfSeg* __restrict__ surf,
+                    int n_surf, int S, const uint32_t* __restrict__ ymax,
+                    unsigned long long* __restrict__ tile_sum, unsigned long long* __restrict__ sub) {
+    __shared__ uint32_t s_in[kScanThreads * (kScanPer + 1)];
+    __shared__ unsigned long long s_warp[33];
+    const TileRef tr = tile_ref(surf, n_surf, S, blockIdx.x);
+    const int64_t n = tr.sg->n;
+    const uint32_t* row =
+        reinterpret_cast<const uint32_t*>(yields + static_cast<int64_t>(tr.k) * N + tr.sg->c0);
+    const int base = cdf_quant_base(ymax[tr.b * S + tr.k], tr.sg->L);
+    load_tile(row, tr.tile * kScanTile, n, s_in);
+    __syncthreads();
+    const uint32_t* mine = s_in + threadIdx.x * (kScanPer + 1);
+    unsigned long long acc = 0;
+#pragma unroll
+    for (int k = 0; k < kScanPer; k++) acc += cdf_quantize(mine[k], base);
+    unsigned long long tot;
+    const unsigned long long ex = block_excl_scan_u64(acc, s_warp, &tot);
+    constexpr int kPerRun = kCdfSub / kScanPer;   // threads per run
+    if (threadIdx.x % kPerRun == 0)
+        sub[static_cast<int64_t>(blockIdx.x) * kCdfSubs + threadIdx.x / kPerRun] = ex;
+    if (threadIdx.x == 0) tile_sum[blockIdx.x] = tot;
+}
+
 // one block per row (b, k): exclusive scan of the row's tile sums, the row
-// total Q, the FP64 yield Q 2^-E, C[n] = Q and the guide sentinel
+// total Q, the FP64 yield Q 2^-E, whether the row is sparse, C[n] = Q and the
+// guide sentinel
 __global__ void __launch_bounds__(kScanThreads)
 cdf_tile_offset_kernel(const SurfSeg* __restrict__ surf, int S,
                        const unsigned long long* __restrict__ tile_sum,
-                       const uint32_t* __restrict__ ymax, unsigned long long* __restrict__ tile_off,
-                       unsigned long long* __restrict__ qtot, double* __restrict__ totals,
-                       unsigned long long* __restrict__ cdf, int32_t* __restrict__ guide) {
+                       const uint32_t* __restrict__ ymax, double ymult, bool allow_sparse,
+                       unsigned long long* __restrict__ tile_off,
+                       unsigned long long* __restrict__ qtot, int32_t* __restrict__ sparse,
+                       double* __restrict__ totals, unsigned long long* __restrict__ cdf,
+                       int32_t* __restrict__ guide) {
     __shared__ unsigned long long s_warp[33];
     const int r = blockIdx.x;
     const int b = r / S, k = r - b * S;
@@ -518,7 +539,10 @@ cdf_tile_offset_kernel(const SurfSeg* __restrict__ surf, int S,
     if (threadIdx.x == 0) {
         const int base = cdf_quant_base(ymax[r], sg.L);
         qtot[r] = carry;
-        totals[r] = carry ? ldexp(static_cast<double>(carry), -(150 + base)) : 0.0;
+        const double total = carry ? ldexp(static_cast<double>(carry), -(150 + base)) : 0.0;
+        totals[r] = total;
+        // a row whose CDF would be written for few draws is left unwritten
+        sparse[r] = allow_sparse && total * ymult * sg.ne * kSparseDraws < static_cast<double>(sg.n);
         cdf[sg.cdf_base + static_cast<int64_t>(k) * (sg.n + 1) + sg.n] = carry;
         const int64_t G = int64_t(1) << sg.g;
         guide[sg.guide_base + static_cast<int64_t>(k) * (G + 1) + G] = static_cast<int32_t>(sg.n - 1);
@@ -531,25 +555,21 @@ __device__ __forceinline__ unsigned long long bucket_start(unsigned long long j,
     return __umul64hi(j << (64 - g), Q);
 }
 
-// Writes row (b, k) of the cell CDF, C[i] = sum of q over cells < i, and
+// Writes tile tile_id of the dense row (b, k) of the cell CDF, C[i] = sum of q over cells < i, and
 // scatters the guide table (indexed search, Chen & Asau 1974): guide[j] is
 // the cell whose interval [C[i], C[i+1]) holds f(j).  The intervals partition
 // [0, Q), so every bucket j < 2^g gets exactly one writer; the cell of any v
 // drawn in bucket j lies in [guide[j], guide[j+1]].
-__global__ void __launch_bounds__(kScanThreads)
-cdf_tile_scan_kernel(const float* __restrict__ yields, int64_t N, const SurfSeg* __restrict__ surf,
-                     int n_surf, int S, const uint32_t* __restrict__ ymax,
-                     const unsigned long long* __restrict__ tile_off,
-                     const unsigned long long* __restrict__ qtot,
-                     unsigned long long* __restrict__ cdf, int32_t* __restrict__ guide) {
-    // padded tile buffers: element e of the tile sits at (e / 8) * 9 + e % 8;
-    // s_in holds the FP32 yield bits, s_c the CDF values on the way out
-    __shared__ uint32_t s_in[kScanThreads * (kScanPer + 1)];
-    __shared__ unsigned long long s_c[kScanThreads * (kScanPer + 1)];
-    __shared__ unsigned long long s_warp[33];
-    const TileRef tr = tile_ref(surf, n_surf, S, blockIdx.x);
+__device__ __forceinline__ void scan_tile(
+    const float* __restrict__ yields, int64_t N, const SurfSeg* __restrict__ surf, int n_surf, int S,
+    const uint32_t* __restrict__ ymax, int64_t tile_id, const unsigned long long* __restrict__ tile_off,
+    const unsigned long long* __restrict__ qtot, const int32_t* __restrict__ sparse,
+    unsigned long long* __restrict__ cdf, int32_t* __restrict__ guide, uint32_t* s_in, unsigned long long* s_c,
+    unsigned long long* s_warp) {
+    const TileRef tr = tile_ref(surf, n_surf, S, tile_id);
     const int64_t n = tr.sg->n;
     const int r = tr.b * S + tr.k;
+    if (sparse[r]) return;   // the whole block: one row per tile
     const int64_t t0 = tr.tile * kScanTile;
     const uint32_t* row =
         reinterpret_cast<const uint32_t*>(yields + static_cast<int64_t>(tr.k) * N + tr.sg->c0);
@@ -559,12 +579,8 @@ cdf_tile_scan_kernel(const float* __restrict__ yields, int64_t N, const SurfSeg*
     int32_t* gd = guide + tr.sg->guide_base + static_cast<int64_t>(tr.k) * (G + 1);
     const int base = cdf_quant_base(ymax[r], tr.sg->L);
     const unsigned long long Q = qtot[r];
-    // coalesced load
-    for (int k = 0; k < kScanPer; k++) {
-        const int e = k * kScanThreads + threadIdx.x;
-        const int64_t i = t0 + e;
-        s_in[(e / kScanPer) * (kScanPer + 1) + e % kScanPer] = i < n ? row[i] : 0u;
-    }
+    __syncthreads();   // the buffers are free of the block's tile before
+    load_tile(row, t0, n, s_in);
     __syncthreads();
     const uint32_t* mine = s_in + threadIdx.x * (kScanPer + 1);
     unsigned long long* mine_c = s_c + threadIdx.x * (kScanPer + 1);
@@ -577,7 +593,7 @@ cdf_tile_scan_kernel(const float* __restrict__ yields, int64_t N, const SurfSeg*
     }
     unsigned long long tot;
     const unsigned long long ex = block_excl_scan_u64(acc, s_warp, &tot);
-    const unsigned long long start = tile_off[blockIdx.x] + ex;
+    const unsigned long long start = tile_off[tile_id] + ex;
     const int64_t e0 = t0 + static_cast<int64_t>(threadIdx.x) * kScanPer;
     // q -> exclusive prefix C, in place
     unsigned long long run = start;
@@ -624,6 +640,24 @@ cdf_tile_scan_kernel(const float* __restrict__ yields, int64_t N, const SurfSeg*
     }
 }
 
+__global__ void __launch_bounds__(kScanThreads, 6)
+cdf_tile_scan_kernel(const float* __restrict__ yields, int64_t N, const SurfSeg* __restrict__ surf,
+                     int n_surf, int S, const uint32_t* __restrict__ ymax, int64_t n_tiles,
+                     int tiles_per_block,
+                     const unsigned long long* __restrict__ tile_off,
+                     const unsigned long long* __restrict__ qtot, const int32_t* __restrict__ sparse,
+                     unsigned long long* __restrict__ cdf, int32_t* __restrict__ guide) {
+    // s_in holds the FP32 yield bits (load_tile), s_c the CDF values on the
+    // way out, in the same padded places
+    __shared__ uint32_t s_in[kScanThreads * (kScanPer + 1)];
+    __shared__ unsigned long long s_c[kScanThreads * (kScanPer + 1)];
+    __shared__ unsigned long long s_warp[33];
+    const int64_t first_tile = static_cast<int64_t>(blockIdx.x) * tiles_per_block;
+    const int64_t last_tile = min(first_tile + tiles_per_block, n_tiles);
+    for (int64_t tile = first_tile; tile < last_tile; tile++)
+        scan_tile(yields, N, surf, n_surf, S, ymax, tile, tile_off, qtot, sparse, cdf, guide, s_in, s_c, s_warp);
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------------
@@ -654,38 +688,27 @@ cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, const S
 int cdf_num_tiles(int64_t n) { return static_cast<int>((n + kScanTile - 1) / kScanTile); }
 
 cudaError_t launch_cdf_head(const float* yields, int64_t N, const SurfSeg* surf, int n_surf,
-                            int64_t n_tiles, int S, uint32_t* ymax, unsigned long long* tile_sum,
-                            unsigned long long* tile_off, unsigned long long* qtot, double* totals,
-                            unsigned long long* cdf, int32_t* guide, cudaStream_t stream) {
+                            int64_t n_tiles, int S, const uint32_t* ymax, double ymult, bool allow_sparse,
+                            const CdfBuffers& b, cudaStream_t stream) {
     if (n_tiles <= 0 || S <= 0 || n_surf <= 0) return cudaSuccess;
     const int rows = n_surf * S;
     const unsigned grid = static_cast<unsigned>(n_tiles);
-    cdf_tile_sum_kernel<<<grid, kScanThreads, 0, stream>>>(yields, N, surf, n_surf, S, ymax,
-                                                          tile_sum);
-    cdf_tile_offset_kernel<<<rows, kScanThreads, 0, stream>>>(surf, S, tile_sum, ymax, tile_off,
-                                                             qtot, totals, cdf, guide);
+    cdf_tile_sum_kernel<<<grid, kScanThreads, 0, stream>>>(yields, N, surf, n_surf, S, ymax, b.tile_sum, b.sub);
+    cdf_tile_offset_kernel<<<rows, kScanThreads, 0, stream>>>(
+        surf, S, b.tile_sum, ymax, ymult, allow_sparse && n_tiles >= kSparseTiles, b.tile_off, b.qtot, b.sparse,
+        b.totals, b.cdf, b.guide);
     return cudaGetLastError();
 }
 
 cudaError_t launch_cdf_scan(const float* yields, int64_t N, const SurfSeg* surf, int n_surf,
-                            int64_t n_tiles, int S, const uint32_t* ymax, const unsigned long long* tile_off,
-                            const unsigned long long* qtot, unsigned long long* cdf, int32_t* guide,
+                            int64_t n_tiles, int S, const uint32_t* ymax, const CdfBuffers& b,
                             cudaStream_t stream) {
     if (n_tiles <= 0 || S <= 0 || n_surf <= 0) return cudaSuccess;
-    const unsigned grid = static_cast<unsigned>(n_tiles);
-    cdf_tile_scan_kernel<<<grid, kScanThreads, 0, stream>>>(yields, N, surf, n_surf, S, ymax,
-                                                           tile_off, qtot, cdf, guide);
+    const int per_block = n_tiles > kScanFewTiles ? kScanTilesPerBlock : 1;
+    const unsigned grid = static_cast<unsigned>((n_tiles + per_block - 1) / per_block);
+    cdf_tile_scan_kernel<<<grid, kScanThreads, 0, stream>>>(yields, N, surf, n_surf, S, ymax, n_tiles, per_block,
+                                                           b.tile_off, b.qtot, b.sparse, b.cdf, b.guide);
     return cudaGetLastError();
-}
-
-cudaError_t launch_cdf(const float* yields, int64_t N, const SurfSeg* surf, int n_surf,
-                       int64_t n_tiles, int S, uint32_t* ymax, unsigned long long* tile_sum,
-                       unsigned long long* tile_off, unsigned long long* qtot, double* totals,
-                       unsigned long long* cdf, int32_t* guide, cudaStream_t stream) {
-    const cudaError_t e = launch_cdf_head(yields, N, surf, n_surf, n_tiles, S, ymax, tile_sum, tile_off,
-                                          qtot, totals, cdf, guide, stream);
-    if (e != cudaSuccess) return e;
-    return launch_cdf_scan(yields, N, surf, n_surf, n_tiles, S, ymax, tile_off, qtot, cdf, guide, stream);
 }
 
 }  // namespace iss

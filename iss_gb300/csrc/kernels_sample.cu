@@ -204,6 +204,9 @@ constexpr float kTwoPiF = 6.2831853071795865f;
 // guide buckets spanning at most this many cells past their first are
 // resolved with one batch of CDF reads (cell_assign_kernel)
 constexpr int kAssignSpan = 3;
+// where a warp takes several work items, the draws of items of up to this many
+// are dealt out to its lanes (cell_assign_kernel)
+constexpr int kDealtDraws = 16;
 
 // Work items are ordered by event chunk (cfg.chunk_events consecutive events),
 // then species, then event: warps that run at the same time mostly sample one
@@ -466,19 +469,83 @@ struct Unit {
     const float* lp;           // learned sampler: the pair's mixture record (null: plain)
 };
 
-// Cell draw from 64 random bits r on the fixed-point CDF row C[0..n]
-// (cdf_quantize): v = floor(r * Q / 2^64), and the cell is the i with
-// C[i] <= v < C[i+1] -- the reference's binarySearch (src/arsenal.cpp:644-678)
-// on integer sums.  The guide bucket j = r >> (64 - g) brackets the cell by
-// guide[j] <= i <= guide[j+1]; when both agree no CDF entry is read.
-__device__ __forceinline__ int cell_search(const unsigned long long* __restrict__ row, int64_t n,
-                                           const int32_t* __restrict__ gd, int g,
-                                           unsigned long long Q, unsigned long long r) {
-    const unsigned long long v = __umul64hi(r, Q);
-    const unsigned j = static_cast<unsigned>(r >> (64 - g));
-    const int2 b = make_int2(__ldg(gd + j), __ldg(gd + j + 1));
-    const int last = static_cast<int>(n - 1);
-    int lo = min(max(b.x, 0), last), hi = min(max(b.y, lo), last);
+// Last index i < n with a[i] <= v, for nondecreasing a with a[0] <= v: eight
+// intervals per round, whose seven reads do not wait for one another.
+__device__ __forceinline__ int last_le(const unsigned long long* __restrict__ a, int n, unsigned long long v) {
+    int at = 0;
+    while (n > 1) {
+        const int step = (n + 7) >> 3;
+        unsigned long long w[7];
+#pragma unroll
+        for (int k = 0; k < 7; k++) w[k] = (k + 1) * step < n ? __ldg(a + at + (k + 1) * step) : ~0ull;
+        int c = 0;
+#pragma unroll
+        for (int k = 0; k < 7; k++) c += w[k] <= v;
+        at += c * step;
+        n = min(step, n - c * step);
+    }
+    return at;
+}
+
+// The cell of v on a sparse row (surface sg, species s, row r = b S + s),
+// relative to the surface's first cell: the tile, the run of kCdfSub cells
+// inside it and the cell inside the run whose interval of the same integer
+// prefix sums C holds v, so the cell is the one a search of the full row finds.
+// Some six rounds of reads and 32 quantised yields: dear per draw, but the row
+// itself need not be written.
+__device__ __noinline__ int sparse_cell(const CellRows& rows, const SurfSeg* __restrict__ surf, int b, int s,
+                                        unsigned long long v) {
+    const SurfSeg sg = surf[b];
+    const int64_t tile0 = sg.tile_base + static_cast<int64_t>(s) * sg.nt;
+    const int tile = last_le(rows.tile_off + tile0, sg.nt, v);
+    v -= __ldg(rows.tile_off + tile0 + tile);
+    const unsigned long long* sub = rows.sub + (tile0 + tile) * kCdfSubs;
+    const int run_at = last_le(sub, kCdfSubs, v);
+    v -= __ldg(sub + run_at);
+    const int first = tile * kCdfTile + run_at * kCdfSub;
+    const int last = static_cast<int>(sg.n - 1);
+    const int len = min(kCdfSub, last + 1 - first);
+    const int base = cdf_quant_base(rows.ymax[b * rows.n_species + s], sg.L);
+    // 16-byte reads of the aligned window around the run; the entries outside
+    // it count nothing
+    const int64_t at = static_cast<int64_t>(s) * rows.n_cells + sg.c0 + first;
+    const int skip = static_cast<int>(at & 3);
+    const uint4* w = reinterpret_cast<const uint4*>(rows.yields + (at - skip));
+    unsigned long long run = 0;
+    int cell = 0;
+#pragma unroll
+    for (int c = 0; c < kCdfSub / 4 + 1; c++) {
+        const uint4 y4 = 4 * c < skip + len ? __ldg(w + c) : make_uint4(0, 0, 0, 0);
+        const uint32_t y[4] = {y4.x, y4.y, y4.z, y4.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int i = 4 * c + k - skip;
+            if (i >= 0 && i < len) {
+                run += cdf_quantize(y[k], base);
+                cell += run <= v;
+            }
+        }
+    }
+    return min(first + cell, last);
+}
+
+// Cell draw from 64 random bits r on row (b, s): v = floor(r * Q / 2^64), and
+// the cell is the i with C[i] <= v < C[i+1] of the fixed-point prefix sums
+// (cdf_quantize) -- the reference's binarySearch (src/arsenal.cpp:644-678) on
+// integer sums.  On a dense row the guide bucket j = r >> (64 - g) brackets the
+// cell by guide[j] <= i <= guide[j+1]; when both agree no CDF entry is read.
+__device__ __noinline__ int cell_search(const CellRows& rows, const SurfSeg* __restrict__ surf, int b, int s,
+                                        unsigned long long r) {
+    const SurfSeg& sg = surf[b];
+    const int q = b * rows.n_species + s;
+    const unsigned long long v = __umul64hi(r, rows.qtot[q]);
+    if (rows.sparse[q]) return sparse_cell(rows, surf, b, s, v);
+    const unsigned long long* row = rows.cdf + sg.cdf_base + static_cast<int64_t>(s) * (sg.n + 1);
+    const int32_t* gd = rows.guide + sg.guide_base + static_cast<int64_t>(s) * ((int64_t(1) << sg.g) + 1);
+    const unsigned j = static_cast<unsigned>(r >> (64 - sg.g));
+    const int2 bk = make_int2(__ldg(gd + j), __ldg(gd + j + 1));
+    const int last = static_cast<int>(sg.n - 1);
+    int lo = min(max(bk.x, 0), last), hi = min(max(bk.y, lo), last);
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (__ldg(row + mid) <= v) lo = mid; else hi = mid - 1;
@@ -1333,40 +1400,98 @@ __device__ __forceinline__ bool setup_hadron(const DevConfig& cfg, const CellArr
     return ok;
 }
 
-// Cell of every hadron's first draw (redraw 0), one warp per work item in
-// species-major order.  Each lane runs independent searches, so the latency
-// of the guide and CDF reads overlaps across many warps; the sampler then
-// starts each hadron from cell_of[slot] instead of a dependent search.
+// Cell of every hadron's first draw (redraw 0).  A warp takes `group`
+// consecutive work items (species-major order, so mostly one species in
+// consecutive events; one item each while there are fewer items than warps)
+// and reads their descriptions with a lane each.  The draws of the items on
+// sparse rows and of those with few draws are then dealt out to the lanes, so
+// that 32 of them are searched at a time whatever items they belong to; the
+// other items are searched by the whole warp, one after another.  Each lane
+// runs independent searches, so the latency of the reads overlaps across lanes
+// and warps; the sampler then starts each hadron from cell_of[slot] instead of
+// a dependent search.  Bound by the latency of those reads.
 constexpr int kAssignThreads = 256;
 
-__global__ void __launch_bounds__(kAssignThreads)
-cell_assign_kernel(DevConfig cfg_in, const unsigned long long* __restrict__ cdf,
-                   const int32_t* __restrict__ guide,
-                   const unsigned long long* __restrict__ qtot, const int64_t* __restrict__ offsets,
+__global__ void __launch_bounds__(kAssignThreads, 4)
+cell_assign_kernel(DevConfig cfg_in, const __grid_constant__ CellRows rows, const int64_t* __restrict__ offsets,
                    const int64_t* __restrict__ item_off, const int32_t* __restrict__ item_seg,
                    int64_t k_begin, int64_t k_end, const SpeciesDev* __restrict__ species,
                    int32_t* __restrict__ cell_of, const int64_t* __restrict__ k_end_dev) {
     const DevConfig cfg = with_run_keys(cfg_in);
     if (k_end_dev) k_end = *k_end_dev;
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t k = k_begin + warp; k < k_end; k += n_warps) {
-        const int q = item_seg[k];
-        const int64_t j = k - item_off[q];
-        int e, s;
-        item_decode(cfg, q, e, s);
-        const int64_t seg = static_cast<int64_t>(e) * cfg.n_species + s;
-        const int64_t base = offsets[seg];
-        const int mult = records_per_draw(cfg, species[s]);
-        const int64_t draws = (offsets[seg + 1] - base) / mult;
-        const int64_t d_begin = j * cfg.item_size;
-        const int64_t d_end = min(d_begin + cfg.item_size, draws);
+    const int group = static_cast<int>(min(static_cast<int64_t>(32), max(static_cast<int64_t>(1),
+                                                                        (k_end - k_begin) / n_warps)));
+    for (int64_t k0 = k_begin + warp * group; k0 < k_end; k0 += n_warps * group) {
+        // this lane's item
+        int e_l = 0, s_l = 0, n_l = 0, mult_l = 1, b_l = 0;
+        uint32_t d_l = 0;
+        int64_t base_l = 0;
+        bool dealt = false;
+        if (lane < group && k0 + lane < k_end) {
+            const int q = item_seg[k0 + lane];
+            item_decode(cfg, q, e_l, s_l);
+            const int64_t seg = static_cast<int64_t>(e_l) * cfg.n_species + s_l;
+            b_l = cfg.ev_surf[e_l];
+            const int64_t first = offsets[seg];
+            const int64_t draws_end = offsets[seg + 1];
+            mult_l = records_per_draw(cfg, species[s_l]);
+            const int64_t d0 = (k0 + lane - item_off[q]) * cfg.item_size;
+            n_l = static_cast<int>(min(static_cast<int64_t>(cfg.item_size), (draws_end - first) / mult_l - d0));
+            d_l = static_cast<uint32_t>(d0);
+            base_l = first - cfg.slot_base;
+            dealt = rows.sparse[b_l * cfg.n_species + s_l] || (group > 1 && n_l <= kDealtDraws);
+        }
+        // draws [pre, pre + n) of the dealt ones are this lane's item's
+        int pre = dealt ? n_l : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(FULL, pre, o);
+            if (lane >= o) pre += x;
+        }
+        const int total = __shfl_sync(FULL, pre, 31);
+        pre -= dealt ? n_l : 0;
+        for (int t0 = 0; t0 < total; t0 += 32) {
+            const int t = t0 + lane;
+            // the last item whose first draw is at or before t (items without
+            // dealt draws share it with the next one)
+            int src = 0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const int x = __shfl_sync(FULL, pre, src + o);
+                if (x <= t) src += o;
+            }
+            const int e = __shfl_sync(FULL, e_l, src), s = __shfl_sync(FULL, s_l, src);
+            const int b = __shfl_sync(FULL, b_l, src);
+            const int mult = __shfl_sync(FULL, mult_l, src);
+            const int64_t base = __shfl_sync(FULL, base_l, src);
+            const uint32_t d = __shfl_sync(FULL, d_l, src) + static_cast<uint32_t>(t - __shfl_sync(FULL, pre, src));
+            if (t < total) {
+                // draws 2j and 2j + 1 take the halves of block j
+                const uint4 w = block(0u, d >> 1, cfg.event_offset + static_cast<uint32_t>(e),
+                                      static_cast<uint32_t>(s) | (kTagCell << 16), cfg.key0, cfg.key1);
+                const uint32_t hi = (d & 1) ? w.z : w.x, lo = (d & 1) ? w.w : w.y;
+                const unsigned long long r = (static_cast<unsigned long long>(hi) << 32) | lo;
+                cell_of[base + static_cast<int64_t>(d) * mult] =
+                    static_cast<int32_t>(cfg.surf[b].c0) + cell_search(rows, cfg.surf, b, s, r);
+            }
+        }
+        unsigned todo = __ballot_sync(FULL, !dealt && n_l > 0);
+        for (; todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1;
+        const int e = __shfl_sync(FULL, e_l, src), s = __shfl_sync(FULL, s_l, src);
+        const int mult = __shfl_sync(FULL, mult_l, src);
+        const int64_t base = __shfl_sync(FULL, base_l, src);
+        const int64_t d_begin = __shfl_sync(FULL, d_l, src);
+        const int64_t d_end = d_begin + __shfl_sync(FULL, n_l, src);
         const int b = cfg.ev_surf[e];
         const SurfSeg sg = cfg.surf[b];
-        const unsigned long long* row = cdf + sg.cdf_base + static_cast<int64_t>(s) * (sg.n + 1);
-        const int32_t* gd = guide + sg.guide_base + static_cast<int64_t>(s) * ((int64_t(1) << sg.g) + 1);
-        const unsigned long long Q = qtot[b * cfg.n_species + s];
+        const unsigned long long* row = rows.cdf + sg.cdf_base + static_cast<int64_t>(s) * (sg.n + 1);
+        const int32_t* gd = rows.guide + sg.guide_base + static_cast<int64_t>(s) * ((int64_t(1) << sg.g) + 1);
+        const unsigned long long Q = rows.qtot[b * cfg.n_species + s];
         const uint32_t eg = cfg.event_offset + static_cast<uint32_t>(e);
         const uint32_t c3 = static_cast<uint32_t>(s) | (kTagCell << 16);
         // 64 draws at a time: each lane takes the pair (2k, 2k + 1), whose
@@ -1437,8 +1562,9 @@ cell_assign_kernel(DevConfig cfg_in, const unsigned long long* __restrict__ cdf,
                 if (c1 <= q1) lo1 = m1; else hi1 = m1 - 1;
             }
         }
-        if (v0) cell_of[base - cfg.slot_base + d0 * mult] = static_cast<int32_t>(sg.c0) + lo0;
-        if (v1) cell_of[base - cfg.slot_base + d1 * mult] = static_cast<int32_t>(sg.c0) + lo1;
+        if (v0) cell_of[base + d0 * mult] = static_cast<int32_t>(sg.c0) + lo0;
+        if (v1) cell_of[base + d1 * mult] = static_cast<int32_t>(sg.c0) + lo1;
+        }
         }
     }
 }
@@ -1454,9 +1580,8 @@ constexpr int kSampleThreads = 256;
 template <bool kLcc, bool kLearned, int kMode>
 __global__ void __launch_bounds__(kSampleThreads, 3)
 sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict__ species,
-               const int32_t* __restrict__ pids, const unsigned long long* __restrict__ cdf,
-               const int32_t* __restrict__ guide,
-               const unsigned long long* __restrict__ qtot, const int64_t* __restrict__ offsets,
+               const int32_t* __restrict__ pids, const __grid_constant__ CellRows rows,
+               const int64_t* __restrict__ offsets,
                const int64_t* __restrict__ item_off, const int32_t* __restrict__ item_seg,
                int64_t k_begin, int64_t k_end, int32_t* __restrict__ cell_of,
                HadronRec* __restrict__ out,
@@ -1564,12 +1689,7 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
                     const unsigned long long r = (static_cast<unsigned long long>(w.x) << 32) |
                                                  static_cast<unsigned long long>(w.y);
                     const int b = cfg.ev_surf[u.eg - cfg.event_offset];
-                    const SurfSeg sg = cfg.surf[b];
-                    l = static_cast<int>(sg.c0) +
-                        cell_search(cdf + sg.cdf_base + static_cast<int64_t>(u.s) * (sg.n + 1), sg.n,
-                                    guide + sg.guide_base +
-                                        static_cast<int64_t>(u.s) * ((int64_t(1) << sg.g) + 1),
-                                    sg.g, qtot[b * cfg.n_species + u.s], r);
+                    l = static_cast<int>(cfg.surf[b].c0) + cell_search(rows, cfg.surf, b, u.s, r);
                 }
                 u.cell = l;
                 u.tries_cell = 0;
@@ -1686,8 +1806,7 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
 template <bool kLcc>
 __global__ void __launch_bounds__(kSampleThreads, 4)
 efa_sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict__ species,
-                   const int32_t* __restrict__ pids, const unsigned long long* __restrict__ cdf,
-                   const int32_t* __restrict__ guide, const unsigned long long* __restrict__ qtot,
+                   const int32_t* __restrict__ pids, const __grid_constant__ CellRows rows,
                    const int64_t* __restrict__ offsets, const int64_t* __restrict__ item_off,
                    const int32_t* __restrict__ item_seg, int64_t k_begin, int64_t k_end,
                    int32_t* __restrict__ cell_of, HadronRec* __restrict__ out,
@@ -1758,11 +1877,7 @@ efa_sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restr
                 const unsigned long long r =
                     (static_cast<unsigned long long>(w.x) << 32) | static_cast<unsigned long long>(w.y);
                 const int b = cfg.ev_surf[e];
-                const SurfSeg sg = cfg.surf[b];
-                l = static_cast<int>(sg.c0) +
-                    cell_search(cdf + sg.cdf_base + static_cast<int64_t>(s) * (sg.n + 1), sg.n,
-                                guide + sg.guide_base + static_cast<int64_t>(s) * ((int64_t(1) << sg.g) + 1),
-                                sg.g, qtot[b * cfg.n_species + s], r);
+                l = static_cast<int>(cfg.surf[b].c0) + cell_search(rows, cfg.surf, b, s, r);
             }
             if (!done) {
                 if (lane < mult)
@@ -2038,9 +2153,7 @@ cudaError_t launch_graph_limits(const int64_t* offsets, const int64_t* item_off,
 }
 
 cudaError_t launch_sampler(const DevConfig& cfg, const CellArrays& cells, const SpeciesDev* sp,
-                           const int32_t* pids, const unsigned long long* cdf,
-                           const int32_t* guide, const unsigned long long* qtot,
-                           const int64_t* offsets,
+                           const int32_t* pids, const CellRows& rows, const int64_t* offsets,
                            const int64_t* item_off, const int32_t* item_seg, int64_t k_begin,
                            int64_t k_end, int32_t* cell_of, HadronRec* out,
                            unsigned long long* work_counter, SampleCounters* counters, int num_sms,
@@ -2054,7 +2167,7 @@ cudaError_t launch_sampler(const DevConfig& cfg, const CellArrays& cells, const 
         const int64_t need = (n_items + (kAssignThreads / 32) - 1) / (kAssignThreads / 32);
         if (blocks > need) blocks = need;
         cell_assign_kernel<<<static_cast<unsigned>(blocks), kAssignThreads, 0, stream>>>(
-            cfg, cdf, guide, qtot, offsets, item_off, item_seg, k_begin, k_end, sp, cell_of,
+            cfg, rows, offsets, item_off, item_seg, k_begin, k_end, sp, cell_of,
             k_end_dev);
     }
     if (cfg.mc_sampling == 2) {
@@ -2065,7 +2178,7 @@ cudaError_t launch_sampler(const DevConfig& cfg, const CellArrays& cells, const 
         if (blocks > need) blocks = need;
         auto efa = cfg.lcc ? efa_sampler_kernel<true> : efa_sampler_kernel<false>;
         efa<<<static_cast<unsigned>(blocks), kSampleThreads, 0, stream>>>(
-            cfg, cells, sp, pids, cdf, guide, qtot, offsets, item_off, item_seg, k_begin, k_end, cell_of, out,
+            cfg, cells, sp, pids, rows, offsets, item_off, item_seg, k_begin, k_end, cell_of, out,
             work_counter, counters, k_end_dev);
         return cudaGetLastError();
     }
@@ -2084,7 +2197,7 @@ cudaError_t launch_sampler(const DevConfig& cfg, const CellArrays& cells, const 
         : mode == 2 ? (cfg.lcc ? sampler_kernel<true, false, 2> : sampler_kernel<false, false, 2>)
                     : (cfg.lcc ? sampler_kernel<true, false, 0> : sampler_kernel<false, false, 0>);
     kernel<<<static_cast<unsigned>(blocks), kSampleThreads, 0, stream>>>(
-        cfg, cells, sp, pids, cdf, guide, qtot, offsets, item_off, item_seg, k_begin,
+        cfg, cells, sp, pids, rows, offsets, item_off, item_seg, k_begin,
         k_end, cell_of, out, work_counter, counters, k_end_dev);
     return cudaGetLastError();
 }
