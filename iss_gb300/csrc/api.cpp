@@ -130,7 +130,7 @@ struct iss_handle {
     DevBuf<float4> d_milne;          // MC_sampling = 2: regulated Milne cells, 6 float4 each
     DevBuf<SpeciesDev> d_species;
     DevBuf<int32_t> d_pids;
-    DevBuf<int32_t> d_yorder;        // yields kernel: species grouped by identical series
+    DevBuf<float4> d_ylist;          // yields kernel: species grouped by identical series
     DevBuf<float> d_yields;
     DevBuf<unsigned long long> d_cdf, d_tile_sum, d_tile_off, d_sub, d_qtot;
     DevBuf<int32_t> d_sparse;        // rows whose CDF is not written (CellRows)
@@ -145,8 +145,7 @@ struct iss_handle {
     DevBuf<int> d_error;
     // tables
     TableKey table_key;
-    DevBuf<float4> d_sfK;
-    DevBuf<float> d_sfE;
+    DevBuf<float4> d_sfK, d_sfE;
     DevBuf<double> d_b14c0, d_b14c1, d_b14c2, d_ce, d_qmu, d_logfact, d_pois;
     Bulk14Table b14;
 
@@ -184,13 +183,14 @@ struct iss_handle {
 
     ~iss_handle() {
         if (cuda_ready) {
-            DevBuf<float>* fb[] = {&d_fo34, &d_yields, &d_sfE};
+            DevBuf<float>* fb[] = {&d_fo34, &d_yields};
             for (auto* b : fb) b->release();
+            d_sfE.release();
             d_cells.release();
             d_milne.release();
             d_species.release();
             d_pids.release();
-            d_yorder.release();
+            d_ylist.release();
             DevBuf<double>* db[] = {&d_totals, &d_b14c0, &d_b14c1, &d_b14c2, &d_ce, &d_qmu,
                                     &d_logfact, &d_pois};
             for (auto* b : db) b->release();
@@ -272,15 +272,16 @@ iss_status fail(iss_handle* h, iss_status st, const char* fmt, ...) {
             return fail((h), ISS_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(_e)); \
     } while (0)
 
-// Species groups of the yields kernel.  The thermal series of
-// calculate_dN_analytic (src/FSSW.cpp:719-848) depends on a species only
-// through its mass, statistics, number of terms and chemical potential, so
-// species that agree in the first three share one series per cell (isospin
-// partners, particles and antiparticles).  Layout: G + 1 group starts into
-// the member list, then the members (species indices, each species once).
-// Groups are ordered by decreasing work (series terms, then members), so
-// that the kernel's interleaving of groups over grid rows stays balanced.
-std::vector<int32_t> yield_group_order(const std::vector<SpeciesDev>& sd) {
+// The species list of the yields kernel (YieldGroup, device_common.cuh).  The
+// thermal series of calculate_dN_analytic (src/FSSW.cpp:719-848) depends on a
+// species only through its mass, statistics, number of terms and chemical
+// potential, so species that agree in the first three share one series per
+// cell (isospin partners, particles and antiparticles).  Groups are ordered
+// by decreasing work (series terms, then members), so that the kernel's
+// interleaving of groups over grid rows stays balanced.  The members of a
+// group that also agree in degeneracy and baryon number form a run: their
+// yields are equal wherever strangeness and charge have no potential.
+std::vector<float4> yield_list(const std::vector<SpeciesDev>& sd, int* n_groups, int* n_runs) {
     std::vector<std::vector<int32_t>> groups;
     for (size_t k = 0; k < sd.size(); k++) {
         const SpeciesDev& a = sd[k];
@@ -300,14 +301,42 @@ std::vector<int32_t> yield_group_order(const std::vector<SpeciesDev>& sd) {
     };
     std::stable_sort(groups.begin(), groups.end(),
                      [&](const auto& x, const auto& y) { return cost(x) > cost(y); });
-    std::vector<int32_t> out;
-    int32_t start = 0;
-    for (const auto& g : groups) {
-        out.push_back(start);
-        start += static_cast<int32_t>(g.size());
+    auto same_run = [&](int32_t x, int32_t y) {
+        return sd[x].degen == sd[y].degen && sd[x].baryon == sd[y].baryon;
+    };
+    std::vector<int32_t> group_runs, run_members, member;
+    for (auto& g : groups) {
+        std::stable_sort(g.begin(), g.end(), [&](int32_t x, int32_t y) {
+            return std::make_pair(sd[x].degen, sd[x].baryon) < std::make_pair(sd[y].degen, sd[y].baryon);
+        });
+        group_runs.push_back(static_cast<int32_t>(run_members.size()));
+        for (size_t i = 0; i < g.size(); i++) {
+            if (i == 0 || !same_run(g[i - 1], g[i])) run_members.push_back(static_cast<int32_t>(member.size()));
+            member.push_back(g[i]);
+        }
     }
-    out.push_back(start);
-    for (const auto& g : groups) out.insert(out.end(), g.begin(), g.end());
+    const int S = static_cast<int>(sd.size()), G = static_cast<int>(groups.size());
+    const int R = static_cast<int>(run_members.size());
+    *n_groups = G;
+    *n_runs = R;
+    group_runs.push_back(R);
+    run_members.push_back(S);
+    std::vector<float4> out(static_cast<size_t>(yield_list_float4(S, G, R)), float4{0.f, 0.f, 0.f, 0.f});
+    for (int t = 0; t < S; t++) {
+        const SpeciesDev& s = sd[static_cast<size_t>(member[t])];
+        out[static_cast<size_t>(t)] = float4{static_cast<float>(s.baryon), static_cast<float>(s.strange),
+                                             static_cast<float>(s.charge), s.degen};
+    }
+    for (int g = 0; g < G; g++) {
+        const SpeciesDev& s = sd[static_cast<size_t>(groups[static_cast<size_t>(g)][0])];
+        const YieldGroup yg{s.m_hi, s.m_lo, s.sign, s.light};
+        static_assert(sizeof(YieldGroup) == sizeof(float4), "a group is one float4");
+        std::memcpy(&out[static_cast<size_t>(S + g)], &yg, sizeof(yg));
+    }
+    int32_t* tail = reinterpret_cast<int32_t*>(out.data() + S + G);
+    tail = std::copy(group_runs.begin(), group_runs.end(), tail);
+    tail = std::copy(run_members.begin(), run_members.end(), tail);
+    std::copy(member.begin(), member.end(), tail);
     return out;
 }
 
@@ -527,8 +556,10 @@ iss_status prepare(iss_handle* h) {
         CUDA_TRY(h, cudaMemcpy(h->d_sfK.ptr, K4.data(), sizeof(float4) * kSfLen,
                                cudaMemcpyHostToDevice));
         if (c.include_diff) {
-            std::vector<float> E32(E.begin(), E.end());
-            CUDA_TRY(h, h->d_sfE.reserve(E32.size()));
+            std::vector<float> E32(static_cast<size_t>(kSfLen) * 12, 0.0f);
+            for (int i = 0; i < kSfLen; i++)
+                for (int j = 0; j < 9; j++) E32[12 * i + j] = static_cast<float>(E[9 * i + j]);
+            CUDA_TRY(h, h->d_sfE.reserve(static_cast<size_t>(kSfLen) * 3));
             CUDA_TRY(h, cudaMemcpy(h->d_sfE.ptr, E32.data(), sizeof(float) * E32.size(),
                                    cudaMemcpyHostToDevice));
         }
@@ -604,18 +635,17 @@ iss_status prepare(iss_handle* h) {
     // (same float-float mass, statistics and number of terms) form one group
     // of the yields kernel; the series runs once per group and cell whenever
     // the members' chemical potentials agree in that cell
-    const std::vector<int32_t> yorder = yield_group_order(sd);
-    c.n_ygroups = static_cast<int>(yorder.size() - sd.size()) - 1;
+    const std::vector<float4> ylist = yield_list(sd, &c.n_ygroups, &c.n_yruns);
     CUDA_TRY(h, h->d_species.reserve(sd.size()));
     CUDA_TRY(h, h->d_pids.reserve(sd.size()));
-    CUDA_TRY(h, h->d_yorder.reserve(yorder.size()));
-    c.yorder = h->d_yorder.ptr;
+    CUDA_TRY(h, h->d_ylist.reserve(ylist.size()));
+    c.ylist = h->d_ylist.ptr;
     if (!sd.empty()) {
         CUDA_TRY(h, cudaMemcpyAsync(h->d_species.ptr, sd.data(), sizeof(SpeciesDev) * sd.size(),
                                     cudaMemcpyHostToDevice, h->stream));
         CUDA_TRY(h, cudaMemcpyAsync(h->d_pids.ptr, pids.data(), 4 * pids.size(),
                                     cudaMemcpyHostToDevice, h->stream));
-        CUDA_TRY(h, cudaMemcpyAsync(h->d_yorder.ptr, yorder.data(), 4 * yorder.size(),
+        CUDA_TRY(h, cudaMemcpyAsync(h->d_ylist.ptr, ylist.data(), sizeof(float4) * ylist.size(),
                                     cudaMemcpyHostToDevice, h->stream));
     }
     h->cfg = c;
@@ -677,13 +707,13 @@ iss_status run_cells(iss_handle* h) {
     CUDA_TRY(h, h->d_totals.reserve(rows));
     CUDA_TRY(h, h->d_sparse.reserve(rows));
     CUDA_TRY(h, h->d_qtot.reserve(rows));
-    CUDA_TRY(h, h->d_ymax.reserve(rows));
+    CUDA_TRY(h, h->d_ymax.reserve(rows + 1));   // and launch_yields' flag
     CUDA_TRY(h, h->d_guide.reserve(static_cast<size_t>(std::max<int64_t>(h->guide_len, 1))));
     const CellArrays cells = cell_arrays(h);
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvStart], st));
     CUDA_TRY(h, launch_cell_prologue(c, h->d_fo34.ptr, n, cells, st));
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvPrologue], st));
-    CUDA_TRY(h, launch_yields(c, cells, h->d_species.ptr, h->d_yields.ptr, h->d_ymax.ptr, st));
+    CUDA_TRY(h, launch_yields(c, cells, h->d_yields.ptr, h->d_ymax.ptr, h->num_sms, st));
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvYields], st));
     // the number of events is not known yet when it follows from the yields
     const bool allow_sparse = h->params.get_or("sample_upto_desired_particle_number", 0) != 1;
@@ -1066,7 +1096,7 @@ cudaError_t enqueue_generate(iss_handle* h, const DevConfig& c) {
     record(h, kEvStart, true);
     GTRY(launch_cell_prologue(c, h->d_fo34.ptr, n, cells, s));
     record(h, kEvPrologue, true);
-    GTRY(launch_yields(c, cells, h->d_species.ptr, h->d_yields.ptr, h->d_ymax.ptr, s));
+    GTRY(launch_yields(c, cells, h->d_yields.ptr, h->d_ymax.ptr, h->num_sms, s));
     record(h, kEvYields, true);
     const CdfBuffers cb = cdf_buffers(h);
     GTRY(launch_cdf_head(h->d_yields.ptr, n, h->d_surf.ptr, c.n_surfaces, h->n_tiles, S, h->d_ymax.ptr,

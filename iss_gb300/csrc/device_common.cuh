@@ -13,7 +13,7 @@ namespace iss {
 
 struct DevTables {
     const float4* sfK;      // [kSfLen] (K1, K2, K3, 0) in FP32, grid x = 0.5 + 0.05 i
-    const float* sfE;       // [kSfLen * 9] E_2, E_4, ..., E_18 in FP32
+    const float4* sfE;      // [kSfLen][3] E_2, E_4, ..., E_18 in FP32, padded to 12 floats
     const double* b14c0;    // OSU 14-moment tables [iT * nmu + imu]
     const double* b14c1;
     const double* b14c2;
@@ -73,10 +73,10 @@ struct DevConfig {
     // launch shape (results do not depend on it; the autotuner picks it)
     int item_size;       // draws per sampler work item (multiple of 32, <= 1024)
     int yield_groups;    // species groups per cell in the yields kernel (grid y)
-    // yields kernel: n_ygroups + 1 group starts, then the species of each
-    // group (species with the same thermal series, yield_group_order)
-    const int32_t* yorder;
-    int n_ygroups;
+    // yields kernel: the yield list (YieldGroup) of n_ygroups groups and
+    // n_yruns runs
+    const float4* ylist;
+    int n_ygroups, n_yruns;
     int sampler_ctas;    // sampler CTAs per SM (1..3)
     int assign_bps;      // cell-assignment blocks per SM
     // graph replays: (key0, key1, event_offset) of the call in device memory,
@@ -106,6 +106,22 @@ struct SpeciesDev {
     int light;               // mass < 0.7 GeV: 10 series terms (src/FSSW.cpp:740-745)
     int baryon, strange, charge, sign;
 };
+
+// The yields kernel's list of species, group by group (species with the same
+// thermal series) and inside a group run by run (the same degeneracy and baryon
+// number): for every member (baryon number, strangeness, charge, degeneracy) as
+// floats; the groups; the G + 1 first runs of the groups; the R + 1 first
+// members of the runs; the members' species indices.
+struct YieldGroup {
+    float m_hi, m_lo;        // FP64 mass as a float-float pair
+    int sign, light;         // statistics; 1: ten series terms
+};
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+inline int yield_list_float4(int n_species, int n_groups, int n_runs) {
+    return n_species + n_groups + (n_groups + 1 + n_runs + 1 + n_species + 3) / 4;
+}
 
 // What a cell draw reads of the (surface, species) rows r = b S + k: the full
 // prefix sums and guide table of dense rows, and for the others (sparse[r])

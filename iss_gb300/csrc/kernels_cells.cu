@@ -79,13 +79,9 @@ __device__ __forceinline__ GridPos grid_pos(float xh, float xl) {
     const float pl = fmaf(20.0f, se, pe);
     int idx = static_cast<int>(floorf(ph));
     float f = (ph - static_cast<float>(idx)) + pl;
-    if (f < 0.0f) {
-        idx -= 1;
-        f += 1.0f;
-    } else if (f >= 1.0f) {
-        idx += 1;
-        f -= 1.0f;
-    }
+    const bool below = f < 0.0f, above = f >= 1.0f;
+    idx += static_cast<int>(above) - static_cast<int>(below);
+    f = below ? f + 1.0f : (above ? f - 1.0f : f);
     g.idx = min(max(idx, 0), 7989);
     g.frac = f;
     return g;
@@ -105,12 +101,16 @@ __device__ __forceinline__ int surface_of(const SurfSeg* __restrict__ surf, int 
     return lo;
 }
 
+// Form of the bulk correction of the yields (include_deltaf_bulk): none (also
+// for the kinds without a yield term), Chapman-Enskog (kinds 1 and 21), the
+// 14-moment form (kind 11)
+constexpr int kNoBulk = 0, kBulkCe = 1, kBulk14 = 2;
+
 // Per-cell quantities shared by every species' yield in cell l.
 struct CellYieldIn {
     float T, b_hi, b_lo;
-    bool warm, with_bulk, kind_ce, kind_14;
-    int bulk_kind;
-    float bulkPi, dsq, pref_q, inv_kappa, unit_pref;
+    bool warm;
+    float da0, bulkPi, dsq, pref_q, inv_kappa, unit_pref;
     float4 th, th2, cf;
 };
 
@@ -121,97 +121,132 @@ struct SeriesSums {
     float Neq, b1, b2, b3, q1, q2;
 };
 
-__device__ __forceinline__ float species_mu(const SpeciesDev& sp, const float4& th) {
-    return static_cast<float>(sp.baryon) * th.y + static_cast<float>(sp.strange) * th.z +
-           static_cast<float>(sp.charge) * th.w;
+// Term nn of the series, with what the terms share: x1 = m beta and
+// bm = beta mu as float-float numbers.  kFirst: nn = 1, where n x and the
+// divisions by n drop out (nine species in ten have this term only).  A
+// division by n = 2, 4, 8 is a multiplication by the exact 1 / n: the same
+// correctly rounded quotient.  kTable: an argument off the special-function
+// table only sets off; without it, it is evaluated directly as well.
+template <int kBulk, bool kDiff, bool kFirst, bool kTable>
+__device__ __forceinline__ void series_term(const DevConfig& cfg, const CellYieldIn& c, int nn, float theta,
+                                            float x1_h, float x1_l, float bm_h, float bm_l, bool no_mu,
+                                            float mbeta, SeriesSums& s, bool& off) {
+    const float fn = kFirst ? 1.0f : static_cast<float>(nn);
+    // x_n = n m beta
+    float xh = x1_h, xl = x1_l;
+    if (!kFirst) {
+        float xe;
+        two_prod(fn, x1_h, xh, xe);
+        xl = fmaf(fn, x1_l, xe);
+    }
+    // lambda^n = exp(n beta mu)
+    float fug = 1.0f;
+    if (!no_mu) {
+        float ah = bm_h, al = bm_l;
+        if (!kFirst) {
+            float ae;
+            two_prod(fn, bm_h, ah, ae);
+            al = fmaf(fn, bm_l, ae);
+        }
+        fug = expf(ah) * (1.0f + al);
+    }
+    const GridPos g = grid_pos(xh, xl);
+    if (!g.on_table) off = true;
+    float K1, K2, K3;
+    if (kTable || g.on_table) {
+        const float4 ka = __ldg(cfg.tab.sfK + g.idx);
+        const float4 kb = __ldg(cfg.tab.sfK + g.idx + 1);
+        K1 = fmaf(g.frac, kb.x - ka.x, ka.x);
+        K2 = fmaf(g.frac, kb.y - ka.y, ka.y);
+        K3 = fmaf(g.frac, kb.z - ka.z, ka.z);
+    } else {
+        const double xd = static_cast<double>(xh) + static_cast<double>(xl);
+        K2 = static_cast<float>(bessel_k_direct(2, xd));
+        K1 = kBulk != kNoBulk ? static_cast<float>(bessel_k_direct(1, xd)) : 0.0f;
+        K3 = kBulk == kBulk14 ? static_cast<float>(bessel_k_direct(3, xd)) : 0.0f;
+    }
+    const float tf = theta * fug;
+    float tf_n = tf, k2_n = 3.0f * K2, k3_n = 3.0f * K3;
+    if (!kFirst) {
+        if ((nn & (nn - 1)) == 0) {
+            const float r = 1.0f / fn;
+            tf_n *= r;
+            k2_n *= r;
+            k3_n *= r;
+        } else {
+            tf_n = tf_n / fn;
+            if (kBulk != kNoBulk) k2_n = k2_n / fn;
+            if (kBulk == kBulk14) k3_n = k3_n / fn;
+        }
+    }
+    s.Neq = fmaf(tf_n, K2, s.Neq);
+    if (kBulk == kBulkCe) {
+        s.b1 = fmaf(tf, fmaf(mbeta, K1, k2_n), s.b1);
+        s.b2 = fmaf(tf, K1, s.b2);
+    } else if (kBulk == kBulk14) {
+        s.b1 = fmaf(tf, K2, s.b1);
+        s.b2 = fmaf(tf, fmaf(mbeta, K1, k2_n), s.b2);
+        s.b3 = fmaf(tf, fmaf(mbeta, K2, k3_n), s.b3);
+    }
+    if (kDiff) {
+        s.q1 = fmaf(tf_n, K2, s.q1);
+        float En[9];
+        if (kTable || g.on_table) {
+            // rows of 12 floats: three 16-byte reads each
+            const float4* ea = cfg.tab.sfE + 3 * g.idx;
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const float4 a = __ldg(ea + i), b = __ldg(ea + 3 + i);
+                En[4 * i] = fmaf(g.frac, b.x - a.x, a.x);
+                if (i < 2) {
+                    En[4 * i + 1] = fmaf(g.frac, b.y - a.y, a.y);
+                    En[4 * i + 2] = fmaf(g.frac, b.z - a.z, a.z);
+                    En[4 * i + 3] = fmaf(g.frac, b.w - a.w, a.w);
+                }
+            }
+        } else {
+            const double xd = static_cast<double>(xh) + static_cast<double>(xl);
+            En[0] = static_cast<float>(expint_direct(2, xd));
+            for (int i = 1; i < 9; i++) En[i] = static_cast<float>(expint_direct(2 * i + 2, xd));
+        }
+        const float arg = xh;
+        const float em = expf(-xh) * (1.0f - xl);
+        float I = em / arg * (2.0f / (arg * arg) + 2.0f / arg - 0.5f) + 0.375f * En[0];
+        // 3 (2k-5)!! / (2^k k!) for k = 3..10
+        const float ck[8] = {0.0625f, 0.0234375f, 0.01171875f, 0.0068359375f,
+                             0.00439453125f, 0.0030212402343750f,
+                             0.0021820068359375f, 0.0016365051269531f};
+#pragma unroll
+        for (int k2 = 0; k2 < 8; k2++) I = fmaf(ck[k2], En[k2 + 1], I);
+        I = -(mbeta * mbeta * mbeta) * I;
+        s.q2 = fmaf(fn * tf, I, s.q2);
+    }
 }
 
-template <bool kDiff>
+template <int kBulk, bool kDiff, bool kTable>
 __device__ __forceinline__ SeriesSums thermal_series(const DevConfig& cfg, const CellYieldIn& c,
-                                                     const SpeciesDev& sp, float mu) {
+                                                     const YieldGroup& gr, float mu, bool& off) {
     const float b_hi = c.b_hi, b_lo = c.b_lo;
-    const bool warm = c.warm, with_bulk = c.with_bulk;
-    constexpr bool with_diff = kDiff;
-    const bool kind_ce = c.kind_ce, kind_14 = c.kind_14;
     // beta*mu and m*beta as float-float numbers
     float bm_h, bm_e;
     two_prod(mu, b_hi, bm_h, bm_e);
     const float bm_l = fmaf(mu, b_lo, bm_e);
     float x1_h, x1_e;
-    two_prod(sp.m_hi, b_hi, x1_h, x1_e);
-    const float x1_l = x1_e + fmaf(sp.m_hi, b_lo, sp.m_lo * b_hi);
-    const int nmax = (sp.light && warm) ? 10 : 1;
-    float Neq = 0.f, b1 = 0.f, b2 = 0.f, b3 = 0.f, q1 = 0.f, q2 = 0.f;
+    two_prod(gr.m_hi, b_hi, x1_h, x1_e);
+    const float x1_l = x1_e + fmaf(gr.m_hi, b_lo, gr.m_lo * b_hi);
+    const bool no_mu = mu == 0.0f;   // exp(0) = 1
     const float mbeta = x1_h + x1_l;
-    for (int nn = 1; nn <= nmax; nn++) {
-        const float fn = static_cast<float>(nn);
-        float theta = 1.0f;
-        if (sp.sign == 1 && (nn % 2 == 0)) theta = -1.0f;
-        if (sp.sign == 0 && nn > 1) theta = 0.0f;
-        // x_n = n m beta
-        float xh, xe;
-        two_prod(fn, x1_h, xh, xe);
-        const float xl = fmaf(fn, x1_l, xe);
-        // lambda^n = exp(n beta mu)
-        float ah, ae;
-        two_prod(fn, bm_h, ah, ae);
-        const float al = fmaf(fn, bm_l, ae);
-        const float fug = expf(ah) * (1.0f + al);
-        const GridPos g = grid_pos(xh, xl);
-        float K1, K2, K3;
-        if (g.on_table) {
-            const float4 ka = __ldg(cfg.tab.sfK + g.idx);
-            const float4 kb = __ldg(cfg.tab.sfK + g.idx + 1);
-            K1 = fmaf(g.frac, kb.x - ka.x, ka.x);
-            K2 = fmaf(g.frac, kb.y - ka.y, ka.y);
-            K3 = fmaf(g.frac, kb.z - ka.z, ka.z);
-        } else {
-            const double xd = static_cast<double>(xh) + static_cast<double>(xl);
-            K2 = static_cast<float>(bessel_k_direct(2, xd));
-            K1 = with_bulk ? static_cast<float>(bessel_k_direct(1, xd)) : 0.0f;
-            K3 = (with_bulk && kind_14) ? static_cast<float>(bessel_k_direct(3, xd)) : 0.0f;
-        }
-        const float tf = theta * fug;
-        Neq = fmaf(tf / fn, K2, Neq);
-        if (with_bulk) {
-            if (kind_ce) {
-                b1 = fmaf(tf, fmaf(mbeta, K1, 3.0f * K2 / fn), b1);
-                b2 = fmaf(tf, K1, b2);
-            } else if (kind_14) {
-                b1 = fmaf(tf, K2, b1);
-                b2 = fmaf(tf, fmaf(mbeta, K1, 3.0f * K2 / fn), b2);
-                b3 = fmaf(tf, fmaf(mbeta, K2, 3.0f * K3 / fn), b3);
-            }
-        }
-        if (with_diff) {
-            q1 = fmaf(tf / fn, K2, q1);
-            float En[9];
-            if (g.on_table) {
-                const float* ea = cfg.tab.sfE + 9 * g.idx;
-#pragma unroll
-                for (int i = 0; i < 9; i++) {
-                    const float a = __ldg(ea + i), b = __ldg(ea + 9 + i);
-                    En[i] = fmaf(g.frac, b - a, a);
-                }
-            } else {
-                const double xd = static_cast<double>(xh) + static_cast<double>(xl);
-                En[0] = static_cast<float>(expint_direct(2, xd));
-                for (int i = 1; i < 9; i++) En[i] = static_cast<float>(expint_direct(2 * i + 2, xd));
-            }
-            const float arg = xh;
-            const float em = expf(-xh) * (1.0f - xl);
-            float I = em / arg * (2.0f / (arg * arg) + 2.0f / arg - 0.5f) + 0.375f * En[0];
-            // 3 (2k-5)!! / (2^k k!) for k = 3..10
-            const float ck[8] = {0.0625f, 0.0234375f, 0.01171875f, 0.0068359375f,
-                                 0.00439453125f, 0.0030212402343750f,
-                                 0.0021820068359375f, 0.0016365051269531f};
-#pragma unroll
-            for (int k2 = 0; k2 < 8; k2++) I = fmaf(ck[k2], En[k2 + 1], I);
-            I = -(mbeta * mbeta * mbeta) * I;
-            q2 = fmaf(fn * tf, I, q2);
+    SeriesSums s{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    series_term<kBulk, kDiff, true, kTable>(cfg, c, 1, 1.0f, x1_h, x1_l, bm_h, bm_l, no_mu, mbeta, s, off);
+    if (gr.light && c.warm) {
+        for (int nn = 2; nn <= 10; nn++) {
+            float theta = 1.0f;
+            if (gr.sign == 1 && (nn % 2 == 0)) theta = -1.0f;
+            if (gr.sign == 0) theta = 0.0f;
+            series_term<kBulk, kDiff, false, kTable>(cfg, c, nn, theta, x1_h, x1_l, bm_h, bm_l, no_mu, mbeta, s, off);
         }
     }
-    return SeriesSums{Neq, b1, b2, b3, q1, q2};
+    return s;
 }
 
 // The yield of calculate_dN_dxtdy_for_one_particle_species
@@ -220,31 +255,29 @@ __device__ __forceinline__ SeriesSums thermal_series(const DevConfig& cfg, const
 // bulk and diffusion terms, and depend on the species only through the
 // quantities its group shares (mass and the series sums).  They are formed
 // once per series; each member then costs one multiply-add.
-template <bool kDiff>
-__device__ __forceinline__ float2 yield_coefs(const CellYieldIn& c, const SpeciesDev& sp,
-                                              const SeriesSums& ss, float4 da) {
+template <int kBulk, bool kDiff>
+__device__ __forceinline__ float2 yield_coefs(const CellYieldIn& c, const YieldGroup& gr,
+                                              const SeriesSums& ss) {
     const float T = c.T;
     const float4 cf = c.cf;
-    const float mass = sp.m_hi + sp.m_lo;
+    const float mass = gr.m_hi + gr.m_lo;
     const float m2 = mass * mass;
-    float x = m2 * T * ss.Neq;
+    // (the products and fused multiply-adds are spelled out: the yields feed the
+    // integer CDF, so every build has to round them alike)
+    float x = __fmul_rn(m2 * T, ss.Neq);
     float y = 0.0f;
-    if (c.with_bulk) {
-        if (c.kind_ce) {
-            // Chapman-Enskog form, bulk_deltaf_kind 1 and 21
-            const float r1 = m2 * T * ss.b1;
-            const float r2 = m2 * mass / 3.0f * ss.b2;
-            x += (-c.bulkPi * cf.x) * (-cf.y * r1 + r2);
-        } else if (c.bulk_kind == 11) {
-            const float r1 = m2 * T * ss.b1;
-            const float r2 = m2 * T * T * ss.b2;
-            const float r3 = m2 * mass * T * T * ss.b3;
-            x += c.bulkPi * (r1 * m2 * cf.x + r3 * cf.z);
-            y += c.bulkPi * r2 * cf.y;
-        }
+    if (kBulk == kBulkCe) {
+        const float r1 = __fmul_rn(m2 * T, ss.b1);
+        x = fmaf(__fmul_rn(-c.bulkPi, cf.x), fmaf(m2 * mass / 3.0f, ss.b2, -__fmul_rn(cf.y, r1)), x);
+    } else if (kBulk == kBulk14) {
+        const float r1 = __fmul_rn(m2 * T, ss.b1);
+        const float r2 = __fmul_rn(m2 * T * T, ss.b2);
+        const float r3 = __fmul_rn(m2 * mass * T * T, ss.b3);
+        x = fmaf(c.bulkPi, fmaf(__fmul_rn(r1, m2), cf.x, __fmul_rn(r3, cf.z)), x);
+        y = __fmul_rn(__fmul_rn(c.bulkPi, r2), cf.y);
     }
-    x *= da.x;
-    y *= da.x;
+    x *= c.da0;
+    y *= c.da0;
     if (kDiff) {
         const float r4 = m2 * T * T * ss.q1;
         const float r5 = (T * T * T / 3.0f) * ss.q2;
@@ -258,141 +291,200 @@ __device__ __forceinline__ float2 yield_coefs(const CellYieldIn& c, const Specie
 // negative -> 0 (FSSW::calculate_dN_dxtdy_for_one_particle_species,
 // src/FSSW.cpp:707); NaN -> 0; +inf -> FLT_MAX so the cell CDF stays
 // finite; -0 -> +0 so the bits order as the values
-__device__ __forceinline__ float member_yield(const SpeciesDev& sp, float2 xy) {
-    const float total = sp.degen * fmaf(static_cast<float>(sp.baryon), xy.y, xy.x);
+__device__ __forceinline__ float member_yield(const float4& q, float2 xy) {
+    const float total = q.w * fmaf(q.x, xy.y, xy.x);
     return __uint_as_float(__float_as_uint(fminf(fmaxf(total, 0.0f), 3.40282347e38f)) & 0x7FFFFFFFu);
 }
 
-// Yields of the species groups k0, k0 + kstep, ... in cell l (not dropped:
-// u.dsigma >= 0).  A group's series runs for its first member and is reused
-// by the next members while their chemical potential in this cell has the
-// same bits (the same inputs, so the same sums); a member with another mu
-// gets its own series.
-template <bool kDiff>
-__device__ __forceinline__ void cell_yields(const DevConfig& cfg, const CellArrays& cells,
-                                            const SpeciesDev* s_sp, const int32_t* s_gst,
-                                            const int32_t* s_mem, int n_groups, int k0, int kstep,
-                                            int64_t n, int64_t l, float4 da, bool valid, bool live,
-                                            uint32_t* s_max, uint32_t* __restrict__ ymax_row,
-                                            float* __restrict__ yields) {
+// Per-cell quantities of cell l (not dropped: u.dsigma >= 0)
+template <int kBulk, bool kDiff>
+__device__ __forceinline__ CellYieldIn cell_yield_in(const DevConfig& cfg, const CellArrays& cells,
+                                                     int64_t l, const float4& da) {
     CellYieldIn c;
-    const int64_t lc = valid ? l : 0;   // lanes past the last cell read cell 0 and store nothing
-    c.th = cells.th[lc];
-    c.th2 = cells.th2[lc];
-    c.cf = cells.coef[lc];
-    const float4 th = c.th, th2 = c.th2, cf = c.cf;
-    const float T = th.x;
+    c.th = cells.th[l];
+    c.th2 = cells.th2[l];
+    c.cf = cells.coef[l];
+    const float T = c.th.x;
     const double beta_d = 1.0 / static_cast<double>(T);
-    const float b_hi = static_cast<float>(beta_d);
-    const float b_lo = static_cast<float>(beta_d - static_cast<double>(b_hi));
-    const bool warm = static_cast<double>(T) > 0.05;
-    const int bulk_kind = cfg.bulk_kind;
-    const bool with_bulk = cfg.include_bulk != 0;
-    constexpr bool with_diff = kDiff;
-    const bool kind_ce = (bulk_kind == 1 || bulk_kind == 21);
-    const bool kind_14 = (bulk_kind == 11 || bulk_kind == 20);
-    float bulkPi = 0.0f;
-    if (with_bulk) bulkPi = (bulk_kind == 21 || bulk_kind == 20 || bulk_kind == 11 || bulk_kind == 0)
-                                ? th2.w : th2.w / kHbarCf;
-    float dsq = 0.0f, pref_q = 0.0f, inv_kappa = 0.0f;
-    if (with_diff) {
-        const float4 p2 = cells.pi2[lc];
-        dsq = p2.y * da.y + p2.z * da.z + p2.w * da.w;
-        pref_q = th2.z / (th2.x + th2.y);
-        inv_kappa = 1.0f / cf.w;
-    }
-    // (1/hbarc^3) / (2 pi^2)
-    const float unit_pref = (1.0f / (0.197327053f * 0.197327053f * 0.197327053f)) /
-                            (2.0f * 9.8696044010893586f);
-
     c.T = T;
-    c.b_hi = b_hi;
-    c.b_lo = b_lo;
-    c.warm = warm;
-    c.with_bulk = with_bulk;
-    c.kind_ce = kind_ce;
-    c.kind_14 = kind_14;
-    c.bulk_kind = bulk_kind;
-    c.bulkPi = bulkPi;
-    c.dsq = dsq;
-    c.pref_q = pref_q;
-    c.inv_kappa = inv_kappa;
-    c.unit_pref = unit_pref;
-    for (int j = k0; j < n_groups; j += kstep) {
-        const int a = s_gst[j], b = s_gst[j + 1];
-        float2 xy = make_float2(0.0f, 0.0f);
-        uint32_t mu_bits = 0;
-        for (int t = a; t < b; t++) {
-            const int k = s_mem[t];
-            const SpeciesDev sp = s_sp[k];
-            float yv = 0.0f;
-            if (live) {
-                const float mu = species_mu(sp, th);
-                if (t == a || __float_as_uint(mu) != mu_bits) {
-                    xy = yield_coefs<kDiff>(c, sp, thermal_series<kDiff>(cfg, c, sp, mu), da);
-                    mu_bits = __float_as_uint(mu);
-                }
-                yv = member_yield(sp, xy);
-            }
-            if (valid) yields[static_cast<int64_t>(k) * n + l] = yv;
-            // the species' largest yield (its float bits: yields are >= +0,
-            // so the unsigned order of the bits is the order of the values)
-            const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(yv));
-            if ((threadIdx.x & 31) == 0 && m) {
-                if (s_max) atomicMax(s_max + k, m);
-                else atomicMax(ymax_row + k, m);
-            }
-        }
+    c.da0 = da.x;
+    c.b_hi = static_cast<float>(beta_d);
+    c.b_lo = static_cast<float>(beta_d - static_cast<double>(c.b_hi));
+    c.warm = T >= 0.05f;   // as double: T > 0.05 (0.05f is the first float above it)
+    c.bulkPi = 0.0f;
+    if (kBulk != kNoBulk) c.bulkPi = cfg.bulk_kind == 1 ? c.th2.w / kHbarCf : c.th2.w;
+    c.dsq = c.pref_q = c.inv_kappa = 0.0f;
+    if (kDiff) {
+        const float4 p2 = cells.pi2[l];
+        c.dsq = p2.y * da.y + p2.z * da.z + p2.w * da.w;
+        c.pref_q = c.th2.z / (c.th2.x + c.th2.y);
+        c.inv_kappa = 1.0f / c.cf.w;
     }
+    // formed once: without this the compiler repeats the FP64 and FP32
+    // divisions in every term rather than hold their results
+    asm volatile("" : "+f"(c.b_hi), "+f"(c.b_lo), "+f"(c.bulkPi));
+    if (kDiff) asm volatile("" : "+f"(c.dsq), "+f"(c.pref_q), "+f"(c.inv_kappa));
+    // (1/hbarc^3) / (2 pi^2)
+    c.unit_pref = (1.0f / (0.197327053f * 0.197327053f * 0.197327053f)) / (2.0f * 9.8696044010893586f);
+    return c;
 }
 
+// Yields of every (cell, species) pair, one cell per thread.  A group's series
+// runs for its first member and is reused by the next members while their
+// chemical potential in this cell is the same; a member with another mu gets
+// its own series.  In a warp whose cells have no strangeness and charge
+// potential, mu and with it the yield is the same for the whole run, so a
+// run costs one multiply-add and one maximum, and a member only its store.
+//
+// Besides the yields, the kernel raises ymax[b S + k] to the largest yield of
+// species k on surface b (its float bits: yields are >= +0, so the unsigned
+// order of the bits is the order of the values; ymax starts at 0): through a
+// per-block maximum in shared memory when the block's cells lie on one surface,
+// else lane by lane.
+//
+// Series with an argument off the special-function tables (x < 0.5: pions
+// above 0.27 GeV; x > 399.95) are left at zero and flagged, for
+// yields_off_table_kernel: the FP64 evaluation, inlined here, had its set-up
+// run for every term of every cell.
+//
+// Bound by instruction issue (about 80 % of the issue slots): some 100 one-term
+// and 5 ten-term series per cell, and 319 stores.  200,000 cells, 319 species,
+// 14-moment bulk: 228 us (345 with the FP64 set-up in the loop, the bulk form
+// tested in every term and a multiply-add and a maximum per member); 100,000
+// cells, 400 species with diffusion: 246 us (590).  7 and 6 blocks per SM:
+// 8 and 5 spill or leave warps out (244 and 265 us).
 // kDiff: include_deltaf_diffusion (a separate instantiation, so the common
-// case carries none of the diffusion series' registers; it is held to 6
-// blocks per SM, whose few spills cost less than the warps they add).  Besides the
-// yields, the kernel raises ymax[b S + k] to the largest yield of species k
-// on surface b (as float bits; ymax starts at 0): through a per-block
-// maximum in shared memory when the block's cells lie on one surface, else
-// lane by lane.
-template <bool kDiff>
-__global__ void __launch_bounds__(kYieldThreads, kDiff ? 4 : 6)
-yields_kernel(DevConfig cfg, CellArrays cells, const SpeciesDev* __restrict__ species,
-              float* __restrict__ yields, uint32_t* __restrict__ ymax) {
-    extern __shared__ SpeciesDev s_sp[];
+// case carries none of the diffusion series' registers).
+template <int kBulk, bool kDiff>
+__global__ void __launch_bounds__(kYieldThreads, kDiff ? 6 : 7)
+yields_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yields, uint32_t* __restrict__ ymax,
+              uint32_t* __restrict__ off_table) {
+    extern __shared__ float4 s_dyn[];
     __shared__ int s_b[2];
     const int nsp = cfg.n_species;
-    const int G = cfg.n_ygroups;
-    int32_t* s_gst = reinterpret_cast<int32_t*>(s_sp + nsp);
-    int32_t* s_mem = s_gst + G + 1;
-    uint32_t* s_max = reinterpret_cast<uint32_t*>(s_mem + nsp);
+    const int G = cfg.n_ygroups, R = cfg.n_yruns;
+    // the yield list (YieldGroup) as it is, then the members' and runs' maxima
+    const int words4 = yield_list_float4(nsp, G, R);
+    uint32_t* s_max = reinterpret_cast<uint32_t*>(s_dyn + words4);
+    uint32_t* s_rmax = s_max + nsp;
+    const float4* s_q = s_dyn;
+    const YieldGroup* s_g = reinterpret_cast<const YieldGroup*>(s_dyn + nsp);
+    const int32_t* s_gst = reinterpret_cast<const int32_t*>(s_dyn + nsp + G);
+    const int32_t* s_rst = s_gst + G + 1;
+    const int32_t* s_mem = s_rst + R + 1;
     const int64_t n = cfg.n_cells;
-    const int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x;
-    for (int k = threadIdx.x; k < nsp; k += blockDim.x) {
-        s_sp[k] = species[k];
-        s_max[k] = 0u;
-    }
-    for (int k = threadIdx.x; k < G + 1 + nsp; k += blockDim.x) s_gst[k] = cfg.yorder[k];
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * kYieldThreads;
+    for (int k = threadIdx.x; k < words4; k += kYieldThreads) s_dyn[k] = cfg.ylist[k];
+    for (int k = threadIdx.x; k < nsp + R; k += kYieldThreads) s_max[k] = 0u;
     if (threadIdx.x < 2) {
-        const int64_t lb = threadIdx.x == 0 ? first : min(first + blockDim.x, n) - 1;
+        const int64_t lb = threadIdx.x == 0 ? first : min(first + kYieldThreads, n) - 1;
         s_b[threadIdx.x] = surface_of(cfg.surf, cfg.n_surfaces, lb);
     }
     __syncthreads();
+    const bool one_surface = s_b[0] == s_b[1];
     const int64_t l = first + threadIdx.x;
     const bool valid = l < n;
-    const bool one_surface = s_b[0] == s_b[1];
-    const int b = one_surface ? s_b[0] : surface_of(cfg.surf, cfg.n_surfaces, valid ? l : n - 1);
+    const int64_t lc = valid ? l : 0;   // lanes past the last cell read cell 0 and store nothing
+    const float4 da = cells.da[lc];
+    const bool live = valid && !(da.x < 0.0f);
+    const CellYieldIn c = cell_yield_in<kBulk, kDiff>(cfg, cells, lc, da);
+    uint32_t* ymax_row = ymax + static_cast<int64_t>(
+        one_surface ? s_b[0] : surface_of(cfg.surf, cfg.n_surfaces, valid ? l : n - 1)) * nsp;
+    float* out = yields + l;
+    const bool by_run = __all_sync(0xffffffffu, c.th.z == 0.0f && c.th.w == 0.0f);
     // blockIdx.y picks every gridDim.y-th species group: the groups come in
     // decreasing order of work, so interleaving keeps the rows' work equal,
     // and the grid has several waves of blocks
-    const int k0 = blockIdx.y, kstep = gridDim.y;
-    const float4 da = cells.da[valid ? l : 0];
-    const bool live = valid && !(da.x < 0.0f);
-    cell_yields<kDiff>(cfg, cells, s_sp, s_gst, s_mem, G, k0, kstep, n, l, da, valid, live,
-                       one_surface ? s_max : nullptr, ymax + static_cast<int64_t>(b) * nsp,
-                       yields);
+    for (int g = blockIdx.y; g < G; g += gridDim.y) {
+        const YieldGroup gr = s_g[g];
+        const int r0 = s_gst[g], r1 = s_gst[g + 1];
+        float2 xy = make_float2(0.0f, 0.0f);
+        float mu_of = __int_as_float(0x7fc00000);   // mu of xy: none yet
+        for (int r = r0; r < r1; r++) {
+            const int t0 = s_rst[r], t1 = s_rst[r + 1];
+            for (int t = t0; t < t1; t++) {
+                const float4 q = s_q[t];    // baryon number, strangeness, charge, degeneracy
+                float yv = 0.0f;
+                if (live) {
+                    const float mu = q.x * c.th.y + q.y * c.th.z + q.z * c.th.w;
+                    if (mu != mu_of) {
+                        bool off = false;
+                        xy = yield_coefs<kBulk, kDiff>(c, gr, thermal_series<kBulk, kDiff, true>(cfg, c, gr, mu, off));
+                        mu_of = mu;
+                        if (off) {   // yields_off_table_kernel
+                            xy = make_float2(0.0f, 0.0f);
+                            *off_table = 1u;
+                        }
+                    }
+                    yv = member_yield(q, xy);
+                }
+                if (one_surface) {
+                    const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(yv));
+                    if ((threadIdx.x & 31) == 0 && m) atomicMax(by_run ? s_rmax + r : s_max + t, m);
+                }
+                if (by_run) {
+                    if (!one_surface && yv > 0.0f)
+                        for (int u = t0; u < t1; u++) atomicMax(ymax_row + s_mem[u], __float_as_uint(yv));
+                    if (valid)
+                        for (int u = t0; u < t1; u++) out[static_cast<int64_t>(s_mem[u]) * n] = yv;
+                    break;
+                }
+                if (!one_surface && yv > 0.0f) atomicMax(ymax_row + s_mem[t], __float_as_uint(yv));
+                if (valid) out[static_cast<int64_t>(s_mem[t]) * n] = yv;
+            }
+        }
+    }
     if (one_surface) {
         __syncthreads();
-        for (int k = threadIdx.x; k < nsp; k += blockDim.x)
-            if (s_max[k]) atomicMax(ymax + static_cast<int64_t>(s_b[0]) * nsp + k, s_max[k]);
+        for (int r = threadIdx.x; r < R; r += kYieldThreads)
+            for (int t = s_rst[r]; t < s_rst[r + 1]; t++) {
+                const uint32_t m = max(s_max[t], s_rmax[r]);
+                if (m) atomicMax(ymax_row + s_mem[t], m);
+            }
+    }
+}
+
+// The yields that yields_kernel left out, where it left out any: the series
+// with an argument off the tables, evaluated directly.  A thread per cell and
+// gridDim.y rows of groups.
+template <int kBulk, bool kDiff>
+__global__ void __launch_bounds__(kYieldThreads)
+yields_off_table_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yields, uint32_t* __restrict__ ymax,
+                        const uint32_t* __restrict__ off_table) {
+    if (*off_table == 0u) return;
+    const int nsp = cfg.n_species;
+    const int G = cfg.n_ygroups;
+    const float4* list = cfg.ylist;
+    const YieldGroup* groups = reinterpret_cast<const YieldGroup*>(list + nsp);
+    const int32_t* gst = reinterpret_cast<const int32_t*>(list + nsp + G);
+    const int32_t* rst = gst + G + 1;
+    const int32_t* mem = rst + cfg.n_yruns + 1;
+    const int64_t n = cfg.n_cells;
+    for (int64_t l = static_cast<int64_t>(blockIdx.x) * kYieldThreads + threadIdx.x; l < n;
+         l += static_cast<int64_t>(gridDim.x) * kYieldThreads) {
+        const float4 da = cells.da[l];
+        if (da.x < 0.0f) continue;
+        const CellYieldIn c = cell_yield_in<kBulk, kDiff>(cfg, cells, l, da);
+        const int64_t row0 = static_cast<int64_t>(surface_of(cfg.surf, cfg.n_surfaces, l)) * nsp;
+        for (int g = blockIdx.y; g < G; g += gridDim.y) {
+            const YieldGroup gr = groups[g];
+            float2 xy = make_float2(0.0f, 0.0f);
+            float mu_of = __int_as_float(0x7fc00000);
+            bool off = false;
+            for (int t = rst[gst[g]]; t < rst[gst[g + 1]]; t++) {
+                const float4 q = list[t];
+                const float mu = q.x * c.th.y + q.y * c.th.z + q.z * c.th.w;
+                if (mu != mu_of) {
+                    off = false;
+                    xy = yield_coefs<kBulk, kDiff>(c, gr, thermal_series<kBulk, kDiff, false>(cfg, c, gr, mu, off));
+                    mu_of = mu;
+                }
+                if (!off) continue;
+                const float yv = member_yield(q, xy);
+                yields[static_cast<int64_t>(mem[t]) * n + l] = yv;
+                if (yv > 0.0f) atomicMax(ymax + row0 + mem[t], __float_as_uint(yv));
+            }
+        }
     }
 }
 
@@ -663,25 +755,44 @@ cdf_tile_scan_kernel(const float* __restrict__ yields, int64_t N, const SurfSeg*
 // ------------------------------------------------------------------------
 // launch wrappers
 
-cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, const SpeciesDev* sp,
-                          float* yields, uint32_t* ymax, cudaStream_t stream) {
-    cudaError_t e0 = cudaMemsetAsync(
-        ymax, 0, sizeof(uint32_t) * static_cast<size_t>(cfg.n_surfaces) * cfg.n_species, stream);
+cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, float* yields, uint32_t* ymax,
+                          int num_sms, cudaStream_t stream) {
+    // ymax and, behind it, the flag of arguments off the tables
+    const size_t rows = static_cast<size_t>(cfg.n_surfaces) * cfg.n_species;
+    uint32_t* off_table = ymax + rows;
+    cudaError_t e0 = cudaMemsetAsync(ymax, 0, sizeof(uint32_t) * (rows + 1), stream);
     if (e0 != cudaSuccess) return e0;
     if (cfg.n_cells <= 0) return cudaSuccess;
     const unsigned blocks = static_cast<unsigned>((cfg.n_cells + kYieldThreads - 1) / kYieldThreads);
-    // species, group starts and members, per-block species maxima
-    const size_t smem = sizeof(SpeciesDev) * static_cast<size_t>(cfg.n_species) +
-                        sizeof(int32_t) * static_cast<size_t>(cfg.n_ygroups + 1 + 2 * cfg.n_species);
-    auto kernel = cfg.include_diff ? yields_kernel<true> : yields_kernel<false>;
+    const size_t smem = sizeof(float4) * static_cast<size_t>(yield_list_float4(cfg.n_species, cfg.n_ygroups,
+                                                                               cfg.n_yruns)) +
+                        sizeof(uint32_t) * static_cast<size_t>(cfg.n_species + cfg.n_yruns);
+    const int bulk = !cfg.include_bulk ? kNoBulk
+                     : (cfg.bulk_kind == 1 || cfg.bulk_kind == 21) ? kBulkCe
+                     : cfg.bulk_kind == 11 ? kBulk14 : kNoBulk;
+    using Kernel = void (*)(DevConfig, CellArrays, float*, uint32_t*, uint32_t*);
+    const Kernel kernels[3][2] = {{yields_kernel<kNoBulk, false>, yields_kernel<kNoBulk, true>},
+                                  {yields_kernel<kBulkCe, false>, yields_kernel<kBulkCe, true>},
+                                  {yields_kernel<kBulk14, false>, yields_kernel<kBulk14, true>}};
+    using OffKernel = void (*)(DevConfig, CellArrays, float*, uint32_t*, const uint32_t*);
+    const OffKernel off_kernels[3][2] = {
+        {yields_off_table_kernel<kNoBulk, false>, yields_off_table_kernel<kNoBulk, true>},
+        {yields_off_table_kernel<kBulkCe, false>, yields_off_table_kernel<kBulkCe, true>},
+        {yields_off_table_kernel<kBulk14, false>, yields_off_table_kernel<kBulk14, true>}};
+    const Kernel kernel = kernels[bulk][cfg.include_diff ? 1 : 0];
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem));
         if (e != cudaSuccess) return e;
     }
-    const int want = cfg.yield_groups > 0 ? cfg.yield_groups : kYieldGroups;
+    // rows of species groups: as tuned, more where the cells alone would leave
+    // SMs idle (1,245 cells: 10 blocks in 4 rows took 41 us, in 76 rows 18 us)
+    int want = cfg.yield_groups > 0 ? cfg.yield_groups : kYieldGroups;
+    want = std::max(want, static_cast<int>((static_cast<int64_t>(num_sms) * 5 + blocks - 1) / blocks));
     const unsigned groups = static_cast<unsigned>(std::max(1, std::min(want, cfg.n_ygroups)));
-    kernel<<<dim3(blocks, groups), kYieldThreads, smem, stream>>>(cfg, cells, sp, yields, ymax);
+    kernel<<<dim3(blocks, groups), kYieldThreads, smem, stream>>>(cfg, cells, yields, ymax, off_table);
+    off_kernels[bulk][cfg.include_diff ? 1 : 0]<<<dim3(std::min(blocks, 2u * static_cast<unsigned>(num_sms)), 4), kYieldThreads, 0, stream>>>(
+        cfg, cells, yields, ymax, off_table);
     return cudaGetLastError();
 }
 
