@@ -56,6 +56,16 @@ struct GraphHost {
     int64_t event_offsets[1];   // n_events + 1 entries (allocated with the struct)
 };
 
+// Page-locked results of an eager generate: the counts' report (CountReport)
+// and the sampler's counters.  `tail` holds the event offsets, then the chunks'
+// first work items.
+struct EagerHost {
+    int64_t sizes[2];
+    int32_t count_err, pad;
+    SampleCounters ctr;
+    int64_t tail[1];
+};
+
 enum Phase { kEvStart = 0, kEvPrologue, kEvYields, kEvCdf, kEvCounts, kEvSampleStart, kEvSample,
              kEvLearnStart, kEvLearnEnd, kEvFwdStart, kEvFwdEnd, kEvCount };
 
@@ -171,6 +181,8 @@ struct iss_handle {
     DevBuf<int64_t> d_limits;
     GraphHost* gh = nullptr;
     size_t gh_events = 0;
+    EagerHost* eh = nullptr;
+    size_t eh_tail = 0;
     // launch shape of the kernels (iss_gpu_set_tuning / iss_gpu_autotune)
     iss_tuning_t tune{64, 4, 3, 8, 16};
     bool tuned = false;
@@ -235,6 +247,7 @@ struct iss_handle {
             learned.release_all();
             if (graph_exec) cudaGraphExecDestroy(graph_exec);
             if (gh) cudaFreeHost(gh);
+            if (eh) cudaFreeHost(eh);
             d_run.release();
             d_limits.release();
             d_lslot.release();
@@ -681,7 +694,8 @@ CellRows cell_rows(iss_handle* h) {
                     static_cast<int>(h->species.size())};
 }
 
-// surface upload + prologue + yields + CDF (the per-cell half of generate)
+// surface upload + prologue + yields + CDF head: the per-cell half of generate
+// up to the per-species totals (run_cdf_scan writes the rows)
 iss_status run_cells(iss_handle* h) {
     const int64_t n = h->n_cells;
     const int S = static_cast<int>(h->species.size());
@@ -717,13 +731,30 @@ iss_status run_cells(iss_handle* h) {
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvYields], st));
     // the number of events is not known yet when it follows from the yields
     const bool allow_sparse = h->params.get_or("sample_upto_desired_particle_number", 0) != 1;
-    const CdfBuffers cb = cdf_buffers(h);
     CUDA_TRY(h, launch_cdf_head(h->d_yields.ptr, n, h->d_surf.ptr, c.n_surfaces, h->n_tiles, S, h->d_ymax.ptr,
-                                c.ymult, allow_sparse, cb, st));
-    CUDA_TRY(h, launch_cdf_scan(h->d_yields.ptr, n, h->d_surf.ptr, c.n_surfaces, h->n_tiles, S, h->d_ymax.ptr,
-                                cb, st));
-    CUDA_TRY(h, cudaEventRecord(h->ev[kEvCdf], st));
+                                c.ymult, allow_sparse, cdf_buffers(h), st));
+    return ISS_OK;
+}
+
+iss_status run_cdf_scan(iss_handle* h) {
+    CUDA_TRY(h, launch_cdf_scan(h->d_yields.ptr, h->n_cells, h->d_surf.ptr, h->cfg.n_surfaces, h->n_tiles,
+                                static_cast<int>(h->species.size()), h->d_ymax.ptr, cdf_buffers(h), h->stream));
+    CUDA_TRY(h, cudaEventRecord(h->ev[kEvCdf], h->stream));
     h->yields_valid = true;
+    return ISS_OK;
+}
+
+// the second stream of a generate (the counts beside the CDF scan), at the
+// highest priority: its blocks go first whenever the scan's leave room (a
+// graph keeps stream priorities as node priorities)
+iss_status ensure_aux_stream(iss_handle* h) {
+    if (!h->aux_stream) {
+        int least = 0, greatest = 0;
+        CUDA_TRY(h, cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        CUDA_TRY(h, cudaStreamCreateWithPriority(&h->aux_stream, cudaStreamNonBlocking, greatest));
+    }
+    for (cudaEvent_t* e : {&h->ev_fork, &h->ev_join})
+        if (!*e) CUDA_TRY(h, cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     return ISS_OK;
 }
 
@@ -1158,16 +1189,8 @@ iss_status capture_graph(iss_handle* h, int64_t n_items) {
     c.run = h->d_run.ptr;
     c.chunk_events = std::max(E, 1);
     cudaStream_t s = h->stream;
-    if (!h->aux_stream) {
-        // the counts branch at the highest priority: its blocks go first
-        // whenever the CDF scan's blocks leave room (the graph keeps stream
-        // priorities as node priorities)
-        int least = 0, greatest = 0;
-        CUDA_TRY(h, cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        CUDA_TRY(h, cudaStreamCreateWithPriority(&h->aux_stream, cudaStreamNonBlocking, greatest));
-    }
-    for (cudaEvent_t* e : {&h->ev_fork, &h->ev_join})
-        if (!*e) CUDA_TRY(h, cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    const iss_status ast = ensure_aux_stream(h);
+    if (ast != ISS_OK) return ast;
     cudaGraph_t graph = nullptr;
     CUDA_TRY(h, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     const cudaError_t ce = enqueue_generate(h, c);
@@ -1307,7 +1330,10 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
 
     // number of events from the thermal pi+ yield when asked for
     // (FSSW::compute_number_of_sampling_needed, src/FSSW.cpp:851-869)
-    if (h->params.get_or("sample_upto_desired_particle_number", 0) == 1) {
+    const bool upto = h->params.get_or("sample_upto_desired_particle_number", 0) == 1;
+    if (upto) {
+        st = run_cdf_scan(h);
+        if (st != ISS_OK) return st;
         double needed, max_ev;
         if (!need(h, "number_of_particles_needed", &needed) ||
             !need(h, "maximum_sampling_events", &max_ev))
@@ -1352,52 +1378,70 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     CUDA_TRY(h, h->d_error.reserve(1));
     CUDA_TRY(h, h->d_work.reserve(static_cast<size_t>(n_chunks)));
     CUDA_TRY(h, h->d_counters.reserve(1));
-    CUDA_TRY(h, cudaMemsetAsync(h->d_error.ptr, 0, sizeof(int), s));
+    CUDA_TRY(h, h->d_item_seg.reserve(1));
     // per species: kPoissonConsts constants, then an inversion table of
     // kInvTable + 1 doubles (the last holds the length)
     CUDA_TRY(h, h->d_pois.reserve(static_cast<size_t>(std::max(S * c.n_surfaces, 1)) *
                                   (kPoissonConsts + kInvTable + 1)));
+    const size_t tail = static_cast<size_t>(E) + 1 + static_cast<size_t>(n_chunks);
+    if (!h->eh || h->eh_tail < tail) {
+        if (h->eh) cudaFreeHost(h->eh);
+        h->eh = nullptr;
+        CUDA_TRY(h, cudaMallocHost(reinterpret_cast<void**>(&h->eh), sizeof(EagerHost) + sizeof(int64_t) * tail));
+        h->eh_tail = tail;
+    }
+    std::fill(h->eh->tail, h->eh->tail + tail, 0);
+    st = ensure_aux_stream(h);
+    if (st != ISS_OK) return st;
+    // The counts need only the per-species totals: they run on a second stream
+    // beside the CDF scan, and the host waits for them alone, so that the
+    // sampler is enqueued while the scan still runs.
+    cudaStream_t a = h->aux_stream;
+    CUDA_TRY(h, cudaMemsetAsync(h->d_work.ptr, 0, sizeof(unsigned long long) * n_chunks, s));
+    CUDA_TRY(h, cudaMemsetAsync(h->d_counters.ptr, 0, sizeof(SampleCounters), s));
+    CUDA_TRY(h, cudaMemsetAsync(h->d_error.ptr, 0, sizeof(int), s));
+    CUDA_TRY(h, cudaEventRecord(h->ev_fork, s));
+    CUDA_TRY(h, cudaStreamWaitEvent(a, h->ev_fork, 0));
     CUDA_TRY(h, launch_counts(c, h->d_species.ptr, h->d_totals.ptr, h->d_pois.ptr, h->d_counts.ptr,
-                              h->d_items.ptr, h->d_error.ptr, s));
-    CUDA_TRY(h, launch_offsets_scan(h->d_counts.ptr, nseg, h->d_off_tiles.ptr, h->d_offsets.ptr, s));
-    CUDA_TRY(h, launch_offsets_scan(h->d_items.ptr, nseg, h->d_off_tiles.ptr, h->d_item_off.ptr, s));
-    int64_t sizes[2] = {0, 0};   // hadrons, work items
-    int count_err = 0;
-    std::vector<int64_t> chunk_item(static_cast<size_t>(n_chunks) + 1, 0);
-    h->event_offsets.assign(static_cast<size_t>(E) + 1, 0);
-    CUDA_TRY(h, cudaMemcpyAsync(&sizes[0], h->d_offsets.ptr + nseg, sizeof(int64_t),
-                                cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(h, cudaMemcpyAsync(&sizes[1], h->d_item_off.ptr + nseg, sizeof(int64_t),
-                                cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(h, cudaMemcpyAsync(&count_err, h->d_error.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
+                              h->d_items.ptr, h->d_error.ptr, a));
+    int n_launches = 6 + (nseg > 0 ? 2 : 0);   // prologue, yields (2), CDF (3); counts (2)
+    bool mapped = false;
+    const CountReport rep{h->eh->sizes, &h->eh->count_err, h->eh->tail, h->eh->tail + E + 1, c.chunk_events, n_chunks};
+    CUDA_TRY(h, launch_count_scans(h->d_counts.ptr, h->d_items.ptr, nseg, S, E, h->d_off_tiles.ptr,
+                                   h->d_offsets.ptr, h->d_item_off.ptr, h->d_item_seg.ptr,
+                                   static_cast<int64_t>(h->d_item_seg.cap), h->d_error.ptr, rep, &n_launches,
+                                   &mapped, a));
+    CUDA_TRY(h, cudaEventRecord(h->ev_join, a));
+    if (!upto) {
+        st = run_cdf_scan(h);
+        if (st != ISS_OK) return st;
+    }
     if (h->use_learned) {
         // per-species totals: which species the learned proposal takes
         h->totals.resize(static_cast<size_t>(S) * c.n_surfaces);
         CUDA_TRY(h, cudaMemcpyAsync(h->totals.data(), h->d_totals.ptr, 8 * h->totals.size(),
-                                    cudaMemcpyDeviceToHost, s));
+                                    cudaMemcpyDeviceToHost, a));
     }
-    if (S > 0) {
-        // event offsets: offsets[e * S] for e = 0..n_events
-        CUDA_TRY(h, cudaMemcpy2DAsync(h->event_offsets.data(), sizeof(int64_t), h->d_offsets.ptr,
-                                      sizeof(int64_t) * static_cast<size_t>(S), sizeof(int64_t),
-                                      static_cast<size_t>(E) + 1, cudaMemcpyDeviceToHost, s));
-        // first work item of each chunk: item_off at segment c * chunk_events * S
-        CUDA_TRY(h, cudaMemcpy2DAsync(chunk_item.data(), sizeof(int64_t), h->d_item_off.ptr,
-                                      sizeof(int64_t) * static_cast<size_t>(c.chunk_events) * S,
-                                      sizeof(int64_t), static_cast<size_t>(n_chunks),
-                                      cudaMemcpyDeviceToHost, s));
-    }
-    CUDA_TRY(h, cudaStreamSynchronize(s));
-    const int64_t n_units = sizes[0], n_items = sizes[1];
-    chunk_item[n_chunks] = n_items;
+    CUDA_TRY(h, cudaStreamWaitEvent(s, h->ev_join, 0));
+    CUDA_TRY(h, cudaStreamSynchronize(a));
+    const int64_t n_units = h->eh->sizes[0], n_items = h->eh->sizes[1];
+    const int count_err = h->eh->count_err;
+    h->event_offsets.assign(h->eh->tail, h->eh->tail + E + 1);
+    std::vector<int64_t> chunk_item(h->eh->tail + E + 1, h->eh->tail + E + 1 + n_chunks);
+    chunk_item.push_back(n_items);
     if (count_err == 2) return fail(h, ISS_ERR_OUT_OF_RANGE, "negative particle yield (dN < 0)");
     if (count_err != 0) return fail(h, ISS_ERR_SAMPLING, "count draw did not converge");
     const bool graph_mode = graph_eligible(h, host_out, sink != nullptr);
     // a call that will be captured gets 15 % headroom in the buffers whose
     // size depends on the draws, so that later calls fit the same graph
     const auto headroom = [&](int64_t v) { return graph_mode ? v + v / 7 + 1024 : std::max<int64_t>(v, 1); };
-    CUDA_TRY(h, h->d_item_seg.reserve(static_cast<size_t>(headroom(n_items))));
-    CUDA_TRY(h, launch_item_map(h->d_items.ptr, h->d_item_off.ptr, nseg, h->d_item_seg.ptr, s));
+    mapped = mapped && n_items <= static_cast<int64_t>(h->d_item_seg.cap) &&
+             headroom(n_items) <= static_cast<int64_t>(h->d_item_seg.cap);
+    if (!mapped) {
+        CUDA_TRY(h, h->d_item_seg.reserve(static_cast<size_t>(headroom(n_items))));
+        CUDA_TRY(h, launch_item_map(h->d_items.ptr, h->d_item_off.ptr, nseg, h->d_item_seg.ptr, s));
+        n_launches += nseg > 0 ? 1 : 0;
+    }
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvCounts], s));
     {
         // per-generate fields; the training fields stay
@@ -1456,10 +1500,8 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     }
     CUDA_TRY(h, h->d_hadrons.reserve(static_cast<size_t>(sink ? 2 * ring : headroom(n_units))));
     CUDA_TRY(h, h->d_cell_of.reserve(static_cast<size_t>(sink ? 2 * ring : headroom(n_units))));
-    CUDA_TRY(h, cudaMemsetAsync(h->d_work.ptr, 0, sizeof(unsigned long long) * n_chunks, s));
-    CUDA_TRY(h, cudaMemsetAsync(h->d_counters.ptr, 0, sizeof(SampleCounters), s));
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvSampleStart], s));
-    int n_launches = sink ? 2 * n_chunks : 0;   // of the cell assignment and the sampler
+    if (sink) n_launches += 2 * n_chunks;   // the cell assignment and the sampler
     // hands chunk ch's records (already copied to the host) to the sink
     std::vector<int64_t> rel;
     const auto deliver = [&](int ch) -> iss_status {
@@ -1551,9 +1593,9 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
         CUDA_TRY(h, cudaStreamWaitEvent(s, h->ev_sample2[1], 0));
     }
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvSample], s));
-    SampleCounters ctr{};
-    CUDA_TRY(h, cudaMemcpyAsync(&ctr, h->d_counters.ptr, sizeof(ctr), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(h, cudaMemcpyAsync(&h->eh->ctr, h->d_counters.ptr, sizeof(SampleCounters), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(h, cudaStreamSynchronize(s));
+    const SampleCounters ctr = h->eh->ctr;
     if (to_host) {
         CUDA_TRY(h, cudaStreamSynchronize(h->copy_stream));
         if (copied) *copied = true;
@@ -1596,7 +1638,7 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     t.n_tries = static_cast<int64_t>(ctr.tries);
     t.n_cell_redraws = static_cast<int64_t>(ctr.redraws);
     t.n_failures = static_cast<int64_t>(ctr.failures + decay_failures);
-    t.kernel_launches = 15 + n_launches;
+    t.kernel_launches = n_launches;
     if (h->use_learned) {
         t.kernel_launches += 4;
         h->lstats.n_tries = static_cast<int64_t>(ctr.learned_tries);

@@ -68,6 +68,21 @@ cudaError_t launch_offsets_scan(const int32_t* counts, int64_t n, int64_t* tile_
 cudaError_t launch_item_map(const int32_t* items, const int64_t* item_off, int64_t nseg,
                             int32_t* item_seg, cudaStream_t stream,
                             const int64_t* limits = nullptr);
+// What the host reads of the counts after one wait, all in page-locked memory
+struct CountReport {
+    int64_t* sizes;           // hadrons, work items
+    int32_t* error;           // of launch_counts
+    int64_t* event_offsets;   // [n_events + 1]
+    int64_t* chunk_items;     // [n_chunks] first work item of each chunk of chunk_events events
+    int chunk_events, n_chunks;
+};
+// the slot scans of the counts (offsets) and work items (item_off), and the
+// report; for few segments also the item map, as far as item_seg's capacity
+// reaches (*mapped).  *launches is raised by the kernels launched.
+cudaError_t launch_count_scans(const int32_t* counts, const int32_t* items, int64_t nseg, int S, int n_events,
+                               int64_t* tiles, int64_t* offsets, int64_t* item_off, int32_t* item_seg,
+                               int64_t cap_items, const int* error, const CountReport& rep, int* launches,
+                               bool* mapped, cudaStream_t stream);
 // graph replays: limits[0] = the call's work items, limits[1] = 1 when the
 // call does not fit the captured buffers (cap_units records, cap_items items)
 cudaError_t launch_graph_limits(const int64_t* offsets, const int64_t* item_off, int64_t nseg,

@@ -108,21 +108,45 @@ __device__ __forceinline__ double log_factorial(const double* __restrict__ table
                      __dmul_rn(r, t));
 }
 
-__device__ void poisson_inv_table(const PoissonC& c, PoissonInv& t) {
-    t.len = 0;
-    if (!(c.mu < 12.0)) return;
-    double p = c.emu, cdf = p;
-    t.icdf[0] = floor_2p53(cdf);
-    for (int k = 1; k < kInvTable; k++) {
-        p = __dmul_rn(p, c.mu / static_cast<double>(k));
-        const double next = __dadd_rn(cdf, p);
-        if (next == cdf && static_cast<double>(k) > c.mu) {
-            t.len = k;
-            return;
-        }
-        cdf = next;
-        t.icdf[k] = floor_2p53(cdf);
+// by a warp: the quotients mu / k, four per lane, in parallel; then every lane
+// forms the sums in the loop's own order and keeps the entries k = lane + 32 j
+__device__ void poisson_inv_table(const PoissonC& c, PoissonInv& t, int lane) {
+    constexpr int kPer = (kInvTable + 31) / 32;
+    if (!(c.mu < 12.0)) {
+        if (lane == 0) t.len = 0;
+        return;
     }
+    double ratio[kPer], entry[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        ratio[j] = c.mu / static_cast<double>(max(lane + 32 * j, 1));
+        entry[j] = 0.0;
+    }
+    double p = c.emu, cdf = p;
+    int len = 0, n = kInvTable;
+    bool end = false;
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        for (int i = 0; i < 32 && !end; i++) {
+            const int k = 32 * j + i;
+            if (k >= kInvTable) break;
+            if (k > 0) {
+                p = __dmul_rn(p, __shfl_sync(0xffffffffu, ratio[j], i));
+                const double next = __dadd_rn(cdf, p);
+                if (next == cdf && static_cast<double>(k) > c.mu) {
+                    len = n = k;
+                    end = true;
+                    break;
+                }
+                cdf = next;
+            }
+            if (lane == i) entry[j] = cdf;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kPer; j++)
+        if (lane + 32 * j < n) t.icdf[lane + 32 * j] = floor_2p53(entry[j]);
+    if (lane == 0) t.len = len;
 }
 
 __device__ int64_t poisson_draw(uint32_t c2, uint32_t c3, uint32_t k0, uint32_t k1, uint32_t iter0,
@@ -239,19 +263,25 @@ __device__ __forceinline__ void item_decode(const DevConfig& cfg, int q, int& e,
     e = e0 + (r - s * ne);
 }
 
-// per-species Poisson constants of the model-30 draws (same mu in every event)
-__global__ void count_consts_kernel(DevConfig cfg, const double* __restrict__ totals,
-                                    PoissonC* __restrict__ pois, PoissonInv* __restrict__ inv) {
-    // one thread per (surface, species) row
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= cfg.n_surfaces * cfg.n_species) return;
+// Poisson constants and inversion table of the model-30 draws (same mu in every
+// event), a warp and a block per (surface, species) row: the FP64 chains are
+// bound by latency, and a block each spreads them over the SMs' narrow FP64
+// pipes (319 rows: 32 us with a thread per row, 4 us so)
+__global__ void __launch_bounds__(32)
+count_consts_kernel(DevConfig cfg, const double* __restrict__ totals, PoissonC* __restrict__ pois,
+                    PoissonInv* __restrict__ inv) {
+    const int s = blockIdx.x;
     const double dN = __dmul_rn(totals[s], cfg.ymult);
     const PoissonC c = poisson_consts(dN);
-    pois[s] = c;
-    poisson_inv_table(c, inv[s]);
+    if (threadIdx.x == 0) pois[s] = c;
+    poisson_inv_table(c, inv[s], threadIdx.x);
 }
 
-__global__ void counts_kernel(DevConfig cfg_in, const SpeciesDev* __restrict__ species,
+// (blocks of 64: one event's 319 draws share the FP64 pipes of five SMs, not two)
+constexpr int kCountThreads = 64;
+
+__global__ void __launch_bounds__(kCountThreads)
+counts_kernel(DevConfig cfg_in, const SpeciesDev* __restrict__ species,
                               const double* __restrict__ totals,
                               const PoissonC* __restrict__ pois,
                               const PoissonInv* __restrict__ inv, int32_t* __restrict__ counts,
@@ -420,6 +450,79 @@ off_tile_scan_kernel(const int32_t* __restrict__ counts, int64_t n,
     for (int k = 0; k < kOffPer; k++) {
         if (e0 + k < n) offsets[e0 + k] = run;
         run += mine[k];
+    }
+}
+
+// What the host needs of the counts, written to its page-locked memory: the
+// hadron and work-item totals, the first hadron of every event and the first
+// work item of every sampling chunk (the kernels' completion makes them
+// visible; one wait instead of a copy each).
+__device__ __forceinline__ void report_offset(const CountReport& rep, int S, int64_t i, long long offset,
+                                              long long item) {
+    if (S <= 0) return;
+    if (i % S == 0) rep.event_offsets[i / S] = offset;
+    const int64_t per = static_cast<int64_t>(rep.chunk_events) * S;
+    if (i % per == 0 && i / per < rep.n_chunks) rep.chunk_items[i / per] = item;
+}
+
+__global__ void count_report_kernel(const int64_t* __restrict__ offsets, const int64_t* __restrict__ item_off,
+                                    int64_t nseg, int S, int n_events, const int* __restrict__ error,
+                                    CountReport rep) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e == 0) {
+        rep.sizes[0] = offsets[nseg];
+        rep.sizes[1] = item_off[nseg];
+        *rep.error = *error;
+    }
+    if (e <= n_events) {
+        const int64_t i = static_cast<int64_t>(e) * S;
+        report_offset(rep, S, i, offsets[i], item_off[i]);
+    }
+}
+
+// Both slot scans, the item map (as far as cap_items reaches) and the report in
+// one block, for up to kSmallScan segments: a call with few events otherwise
+// waits for eight launches of a few microseconds each
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallPer = 8;
+constexpr int64_t kSmallScan = kSmallThreads * kSmallPer;
+__global__ void __launch_bounds__(kSmallThreads)
+small_scans_kernel(const int32_t* __restrict__ counts, const int32_t* __restrict__ items, int nseg, int S,
+                   int64_t* __restrict__ offsets, int64_t* __restrict__ item_off, int32_t* __restrict__ item_seg,
+                   int64_t cap_items, const int* __restrict__ error, CountReport rep) {
+    __shared__ long long s_warp[33];
+    const int i0 = threadIdx.x * kSmallPer;
+    int32_t c[kSmallPer], m[kSmallPer];
+    long long ca = 0, ma = 0;
+#pragma unroll
+    for (int k = 0; k < kSmallPer; k++) {
+        c[k] = i0 + k < nseg ? counts[i0 + k] : 0;
+        m[k] = i0 + k < nseg ? items[i0 + k] : 0;
+        ca += c[k];
+        ma += m[k];
+    }
+    long long units, n_items;
+    long long off = block_excl_scan_ll(ca, s_warp, &units);
+    long long item = block_excl_scan_ll(ma, s_warp, &n_items);
+#pragma unroll
+    for (int k = 0; k < kSmallPer; k++) {
+        const int i = i0 + k;
+        if (i < nseg) {
+            offsets[i] = off;
+            item_off[i] = item;
+            report_offset(rep, S, i, off, item);
+            for (int j = 0; j < m[k] && item + j < cap_items; j++) item_seg[item + j] = i;
+            off += c[k];
+            item += m[k];
+        }
+    }
+    if (threadIdx.x == 0) {
+        offsets[nseg] = units;
+        item_off[nseg] = n_items;
+        report_offset(rep, S, nseg, units, n_items);
+        rep.sizes[0] = units;
+        rep.sizes[1] = n_items;
+        *rep.error = *error;
     }
 }
 
@@ -2119,9 +2222,9 @@ cudaError_t launch_counts(const DevConfig& cfg, const SpeciesDev* species, const
     const int rows = cfg.n_surfaces * cfg.n_species;
     PoissonC* pc = reinterpret_cast<PoissonC*>(pois);
     PoissonInv* inv = reinterpret_cast<PoissonInv*>(pc + rows);
-    count_consts_kernel<<<(rows + 127) / 128, 128, 0, stream>>>(cfg, totals, pc, inv);
-    const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-    counts_kernel<<<blocks, 256, 0, stream>>>(cfg, species, totals, pc, inv, counts, items, error);
+    count_consts_kernel<<<rows, 32, 0, stream>>>(cfg, totals, pc, inv);
+    const unsigned blocks = static_cast<unsigned>((total + kCountThreads - 1) / kCountThreads);
+    counts_kernel<<<blocks, kCountThreads, 0, stream>>>(cfg, species, totals, pc, inv, counts, items, error);
     return cudaGetLastError();
 }
 
@@ -2142,6 +2245,26 @@ cudaError_t launch_item_map(const int32_t* items, const int64_t* item_off, int64
     if (nseg <= 0) return cudaSuccess;
     item_map_kernel<<<static_cast<unsigned>((nseg + 255) / 256), 256, 0, stream>>>(
         items, item_off, nseg, item_seg, limits);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_count_scans(const int32_t* counts, const int32_t* items, int64_t nseg, int S, int n_events,
+                               int64_t* tiles, int64_t* offsets, int64_t* item_off, int32_t* item_seg,
+                               int64_t cap_items, const int* error, const CountReport& rep, int* launches,
+                               bool* mapped, cudaStream_t stream) {
+    *mapped = nseg > 0 && nseg <= kSmallScan;
+    if (*mapped) {
+        small_scans_kernel<<<1, kSmallThreads, 0, stream>>>(counts, items, static_cast<int>(nseg), S, offsets,
+                                                            item_off, item_seg, cap_items, error, rep);
+        *launches += 1;
+        return cudaGetLastError();
+    }
+    cudaError_t e = launch_offsets_scan(counts, nseg, tiles, offsets, stream);
+    if (e == cudaSuccess) e = launch_offsets_scan(items, nseg, tiles, item_off, stream);
+    if (e != cudaSuccess) return e;
+    count_report_kernel<<<static_cast<unsigned>(n_events / 256 + 1), 256, 0, stream>>>(offsets, item_off, nseg, S,
+                                                                                     n_events, error, rep);
+    *launches += nseg > 0 ? 7 : 1;
     return cudaGetLastError();
 }
 
