@@ -785,10 +785,12 @@ cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, float* 
                                              static_cast<int>(smem));
         if (e != cudaSuccess) return e;
     }
-    // rows of species groups: as tuned, more where the cells alone would leave
-    // SMs idle (1,245 cells: 10 blocks in 4 rows took 41 us, in 76 rows 18 us)
+    // rows of species groups: as tuned, more where that leaves fewer than three
+    // waves of 7 blocks per SM (a call of 1.1 waves runs two: 37,211 cells took
+    // 80 us in 4 rows, 62 us so; 1,245 cells 41 and 18 us).  More waves repeat
+    // the cells' set-up too often (5, 8 and 12 waves: 64, 70 and 78 us).
     int want = cfg.yield_groups > 0 ? cfg.yield_groups : kYieldGroups;
-    want = std::max(want, static_cast<int>((static_cast<int64_t>(num_sms) * 5 + blocks - 1) / blocks));
+    want = std::max(want, static_cast<int>((static_cast<int64_t>(num_sms) * 21 + blocks - 1) / blocks));
     const unsigned groups = static_cast<unsigned>(std::max(1, std::min(want, cfg.n_ygroups)));
     kernel<<<dim3(blocks, groups), kYieldThreads, smem, stream>>>(cfg, cells, yields, ymax, off_table);
     off_kernels[bulk][cfg.include_diff ? 1 : 0]<<<dim3(std::min(blocks, 2u * static_cast<unsigned>(num_sms)), 4), kYieldThreads, 0, stream>>>(
