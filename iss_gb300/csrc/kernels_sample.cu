@@ -457,12 +457,10 @@ off_tile_scan_kernel(const int32_t* __restrict__ counts, int64_t n,
 // hadron and work-item totals, the first hadron of every event and the first
 // work item of every sampling chunk (the kernels' completion makes them
 // visible; one wait instead of a copy each).
-__device__ __forceinline__ void report_offset(const CountReport& rep, int S, int64_t i, long long offset,
-                                              long long item) {
-    if (S <= 0) return;
-    if (i % S == 0) rep.event_offsets[i / S] = offset;
-    const int64_t per = static_cast<int64_t>(rep.chunk_events) * S;
-    if (i % per == 0 && i / per < rep.n_chunks) rep.chunk_items[i / per] = item;
+__device__ __forceinline__ void report_event(const CountReport& rep, int e, long long offset, long long item) {
+    rep.event_offsets[e] = offset;
+    if (e % rep.chunk_events == 0 && e / rep.chunk_events < rep.n_chunks)
+        rep.chunk_items[e / rep.chunk_events] = item;
 }
 
 __global__ void count_report_kernel(const int64_t* __restrict__ offsets, const int64_t* __restrict__ item_off,
@@ -474,9 +472,9 @@ __global__ void count_report_kernel(const int64_t* __restrict__ offsets, const i
         rep.sizes[1] = item_off[nseg];
         *rep.error = *error;
     }
-    if (e <= n_events) {
+    if (e <= n_events && S > 0) {
         const int64_t i = static_cast<int64_t>(e) * S;
-        report_offset(rep, S, i, offsets[i], item_off[i]);
+        report_event(rep, e, offsets[i], item_off[i]);
     }
 }
 
@@ -504,13 +502,18 @@ small_scans_kernel(const int32_t* __restrict__ counts, const int32_t* __restrict
     long long units, n_items;
     long long off = block_excl_scan_ll(ca, s_warp, &units);
     long long item = block_excl_scan_ll(ma, s_warp, &n_items);
+    int e = i0 / S, s = i0 - e * S;   // event and species of segment i0
 #pragma unroll
     for (int k = 0; k < kSmallPer; k++) {
         const int i = i0 + k;
         if (i < nseg) {
             offsets[i] = off;
             item_off[i] = item;
-            report_offset(rep, S, i, off, item);
+            if (s == 0) report_event(rep, e, off, item);
+            if (++s == S) {
+                s = 0;
+                e++;
+            }
             for (int j = 0; j < m[k] && item + j < cap_items; j++) item_seg[item + j] = i;
             off += c[k];
             item += m[k];
@@ -519,7 +522,7 @@ small_scans_kernel(const int32_t* __restrict__ counts, const int32_t* __restrict
     if (threadIdx.x == 0) {
         offsets[nseg] = units;
         item_off[nseg] = n_items;
-        report_offset(rep, S, nseg, units, n_items);
+        report_event(rep, nseg / S, units, n_items);
         rep.sizes[0] = units;
         rep.sizes[1] = n_items;
         *rep.error = *error;
