@@ -181,6 +181,11 @@ struct iss_handle {
     DevBuf<int64_t> d_limits;
     GraphHost* gh = nullptr;
     size_t gh_events = 0;
+    // OSCAR output: event tables, the chunks' text on either side
+    DevBuf<int64_t> d_oscar_off, d_oscar_byte;
+    DevBuf<char> d_oscar_text;
+    char* oscar_host = nullptr;
+    cudaEvent_t oscar_ev[2] = {nullptr, nullptr};
     EagerHost* eh = nullptr;
     size_t eh_tail = 0;
     // launch shape of the kernels (iss_gpu_set_tuning / iss_gpu_autotune)
@@ -248,6 +253,12 @@ struct iss_handle {
             if (graph_exec) cudaGraphExecDestroy(graph_exec);
             if (gh) cudaFreeHost(gh);
             if (eh) cudaFreeHost(eh);
+            if (oscar_host) cudaFreeHost(oscar_host);
+            d_oscar_off.release();
+            d_oscar_byte.release();
+            d_oscar_text.release();
+            for (auto& e : oscar_ev)
+                if (e) cudaEventDestroy(e);
             d_run.release();
             d_limits.release();
             d_lslot.release();
@@ -1796,15 +1807,23 @@ iss_status ensure_host_copy(iss_handle* h) {
     return ISS_OK;
 }
 
-// OSCAR output with the text made on the GPU: the header file is copied,
-// then chunks of whole events are formatted on the device, copied to
-// page-locked host memory and written, two chunks in flight.
+// OSCAR output with the text made on the GPU: the header file is copied, then
+// chunks of lines are formatted on the device, copied to page-locked memory
+// and written, one chunk being formatted and copied while another is written.
+// The chunks' buffers (kOscarBuffers x kOscarChunk on either side) stay with
+// the handle: allocating and pinning them for each call took longer than the
+// write itself (222,078 hadrons, 57 MB to a RAM disk: 8.3 ms, now 4.6, of which
+// the write is 4.5).  Chunks of 8 MB start the write after some 60 us.
+constexpr int64_t kOscarChunk = int64_t(8) << 20;
+constexpr int kOscarBuffers = 2;
+
 iss_status write_oscar_gpu(iss_handle* h, const char* filename) {
     const std::string header_file = h->table_path + "/OSCAR_header.txt";
     std::ifstream header(header_file);
     if (!header) return fail(h, ISS_ERR_IO, "OSCAR header file %s not found", header_file.c_str());
     std::remove(filename);
-    std::FILE* f = std::fopen(filename, "w");
+    const std::unique_ptr<std::FILE, int (*)(std::FILE*)> file(std::fopen(filename, "w"), &std::fclose);
+    std::FILE* f = file.get();
     if (!f) return fail(h, ISS_ERR_IO, "can not open %s", filename);
     std::string line;
     while (std::getline(header, line)) std::fprintf(f, "%s\n", line.c_str());
@@ -1815,79 +1834,58 @@ iss_status write_oscar_gpu(iss_handle* h, const char* filename) {
         const int64_t n = off[e + 1] - off[e];
         ev_byte[e + 1] = ev_byte[e] + (n > 0 ? kOscarSubHeader + n * kOscarLine : 0);
     }
-    const int64_t kChunk = int64_t(256) << 20;
-    DevBuf<int64_t> d_off, d_byte;
-    DevBuf<char> d_text[2];
-    char* host[2] = {nullptr, nullptr};
-    cudaStream_t s = h->stream;
-    cudaEvent_t done[2] = {nullptr, nullptr};
-    iss_status st = ISS_OK;
-    auto cleanup = [&]() {
-        for (int k = 0; k < 2; k++) {
-            if (done[k]) cudaEventDestroy(done[k]);
-            if (host[k]) cudaFreeHost(host[k]);
-            d_text[k].release();
+    // chunks: runs of lines of at most kOscarChunk bytes, each with the
+    // sub-headers of the events that start in it
+    struct Chunk { int64_t h0, h1, byte0, bytes; int e_lo, e_hi; };
+    std::vector<Chunk> chunks;
+    for (int e = 0; e < E; e++) {
+        int64_t hd = off[e];
+        while (hd < off[e + 1]) {
+            const int64_t head = hd == off[e] ? kOscarSubHeader : 0;
+            if (chunks.empty() || chunks.back().bytes + head + kOscarLine > kOscarChunk)
+                chunks.push_back({hd, hd, ev_byte[e] + (hd - off[e]) * kOscarLine + (head ? 0 : kOscarSubHeader), 0, e, e});
+            Chunk& c = chunks.back();
+            const int64_t n = std::min(off[e + 1] - hd, (kOscarChunk - c.bytes - head) / kOscarLine);
+            c.bytes += head + n * kOscarLine;
+            hd += n;
+            c.h1 = hd;
+            c.e_hi = e + 1;
         }
-        d_off.release();
-        d_byte.release();
-        std::fclose(f);
-    };
-#define OSCAR_TRY(x)                                                                   \
-    do {                                                                               \
-        const cudaError_t e_ = (x);                                                    \
-        if (e_ != cudaSuccess) {                                                       \
-            cleanup();                                                                 \
-            return fail(h, ISS_ERR_CUDA, "%s: %s", #x, cudaGetErrorString(e_));        \
-        }                                                                              \
-    } while (0)
-    // chunks: runs of whole events of at most kChunk bytes (an event larger
-    // than that is a chunk by itself)
-    std::vector<std::pair<int, int>> chunks;
-    int64_t max_bytes = 0;
-    for (int e = 0; e < E;) {
-        int e1 = e + 1;
-        while (e1 < E && ev_byte[e1 + 1] - ev_byte[e] <= kChunk) e1++;
-        chunks.push_back({e, e1});
-        max_bytes = std::max(max_bytes, ev_byte[e1] - ev_byte[e]);
-        e = e1;
     }
-    OSCAR_TRY(d_off.reserve(off.size()));
-    OSCAR_TRY(d_byte.reserve(ev_byte.size()));
-    OSCAR_TRY(cudaMemcpyAsync(d_off.ptr, off.data(), 8 * off.size(), cudaMemcpyHostToDevice, s));
-    OSCAR_TRY(cudaMemcpyAsync(d_byte.ptr, ev_byte.data(), 8 * ev_byte.size(), cudaMemcpyHostToDevice, s));
-    for (int k = 0; k < 2 && k < static_cast<int>(chunks.size()); k++) {
-        OSCAR_TRY(d_text[k].reserve(static_cast<size_t>(std::max<int64_t>(max_bytes, 1))));
-        OSCAR_TRY(cudaHostAlloc(reinterpret_cast<void**>(&host[k]),
-                                static_cast<size_t>(std::max<int64_t>(max_bytes, 1)), cudaHostAllocDefault));
-        OSCAR_TRY(cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming));
-    }
-    auto enqueue = [&](size_t c) -> cudaError_t {
-        const int k = static_cast<int>(c & 1);
-        const int ea = chunks[c].first, eb = chunks[c].second;
-        const int64_t bytes = ev_byte[eb] - ev_byte[ea];
-        cudaError_t e = launch_oscar_lines(h->d_hadrons.ptr, off[ea], off[eb], d_off.ptr, d_byte.ptr,
-                                           ea, eb, ev_byte[ea], d_text[k].ptr, h->num_sms, s);
-        if (e != cudaSuccess) return e;
-        if (bytes > 0) e = cudaMemcpyAsync(host[k], d_text[k].ptr, static_cast<size_t>(bytes),
-                                           cudaMemcpyDeviceToHost, s);
-        if (e != cudaSuccess) return e;
-        return cudaEventRecord(done[k], s);
+    if (chunks.empty()) return ISS_OK;
+    cudaStream_t s = h->stream;
+    CUDA_TRY(h, h->d_oscar_off.reserve(off.size()));
+    CUDA_TRY(h, h->d_oscar_byte.reserve(ev_byte.size()));
+    CUDA_TRY(h, h->d_oscar_text.reserve(static_cast<size_t>(kOscarBuffers * kOscarChunk)));
+    if (!h->oscar_host)
+        CUDA_TRY(h, cudaHostAlloc(reinterpret_cast<void**>(&h->oscar_host),
+                                  static_cast<size_t>(kOscarBuffers * kOscarChunk), cudaHostAllocDefault));
+    for (auto& e : h->oscar_ev)
+        if (!e) CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    CUDA_TRY(h, cudaMemcpyAsync(h->d_oscar_off.ptr, off.data(), 8 * off.size(), cudaMemcpyHostToDevice, s));
+    CUDA_TRY(h, cudaMemcpyAsync(h->d_oscar_byte.ptr, ev_byte.data(), 8 * ev_byte.size(), cudaMemcpyHostToDevice, s));
+    const auto enqueue = [&](size_t k) -> iss_status {
+        const Chunk& c = chunks[k];
+        const int64_t at = static_cast<int64_t>(k % kOscarBuffers) * kOscarChunk;
+        CUDA_TRY(h, launch_oscar_lines(h->d_hadrons.ptr, c.h0, c.h1, h->d_oscar_off.ptr, h->d_oscar_byte.ptr, c.e_lo,
+                                       c.e_hi, c.byte0, h->d_oscar_text.ptr + at, h->num_sms, s));
+        CUDA_TRY(h, cudaMemcpyAsync(h->oscar_host + at, h->d_oscar_text.ptr + at, static_cast<size_t>(c.bytes),
+                                    cudaMemcpyDeviceToHost, s));
+        CUDA_TRY(h, cudaEventRecord(h->oscar_ev[k % kOscarBuffers], s));
+        return ISS_OK;
     };
-    if (!chunks.empty()) OSCAR_TRY(enqueue(0));
-    for (size_t c = 0; c < chunks.size(); c++) {
-        // chunk c + 1 is formatted while chunk c is written; chunk c + 1 uses
-        // the other buffer, which chunk c - 1 released when it was written
-        if (c + 1 < chunks.size()) OSCAR_TRY(enqueue(c + 1));
-        const int k = static_cast<int>(c & 1);
-        OSCAR_TRY(cudaEventSynchronize(done[k]));
-        const int64_t bytes = ev_byte[chunks[c].second] - ev_byte[chunks[c].first];
-        if (bytes > 0 && std::fwrite(host[k], 1, static_cast<size_t>(bytes), f) != static_cast<size_t>(bytes)) {
-            cleanup();
+    iss_status st = enqueue(0);
+    for (size_t k = 0; k < chunks.size() && st == ISS_OK; k++) {
+        // chunk k + 1 takes the buffer that chunk k - 1 left when it was written
+        if (k + 1 < chunks.size()) st = enqueue(k + 1);
+        if (st != ISS_OK) break;
+        CUDA_TRY(h, cudaEventSynchronize(h->oscar_ev[k % kOscarBuffers]));
+        const size_t bytes = static_cast<size_t>(chunks[k].bytes);
+        if (std::fwrite(h->oscar_host + static_cast<int64_t>(k % kOscarBuffers) * kOscarChunk, 1, bytes, f) != bytes) {
+            cudaStreamSynchronize(s);
             return fail(h, ISS_ERR_IO, "write error on %s", filename);
         }
     }
-#undef OSCAR_TRY
-    cleanup();
     return st;
 }
 

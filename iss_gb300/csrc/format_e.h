@@ -68,10 +68,33 @@ FMT_HD U192 shr_round(const U192& a, int s, int* half, int* sticky) {
     return r;
 }
 
+// 5^k, 0 <= k <= 27 (below 2^63), by squaring
+FMT_HD uint64_t pow5(int k) {
+    uint64_t r = (k & 1) ? 5u : 1u;
+    if (k & 2) r *= 25u;
+    if (k & 4) r *= 625u;
+    if (k & 8) r *= 390625u;
+    if (k & 16) r *= 152587890625ull;
+    return r;
+}
+
 // D = round_half_even(|v| * 10^(16 - p)) for |v| = m 2^e, m > 0
 FMT_HD uint64_t scaled_digits(uint32_t m, int e, int p) {
     const int b = 16 - p;
     const int a = e + b;
+    if (b >= 0 && b <= 27 && a < 0 && a > -64) {
+        // 1e-11 <= |v| < 1e17 and the like: m 5^b has at most 87 bits, and less
+        // than 64 of them are shifted out
+        const unsigned __int128 x = static_cast<unsigned __int128>(pow5(b)) * m;
+        const int s = -a;
+        const unsigned __int128 q = x >> s;
+        if (static_cast<uint64_t>(q >> 64)) return ~0ull;
+        uint64_t d = static_cast<uint64_t>(q);
+        const uint64_t dropped = static_cast<uint64_t>(x) << (64 - s);   // the s low bits, at the top
+        const uint64_t half = 1ull << 63;
+        if (dropped > half || (dropped == half && (d & 1))) d++;
+        return d;
+    }
     if (b >= 0) {
         U192 x = {{m, 0, 0}};
         int k = b;
@@ -79,9 +102,7 @@ FMT_HD uint64_t scaled_digits(uint32_t m, int e, int p) {
             mul_small(x, 7450580596923828125ull);
             k -= 27;
         }
-        uint64_t f = 1;
-        for (int i = 0; i < k; i++) f *= 5;
-        mul_small(x, f);
+        mul_small(x, pow5(k));
         if (a >= 0) {
             // |v| 10^b is an integer; below 10^17 whenever p is right, so a
             // result of 64 bits or more only says that p is too small
@@ -97,8 +118,7 @@ FMT_HD uint64_t scaled_digits(uint32_t m, int e, int p) {
         return d;
     }
     // b < 0: m 2^a / 5^-b with a > 0
-    uint64_t den = 1;
-    for (int i = 0; i < -b; i++) den *= 5;
+    const uint64_t den = pow5(-b);   // -b <= 22
     if (a >= 128 - 24) return ~0ull;
     const unsigned __int128 num = static_cast<unsigned __int128>(m) << a;
     const unsigned __int128 q = num / den;
@@ -110,7 +130,17 @@ FMT_HD uint64_t scaled_digits(uint32_t m, int e, int p) {
     return d;
 }
 
+// n decimal digits of v (zero-padded) to out
+FMT_HD void put_digits(uint32_t v, int n, char* out) {
+    for (int i = n - 1; i >= 0; i--) {
+        out[i] = static_cast<char>('0' + v % 10);
+        v /= 10;
+    }
+}
+
 // Writes exactly 24 characters (no terminator): printf("%24.16e", (double)x).
+// A float's exponent has two digits, so a finite value is two places of blanks
+// or sign, the digit, the point, 16 digits and the exponent.
 FMT_HD void format_e24_16(float x, char* out) {
     uint32_t bits;
 #if defined(__CUDA_ARCH__)
@@ -121,62 +151,60 @@ FMT_HD void format_e24_16(float x, char* out) {
     const int neg = static_cast<int>(bits >> 31);
     const int ex = static_cast<int>((bits >> 23) & 0xFFu);
     uint32_t m = bits & 0x7FFFFFu;
-    char buf[24];
-    int len = 0;
     if (ex == 0xFF) {
-        const char* s = m ? "nan" : "inf";
-        if (neg) buf[len++] = '-';
-        for (int i = 0; i < 3; i++) buf[len++] = s[i];
-    } else {
-        int e;
-        if (ex) {
-            m |= 0x800000u;
-            e = ex - 150;
-        } else {
-            e = -149;
-        }
-        uint64_t D = 0;
-        int p = 0;
-        if (m != 0) {
-            // estimate p = floor(log10(m 2^e)) from the bit length
-            int nb = 0;
-            for (uint32_t t = m; t; t >>= 1) nb++;
-            const int e2 = e + nb - 1;                     // 2^e2 <= |v| < 2^(e2+1)
-            p = (e2 >= 0) ? (e2 * 78913) >> 18 : -(((-e2) * 78913 + 262143) >> 18);
-            for (int it = 0; it < 4; it++) {
-                D = scaled_digits(m, e, p);
-                if (D >= 100000000000000000ull) {
-                    p++;
-                } else if (D < 10000000000000000ull) {
-                    p--;
-                } else {
-                    break;
-                }
-            }
-            if (D == 100000000000000000ull) {   // rounding carried into a new digit
-                D = 10000000000000000ull;
-                p++;
-            }
-        }
-        char dig[17];
-        for (int i = 16; i >= 0; i--) {
-            dig[i] = static_cast<char>('0' + D % 10);
-            D /= 10;
-        }
-        if (neg) buf[len++] = '-';
-        buf[len++] = dig[0];
-        buf[len++] = '.';
-        for (int i = 1; i < 17; i++) buf[len++] = dig[i];
-        buf[len++] = 'e';
-        buf[len++] = p < 0 ? '-' : '+';
-        const int ap = p < 0 ? -p : p;
-        if (ap >= 100) buf[len++] = static_cast<char>('0' + ap / 100);
-        buf[len++] = static_cast<char>('0' + (ap / 10) % 10);
-        buf[len++] = static_cast<char>('0' + ap % 10);
+        for (int i = 0; i < 20; i++) out[i] = ' ';
+        out[20] = neg ? '-' : ' ';
+        out[21] = m ? 'n' : 'i';
+        out[22] = m ? 'a' : 'n';
+        out[23] = m ? 'n' : 'f';
+        return;
     }
-    const int pad = 24 - len;
-    for (int i = 0; i < pad; i++) out[i] = ' ';
-    for (int i = 0; i < len; i++) out[pad + i] = buf[i];
+    int e;
+    if (ex) {
+        m |= 0x800000u;
+        e = ex - 150;
+    } else {
+        e = -149;
+    }
+    uint64_t D = 0;
+    int p = 0;
+    if (m != 0) {
+        // estimate p = floor(log10(m 2^e)) from the bit length
+#if defined(__CUDA_ARCH__)
+        const int nb = 32 - __clz(static_cast<int>(m));
+#else
+        const int nb = 32 - __builtin_clz(m);
+#endif
+        const int e2 = e + nb - 1;                     // 2^e2 <= |v| < 2^(e2+1)
+        p = (e2 >= 0) ? (e2 * 78913) >> 18 : -(((-e2) * 78913 + 262143) >> 18);
+        for (int it = 0; it < 4; it++) {
+            D = scaled_digits(m, e, p);
+            if (D >= 100000000000000000ull) {
+                p++;
+            } else if (D < 10000000000000000ull) {
+                p--;
+            } else {
+                break;
+            }
+        }
+        if (D == 100000000000000000ull) {   // rounding carried into a new digit
+            D = 10000000000000000ull;
+            p++;
+        }
+    }
+    // 17 digits: 1 + 8 in the upper word, 8 in the lower one
+    const uint32_t upper = static_cast<uint32_t>(D / 100000000u);
+    const uint32_t lower = static_cast<uint32_t>(D - static_cast<uint64_t>(upper) * 100000000u);
+    const uint32_t lead = upper / 100000000u;
+    out[0] = ' ';
+    out[1] = neg ? '-' : ' ';
+    out[2] = static_cast<char>('0' + lead);
+    out[3] = '.';
+    put_digits(upper - lead * 100000000u, 8, out + 4);
+    put_digits(lower, 8, out + 12);
+    out[20] = 'e';
+    out[21] = p < 0 ? '-' : '+';
+    put_digits(static_cast<uint32_t>(p < 0 ? -p : p), 2, out + 22);
 }
 
 // Right-aligned decimal integer in `width` characters (std::setw(width) << v).
