@@ -277,72 +277,72 @@ __device__ __forceinline__ float langevin_over_kappa(float kappa) {
     return ((1.0f + e) / (1.0f - e) - 1.0f / kappa) / kappa;
 }
 
+// maximum and sum over the eight lanes of a row
+__device__ __forceinline__ float row_max(float v) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float row_sum(float v) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Eight lanes per row, lane k the k-th component: each transcendental once, and
+// rows enough in flight for small batches.  (50,001 rows: 35 us with a thread
+// per row, 10 us so.)
+static_assert(kComp == 8, "eight lanes per row");
 __global__ void __launch_bounds__(256)
 mlp_loss_kernel(const float* __restrict__ out, const float4* __restrict__ target, int64_t n,
                 float inv_n, float* __restrict__ dout, double* __restrict__ loss_base,
                 const int* __restrict__ step) {
-    const int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    float nll = 0.0f;
-    if (row < n && !(target[row].x > 0.0f)) {
-        // a row without a target (K <= 0) contributes nothing
-        for (int j = 0; j < kOut; j++) dout[row * kOut + j] = 0.0f;
-    } else if (row < n) {
-        const float* z = out + row * kOut;
-        const float4 tg = target[row];
-        const float lK = logf(tg.x);
-        float lmax = -INFINITY;
-        for (int k = 0; k < kComp; k++) lmax = fmaxf(lmax, z[k]);
-        float se = 0.0f;
-        for (int k = 0; k < kComp; k++) se += expf(z[k] - lmax);
-        const float lse_w = lmax + logf(se);
-        float lc[kComp];
-        float cmax = -INFINITY;
-        const float half_l2pi = 0.91893853320467274f;
-        for (int k = 0; k < kComp; k++) {
-            const float s = fminf(fmaxf(z[16 + k], kLogSigMin), kLogSigMax);
-            const float is2 = expf(-2.0f * s);
-            const float d = lK - z[8 + k];
-            const float vx = z[24 + 3 * k], vy = z[25 + 3 * k], vz = z[26 + 3 * k];
-            const float kap = sqrtf(vx * vx + vy * vy + vz * vz);
-            lc[k] = z[k] - lse_w - s - half_l2pi - 0.5f * d * d * is2 + log_vmf_norm(kap) +
-                    vx * tg.y + vy * tg.z + vz * tg.w;
-            cmax = fmaxf(cmax, lc[k]);
-        }
-        float sc = 0.0f;
-        for (int k = 0; k < kComp; k++) sc += expf(lc[k] - cmax);
-        const float L = cmax + logf(sc);
-        nll = -(L - lK);
+    const int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 3;
+    const int k = threadIdx.x & 7;
+    const bool on = row < n;
+    const float4 tg = on ? target[row] : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+    // a row without a target (K <= 0) contributes nothing
+    const bool live = tg.x > 0.0f;
+    const float* z = out + (on ? row : 0) * kOut;
+    const float zk = z[k], mu = z[8 + k], sraw = z[16 + k];
+    const float vx = z[24 + 3 * k], vy = z[25 + 3 * k], vz = z[26 + 3 * k];
+    const float half_l2pi = 0.91893853320467274f;
+    const float lK = logf(live ? tg.x : 1.0f);
+    const float lmax = row_max(zk);
+    const float lse_w = lmax + logf(row_sum(expf(zk - lmax)));
+    const float s = fminf(fmaxf(sraw, kLogSigMin), kLogSigMax);
+    const float is2 = expf(-2.0f * s);
+    const float d = lK - mu;
+    const float kap = sqrtf(vx * vx + vy * vy + vz * vz);
+    const float lc = zk - lse_w - s - half_l2pi - 0.5f * d * d * is2 + log_vmf_norm(kap) + vx * tg.y +
+                     vy * tg.z + vz * tg.w;
+    const float cmax = row_max(lc);
+    const float L = cmax + logf(row_sum(expf(lc - cmax)));
+    if (on) {
+        const float r = live ? expf(lc - L) : 0.0f;
+        const float w = live ? expf(zk - lse_w) : 0.0f;
+        const float gk = langevin_over_kappa(kap);
         float* g = dout + row * kOut;
-        for (int k = 0; k < kComp; k++) {
-            const float r = expf(lc[k] - L);
-            const float w = expf(z[k] - lse_w);
-            const float sraw = z[16 + k];
-            const float s = fminf(fmaxf(sraw, kLogSigMin), kLogSigMax);
-            const float is2 = expf(-2.0f * s);
-            const float d = lK - z[8 + k];
-            const float vx = z[24 + 3 * k], vy = z[25 + 3 * k], vz = z[26 + 3 * k];
-            const float kap = sqrtf(vx * vx + vy * vy + vz * vz);
-            const float gk = langevin_over_kappa(kap);
-            g[k] = (w - r) * inv_n;
-            g[8 + k] = -r * d * is2 * inv_n;
-            g[16 + k] = (sraw > kLogSigMin && sraw < kLogSigMax) ? -r * (d * d * is2 - 1.0f) * inv_n : 0.0f;
-            g[24 + 3 * k] = -r * (tg.y - gk * vx) * inv_n;
-            g[25 + 3 * k] = -r * (tg.z - gk * vy) * inv_n;
-            g[26 + 3 * k] = -r * (tg.w - gk * vz) * inv_n;
-        }
-        for (int j = kOutUsed; j < kOut; j++) g[j] = 0.0f;
+        g[k] = (w - r) * inv_n;
+        g[8 + k] = -r * d * is2 * inv_n;
+        g[16 + k] = (live && sraw > kLogSigMin && sraw < kLogSigMax) ? -r * (d * d * is2 - 1.0f) * inv_n : 0.0f;
+        g[24 + 3 * k] = -r * (tg.y - gk * vx) * inv_n;
+        g[25 + 3 * k] = -r * (tg.z - gk * vy) * inv_n;
+        g[26 + 3 * k] = -r * (tg.w - gk * vz) * inv_n;
+#pragma unroll
+        for (int j = kOutUsed; j < kOut; j += 8) g[j + k] = 0.0f;
     }
     // block sum of the loss
     __shared__ float s_part[8];
-    float v = nll;
+    float v = live && k == 0 ? -(L - lK) : 0.0f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < static_cast<int>(blockDim.x >> 5); w++) s += s_part[w];
-        atomicAdd(step ? loss_base + *step : loss_base, s);
+        double sum = 0.0;
+        for (int i = 0; i < static_cast<int>(blockDim.x >> 5); i++) sum += s_part[i];
+        atomicAdd(step ? loss_base + *step : loss_base, sum);
     }
 }
 
@@ -350,48 +350,71 @@ mlp_loss_kernel(const float* __restrict__ out, const float4* __restrict__ target
 // backward: parameter gradients of the mean loss, accumulated into grad
 // (FP32, flat parameter layout) with atomics per tile
 
+// Four warpgroups share a tile: thread (row t, quarter q) owns a quarter of the
+// columns of row t in every epilogue.  Both GEMMs of a layer, dH = dZ W and
+// dW^T = H^T dZ, start from one barrier; while they run, the next layer's
+// activations and weights are read.  dW^T has the inputs in TMEM lanes, so that
+// the 32 lanes of an atomic add to consecutive weights; the bias gradients
+// are column sums in FP32, 32 columns in 31 shuffles.  Bound by the latency of
+// the five layers' chain of barriers, GEMMs and epilogues per tile.  (50,001
+// rows: 87 us; 433 with one warpgroup, 32 sectors per atomic and five shuffles
+// per column.)
+constexpr int kBwdThreads = 512;
 constexpr int kBwdSmem = 4 * kTile * kHid * 2 + 64;
 
-__device__ __forceinline__ float warp_sum(float v) {
+// column sums over a warp's 32 rows, in lane j the sum of column j (j % N)
+template <int N>
+__device__ __forceinline__ float column_sums(float (&v)[N], int lane) {
+    static_assert(N == 32 || N == 16, "two or one column per lane pair");
+    if (N == 16) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// stage 8 gradient values of row t at columns c..c+7 of a dZ tile with Kz
-// columns: K-major copy sDZ[t][.] and transposed copy sDZt[c + j][t]
-// (K = 128 rows of the tile); the bias gradient gets the column sums
-__device__ __forceinline__ void stage_dz8(uint8_t* sDZ, uint8_t* sDZt, int t, int c, int Kz,
-                                          const float (&d)[8], float* gbias) {
-    uint4 pk;
-    uint32_t* pw = reinterpret_cast<uint32_t*>(&pk);
-#pragma unroll
-    for (int j = 0; j < 4; j++) pw[j] = pack_bf16x2(d[2 * j], d[2 * j + 1]);
-    *reinterpret_cast<uint4*>(sDZ + kmajor_offset(t, c, Kz)) = pk;
-    const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&pk);
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-        *reinterpret_cast<__nv_bfloat16*>(sDZt + kmajor_offset(c + j, t, kTile)) = hb[j];
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const float s = warp_sum(d[j]);
-        if ((t & 31) == 0 && s != 0.0f) atomicAdd(gbias + c + j, s);
+        for (int j = 0; j < N; j++) v[j] += __shfl_xor_sync(0xffffffffu, v[j], 16);
     }
+#pragma unroll
+    for (int o = N / 2; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int j = 0; j < o; j++) {
+            const float send = up ? v[j] : v[j + o];
+            const float keep = up ? v[j + o] : v[j];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0];
 }
 
-// transposed copy of row t of an activation tile: sHt[i][t] for i < width
-__device__ __forceinline__ void stage_ht(uint8_t* sHt, int t, const __nv_bfloat16* src, int width,
-                                         bool valid) {
-    for (int c = 0; c < width; c += 8) {
-        uint4 v = valid ? *reinterpret_cast<const uint4*>(src + c) : make_uint4(0, 0, 0, 0);
-        const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&v);
+// stage N gradient values of row t at columns c0 .. c0 + N - 1 of a dZ tile with
+// Kz columns: K-major copy sDZ[t][.] and transposed copy sDZt[c][t] (K = 128
+// rows of the tile); the bias gradient gets the column sums
+template <int N>
+__device__ __forceinline__ void stage_dz(uint8_t* sDZ, uint8_t* sDZt, int t, int c0, int Kz, float (&d)[N],
+                                         float* gbias) {
+#pragma unroll
+    for (int c = 0; c < N; c += 8) {
+        uint4 pk;
+        uint32_t* pw = reinterpret_cast<uint32_t*>(&pk);
+#pragma unroll
+        for (int j = 0; j < 4; j++) pw[j] = pack_bf16x2(d[c + 2 * j], d[c + 2 * j + 1]);
+        *reinterpret_cast<uint4*>(sDZ + kmajor_offset(t, c0 + c, Kz)) = pk;
+        const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&pk);
 #pragma unroll
         for (int j = 0; j < 8; j++)
-            *reinterpret_cast<__nv_bfloat16*>(sHt + kmajor_offset(c + j, t, kTile)) = hb[j];
+            *reinterpret_cast<__nv_bfloat16*>(sDZt + kmajor_offset(c0 + c + j, t, kTile)) = hb[j];
     }
+    const int lane = t & 31;
+    const float s = column_sums<N>(d, lane);
+    if (lane < N) atomicAdd(gbias + c0 + lane, s);
 }
 
-__global__ void __launch_bounds__(128, 1)
+// transposed copy of 8 activations of row t: sHt[c + j][t]
+__device__ __forceinline__ void stage_ht8(uint8_t* sHt, int t, int c, const uint4& v) {
+    const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        *reinterpret_cast<__nv_bfloat16*>(sHt + kmajor_offset(c + j, t, kTile)) = hb[j];
+}
+
+__global__ void __launch_bounds__(kBwdThreads, 1)
 mlp_bwd_kernel(const __nv_bfloat16* __restrict__ img, const __nv_bfloat16* __restrict__ X,
                const __nv_bfloat16* __restrict__ acts, const float* __restrict__ dout, int64_t n,
                float* __restrict__ grad, int* __restrict__ err) {
@@ -402,8 +425,8 @@ mlp_bwd_kernel(const __nv_bfloat16* __restrict__ img, const __nv_bfloat16* __res
     uint8_t* sHt = sDZt + kTile * kHid * 2;
     uint64_t* bar = reinterpret_cast<uint64_t*>(sHt + kTile * kHid * 2);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
-    const int t = threadIdx.x, warp = t >> 5;
-    if (t == 0) {
+    const int t = threadIdx.x & 127, q = threadIdx.x >> 7, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         barrier_init_fence();
     }
@@ -418,31 +441,67 @@ mlp_bwd_kernel(const __nv_bfloat16* __restrict__ img, const __nv_bfloat16* __res
     const uint32_t tm_dh = tmem, tm_dw = tmem + 128;
     uint32_t phase = 0;
     bool ok = true;
+    const uint4 zero4 = make_uint4(0, 0, 0, 0);
     const int64_t n_tiles = (n + kTile - 1) / kTile;
     for (int64_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         const int64_t row = tile * kTile + t;
         const bool valid = row < n;
-        // dZ of the output layer from the loss gradient
-        for (int c = 0; c < kOut; c += 8) {
-            float d[8];
+        // this thread's quarter of layer l's inputs (32 columns, 8 of X) ...
+        uint4 h[4], w[4];
+        const auto read_inputs = [&](int l) {
+            if (l == 0) {
+                h[0] = valid ? *reinterpret_cast<const uint4*>(X + row * kIn0 + 8 * q) : zero4;
+                return;
+            }
+            const uint4* src = reinterpret_cast<const uint4*>(
+                acts + (static_cast<int64_t>(l - 1) * n + (valid ? row : 0)) * kHid + 32 * q);
 #pragma unroll
-            for (int j = 0; j < 8; j++) d[j] = valid ? dout[row * kOut + c + j] : 0.0f;
-            stage_dz8(sDZ, sDZt, t, c, kOut, d, grad + b_offset(kLayers - 1));
+            for (int c = 0; c < 4; c++) h[c] = valid ? src[c] : zero4;
+        };
+        // ... and its share of the transposed weights' image
+        const auto read_weights = [&](int l) {
+            const uint4* src = reinterpret_cast<const uint4*>(img + bwd_img_offset(l)) + threadIdx.x;
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                if (c * kBwdThreads < dim_in(l) * dim_out(l) / 8) w[c] = src[c * kBwdThreads];
+        };
+        read_inputs(kLayers - 1);
+        read_weights(kLayers - 1);
+        {
+            // dZ of the output layer from the loss gradient: 16 columns each
+            float d[16];
+            const float4* src = reinterpret_cast<const float4*>(dout + (valid ? row : 0) * kOut + 16 * q);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const float4 v = valid ? src[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                d[4 * c] = v.x;
+                d[4 * c + 1] = v.y;
+                d[4 * c + 2] = v.z;
+                d[4 * c + 3] = v.w;
+            }
+            stage_dz<16>(sDZ, sDZt, t, 16 * q, kOut, d, grad + b_offset(kLayers - 1));
         }
+#pragma unroll 1
         for (int l = kLayers - 1; l >= 0; l--) {
             const int K_in = dim_in(l), K_out = dim_out(l);
-            // input of layer l, transposed
-            if (l == 0)
-                stage_ht(sHt, t, X + row * kIn0, kIn0, valid);
-            else
-                stage_ht(sHt, t, acts + (static_cast<int64_t>(l - 1) * n + row) * kHid, kHid, valid);
-            if (l > 0) {
-                const uint4* src = reinterpret_cast<const uint4*>(img + bwd_img_offset(l));
-                uint4* dst = reinterpret_cast<uint4*>(sWt);
-                for (int i = t; i < K_in * K_out * 2 / 16; i += 128) dst[i] = src[i];
+            // (every GEMM that read these buffers has completed: all threads
+            // waited for the last commit)
+            if (l == 0) {
+                stage_ht8(sHt, t, 8 * q, h[0]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    stage_ht8(sHt, t, 32 * q + 8 * c, h[c]);
+                    if (c * kBwdThreads < K_in * K_out / 8)
+                        reinterpret_cast<uint4*>(sWt)[threadIdx.x + c * kBwdThreads] = w[c];
+                }
             }
-            sync_for_mma();
-            if (t == 0) {
+            fence_smem_to_async();
+            fence_before_sync();
+            ok = __syncthreads_and(ok);
+            if (!ok) break;
+            fence_after_sync();
+            if (threadIdx.x == 0) {
                 if (l > 0) {
                     // dH[b][i] = sum_o dZ[b][o] W[o][i]
                     const uint32_t id = idesc_bf16_f32(128, K_in);
@@ -450,66 +509,47 @@ mlp_bwd_kernel(const __nv_bfloat16* __restrict__ img, const __nv_bfloat16* __res
                         mma_bf16(tm_dh, kslice_desc(smem_addr(sDZ), K_out, ks),
                                  kslice_desc(smem_addr(sWt), K_out, ks), id, ks > 0);
                 }
-                if (l == kLayers - 1) {
-                    // dW^T[i][o] = sum_b H[b][i] dZ[b][o]
-                    const uint32_t id = idesc_bf16_f32(128, K_out);
-                    for (int ks = 0; ks < kTile / 16; ks++)
-                        mma_bf16(tm_dw, kslice_desc(smem_addr(sHt), kTile, ks),
-                                 kslice_desc(smem_addr(sDZt), kTile, ks), id, ks > 0);
-                } else {
-                    // dW[o][i] = sum_b dZ[b][o] H[b][i]
-                    const uint32_t id = idesc_bf16_f32(128, K_in);
-                    for (int ks = 0; ks < kTile / 16; ks++)
-                        mma_bf16(tm_dw, kslice_desc(smem_addr(sDZt), kTile, ks),
-                                 kslice_desc(smem_addr(sHt), kTile, ks), id, ks > 0);
-                }
+                // dW^T[i][o] = sum_b H[b][i] dZ[b][o] (layer 0: lanes 32 and up
+                // hold products of stale rows of sHt, which nothing reads)
+                const uint32_t id = idesc_bf16_f32(128, K_out);
+                for (int ks = 0; ks < kTile / 16; ks++)
+                    mma_bf16(tm_dw, kslice_desc(smem_addr(sHt), kTile, ks),
+                             kslice_desc(smem_addr(sDZt), kTile, ks), id, ks > 0);
                 mma_commit(bar);
             }
-            ok = __syncthreads_and(mbar_wait(bar, phase, err, 3));
-            phase ^= 1u;
-            if (!ok) break;
-            fence_after_sync();
-            // weight gradient
-            float* gw = grad + w_offset(l);
-            if (l == kLayers - 1) {
-                for (int c0 = 0; c0 < K_out; c0 += 32) {
-                    float v[32];
-                    tmem_ld32(tmem_lane_addr(tm_dw, warp, c0), v);
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (v[j] != 0.0f) atomicAdd(gw + (c0 + j) * K_in + t, v[j]);
-                }
-            } else {
-                for (int c0 = 0; c0 < K_in; c0 += 32) {
-                    float v[32];
-                    tmem_ld32(tmem_lane_addr(tm_dw, warp, c0), v);
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (v[j] != 0.0f) atomicAdd(gw + t * K_in + c0 + j, v[j]);
-                }
-            }
-            // dZ of layer l - 1: dH masked by the ReLU of H_{l-1}
+            // the ReLU mask of dZ of layer l - 1 (its outputs H are layer l's inputs)
+            uint32_t positive = 0u;
             if (l > 0) {
-                const __nv_bfloat16* h = acts + (static_cast<int64_t>(l - 1) * n + row) * kHid;
-                for (int c0 = 0; c0 < kHid; c0 += 32) {
-                    float v[32];
-                    tmem_ld32(tmem_lane_addr(tm_dh, warp, c0), v);
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        uint4 hv = valid ? *reinterpret_cast<const uint4*>(h + c0 + 8 * q)
-                                         : make_uint4(0, 0, 0, 0);
-                        const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&hv);
-                        float d[8];
+                for (int c = 0; c < 4; c++) {
+                    const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&h[c]);
 #pragma unroll
-                        for (int j = 0; j < 8; j++)
-                            d[j] = __bfloat162float(hb[j]) > 0.0f ? v[8 * q + j] : 0.0f;
-                        stage_dz8(sDZ, sDZt, t, c0 + 8 * q, kHid, d, grad + b_offset(l - 1));
-                    }
+                    for (int j = 0; j < 8; j++)
+                        positive |= static_cast<uint32_t>(__bfloat162float(hb[j]) > 0.0f) << (8 * c + j);
                 }
+                read_inputs(l - 1);
+                if (l > 1) read_weights(l - 1);
             }
-            fence_before_sync();
-            __syncthreads();
+            ok = mbar_wait(bar, phase, err, 3);   // agreed on at the next barrier
+            phase ^= 1u;
+            fence_after_sync();
+            if (l > 0) {
+                float v[32];
+                tmem_ld32(tmem_lane_addr(tm_dh, warp, 32 * q), v);
+#pragma unroll
+                for (int j = 0; j < 32; j++) v[j] = (positive >> j) & 1u ? v[j] : 0.0f;
+                stage_dz<32>(sDZ, sDZt, t, 32 * q, kHid, v, grad + b_offset(l - 1));
+            }
+            // weight gradient: 32 outputs of input t
+            if (32 * q < K_out && (t & ~31) < K_in) {
+                float v[32];
+                tmem_ld32(tmem_lane_addr(tm_dw, warp, 32 * q), v);
+                float* gw = grad + w_offset(l) + t;
+#pragma unroll
+                for (int j = 0; j < 32; j++) atomicAdd(gw + (32 * q + j) * K_in, v[j]);
+            }
         }
+        ok = __syncthreads_and(ok);   // every thread has read its accumulators
     }
     fence_before_sync();
     __syncthreads();
@@ -660,7 +700,7 @@ cudaError_t launch_mlp_forward(const void* img, const float* params, const void*
 cudaError_t launch_mlp_loss(const float* out, const void* target, int64_t n, float* dout,
                             double* loss_base, const int* step, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    mlp_loss_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(
+    mlp_loss_kernel<<<static_cast<unsigned>((n * kComp + 255) / 256), 256, 0, s>>>(
         out, static_cast<const float4*>(target), n, 1.0f / static_cast<float>(n), dout, loss_base,
         step);
     return cudaGetLastError();
@@ -673,7 +713,7 @@ cudaError_t launch_mlp_backward(const void* img, const void* X, const void* acts
     if (e != cudaSuccess) return e;
     const int64_t tiles = (n + kTile - 1) / kTile;
     const int grid = static_cast<int>(tiles < num_sms ? tiles : num_sms);
-    mlp_bwd_kernel<<<grid, 128, kBwdSmem, s>>>(static_cast<const __nv_bfloat16*>(img),
+    mlp_bwd_kernel<<<grid, kBwdThreads, kBwdSmem, s>>>(static_cast<const __nv_bfloat16*>(img),
                                                static_cast<const __nv_bfloat16*>(X),
                                                static_cast<const __nv_bfloat16*>(acts), dout, n, grad,
                                                err);
