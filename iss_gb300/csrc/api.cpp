@@ -788,6 +788,7 @@ constexpr int kDecayBatch = 8;
 
 // hadrons of one sampler launch of iss_gpu_generate_into, at least (run_generate)
 constexpr int64_t kGroupRecords = 256 << 10;
+constexpr int64_t kLearnedGroupRecords = 512 << 10;
 
 iss_status run_decays(iss_handle* h, unsigned long long* failures_out) {
     DevConfig& c = h->cfg;
@@ -1559,11 +1560,15 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     // it holds kGroupRecords hadrons (or half of them all).  A launch ends with
     // a tail of some 50 us (its longest work items), in which the link copies
     // 256k records, so smaller launches only add tails; larger ones leave the
-    // link idle for longer before the first copy.  The launches alternate
+    // link idle for longer before the first copy (512k, 1M and 4M records: 300
+    // events of 200,000 cells 3.81, 3.86 and 4.07 ms, 3.80 so).  The learned
+    // sampler, slower than the link, takes twice as many (1.77 -> 1.65 ms on
+    // 50,000 cells and 200 events).  The launches alternate
     // between two streams, so that one's tail runs beside the next one.
     // (37,211 cells, 37 events, 146,000 hadrons: 13 launches in a row took
     // 0.77 ms.)
-    const int64_t group_records = std::min(kGroupRecords, (n_units + 1) / 2);
+    const int64_t group_records =
+        std::min(h->use_learned ? kLearnedGroupRecords : kGroupRecords, (n_units + 1) / 2);
     if (to_host && n_chunks > 1) {
         if (!h->sample_stream) {
             CUDA_TRY(h, cudaStreamCreateWithFlags(&h->sample_stream, cudaStreamNonBlocking));

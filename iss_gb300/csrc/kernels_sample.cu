@@ -1683,8 +1683,11 @@ constexpr int kSampleThreads = 256;
 // correction (both compile out, which frees registers), 2 the same with
 // diffusion; 1 and 2 read the prologue's lean cell records (the learned
 // proposal's plain component uses the same Prop fields)
+// Blocks per SM: three of 80 registers; the learned instantiations two of 128,
+// since at 80 some 300 bytes per thread spill into the loop over the proposals
+// (50,000 cells, 200 events: sample phase 1093 us with three, 935 with two).
 template <bool kLcc, bool kLearned, int kMode>
-__global__ void __launch_bounds__(kSampleThreads, 3)
+__global__ void __launch_bounds__(kSampleThreads, kLearned ? 2 : 3)
 sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict__ species,
                const int32_t* __restrict__ pids, const __grid_constant__ CellRows rows,
                const int64_t* __restrict__ offsets,
@@ -2308,7 +2311,7 @@ cudaError_t launch_sampler(const DevConfig& cfg, const CellArrays& cells, const 
             work_counter, counters, k_end_dev);
         return cudaGetLastError();
     }
-    const int per_sm = std::min(3, std::max(1, cfg.sampler_ctas));
+    const int per_sm = std::min(cfg.lpairs ? 2 : 3, std::max(1, cfg.sampler_ctas));
     int64_t blocks = static_cast<int64_t>(num_sms) * per_sm;
     const int64_t max_blocks = (n_items + (kSampleThreads / 32) - 1) / (kSampleThreads / 32);
     if (blocks > max_blocks) blocks = max_blocks;
