@@ -1075,6 +1075,7 @@ __device__ float ea_f0_max(int sign, int A, float m, float T, float mu, float f0
 
 struct PropEfa {
     float tau, T, mu, m, bmax;     // bmax: the reference's maximum / (degen prefactor)
+    float dsig;                    // |u.dsigma| + |dsigma_T|, tau included
     float da0, da1, da2, da3, u0, u1, u2, u3;
     float pi00, pi01, pi02, pi03, pi11, pi12, pi13, pi22, pi23, pi33;
     float q0, q1, q2, q3;
@@ -1110,13 +1111,14 @@ __device__ bool setup_efa(const DevConfig& cfg, const CellArrays& cells, const S
     p.bulk_c1 = cf.y;
     p.qpref = cfg.include_diff ? th2.z / ep : 0.0f;
     p.ikappa = cfg.include_diff ? 1.0f / cf.w : 0.0f;
-    if (keep_max) return true;
     // estimate_maximum (src/emissionfunction.cpp:4309-4421)
     const float udsig = p.tau * (p.u0 * p.da0 + p.u1 * p.da1 + p.u2 * p.da2 + p.u3 * p.da3 / p.tau);
     const float dsig2 = p.tau * p.tau * (p.da0 * p.da0 - p.da1 * p.da1 - p.da2 * p.da2 -
                                          p.da3 * p.da3 / (p.tau * p.tau));
     const float dsigT = sqrtf(fabsf(dsig2 - udsig * udsig));
     const float dsig_all = fabsf(udsig) + dsigT;
+    p.dsig = dsig_all;
+    if (keep_max) return true;
     const float f0m = 1.0f / (expf((p.m - p.mu) / p.T) + p.sign);
     const float g_ideal = ea_f0_max(p.sign, 1, p.m, p.T, p.mu, f0m);
     float g = g_ideal;
@@ -1198,6 +1200,93 @@ __device__ __forceinline__ bool try_efa(const DevConfig& cfg, const PropEfa& p, 
         u_rap = u01f(B.x);
     }
     return true;
+}
+
+// Proposals in bulk.  A proposal's pT^2 is uniform, and pT alone bounds its
+// acceptance: the energy in the rest frame is at least
+// E = sqrt(1 + u_T^2) m_T - u_T p_T, p.dsigma at most E (|u.dsigma| + |dsigma_T|),
+// and E f0(E) falls with E above its peak.  efa_bin_bound gives, for the b-th of
+// 32 equal bins in pT^2, a bound of the acceptance over the bin (all phi, y and
+// |delta f| <= df_max_ratio); a proposal whose uniform is not below it is
+// rejected whatever its phi and y are.  About one in twenty survives.  The
+// margins (epsilons of 2e-6 of the largest terms, 1 % on the whole) are far above
+// the rounding of try_efa's own sums; where the bound does not hold (no
+// restrict_deltaf, energies at the peak or below a boson's mu) it is infinite,
+// and a NaN rejects nothing.
+constexpr int kEfaBins = 32;
+__device__ float efa_bin_bound(const DevConfig& cfg, const PropEfa& p, int bin) {
+    const float inf = __int_as_float(0x7f800000);
+    if (!cfg.restrict_df) return inf;
+    const float pa = cfg.pt_max * sqrtf(bin * (1.0f / kEfaBins));
+    const float pb = cfg.pt_max * sqrtf((bin + 1) * (1.0f / kEfaBins));
+    const float uT2 = p.u1 * p.u1 + p.u2 * p.u2;
+    const float uT = sqrtf(uT2), g = sqrtf(1.0f + uT2);
+    // the minimum over the bin: E is convex in pT, least (m) at pT = m u_T
+    const float ps = p.m * uT;
+    const float at = fminf(fmaxf(ps, pa), pb);
+    const float mTb = sqrtf(p.m * p.m + pb * pb);
+    const float ch = coshf(cfg.yme_range);
+    const float eps_e = 2e-6f * (mTb * ch * (p.u0 + fabsf(p.u3)) + pb * uT);
+    const float eps_s = 2e-6f * p.tau * (mTb * ch * (fabsf(p.da0) + fabsf(p.da3) / p.tau) +
+                                         pb * (fabsf(p.da1) + fabsf(p.da2)));
+    const float E = g * sqrtf(p.m * p.m + at * at) - uT * at - eps_e;
+    const float x = (E - p.mu) / p.T;
+    if (p.sign == -1 && !(x > 0.01f)) return inf;
+    const float ex = expf(x);
+    if (!(E >= p.T * (1.0f + (p.sign == 1 ? 1.0f / ex : 0.0f)))) return inf;
+    return 1.01f * (1.0f + fabsf(cfg.df_max_ratio)) * (E * p.dsig + eps_s) / ((ex + p.sign) * p.bmax);
+}
+
+// Words x and w of the Philox block (t, i, eg, c3) for many t: the halves of the
+// first two rounds that do not see t are formed once
+struct EfaStream {
+    uint32_t a0, a1, h0, l0;   // after round 1: x, y; round 2's products of x
+};
+__device__ __forceinline__ EfaStream efa_stream(uint32_t i, uint32_t eg, uint32_t k0) {
+    EfaStream s;
+    s.a0 = __umulhi(0xCD9E8D57u, eg) ^ i ^ k0;
+    s.a1 = 0xCD9E8D57u * eg;
+    s.h0 = __umulhi(0xD2511F53u, s.a0);
+    s.l0 = 0xD2511F53u * s.a0;
+    return s;
+}
+// The round keys are the same for every proposal of a call: forming them costs
+// as many instructions as the rounds' xors, so a lane makes kEfaUnroll
+// proposals (t, t + 32, ...) side by side.
+constexpr int kEfaUnroll = 4;
+constexpr int kEfaBatch = 24;   // queued proposals that are evaluated together, at least
+__device__ __forceinline__ uint2 mul_wide(uint32_t a, uint32_t b) {   // low, high
+    const unsigned long long p = static_cast<unsigned long long>(a) * b;
+    return make_uint2(static_cast<uint32_t>(p), static_cast<uint32_t>(p >> 32));
+}
+__device__ __forceinline__ void efa_words(const EfaStream& s, uint32_t t, uint32_t c3, uint32_t k0, uint32_t k1,
+                                          uint32_t (&x)[kEfaUnroll], uint32_t (&w)[kEfaUnroll]) {
+    uint4 c[kEfaUnroll];
+    const uint32_t k1_1 = k1;
+    k0 += 0x9E3779B9u;
+    k1 += 0xBB67AE85u;
+#pragma unroll
+    for (int j = 0; j < kEfaUnroll; j++) {
+        const uint2 p = mul_wide(0xD2511F53u, t + 32u * j);
+        const uint2 q = mul_wide(0xCD9E8D57u, p.y ^ c3 ^ k1_1);
+        c[j] = make_uint4(q.y ^ s.a1 ^ k0, q.x, s.h0 ^ p.x ^ k1, s.l0);
+    }
+#pragma unroll
+    for (int r = 2; r < 10; r++) {
+        k0 += 0x9E3779B9u;
+        k1 += 0xBB67AE85u;
+#pragma unroll
+        for (int j = 0; j < kEfaUnroll; j++) {
+            const uint2 p = mul_wide(0xD2511F53u, c[j].x);
+            const uint2 q = mul_wide(0xCD9E8D57u, c[j].z);
+            c[j] = make_uint4(q.y ^ c[j].y ^ k0, q.x, p.y ^ c[j].w ^ k1, p.x);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kEfaUnroll; j++) {
+        x[j] = c[j].x;
+        w[j] = c[j].w;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1905,13 +1994,17 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
 
 // The lab-frame sampler (MC_sampling = 2).  A hadron takes about 1,900
 // proposals on average and up to max_tries x (max_redraws + 1), so one hadron
-// belongs to a whole warp: the 32 lanes make proposals t .. t + 31 and the
-// first accepted one (lowest counter) is the hadron, which is the draw a single
-// lane would have made one by one.  A lane per hadron, as the FSSW kernel has
-// it, left the chip waiting for the few lanes with the longest chains: 50,000
-// cells, 40 events, 213,000 hadrons took 194 ms and now take 8.2 ms.  The
-// kernel is bound by instruction issue (Philox, the hyperbolic functions and
-// the exponential of every proposal).
+// belongs to a whole warp: the 32 lanes make proposals t .. t + 31, those that
+// the bound of their pT bin does not reject are queued, and whenever 32 are
+// queued the warp evaluates them; the first accepted one (lowest counter) is
+// the hadron, which is the draw a single lane would have made one by one.  A
+// lane per hadron, as the FSSW kernel has it, left the chip waiting for the few
+// lanes with the longest chains: 50,000 cells, 40 events, 213,000 hadrons took
+// 194 ms; 2.84 ms with every proposal evaluated, 1.87 so.  The kernel is bound
+// by instruction issue: Philox, the bounds' look-up and the queue for each
+// proposal, and some 3,000 instructions per hadron for its cell's maximum and
+// the queue's evaluations.  (Bins in pT^2 and y, 64 to 256 of them, reject more
+// but cost more to form: 2.1 ms.)
 template <bool kLcc>
 __global__ void __launch_bounds__(kSampleThreads, 4)
 efa_sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict__ species,
@@ -1927,6 +2020,8 @@ efa_sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restr
     const int lane = threadIdx.x & 31;
     unsigned long long n_tries = 0;
     unsigned n_redraws = 0, n_fail = 0, n_viol = 0;   // warp-uniform
+    __shared__ uint32_t s_queue[kSampleThreads / 32][32 * (kEfaUnroll + 1)];
+    uint32_t* queue = s_queue[threadIdx.x >> 5];
     for (;;) {
         long long k = 0;
         if (lane == 0) k = k_begin + static_cast<long long>(atomicAdd(work_counter, 1ull));
@@ -1949,25 +2044,58 @@ efa_sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restr
             const uint32_t i = static_cast<uint32_t>(d);
             uint32_t t = 0;               // proposals of this hadron so far (counter)
             int redraw = 0, tries_cell = 0;
+            const uint32_t c3 = static_cast<uint32_t>(s) | (kTagEfa << 16);
+            const EfaStream stream = efa_stream(i, eg, cfg.key0);
             // up to `limit` proposals from counter t; the accepted one is emitted
             const auto propose = [&](const PropEfa& p, int l, int limit, int phase) {
-                for (int b0 = 0; b0 < limit; b0 += 32) {
-                    float4 pl;
-                    float u_rap;
-                    bool viol = false;
-                    const bool ok = b0 + lane < limit &&
-                                    try_efa(cfg, p, t + static_cast<uint32_t>(b0 + lane), i, eg, s, pl, u_rap, viol);
-                    const unsigned hit = __ballot_sync(FULL, ok);
-                    const int made = hit ? __ffs(hit) : min(32, limit - b0);
-                    n_viol += __popc(__ballot_sync(FULL, viol && lane < made));
-                    n_tries += made;
-                    if (hit) {
-                        if (lane == made - 1)
-                            emit_efa(cfg, cells, p, l, phase ? -pid : pid, pl, u_rap, out, slot + phase);
-                        t += static_cast<uint32_t>(b0 + made);
-                        return true;
+                const float bound = efa_bin_bound(cfg, p, lane);
+                int queued = 0;
+                for (int b0 = 0; b0 < limit; b0 += 32 * kEfaUnroll) {
+                    uint32_t x[kEfaUnroll], w[kEfaUnroll];
+                    const uint32_t t0 = t + static_cast<uint32_t>(b0 + lane);
+                    efa_words(stream, t0, c3, cfg.key0, cfg.key1, x, w);
+#pragma unroll
+                    for (int j = 0; j < kEfaUnroll; j++) {
+                        const float bnd = __shfl_sync(FULL, bound, static_cast<int>(x[j] >> 27));
+                        const bool keep = b0 + 32 * j + lane < limit && !(u01f(w[j]) >= bnd);
+                        const unsigned kept = __ballot_sync(FULL, keep);
+                        if (keep) queue[queued + __popc(kept & ((1u << lane) - 1u))] = t0 + 32u * j;
+                        queued += __popc(kept);
                     }
+                    __syncwarp();
+                    // evaluate the queue when it is worth a warp's while, at the end
+                    // all of it (a hadron found late has cost proposals too many)
+                    const int enough = b0 + 32 * kEfaUnroll < limit ? kEfaBatch : 1;
+                    int head = 0;
+                    for (; queued - head >= enough; head += 32) {
+                        float4 pl;
+                        float u_rap;
+                        bool viol = false;
+                        const bool on = head + lane < queued;
+                        const uint32_t mine = on ? queue[head + lane] : 0u;
+                        const bool ok = on && try_efa(cfg, p, mine, i, eg, s, pl, u_rap, viol);
+                        const unsigned hit = __ballot_sync(FULL, ok);
+                        const int made = hit ? __ffs(hit) : 32;
+                        n_viol += __popc(__ballot_sync(FULL, viol && lane < made));
+                        if (hit) {
+                            if (lane == made - 1)
+                                emit_efa(cfg, cells, p, l, phase ? -pid : pid, pl, u_rap, out, slot + phase);
+                            const uint32_t next = __shfl_sync(FULL, mine, made - 1) + 1u;
+                            n_tries += next - t;
+                            t = next;
+                            return true;
+                        }
+                    }
+                    if (head > 0) {
+                        const int left = max(queued - head, 0);   // < kEfaBatch
+                        const uint32_t keep = lane < left ? queue[head + lane] : 0u;
+                        __syncwarp();
+                        if (lane < left) queue[lane] = keep;
+                        queued = left;
+                    }
+                    __syncwarp();
                 }
+                n_tries += limit;
                 t += static_cast<uint32_t>(limit);
                 return false;
             };

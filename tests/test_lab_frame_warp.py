@@ -98,8 +98,37 @@ def test_any_cap_gives_the_same_hadrons(lcc):
     s, ref, off = sample(local_charge_conservation=lcc)
     tries = s.timings()["n_tries"]
     assert len(ref) > 100
-    for cap in (1, 31, 32, 33, 1000):
+    for cap in (1, 31, 32, 33, 127, 128, 129, 1000):
         s, had, o = sample(local_charge_conservation=lcc, gpu_max_tries=cap)
         assert had.tobytes() == ref.tobytes() and np.array_equal(o, off), cap
         assert s.timings()["n_tries"] == tries
         assert cap > 1000 or s.timings()["n_cell_redraws"] > 0
+
+
+@pytest.mark.parametrize("density,bulk", [(0, 0), (1, 0), (0, 1)])
+def test_bulk_rejection_changes_nothing(density, bulk):
+    """The bound that rejects proposals in bulk scales with the cap of delta f: a
+    cap of 1e6 rejects none.  Where |delta f| stays below 1 anyway (shear and
+    bulk scaled down a thousandfold) the cap itself changes nothing, so both
+    must sample the same hadrons: moving and space-like cells, bosons and
+    fermions, with and without chemical potentials."""
+    make = S.finite_density_3d if density else S.viscous_3d
+    fo = make(700, seed=14).fo_surf()
+    fo[:, 19:30] *= 1e-3
+    ref = None
+    for cap in (1.0, 1e6):
+        s = iSS(".", inputfile="")
+        s.set_params(**dict(S.DEFAULT_PARAMETERS, hydro_mode=2, afterburner_type=2 if density else 0,
+                            include_deltaf_shear=1, include_deltaf_bulk=bulk, bulk_deltaf_kind=1,
+                            quantum_statistics=1, number_of_repeated_sampling=20, MC_sampling=2,
+                            restrict_deltaf=1, deltaf_max_ratio=cap, sample_pT_up_to=-1,
+                            sample_y_minus_eta_s_range=Y_RANGE))
+        s.set_surface(fo)
+        s.set_random_seed(8)
+        s.generate_samples()
+        had = s.all_hadrons()[0].copy()
+        tries = s.timings()["n_tries"]
+        assert len(had) > 500
+        if ref is None:
+            ref, ref_tries = had, tries
+    assert had.tobytes() == ref.tobytes() and tries == ref_tries
