@@ -194,6 +194,7 @@ struct iss_handle {
     // the learned proposal: network, training set, per-pair mixture tables
     Learned learned;
     bool use_learned = false;            // gpu_sampler = 1
+    bool want_records = false;           // the generates of iss_gpu_learned_train
     DevBuf<int32_t> d_lslot, d_lspecies, d_spid;
     DevBuf<float> d_lpairs;
     iss_learned_stats_t lstats{};
@@ -635,8 +636,8 @@ iss_status prepare(iss_handle* h) {
     c.tab.b14_nmu = h->b14.nmu;
     c.tab.b14_T0 = h->b14.T0;
     c.tab.b14_mu0 = h->b14.mu0;
-    c.tab.b14_dT = h->b14.dT;
-    c.tab.b14_dmu = h->b14.dmu;
+    c.tab.b14_rdT = 1.0 / h->b14.dT;
+    c.tab.b14_rdmu = 1.0 / h->b14.dmu;
     c.tab.ce = h->d_ce.ptr;
     c.tab.qmu = h->d_qmu.ptr;
 
@@ -688,7 +689,9 @@ CellArrays cell_arrays(iss_handle* h) {
     a.pi1 = b + 5 * n;
     a.pi2 = b + 6 * n;
     a.coef = b + 7 * n;
-    a.rec = b + 8 * n;   // 128-byte records, 128-byte aligned
+    // 128-byte records, 128-byte aligned: for the samplers without the lean
+    // records, and the learned proposal's features and training rows
+    a.rec = h->cfg.mc_sampling == 2 || h->cfg.compat_fermion || h->use_learned || h->want_records ? b + 8 * n : nullptr;
     a.srec = b + 16 * n;  // the lean sampler's 128-byte records
     a.milne = h->cfg.mc_sampling == 2 ? h->d_milne.ptr : nullptr;
     return a;
@@ -1104,7 +1107,8 @@ std::vector<unsigned char> graph_key_of(iss_handle* h) {
     const unsigned char* pb = reinterpret_cast<const unsigned char*>(ptrs);
     k.insert(k.end(), pb, pb + sizeof(ptrs));
     const int64_t nums[] = {h->n_cells, h->n_tiles, h->cdf_len, h->guide_len, h->graph_cap_units,
-                            h->graph_cap_items, h->num_sms, static_cast<int64_t>(h->gh_events)};
+                            h->graph_cap_items, h->num_sms, static_cast<int64_t>(h->gh_events),
+                            static_cast<int64_t>(h->want_records)};
     const unsigned char* nb = reinterpret_cast<const unsigned char*>(nums);
     k.insert(k.end(), nb, nb + sizeof(nums));
     const unsigned char* tb = reinterpret_cast<const unsigned char*>(&h->tune);
@@ -2484,7 +2488,9 @@ iss_status iss_gpu_learned_train(iss_handle* h, const iss_learned_train_t* opt, 
         h->seed = saved_seed;
         h->seed_set = saved_seed_set;
         h->samples_valid = false;
+        h->want_records = false;
     };
+    h->want_records = true;
     h->params.set("gpu_sampler", 0);
     h->params.set("perform_decays", 0);
     h->params.set("sample_upto_desired_particle_number", 0);

@@ -18,7 +18,7 @@ struct DevTables {
     const double* b14c1;
     const double* b14c2;
     int b14_nT, b14_nmu;
-    double b14_T0, b14_mu0, b14_dT, b14_dmu;
+    double b14_T0, b14_mu0, b14_rdT, b14_rdmu;   // first entries, 1 / steps
     const double* ce;       // NEoS-BQS Chapman-Enskog, 200 * 200 rows of 5
     const double* qmu;      // RTA diffusion coefficient, 150 * 100
     const double* logfact;  // [kLogFactLen] log(k!) from the C library's lgamma

@@ -43,6 +43,24 @@ __device__ __forceinline__ ff ff_add(ff a, ff b) {
     s.lo += t.lo;
     return ff_quick_two_sum(s.hi, s.lo);
 }
+// a + b with a float b: what ff_add(a, ff_of(b)) returns, without its steps
+// on the zero low part (adding 0 and renormalising a normal pair change nothing)
+__device__ __forceinline__ ff ff_add_f(ff a, float b) {
+    const ff s = ff_two_sum(a.hi, b);
+    return ff_quick_two_sum(s.hi, s.lo + a.lo);
+}
+// the float nearest to a + b: the high part of ff_add, which ends normal
+__device__ __forceinline__ float ff_add_float(ff a, ff b) {
+    ff s = ff_two_sum(a.hi, b.hi);
+    const ff t = ff_two_sum(a.lo, b.lo);
+    s.lo += t.hi;
+    s = ff_quick_two_sum(s.hi, s.lo);
+    return s.hi + (s.lo + t.lo);
+}
+__device__ __forceinline__ float ff_add_f_float(ff a, float b) {
+    const ff s = ff_two_sum(a.hi, b);
+    return s.hi + (s.lo + a.lo);
+}
 __device__ __forceinline__ ff ff_neg(ff a) { return ff{-a.hi, -a.lo}; }
 __device__ __forceinline__ ff ff_sub(ff a, ff b) { return ff_add(a, ff_neg(b)); }
 
@@ -66,7 +84,7 @@ __device__ __forceinline__ ff ff_div(ff a, ff b) {
     r = ff_sub(r, ff_mul_f(b, q2));
     const float q3 = r.hi / b.hi;
     const ff q = ff_quick_two_sum(q1, q2);
-    return ff_add(q, ff_of(q3));
+    return ff_add_f(q, q3);
 }
 
 // sqrt(a), a > 0: one Newton step from the float root (Karp-Markstein form)

@@ -26,29 +26,32 @@ namespace {
 
 constexpr int kPrologueThreads = 128;
 
+// bilinear in (T, muB).  One FP64 division, the table's steps as reciprocals:
+// a division is about ten FP64 instructions, and the FP64 pipe bounds this
+// kernel (see below).
 __device__ void bulk14_coeff(const DevTables& t, double T, double muB, double* out) {
-    const int idx_T = static_cast<int>((T - t.b14_T0) / t.b14_dT);
-    const int idx_mu = static_cast<int>((muB - t.b14_mu0) / t.b14_dmu);
-    const double xf = (T - t.b14_T0) / t.b14_dT - idx_T;
-    const double yf = (muB - t.b14_mu0) / t.b14_dmu - idx_mu;
+    const double x = (T - t.b14_T0) * t.b14_rdT, y = (muB - t.b14_mu0) * t.b14_rdmu;
+    const int idx_T = static_cast<int>(x);
+    const int idx_mu = static_cast<int>(y);
+    const double xf = x - idx_T;
+    const double yf = y - idx_mu;
     const int nT = t.b14_nT, nmu = t.b14_nmu;
     const int iT1 = min(max(idx_T, 0), nT - 1), iT2 = min(max(idx_T + 1, 0), nT - 1);
     const int im1 = min(max(idx_mu, 0), nmu - 1), im2 = min(max(idx_mu + 1, 0), nmu - 1);
+    const double w1 = (1. - xf) * (1. - yf), w2 = (1. - xf) * yf, w3 = xf * yf, w4 = xf * (1. - yf);
     const double* tabs[3] = {t.b14c0, t.b14c1, t.b14c2};
     double v[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const double* tb = tabs[k];
-        const double f1 = tb[iT1 * nmu + im1], f2 = tb[iT1 * nmu + im2];
-        const double f3 = tb[iT2 * nmu + im2], f4 = tb[iT2 * nmu + im1];
-        v[k] = f1 * (1. - xf) * (1. - yf) + f2 * (1. - xf) * yf + f3 * xf * yf +
-               f4 * xf * (1. - yf);
+        v[k] = fma(tb[iT2 * nmu + im1], w4,
+                   fma(tb[iT2 * nmu + im2], w3, fma(tb[iT1 * nmu + im2], w2, tb[iT1 * nmu + im1] * w1)));
     }
-    const double T3 = T * T * T;
-    const double T4 = T3 * T;
-    out[0] = (v[0] - v[2]) / T4;
-    out[1] = v[1] / T3;
-    out[2] = (4. * v[2] - v[0]) / T4;
+    const double T2 = T * T;
+    const double r = 1.0 / (T2 * T2);
+    out[0] = (v[0] - v[2]) * r;
+    out[1] = v[1] * (T * r);
+    out[2] = fma(4., v[2], -v[0]) * r;
 }
 
 // polynomial fits of FSSW::getbulkvisCoefficients(T), bulk_deltaf_kind 1
@@ -99,17 +102,28 @@ __device__ void ce_neos_coeff(const double* tb, double Edec, double nB, double* 
 }
 
 __device__ double qmu_coeff(const double* tb, double T, double muB) {
-    const int idx_T = static_cast<int>((T - 0.05) / 0.001);
-    const int idx_mu = static_cast<int>((muB - 0.0) / 0.007892);
-    const double xf = (T - 0.05) / 0.001 - idx_T;
-    const double yf = (muB - 0.0) / 0.007892 - idx_mu;
+    const double x = (T - 0.05) * (1. / 0.001), y = muB * (1. / 0.007892);
+    const int idx_T = static_cast<int>(x);
+    const int idx_mu = static_cast<int>(y);
+    const double xf = x - idx_T;
+    const double yf = y - idx_mu;
     if (idx_mu > 98 || idx_T > 148 || idx_mu < 0 || idx_T < 0) return 1e30;
     const double f1 = tb[idx_T * 100 + idx_mu], f2 = tb[idx_T * 100 + idx_mu + 1];
     const double f3 = tb[(idx_T + 1) * 100 + idx_mu + 1], f4 = tb[(idx_T + 1) * 100 + idx_mu];
     return f1 * (1. - xf) * (1. - yf) + f2 * (1. - xf) * yf + f3 * xf * yf + f4 * xf * (1. - yf);
 }
 
-__global__ void __launch_bounds__(kPrologueThreads)
+// Bound by the FP64 pipe (two lanes per SM and clock: at 200,000 cells 975,000
+// warp instructions of cosh, sinh and the coefficient lookups took 50 of 108 us)
+// and by the serial float-float sums.  Hence one expm1 for cosh and sinh, one
+// division in the 14-moment lookup, the sums that round to float after each term
+// without the steps that cannot change that float (ff_add_f_float), the products
+// that several components share taken once, and the 128-byte records written
+// only where a kernel reads them: 200,000 cells 108 -> 65 us, 100,000 cells of a
+// baryon-rich surface 68 -> 50 us.  Unrolling the sums' outer loops as well costs
+// more in instruction fetch than it saves; 4 to 8 blocks per SM measure the same
+// at one wave, and 8 are 10 % faster over several (16 surfaces, 75 -> 68 us).
+__global__ void __launch_bounds__(kPrologueThreads, 8)
 cell_prologue_kernel(DevConfig cfg, const float* __restrict__ fo34, int64_t n, CellArrays cells) {
     __shared__ float s_rec[kPrologueThreads * 34];
     const int64_t base = static_cast<int64_t>(blockIdx.x) * kPrologueThreads;
@@ -132,7 +146,7 @@ cell_prologue_kernel(DevConfig cfg, const float* __restrict__ fo34, int64_t n, C
     // reference's order (C++ promotes a float product to double only after
     // rounding it to float).
     const float u0 = ff_to_float(ff_sqrt(
-        ff_add(ff_add(ff_two_sum(1.0f, u1 * u1), ff_of(u2 * u2)), ff_of(u3 * u3))));
+        ff_add_f(ff_add_f(ff_two_sum(1.0f, u1 * u1), u2 * u2), u3 * u3)));
     const float q0 = ((u1 * q1 + u2 * q2 + u3 * q3) / u0);
     {
         const float g[4] = {-1.f, 1.f, 1.f, 1.f};
@@ -148,7 +162,7 @@ cell_prologue_kernel(DevConfig cfg, const float* __restrict__ fo34, int64_t n, C
             t = ff_add(t, ff_two_prod(u[2], W[2][i]));
             udp[i] = ff_add(t, ff_two_prod(u[3], W[3][i]));
         }
-        const ff tr = ff_add(ff_add(ff_two_sum(-W[0][0], W[1][1]), ff_of(W[2][2])), ff_of(W[3][3]));
+        const ff tr = ff_add_f(ff_add_f(ff_two_sum(-W[0][0], W[1][1]), W[2][2]), W[3][3]);
         ff udpdu = ff_of(0.0f);
         for (int i = 0; i < 4; i++)
             for (int j = 0; j < 4; j++)
@@ -159,49 +173,59 @@ cell_prologue_kernel(DevConfig cfg, const float* __restrict__ fo34, int64_t n, C
         const int jj[10] = {0, 1, 2, 3, 1, 2, 3, 2, 3, 3};
         for (int k = 0; k < 10; k++) {
             const int i = ii[k], j = jj[k];
-            const float gij = (i == j) ? g[i] : 0.0f;
             const ff uu = ff_two_prod(u[i], u[j]);
-            ff v = ff_add(ff_of(W[i][j]), ff_mul_f(udp[j], u[i]));
+            const ff delta = (i == j) ? ff_add_f(uu, g[i]) : uu;
+            ff v = ff_add_f(ff_mul_f(udp[j], u[i]), W[i][j]);
             v = ff_add(v, ff_mul_f(udp[i], u[j]));
             v = ff_add(v, ff_mul(uu, udpdu));
-            v = ff_sub(v, ff_mul(ff_mul(third, ff_add(ff_of(gij), uu)), trsum));
-            pi[k] = ff_to_float(v);
+            pi[k] = ff_add_float(v, ff_neg(ff_mul(ff_mul(third, delta), trsum)));
         }
     }
 
     // transform_to_local_rest_frame (cosh and sinh of the double eta, rounded
-    // to float, stay in FP64: every later rounding point depends on them)
-    const float ch = static_cast<float>(cosh(static_cast<double>(eta)));
-    const float sh = static_cast<float>(sinh(static_cast<double>(eta)));
+    // to float, stay in FP64: every later rounding point depends on them).
+    // Both from one expm1 and one division, with E = e^|eta| - 1:
+    // cosh = 1 + E^2 / (2 (E + 1)), |sinh| = (E + E / (E + 1)) / 2; 3.8e8 random
+    // eta in [-12, 12] round to the same floats as cosh() and sinh().
+    const double em = expm1(fabs(static_cast<double>(eta)));
+    const double er = em > 1e300 ? 1.0 : em / (em + 1.0);
+    const float ch = static_cast<float>(1.0 + 0.5 * em * er);
+    const float sh = static_cast<float>(copysign(0.5 * (em + er), static_cast<double>(eta)));
     const float ut = u0 * ch + u3 * sh;
     const float uz = u3 * ch + u0 * sh;
     const float ux = u1, uy = u2;
     const ff den = ff_two_sum(ut, 1.0f);
-    const ff Lxx = ff_add(ff_of(1.0f), ff_div(ff_of(ux * ux), den));
-    const ff Lyy = ff_add(ff_of(1.0f), ff_div(ff_of(uy * uy), den));
-    const ff Lzz = ff_add(ff_of(1.0f), ff_div(ff_of(uz * uz), den));
+    const ff Lxx = ff_add_f(ff_div(ff_of(ux * ux), den), 1.0f);
+    const ff Lyy = ff_add_f(ff_div(ff_of(uy * uy), den), 1.0f);
+    const ff Lzz = ff_add_f(ff_div(ff_of(uz * uz), den), 1.0f);
     const ff Lxy = ff_div(ff_of(ux * uy), den);
     const ff Lxz = ff_div(ff_of(ux * uz), den);
     const ff Lyz = ff_div(ff_of(uy * uz), den);
-    const ff L[4][4] = {{ff_of(ut), ff_of(-ux), ff_of(-uy), ff_of(-uz)},
-                        {ff_of(-ux), Lxx, Lxy, Lxz},
-                        {ff_of(-uy), Lxy, Lyy, Lyz},
-                        {ff_of(-uz), Lxz, Lyz, Lzz}};
+    // the boost: row and column 0 are floats (f0), the space part Ls is float-float
+    const float f0[4] = {ut, -ux, -uy, -uz};
+    const ff Ls[3][3] = {{Lxx, Lxy, Lxz}, {Lxy, Lyy, Lyz}, {Lxz, Lyz, Lzz}};
+    // row i of the boost times a float vector, rounded to float after each term
+    const auto boost = [&](int i, const float* v) {
+        float x = ff_add_f_float(ff_two_prod(f0[i], v[0]), 0.0f);
+#pragma unroll
+        for (int j = 1; j < 4; j++)
+            x = ff_add_f_float(i == 0 ? ff_two_prod(f0[j], v[j]) : ff_mul_f(Ls[i - 1][j - 1], v[j]), x);
+        return x;
+    };
     const float da_up[4] = {tau * da0 * ch - da3 * sh, -tau * da1, -tau * da2,
                             -da3 * ch + tau * da0 * sh};
-    float dl[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++) dl[i] = ff_to_float(ff_add(ff_of(dl[i]), ff_mul_f(L[i][j], da_up[j])));
+    float dl[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) dl[i] = boost(i, da_up);
     const float qt[4] = {q0 * ch + q3 * sh, q1, q2, q3 * ch + q0 * sh};
-    float ql[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++) ql[i] = ff_to_float(ff_add(ff_of(ql[i]), ff_mul_f(L[i][j], qt[j])));
+    float ql[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) ql[i] = boost(i, qt);
     float pt[4][4];
     // 2. * pi * ch * sh is a double product in the reference; the float terms
     // around it are rounded to float first
-    pt[0][0] = ff_to_float(ff_add(ff_add(ff_of(pi[0] * ch * ch),
-                                         ff_mul_f(ff_two_prod(2.0f * pi[3], ch), sh)),
-                                  ff_of(pi[9] * sh * sh)));
+    pt[0][0] = ff_add_f_float(ff_add_f(ff_mul_f(ff_two_prod(2.0f * pi[3], ch), sh),
+                                       pi[0] * ch * ch), pi[9] * sh * sh);
     pt[0][1] = pi[1] * ch + pi[6] * sh;
     pt[0][2] = pi[2] * ch + pi[8] * sh;
     pt[0][3] = (pi[0] * ch * sh + pi[3] * (ch * ch + sh * sh) + pi[9] * sh * ch);
@@ -216,19 +240,26 @@ cell_prologue_kernel(DevConfig cfg, const float* __restrict__ fo34, int64_t n, C
     pt[3][0] = pt[0][3];
     pt[3][1] = pt[1][3];
     pt[3][2] = pt[2][3];
-    pt[3][3] = ff_to_float(ff_add(ff_add(ff_of(pi[0] * sh * sh),
-                                         ff_mul_f(ff_two_prod(2.0f * pi[3], sh), ch)),
-                                  ff_of(pi[9] * ch * ch)));
-    const int pi_i[5] = {1, 1, 1, 2, 2};
-    const int pi_j[5] = {1, 2, 3, 2, 3};
+    pt[3][3] = ff_add_f_float(ff_add_f(ff_mul_f(ff_two_prod(2.0f * pi[3], sh), ch),
+                                       pi[0] * sh * sh), pi[9] * ch * ch);
+    // pl = components 11 12 13 22 23 of L pt L, rounded to float after each term;
+    // the components of one row i share the products L[i][a] pt[a][b]
     float pl[5];
-    for (int k = 0; k < 5; k++) {
-        const int i = pi_i[k], j = pi_j[k];
-        float acc = 0.f;
+#pragma unroll
+    for (int i = 1; i < 3; i++) {
+        float acc[3] = {0.f, 0.f, 0.f};
+#pragma unroll
         for (int a = 0; a < 4; a++)
-            for (int b = 0; b < 4; b++)
-                acc = ff_to_float(ff_add(ff_of(acc), ff_mul(ff_mul_f(L[i][a], pt[a][b]), L[b][j])));
-        pl[k] = acc;
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const ff f = a == 0 ? ff_two_prod(f0[i], pt[a][b]) : ff_mul_f(Ls[i - 1][a - 1], pt[a][b]);
+#pragma unroll
+                for (int j = i; j < 4; j++)
+                    acc[j - 1] = ff_add_f_float(b == 0 ? ff_mul_f(f, f0[j]) : ff_mul(f, Ls[b - 1][j - 1]),
+                                                acc[j - 1]);
+            }
+#pragma unroll
+        for (int j = i; j < 4; j++) pl[(i - 1) * 2 + j - 1] = acc[j - 1];
     }
 
     if (cells.milne) {
@@ -242,14 +273,20 @@ cell_prologue_kernel(DevConfig cfg, const float* __restrict__ fo34, int64_t n, C
         m[4] = make_float4(pi[8], pi[9], q0, q1);
         m[5] = make_float4(q2, q3, s[29], 0.0f);
     }
-    float4* rec = cells.rec + 8 * l;
-    rec[0] = cells.pos[l] = make_float4(tau, xpt, ypt, eta);
-    rec[1] = cells.da[l] = make_float4(dl[0], -dl[1], -dl[2], -dl[3]);
-    rec[2] = cells.u[l] = make_float4(ut, ux, uy, uz);
-    rec[3] = cells.th[l] = make_float4(Tdec, s[16], s[17], s[18]);
-    rec[4] = cells.th2[l] = make_float4(Edec, Pdec, Bn, s[29]);
-    rec[5] = cells.pi1[l] = make_float4(pl[0], pl[1], pl[2], pl[3]);
-    rec[6] = cells.pi2[l] = make_float4(pl[4], ql[1], ql[2], ql[3]);
+    const float4 vpos = make_float4(tau, xpt, ypt, eta);
+    const float4 vda = make_float4(dl[0], -dl[1], -dl[2], -dl[3]);
+    const float4 vu = make_float4(ut, ux, uy, uz);
+    const float4 vth = make_float4(Tdec, s[16], s[17], s[18]);
+    const float4 vth2 = make_float4(Edec, Pdec, Bn, s[29]);
+    const float4 vp1 = make_float4(pl[0], pl[1], pl[2], pl[3]);
+    const float4 vp2 = make_float4(pl[4], ql[1], ql[2], ql[3]);
+    cells.pos[l] = vpos;
+    cells.da[l] = vda;
+    cells.u[l] = vu;
+    cells.th[l] = vth;
+    cells.th2[l] = vth2;
+    cells.pi1[l] = vp1;
+    cells.pi2[l] = vp2;
 
     double c[3] = {0.0, 0.0, 0.0};
     double kappa = 1.0;
@@ -260,17 +297,23 @@ cell_prologue_kernel(DevConfig cfg, const float* __restrict__ fo34, int64_t n, C
         else if (cfg.bulk_kind == 1) bulk_rta_coeff(Tdec, c);
     }
     if (cfg.include_diff) kappa = qmu_coeff(cfg.tab.qmu, Tdec, s[16]);
-    rec[7] = cells.coef[l] = make_float4(static_cast<float>(c[0]), static_cast<float>(c[1]),
-                                         static_cast<float>(c[2]), static_cast<float>(kappa));
+    const float4 vcoef = make_float4(static_cast<float>(c[0]), static_cast<float>(c[1]),
+                                     static_cast<float>(c[2]), static_cast<float>(kappa));
+    cells.coef[l] = vcoef;
+    if (cells.rec) {
+        float4* rec = cells.rec + 8 * l;
+        rec[0] = vpos;
+        rec[1] = vda;
+        rec[2] = vu;
+        rec[3] = vth;
+        rec[4] = vth2;
+        rec[5] = vp1;
+        rec[6] = vp2;
+        rec[7] = vcoef;
+    }
     if (cells.srec) {
         // the lean sampler's per-cell constants, from the record's floats
-        const float4 da = make_float4(dl[0], -dl[1], -dl[2], -dl[3]);
-        const float4 th = make_float4(Tdec, s[16], s[17], s[18]);
-        const float4 th2 = make_float4(Edec, Pdec, Bn, s[29]);
-        const float4 p1 = make_float4(pl[0], pl[1], pl[2], pl[3]);
-        const float4 p2 = make_float4(pl[4], ql[1], ql[2], ql[3]);
-        const float4 cf = make_float4(static_cast<float>(c[0]), static_cast<float>(c[1]),
-                                      static_cast<float>(c[2]), static_cast<float>(kappa));
+        const float4 da = vda, th = vth, th2 = vth2, p1 = vp1, p2 = vp2, cf = vcoef;
         const float T = th.x;
         const float d0 = fabsf(da.x);
         float D = sqrtf(da.y * da.y + da.z * da.z + da.w * da.w);
