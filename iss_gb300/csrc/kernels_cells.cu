@@ -552,8 +552,8 @@ __device__ __forceinline__ TileRef tile_ref(const SurfSeg* __restrict__ surf, in
     TileRef r;
     r.sg = surf + lo;
     r.b = lo;
-    const int64_t local = t - r.sg->tile_base;
-    r.k = static_cast<int>(local / r.sg->nt);
+    const int64_t local = t - r.sg->tile_base;   // below 2^31: a tile is a block of a grid
+    r.k = static_cast<int>(static_cast<uint32_t>(local) / static_cast<uint32_t>(r.sg->nt));
     r.tile = local - static_cast<int64_t>(r.k) * r.sg->nt;
     if (r.k >= S) r.k = S - 1;   // not reached: the grid has exactly the batch's tiles
     return r;
@@ -576,31 +576,91 @@ __device__ __forceinline__ void load_tile(const uint32_t* __restrict__ row, int6
     }
 }
 
+constexpr int kSumThreads = 128;
+constexpr int kSumRuns = kCdfTile / kSumThreads;   // runs of a warp
+
+// Sums over the warp of the quantised yields of kSumRuns runs (32 cells each,
+// one per lane): the sum of run `lane`, of the last run in the lanes past it.
+// q = floor(y 2^s) (cdf_quantize) with s = 188 - L - exponent(ymax), in limbs of
+// 23 bits: y times 2^s less the low limbs is exact (what a denormal loses is
+// below 1); adding 2^23 rounded down leaves the floor in the mantissa, and the
+// rest goes on to the next limb.  q < 2^(62 - L), so two limbs hold it from
+// L = 16 on and three always.  The float bits are summed as they are, modulo
+// 2^32: 32 limbs add up below 2^28, 32 exponents of 2^23 to kExp.
+template <int kLimbs>
+__device__ __forceinline__ unsigned long long warp_runs(float* y, int s) {
+    constexpr float kTwo23 = 8388608.0f;
+    constexpr uint32_t kExp = 0x60000000u;   // 32 * 0x4B000000
+    int e = s - 23 * (kLimbs - 1);
+    if (e < -126 || e > 127) {
+        const int e1 = e / 2;
+        const float f1 = __uint_as_float(static_cast<uint32_t>(127 + e1) << 23);
+#pragma unroll
+        for (int k = 0; k < kSumRuns; k++) y[k] *= f1;
+        e -= e1;
+    }
+    const float f = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+    const int lane = threadIdx.x & 31;
+    uint32_t mine[kLimbs];
+#pragma unroll
+    for (int k = 0; k < kSumRuns; k++) {
+        const float t = y[k] * f;
+        float a = __fadd_rz(t, kTwo23), r = t - (a - kTwo23);
+#pragma unroll
+        for (int j = kLimbs - 1; j >= 0; j--) {
+            const uint32_t sum = __reduce_add_sync(0xffffffffu, __float_as_uint(a));
+            mine[j] = lane >= k ? sum : mine[j];
+            if (j == 0) break;
+            a = __fmaf_rz(r, kTwo23, kTwo23);
+            if (j > 1) r = fmaf(r, kTwo23, kTwo23 - a);
+        }
+    }
+    unsigned long long q = mine[kLimbs - 1] - kExp;
+#pragma unroll
+    for (int j = kLimbs - 2; j >= 0; j--) q = (q << 23) + (mine[j] - kExp);
+    return q;
+}
+
 // Sum of every tile, and inside it the prefix sums of its runs of kCdfSub
-// cells, which are what the cell draws of sparse rows search.
-__global__ void __launch_bounds__(kScanThreads)
+// cells, which are what the cell draws of sparse rows search.  A warp reads
+// kSumRuns runs, a cell per lane, and only the first warp goes on to the prefix
+// sums of the tile.  Bound by memory (64 M yields of 200,000 cells: 255 MB, 48 us)
+// once the integer work is out of the way: quantising each yield by shifts of
+// 64 bits and scanning them in shared memory, eight cells per thread, took 91 us;
+// warps of eight runs instead of sixteen, which repeat the tile's look-up twice
+// as often, 55 us.  16 surfaces of 225,000 cells together: 126 -> 71 us.
+__global__ void __launch_bounds__(kSumThreads)
 cdf_tile_sum_kernel(const float* __restrict__ yields, int64_t N, const SurfSeg* __restrict__ surf,
                     int n_surf, int S, const uint32_t* __restrict__ ymax,
                     unsigned long long* __restrict__ tile_sum, unsigned long long* __restrict__ sub) {
-    __shared__ uint32_t s_in[kScanThreads * (kScanPer + 1)];
-    __shared__ unsigned long long s_warp[33];
+    static_assert(kCdfSub == 32 && kCdfSubs == 64 && kSumRuns * kSumThreads == kCdfTile, "a run per warp load");
+    __shared__ __align__(16) unsigned long long s_run[kCdfSubs];
     const TileRef tr = tile_ref(surf, n_surf, S, blockIdx.x);
-    const int64_t n = tr.sg->n;
-    const uint32_t* row =
-        reinterpret_cast<const uint32_t*>(yields + static_cast<int64_t>(tr.k) * N + tr.sg->c0);
-    const int base = cdf_quant_base(ymax[tr.b * S + tr.k], tr.sg->L);
-    load_tile(row, tr.tile * kScanTile, n, s_in);
-    __syncthreads();
-    const uint32_t* mine = s_in + threadIdx.x * (kScanPer + 1);
-    unsigned long long acc = 0;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int64_t i0 = tr.tile * kScanTile + wid * (kSumRuns * 32) + lane;
+    const int64_t left = tr.sg->n - i0;
+    const float* row = yields + static_cast<int64_t>(tr.k) * N + tr.sg->c0 + i0;
+    float y[kSumRuns];
+    if (left > (kSumRuns - 1) * 32) {
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) acc += cdf_quantize(mine[k], base);
-    unsigned long long tot;
-    const unsigned long long ex = block_excl_scan_u64(acc, s_warp, &tot);
-    constexpr int kPerRun = kCdfSub / kScanPer;   // threads per run
-    if (threadIdx.x % kPerRun == 0)
-        sub[static_cast<int64_t>(blockIdx.x) * kCdfSubs + threadIdx.x / kPerRun] = ex;
-    if (threadIdx.x == 0) tile_sum[blockIdx.x] = tot;
+        for (int k = 0; k < kSumRuns; k++) y[k] = __ldg(row + k * 32);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kSumRuns; k++) y[k] = k * 32 < left ? __ldg(row + k * 32) : 0.0f;
+    }
+    const int L = tr.sg->L;
+    const int s = 150 + cdf_quant_base(ymax[tr.b * S + tr.k], L);
+    const unsigned long long q = L >= 16 ? warp_runs<2>(y, s) : warp_runs<3>(y, s);
+    if (lane < kSumRuns) s_run[wid * kSumRuns + lane] = q;
+    __syncthreads();
+    if (wid != 0) return;
+    const unsigned long long a = s_run[2 * lane], b = s_run[2 * lane + 1];
+    const unsigned long long inc = warp_incl_scan_u64(a + b);
+    ulonglong2 out;
+    out.x = inc - (a + b);
+    out.y = out.x + a;
+    reinterpret_cast<ulonglong2*>(sub + static_cast<int64_t>(blockIdx.x) * kCdfSubs)[lane] = out;
+    if (lane == 31) tile_sum[blockIdx.x] = inc;
 }
 
 // one block per row (b, k): exclusive scan of the row's tile sums, the row
@@ -806,7 +866,7 @@ cudaError_t launch_cdf_head(const float* yields, int64_t N, const SurfSeg* surf,
     if (n_tiles <= 0 || S <= 0 || n_surf <= 0) return cudaSuccess;
     const int rows = n_surf * S;
     const unsigned grid = static_cast<unsigned>(n_tiles);
-    cdf_tile_sum_kernel<<<grid, kScanThreads, 0, stream>>>(yields, N, surf, n_surf, S, ymax, b.tile_sum, b.sub);
+    cdf_tile_sum_kernel<<<grid, kSumThreads, 0, stream>>>(yields, N, surf, n_surf, S, ymax, b.tile_sum, b.sub);
     cdf_tile_offset_kernel<<<rows, kScanThreads, 0, stream>>>(
         surf, S, b.tile_sum, ymax, ymult, allow_sparse && n_tiles >= kSparseTiles, b.tile_off, b.qtot, b.sparse,
         b.totals, b.cdf, b.guide);
