@@ -26,9 +26,17 @@ double string_to_double(const std::string& s) {
 }
 
 long ParamStore::find(const std::string& key) const {
-    const std::string k = to_lower(trim(key));
+    // trimmed and lower case like the stored keys, without a copy (a call looks
+    // some fifty keys up)
+    size_t b = 0, e = key.size();
+    while (b < e && std::isspace(static_cast<unsigned char>(key[b]))) b++;
+    while (e > b && std::isspace(static_cast<unsigned char>(key[e - 1]))) e--;
     for (size_t i = 0; i < items_.size(); i++) {
-        if (items_[i].first == k) return static_cast<long>(i);
+        const std::string& k = items_[i].first;
+        if (k.size() != e - b) continue;
+        size_t j = 0;
+        while (j < k.size() && k[j] == static_cast<char>(std::tolower(static_cast<unsigned char>(key[b + j])))) j++;
+        if (j == k.size()) return static_cast<long>(i);
     }
     return -1;
 }
