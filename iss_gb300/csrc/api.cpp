@@ -343,7 +343,9 @@ std::vector<float4> yield_list(const std::vector<SpeciesDev>& sd, int* n_groups,
         });
         group_runs.push_back(static_cast<int32_t>(run_members.size()));
         for (size_t i = 0; i < g.size(); i++) {
-            if (i == 0 || !same_run(g[i - 1], g[i])) run_members.push_back(static_cast<int32_t>(member.size()));
+            if (i == 0 || !same_run(g[i - 1], g[i]) ||
+                static_cast<int32_t>(member.size()) - run_members.back() == kRunMembers)
+                run_members.push_back(static_cast<int32_t>(member.size()));
             member.push_back(g[i]);
         }
     }
@@ -354,18 +356,28 @@ std::vector<float4> yield_list(const std::vector<SpeciesDev>& sd, int* n_groups,
     group_runs.push_back(R);
     run_members.push_back(S);
     std::vector<float4> out(static_cast<size_t>(yield_list_float4(S, G, R)), float4{0.f, 0.f, 0.f, 0.f});
-    for (int t = 0; t < S; t++) {
-        const SpeciesDev& s = sd[static_cast<size_t>(member[t])];
-        out[static_cast<size_t>(t)] = float4{static_cast<float>(s.baryon), static_cast<float>(s.strange),
-                                             static_cast<float>(s.charge), s.degen};
-    }
     for (int g = 0; g < G; g++) {
         const SpeciesDev& s = sd[static_cast<size_t>(groups[static_cast<size_t>(g)][0])];
         const YieldGroup yg{s.m_hi, s.m_lo, s.sign, s.light};
         static_assert(sizeof(YieldGroup) == sizeof(float4), "a group is one float4");
-        std::memcpy(&out[static_cast<size_t>(S + g)], &yg, sizeof(yg));
+        std::memcpy(&out[static_cast<size_t>(g)], &yg, sizeof(yg));
     }
-    int32_t* tail = reinterpret_cast<int32_t*>(out.data() + S + G);
+    for (int r = 0; r < R; r++) {
+        const int t0 = run_members[static_cast<size_t>(r)], k = run_members[static_cast<size_t>(r) + 1] - t0;
+        const SpeciesDev& s = sd[static_cast<size_t>(member[static_cast<size_t>(t0)])];
+        uint32_t id[kRunMembers];
+        for (int i = 0; i < kRunMembers; i++)
+            id[i] = i < k ? static_cast<uint32_t>(member[static_cast<size_t>(t0 + i)]) & 0xFFFFu : 0xFFFFu;
+        const YieldRun yr{static_cast<float>(s.baryon), s.degen, id[0] | id[1] << 16, id[2] | id[3] << 16};
+        static_assert(sizeof(YieldRun) == sizeof(float4) && kRunMembers == 4, "a run is one float4");
+        std::memcpy(&out[static_cast<size_t>(G + r)], &yr, sizeof(yr));
+    }
+    for (int t = 0; t < S; t++) {
+        const SpeciesDev& s = sd[static_cast<size_t>(member[t])];
+        out[static_cast<size_t>(G + R + t)] = float4{static_cast<float>(s.baryon), static_cast<float>(s.strange),
+                                                     static_cast<float>(s.charge), s.degen};
+    }
+    int32_t* tail = reinterpret_cast<int32_t*>(out.data() + G + R + S);
     tail = std::copy(group_runs.begin(), group_runs.end(), tail);
     tail = std::copy(run_members.begin(), run_members.end(), tail);
     std::copy(member.begin(), member.end(), tail);
@@ -716,6 +728,7 @@ CellArrays cell_arrays(iss_handle* h) {
     // records, and the learned proposal's features and training rows
     a.rec = h->cfg.mc_sampling == 2 || h->cfg.compat_fermion || h->use_learned || h->want_records ? b + 8 * n : nullptr;
     a.srec = b + 16 * n;  // the lean sampler's 128-byte records
+    a.beta = reinterpret_cast<float2*>(b + 24 * n);
     a.milne = h->cfg.mc_sampling == 2 ? h->d_milne.ptr : nullptr;
     return a;
 }
@@ -745,8 +758,8 @@ iss_status run_cells(iss_handle* h) {
                                     cudaMemcpyHostToDevice, st));
         h->surface_on_device = true;
     }
-    // 8 SoA arrays, the records and the lean sampler's records
-    CUDA_TRY(h, h->d_cells.reserve(static_cast<size_t>(n) * 24));
+    // 8 SoA arrays, the records, the lean sampler's records and 1/T
+    CUDA_TRY(h, h->d_cells.reserve(static_cast<size_t>(n) * 25));
     if (c.mc_sampling == 2) CUDA_TRY(h, h->d_milne.reserve(static_cast<size_t>(n) * 6));
     // (sparse_cell reads the yields 16 bytes at a time)
     CUDA_TRY(h, h->d_yields.reserve(static_cast<size_t>(n) * S + 4));

@@ -108,10 +108,17 @@ struct SpeciesDev {
 };
 
 // The yields kernel's list of species, group by group (species with the same
-// thermal series) and inside a group run by run (the same degeneracy and baryon
-// number): for every member (baryon number, strangeness, charge, degeneracy) as
-// floats; the groups; the G + 1 first runs of the groups; the R + 1 first
-// members of the runs; the members' species indices.
+// thermal series) and inside a group run by run (up to kRunMembers of the same
+// degeneracy and baryon number): the groups; the runs (YieldRun); for every
+// member (baryon number, strangeness, charge, degeneracy) as floats; the G + 1
+// first runs of the groups; the R + 1 first members of the runs; the members'
+// species indices.
+constexpr int kRunMembers = 4;
+constexpr int kMaxRunSpecies = 65535;   // species a YieldRun can name
+struct YieldRun {
+    float baryon, degen;
+    uint32_t m01, m23;       // species indices of the members, 16 bits each, 0xFFFF: none
+};
 struct YieldGroup {
     float m_hi, m_lo;        // FP64 mass as a float-float pair
     int sign, light;         // statistics; 1: ten series terms
@@ -120,7 +127,7 @@ struct YieldGroup {
 __host__ __device__
 #endif
 inline int yield_list_float4(int n_species, int n_groups, int n_runs) {
-    return n_species + n_groups + (n_groups + 1 + n_runs + 1 + n_species + 3) / 4;
+    return n_groups + n_runs + n_species + (n_groups + 1 + n_runs + 1 + n_species + 3) / 4;
 }
 
 // What a cell draw reads of the (surface, species) rows r = b S + k: the full
@@ -170,6 +177,7 @@ struct CellArrays {
     // float4 per cell: (da0..da3), (u0..u3), (pi00 pi01 pi02 pi03),
     // (pi11 pi12 pi13 pi22), (pi23 pi33 q0 q1), (q2 q3 bulkPi 0)
     float4* milne;
+    float2* beta;   // 1/T as a float-float pair
 };
 
 // Resonance decay table (particle_decay::read_resonances_list): particles

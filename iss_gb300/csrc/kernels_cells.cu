@@ -89,6 +89,7 @@ __device__ __forceinline__ GridPos grid_pos(float xh, float xl) {
 
 // ------------------------------------------------------------------------
 constexpr int kYieldThreads = 128;
+constexpr int64_t kTwoCellsFrom = 2500;
 constexpr int kYieldGroups = 4;   // species groups per cell (grid y)
 
 // Surface of cell l in a batch: the last b with surf[b].c0 <= l.
@@ -305,11 +306,11 @@ __device__ __forceinline__ CellYieldIn cell_yield_in(const DevConfig& cfg, const
     c.th2 = cells.th2[l];
     c.cf = cells.coef[l];
     const float T = c.th.x;
-    const double beta_d = 1.0 / static_cast<double>(T);
+    const float2 beta = cells.beta[l];
     c.T = T;
     c.da0 = da.x;
-    c.b_hi = static_cast<float>(beta_d);
-    c.b_lo = static_cast<float>(beta_d - static_cast<double>(c.b_hi));
+    c.b_hi = beta.x;
+    c.b_lo = beta.y;
     c.warm = T >= 0.05f;   // as double: T > 0.05 (0.05f is the first float above it)
     c.bulkPi = 0.0f;
     if (kBulk != kNoBulk) c.bulkPi = cfg.bulk_kind == 1 ? c.th2.w / kHbarCf : c.th2.w;
@@ -329,72 +330,28 @@ __device__ __forceinline__ CellYieldIn cell_yield_in(const DevConfig& cfg, const
     return c;
 }
 
-// Yields of every (cell, species) pair, one cell per thread.  A group's series
-// runs for its first member and is reused by the next members while their
-// chemical potential in this cell is the same; a member with another mu gets
-// its own series.  In a warp whose cells have no strangeness and charge
-// potential, mu and with it the yield is the same for the whole run, so a
-// run costs one multiply-add and one maximum, and a member only its store.
-//
-// Besides the yields, the kernel raises ymax[b S + k] to the largest yield of
-// species k on surface b (its float bits: yields are >= +0, so the unsigned
-// order of the bits is the order of the values; ymax starts at 0): through a
-// per-block maximum in shared memory when the block's cells lie on one surface,
-// else lane by lane.
-//
-// Series with an argument off the special-function tables (x < 0.5: pions
-// above 0.27 GeV; x > 399.95) are left at zero and flagged, for
-// yields_off_table_kernel: the FP64 evaluation, inlined here, had its set-up
-// run for every term of every cell.
-//
-// Bound by instruction issue (about 80 % of the issue slots): some 100 one-term
-// and 5 ten-term series per cell, and 319 stores.  200,000 cells, 319 species,
-// 14-moment bulk: 228 us (345 with the FP64 set-up in the loop, the bulk form
-// tested in every term and a multiply-add and a maximum per member); 100,000
-// cells, 400 species with diffusion: 246 us (590).  7 and 6 blocks per SM:
-// 8 and 5 spill or leave warps out (244 and 265 us).
-// kDiff: include_deltaf_diffusion (a separate instantiation, so the common
-// case carries none of the diffusion series' registers).
+// The yields of cell l (a lane's; past the last cell the lane only takes part)
+// for the groups of row blockIdx.y, whatever the chemical potentials and the
+// surfaces of the warp's cells: b is the block's surface, or -1 where it has
+// several.
 template <int kBulk, bool kDiff>
-__global__ void __launch_bounds__(kYieldThreads, kDiff ? 6 : 7)
-yields_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yields, uint32_t* __restrict__ ymax,
-              uint32_t* __restrict__ off_table) {
-    extern __shared__ float4 s_dyn[];
-    __shared__ int s_b[2];
-    const int nsp = cfg.n_species;
-    const int G = cfg.n_ygroups, R = cfg.n_yruns;
-    // the yield list (YieldGroup) as it is, then the members' and runs' maxima
-    const int words4 = yield_list_float4(nsp, G, R);
-    uint32_t* s_max = reinterpret_cast<uint32_t*>(s_dyn + words4);
-    uint32_t* s_rmax = s_max + nsp;
-    const float4* s_q = s_dyn;
-    const YieldGroup* s_g = reinterpret_cast<const YieldGroup*>(s_dyn + nsp);
-    const int32_t* s_gst = reinterpret_cast<const int32_t*>(s_dyn + nsp + G);
-    const int32_t* s_rst = s_gst + G + 1;
-    const int32_t* s_mem = s_rst + R + 1;
+__device__ __forceinline__ void yields_any(const DevConfig& cfg, const CellArrays& cells, float* __restrict__ yields,
+                                        uint32_t* __restrict__ ymax, uint32_t* __restrict__ off_table, int64_t l,
+                                        int b, const YieldGroup* s_g, const int32_t* s_gst,
+                                        const float4* s_q, const int32_t* s_rst, const int32_t* s_mem,
+                                        uint32_t* s_rmax, uint32_t* s_max) {
+    const int nsp = cfg.n_species, G = cfg.n_ygroups;
     const int64_t n = cfg.n_cells;
-    const int64_t first = static_cast<int64_t>(blockIdx.x) * kYieldThreads;
-    for (int k = threadIdx.x; k < words4; k += kYieldThreads) s_dyn[k] = cfg.ylist[k];
-    for (int k = threadIdx.x; k < nsp + R; k += kYieldThreads) s_max[k] = 0u;
-    if (threadIdx.x < 2) {
-        const int64_t lb = threadIdx.x == 0 ? first : min(first + kYieldThreads, n) - 1;
-        s_b[threadIdx.x] = surface_of(cfg.surf, cfg.n_surfaces, lb);
-    }
-    __syncthreads();
-    const bool one_surface = s_b[0] == s_b[1];
-    const int64_t l = first + threadIdx.x;
+    const bool one_surface = b >= 0;
     const bool valid = l < n;
     const int64_t lc = valid ? l : 0;   // lanes past the last cell read cell 0 and store nothing
     const float4 da = cells.da[lc];
     const bool live = valid && !(da.x < 0.0f);
     const CellYieldIn c = cell_yield_in<kBulk, kDiff>(cfg, cells, lc, da);
     uint32_t* ymax_row = ymax + static_cast<int64_t>(
-        one_surface ? s_b[0] : surface_of(cfg.surf, cfg.n_surfaces, valid ? l : n - 1)) * nsp;
+        one_surface ? b : surface_of(cfg.surf, cfg.n_surfaces, valid ? l : n - 1)) * nsp;
     float* out = yields + l;
     const bool by_run = __all_sync(0xffffffffu, c.th.z == 0.0f && c.th.w == 0.0f);
-    // blockIdx.y picks every gridDim.y-th species group: the groups come in
-    // decreasing order of work, so interleaving keeps the rows' work equal,
-    // and the grid has several waves of blocks
     for (int g = blockIdx.y; g < G; g += gridDim.y) {
         const YieldGroup gr = s_g[g];
         const int r0 = s_gst[g], r1 = s_gst[g + 1];
@@ -434,12 +391,164 @@ yields_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yields, uint3
             }
         }
     }
+}
+
+// Yields of every (cell, species) pair, kCells cells per thread.  A group's
+// series runs for its first run and is reused by the next ones while their
+// chemical potential is the same in the warp's cells.  In a warp whose cells
+// have no strangeness and charge potential (and lie, with the block's others, on
+// one surface) mu and with it the yield is the same for a whole run: a run costs
+// one multiply-add and one maximum, a member only its store.  Other warps take
+// yields_any, where each member forms its mu.
+//
+// Besides the yields, the kernel raises ymax[b S + k] to the largest yield of
+// species k on surface b (its float bits: yields are >= +0, so the unsigned
+// order of the bits is the order of the values; ymax starts at 0): through a
+// per-block maximum in shared memory when the block's cells lie on one surface,
+// else lane by lane.
+//
+// Series with an argument off the special-function tables (x < 0.5: pions
+// above 0.27 GeV; x > 399.95) are left at zero and flagged, for
+// yields_off_table_kernel: the FP64 evaluation, inlined here, had its set-up
+// run for every term of every cell.
+//
+// Bound by instruction issue (75 % of the issue slots; 64 M of 136 M warp
+// instructions are the series of 200,000 cells): some 100 one-term and 5
+// ten-term series per cell, and 319 stores.  Two cells per thread share a run's
+// look-up, maximum and addresses; with 1/T from the prologue (its FP64 division
+// ran once per row of groups) and the runs as one 16-byte record each, 200,000
+// cells with 319 species and 14-moment bulk take 168 us (228 with a look-up per
+// member, 345 with the FP64 set-up in the loop).  Three cells measure the same,
+// four 4 us more, one cell 12 to 30 us more.  With diffusion, whose longer
+// series leave less to share, two cells gain nothing at 100,000 cells (231 us
+// either way; 246 and 590 before) and lose below (6,000 cells: 40 us, 34 with
+// one), so there is no such variant.  Where every cell has a strangeness and
+// charge potential 100,000 cells take 212 us, with diffusion 456 us.  7 blocks
+// per SM, 5 with diffusion: 6 and 5 take 172 and 182 us, 6 and 7 with
+// diffusion 237 us.
+// kDiff: include_deltaf_diffusion (a separate instantiation, so the common
+// case carries none of the diffusion series' registers).
+template <int kBulk, bool kDiff, int kCells>
+__global__ void __launch_bounds__(kYieldThreads, kDiff ? 5 : 7)
+yields_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yields, uint32_t* __restrict__ ymax,
+              uint32_t* __restrict__ off_table) {
+    extern __shared__ float4 s_dyn[];
+    __shared__ int s_b[2];
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int kBlockCells = kYieldThreads * kCells;
+    const int nsp = cfg.n_species;
+    const int G = cfg.n_ygroups, R = cfg.n_yruns;
+    // the yield list as it is, then the runs' and members' maxima; the members'
+    // own entries (s_q, s_rst, s_mem) are staged only in blocks that read them
+    const int words4 = yield_list_float4(nsp, G, R);
+    const YieldGroup* s_g = reinterpret_cast<const YieldGroup*>(s_dyn);
+    const float4* s_run = s_dyn + G;   // YieldRun
+    const float4* s_q = s_run + R;
+    const int32_t* s_gst = reinterpret_cast<const int32_t*>(s_q + nsp);
+    const int32_t* s_rst = s_gst + G + 1;
+    const int32_t* s_mem = s_rst + R + 1;
+    const int32_t* rst = reinterpret_cast<const int32_t*>(cfg.ylist + G + R + nsp) + G + 1;
+    const int32_t* mem = rst + R + 1;
+    uint32_t* s_rmax = reinterpret_cast<uint32_t*>(s_dyn + words4);
+    uint32_t* s_max = s_rmax + R;
+    const int64_t n = cfg.n_cells;
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * kBlockCells;
+    const int gst4 = G + R + nsp;      // the float4 of s_gst
+    for (int k = threadIdx.x; k < G + R; k += kYieldThreads) s_dyn[k] = cfg.ylist[k];
+    for (int k = gst4 + threadIdx.x; k < gst4 + (G + 4) / 4; k += kYieldThreads) s_dyn[k] = cfg.ylist[k];
+    for (int k = threadIdx.x; k < nsp + R; k += kYieldThreads) s_rmax[k] = 0u;
+    if (threadIdx.x < 2) {
+        const int64_t lb = threadIdx.x == 0 ? first : min(first + kBlockCells, n) - 1;
+        s_b[threadIdx.x] = surface_of(cfg.surf, cfg.n_surfaces, lb);
+    }
+    __syncthreads();
+    const bool one_surface = s_b[0] == s_b[1];
+    // a warp's cells are consecutive, a lane's 32 apart
+    const int64_t l0 = first + (threadIdx.x >> 5) * (32 * kCells) + (threadIdx.x & 31);
+    CellYieldIn c[kCells];
+    bool live[kCells];
+    bool usual = one_surface && first + kBlockCells <= n && n < (int64_t(1) << 30) && nsp <= kMaxRunSpecies;
+#pragma unroll
+    for (int j = 0; j < kCells; j++) {
+        const int64_t l = min(l0 + 32 * j, n - 1);
+        const float4 da = cells.da[l];
+        live[j] = !(da.x < 0.0f);
+        c[j] = cell_yield_in<kBulk, kDiff>(cfg, cells, l, da);
+        usual = usual && c[j].th.z == 0.0f && c[j].th.w == 0.0f;
+    }
+    if (__syncthreads_or(!usual)) {
+        for (int k = G + R + threadIdx.x; k < words4; k += kYieldThreads) s_dyn[k] = cfg.ylist[k];
+        __syncthreads();
+    }
+    // blockIdx.y picks every gridDim.y-th species group: the groups come in
+    // decreasing order of work, so interleaving keeps the rows' work equal,
+    // and the grid has several waves of blocks
+    if (__all_sync(FULL, usual)) {
+        // the usual warp: mu is B muB for all its cells, so the loop over the
+        // runs has no branch that lanes take apart
+        const uint32_t row_bytes = static_cast<uint32_t>(n) * 4u;
+        char* const out_bytes = reinterpret_cast<char*>(yields + l0);
+        for (int g = blockIdx.y; g < G; g += gridDim.y) {
+            const YieldGroup gr = s_g[g];
+            const int r1 = s_gst[g + 1];
+            float2 xy[kCells];
+            float mu_of[kCells];   // mu of xy: none yet
+#pragma unroll
+            for (int j = 0; j < kCells; j++) mu_of[j] = __int_as_float(0x7fc00000);
+#pragma unroll 1
+            for (int r = s_gst[g]; r < r1; r++) {
+                const float4 run = s_run[r];   // YieldRun
+                bool other_mu = false;
+#pragma unroll
+                for (int j = 0; j < kCells; j++) other_mu = other_mu || run.x * c[j].th.y != mu_of[j];
+                if (__any_sync(FULL, other_mu)) {
+#pragma unroll
+                    for (int j = 0; j < kCells; j++) {
+                        bool off = false;
+                        mu_of[j] = run.x * c[j].th.y;
+                        xy[j] = yield_coefs<kBulk, kDiff>(
+                            c[j], gr, thermal_series<kBulk, kDiff, true>(cfg, c[j], gr, mu_of[j], off));
+                        if (off) {   // yields_off_table_kernel
+                            xy[j] = make_float2(0.0f, 0.0f);
+                            if (live[j]) *off_table = 1u;
+                        }
+                    }
+                }
+                const float4 q = make_float4(run.x, 0.0f, 0.0f, run.y);
+                float yv[kCells];
+                uint32_t m = 0u;
+#pragma unroll
+                for (int j = 0; j < kCells; j++) {
+                    yv[j] = live[j] ? member_yield(q, xy[j]) : 0.0f;
+                    m = max(m, __float_as_uint(yv[j]));
+                }
+                m = __reduce_max_sync(FULL, m);
+                if ((threadIdx.x & 31) == 0) atomicMax(s_rmax + r, m);
+                const uint32_t m01 = __float_as_uint(run.z), m23 = __float_as_uint(run.w);
+                const uint32_t id[kRunMembers] = {m01 & 0xFFFFu, m01 >> 16, m23 & 0xFFFFu, m23 >> 16};
+#pragma unroll
+                for (int i = 0; i < kRunMembers; i++) {
+                    if (i > 0 && id[i] == 0xFFFFu) continue;
+                    char* const at = out_bytes + static_cast<uint64_t>(id[i]) * row_bytes;
+#pragma unroll
+                    for (int j = 0; j < kCells; j++) reinterpret_cast<float*>(at)[32 * j] = yv[j];
+                }
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int j = 0; j < kCells; j++) {
+            const int64_t l = l0 + 32 * j;
+            yields_any<kBulk, kDiff>(cfg, cells, yields, ymax, off_table, l, one_surface ? s_b[0] : -1, s_g, s_gst,
+                                     s_q, s_rst, s_mem, s_rmax, s_max);
+        }
+    }
     if (one_surface) {
         __syncthreads();
         for (int r = threadIdx.x; r < R; r += kYieldThreads)
-            for (int t = s_rst[r]; t < s_rst[r + 1]; t++) {
+            for (int t = rst[r]; t < rst[r + 1]; t++) {
                 const uint32_t m = max(s_max[t], s_rmax[r]);
-                if (m) atomicMax(ymax_row + s_mem[t], m);
+                if (m) atomicMax(ymax + static_cast<int64_t>(s_b[0]) * nsp + mem[t], m);
             }
     }
 }
@@ -454,9 +563,9 @@ yields_off_table_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yie
     if (*off_table == 0u) return;
     const int nsp = cfg.n_species;
     const int G = cfg.n_ygroups;
-    const float4* list = cfg.ylist;
-    const YieldGroup* groups = reinterpret_cast<const YieldGroup*>(list + nsp);
-    const int32_t* gst = reinterpret_cast<const int32_t*>(list + nsp + G);
+    const YieldGroup* groups = reinterpret_cast<const YieldGroup*>(cfg.ylist);
+    const float4* list = cfg.ylist + G + cfg.n_yruns;
+    const int32_t* gst = reinterpret_cast<const int32_t*>(list + nsp);
     const int32_t* rst = gst + G + 1;
     const int32_t* mem = rst + cfg.n_yruns + 1;
     const int64_t n = cfg.n_cells;
@@ -823,7 +932,11 @@ cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, float* 
     cudaError_t e0 = cudaMemsetAsync(ymax, 0, sizeof(uint32_t) * (rows + 1), stream);
     if (e0 != cudaSuccess) return e0;
     if (cfg.n_cells <= 0) return cudaSuccess;
-    const unsigned blocks = static_cast<unsigned>((cfg.n_cells + kYieldThreads - 1) / kYieldThreads);
+    // two cells per thread once a row of blocks is more than the groups can
+    // spread over the chip (3,000 cells: 22 us, 24 with one; 1,245 cells: 22 and 18)
+    const int per_thread = !cfg.include_diff && cfg.n_cells >= kTwoCellsFrom ? 2 : 1;
+    const int64_t block_cells = kYieldThreads * per_thread;
+    const unsigned blocks = static_cast<unsigned>((cfg.n_cells + block_cells - 1) / block_cells);
     const size_t smem = sizeof(float4) * static_cast<size_t>(yield_list_float4(cfg.n_species, cfg.n_ygroups,
                                                                                cfg.n_yruns)) +
                         sizeof(uint32_t) * static_cast<size_t>(cfg.n_species + cfg.n_yruns);
@@ -831,26 +944,28 @@ cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, float* 
                      : (cfg.bulk_kind == 1 || cfg.bulk_kind == 21) ? kBulkCe
                      : cfg.bulk_kind == 11 ? kBulk14 : kNoBulk;
     using Kernel = void (*)(DevConfig, CellArrays, float*, uint32_t*, uint32_t*);
-    const Kernel kernels[3][2] = {{yields_kernel<kNoBulk, false>, yields_kernel<kNoBulk, true>},
-                                  {yields_kernel<kBulkCe, false>, yields_kernel<kBulkCe, true>},
-                                  {yields_kernel<kBulk14, false>, yields_kernel<kBulk14, true>}};
+    const Kernel kernels[3][3] = {
+        {yields_kernel<kNoBulk, false, 1>, yields_kernel<kNoBulk, false, 2>, yields_kernel<kNoBulk, true, 1>},
+        {yields_kernel<kBulkCe, false, 1>, yields_kernel<kBulkCe, false, 2>, yields_kernel<kBulkCe, true, 1>},
+        {yields_kernel<kBulk14, false, 1>, yields_kernel<kBulk14, false, 2>, yields_kernel<kBulk14, true, 1>}};
     using OffKernel = void (*)(DevConfig, CellArrays, float*, uint32_t*, const uint32_t*);
     const OffKernel off_kernels[3][2] = {
         {yields_off_table_kernel<kNoBulk, false>, yields_off_table_kernel<kNoBulk, true>},
         {yields_off_table_kernel<kBulkCe, false>, yields_off_table_kernel<kBulkCe, true>},
         {yields_off_table_kernel<kBulk14, false>, yields_off_table_kernel<kBulk14, true>}};
-    const Kernel kernel = kernels[bulk][cfg.include_diff ? 1 : 0];
+    const Kernel kernel = kernels[bulk][cfg.include_diff ? 2 : per_thread - 1];
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem));
         if (e != cudaSuccess) return e;
     }
-    // rows of species groups: as tuned, more where that leaves fewer than three
-    // waves of 7 blocks per SM (a call of 1.1 waves runs two: 37,211 cells took
-    // 80 us in 4 rows, 62 us so; 1,245 cells 41 and 18 us).  More waves repeat
-    // the cells' set-up too often (5, 8 and 12 waves: 64, 70 and 78 us).
-    int want = cfg.yield_groups > 0 ? cfg.yield_groups : kYieldGroups;
-    want = std::max(want, static_cast<int>((static_cast<int64_t>(num_sms) * 21 + blocks - 1) / blocks));
+    // rows of species groups: as tuned (per 128 cells), more where that leaves
+    // fewer than three waves of blocks (16 per SM of two cells per thread, 21 of
+    // one): a call of 1.1 waves runs two, and more waves repeat the cells' set-up
+    // too often (45,000 cells in 12, 16, 26 and 40 blocks per SM: 63, 59, 61 and
+    // 63 us; 12,000 cells 30, 30, 36 and 38 us).
+    int want = per_thread * (cfg.yield_groups > 0 ? cfg.yield_groups : kYieldGroups);
+    want = std::max(want, static_cast<int>((static_cast<int64_t>(num_sms) * (per_thread == 2 ? 16 : 21) + blocks - 1) / blocks));
     const unsigned groups = static_cast<unsigned>(std::max(1, std::min(want, cfg.n_ygroups)));
     kernel<<<dim3(blocks, groups), kYieldThreads, smem, stream>>>(cfg, cells, yields, ymax, off_table);
     off_kernels[bulk][cfg.include_diff ? 1 : 0]<<<dim3(std::min(blocks, 2u * static_cast<unsigned>(num_sms)), 4), kYieldThreads, 0, stream>>>(

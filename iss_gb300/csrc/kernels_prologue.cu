@@ -119,7 +119,8 @@ __device__ double qmu_coeff(const double* tb, double T, double muB) {
 // division in the 14-moment lookup, the sums that round to float after each term
 // without the steps that cannot change that float (ff_add_f_float), the products
 // that several components share taken once, and the 128-byte records written
-// only where a kernel reads them: 200,000 cells 108 -> 65 us, 100,000 cells of a
+// only where a kernel reads them: 200,000 cells 108 -> 65 us (69 with the FP64 1/T
+// of the yields, which costs them more), 100,000 cells of a
 // baryon-rich surface 68 -> 50 us.  Unrolling the sums' outer loops as well costs
 // more in instruction fetch than it saves; 4 to 8 blocks per SM measure the same
 // at one wave, and 8 are 10 % faster over several (16 surfaces, 75 -> 68 us).
@@ -285,6 +286,11 @@ cell_prologue_kernel(DevConfig cfg, const float* __restrict__ fo34, int64_t n, C
     cells.u[l] = vu;
     cells.th[l] = vth;
     cells.th2[l] = vth2;
+    {
+        const double beta_d = 1.0 / static_cast<double>(Tdec);
+        const float hi = static_cast<float>(beta_d);
+        cells.beta[l] = make_float2(hi, static_cast<float>(beta_d - static_cast<double>(hi)));
+    }
     cells.pi1[l] = vp1;
     cells.pi2[l] = vp2;
 
