@@ -98,10 +98,11 @@ struct iss_handle {
     // decay work buffers (grow-only): one generation's records (ping-pong),
     // the per-input arrays of all generations, per-(generation, event) tables
     // and the final lists
-    DevBuf<HadronRec> dk_u[2], dk_final;
+    DevBuf<HadronRec> dk_u, dk_final;
     DevBuf<int32_t> dk_ev, dk_pid, dk_chan, dk_etot;
-    DevBuf<int64_t> dk_cnt, dk_coff, dk_tiles, dk_first, dk_last, dk_scnt, dk_shift, dk_meta,
-        dk_off, dk_etiles, dk_evoff;
+    DevBuf<uint8_t> dk_cnt;
+    DevBuf<int64_t> dk_coff, dk_tiles, dk_first, dk_last, dk_shift, dk_meta,
+        dk_off, dk_etiles;
     DevBuf<unsigned long long> dk_fail;
     int64_t dk_scap_hint = 0, dk_ucap_hint = 0, dk_icap_hint = 0;   // sizes the last call needed
     int dk_gen_hint = 0;                           // generations the last call had
@@ -251,10 +252,11 @@ struct iss_handle {
             d_dchannels.release();
             d_dsorted.release();
             d_dhash.release();
-            for (auto* b : {&dk_u[0], &dk_u[1], &dk_final}) b->release();
+            for (auto* b : {&dk_u, &dk_final}) b->release();
             for (auto* b : {&dk_ev, &dk_pid, &dk_chan, &dk_etot}) b->release();
-            for (auto* b : {&dk_cnt, &dk_coff, &dk_tiles, &dk_first, &dk_last, &dk_scnt, &dk_shift,
-                            &dk_meta, &dk_off, &dk_etiles, &dk_evoff})
+            dk_cnt.release();
+            for (auto* b : {&dk_coff, &dk_tiles, &dk_first, &dk_last, &dk_shift,
+                            &dk_meta, &dk_off, &dk_etiles})
                 b->release();
             dk_fail.release();
             learned.release_all();
@@ -829,10 +831,41 @@ constexpr int kDecayBatch = 8;
 constexpr int64_t kGroupRecords = 256 << 10;
 constexpr int64_t kLearnedGroupRecords = 512 << 10;
 
-iss_status run_decays(iss_handle* h, unsigned long long* failures_out) {
-    DevConfig& c = h->cfg;
-    cudaStream_t s = h->stream;
-    const int E = c.n_events;
+// iss_gpu_generate_into with decays: event groups of the write sweep, of at
+// least so many sampled hadrons (some 1.7 records each) and not more than so
+// many groups (run_decays)
+constexpr int64_t kDecayGroupRecords = 256 << 10;
+constexpr int64_t kDecayGroups = 8;
+
+// the copy stream and at least n chunk events
+iss_status ensure_copy_stream(iss_handle* h, int n) {
+    if (!h->copy_stream) CUDA_TRY(h, cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
+    while (static_cast<int>(h->chunk_ev.size()) < n) {
+        cudaEvent_t e;
+        CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        h->chunk_ev.push_back(e);
+    }
+    return ISS_OK;
+}
+
+// sample_stream goes on from the stream's present work, and back
+iss_status fork_sample_stream(iss_handle* h) {
+    if (!h->sample_stream) {
+        CUDA_TRY(h, cudaStreamCreateWithFlags(&h->sample_stream, cudaStreamNonBlocking));
+        for (auto& e : h->ev_sample2) CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    CUDA_TRY(h, cudaEventRecord(h->ev_sample2[0], h->stream));
+    CUDA_TRY(h, cudaStreamWaitEvent(h->sample_stream, h->ev_sample2[0], 0));
+    return ISS_OK;
+}
+
+iss_status join_sample_stream(iss_handle* h) {
+    CUDA_TRY(h, cudaEventRecord(h->ev_sample2[1], h->sample_stream));
+    CUDA_TRY(h, cudaStreamWaitEvent(h->stream, h->ev_sample2[1], 0));
+    return ISS_OK;
+}
+
+iss_status decay_tables(iss_handle* h, DecayTablesDev* out) {
     if (h->decay_table_afterburner != h->afterburner) {
         DecayTable tab;
         std::string err;
@@ -885,151 +918,235 @@ iss_status run_decays(iss_handle* h, unsigned long long* failures_out) {
                                cudaMemcpyHostToDevice));
         h->decay_table_afterburner = h->afterburner;
     }
-    DecayTablesDev t;
+    DecayTablesDev& t = *out;
     t.particles = h->d_dparticles.ptr;
     t.channels = h->d_dchannels.ptr;
     t.sorted_pid = h->d_dsorted.ptr;
     t.sorted_idx = h->d_dsorted.ptr + h->n_decay_particles;
     t.hash = h->d_dhash.ptr;
     t.n_particles = h->n_decay_particles;
+    return ISS_OK;
+}
 
-    const int64_t n0 = h->n_hadrons;
+// The count sweep of a call: sizes and buffers, then what it found.
+struct DecayRun {
+    DecayTablesDev t{};
+    DecayBuffers b{};
+    int64_t n0 = 0;                       // sampled hadrons
+    int64_t s_cap = 0, u_cap = 0, i_cap = 0;
+    std::vector<int64_t> meta;
+    int g = 0;                            // generations enqueued
+    int n_gen = 0;                        // generations with inputs
+    int64_t total = 0;                    // hadrons of the final lists
+};
+
+// the scans add (stable << 32 | unstable) counts of at most 3 each: the
+// unstable half stays below 2^32 while a generation has < 2^32 / 3 inputs
+constexpr int64_t kMaxDecayInputs = (int64_t(1) << 32) / 3 - 1;
+
+// Enqueues the first batch of the count sweep on s: generation 0's inputs from
+// the segments' offsets, or with from_records their ids from the records.
+iss_status decays_enqueue(iss_handle* h, DecayRun* run, bool from_records, cudaStream_t s) {
+    DevConfig& c = h->cfg;
+    const int E = c.n_events, G = kDecayMaxGenerations;
+    const int64_t n0 = run->n0;
+    const size_t GE = static_cast<size_t>(G) * static_cast<size_t>(E);
+    run->u_cap = std::min(run->u_cap, kMaxDecayInputs);
+    run->i_cap = std::max(run->i_cap, n0);
+    const int64_t gen_cap = std::max(n0, run->u_cap);
+    CUDA_TRY(h, h->dk_u.reserve(static_cast<size_t>(std::max<int64_t>(run->i_cap - n0, 1))));
+    CUDA_TRY(h, h->dk_final.reserve(static_cast<size_t>(run->s_cap)));
+    CUDA_TRY(h, h->dk_ev.reserve(static_cast<size_t>(run->i_cap)));
+    CUDA_TRY(h, h->dk_pid.reserve(static_cast<size_t>(run->i_cap)));
+    CUDA_TRY(h, h->dk_chan.reserve(static_cast<size_t>(run->i_cap)));
+    CUDA_TRY(h, h->dk_coff.reserve(static_cast<size_t>(run->i_cap) + G + 1));
+    CUDA_TRY(h, h->dk_cnt.reserve(static_cast<size_t>(gen_cap)));
+    CUDA_TRY(h, h->dk_tiles.reserve(static_cast<size_t>(gen_cap / kDecayTile + 1)));
+    CUDA_TRY(h, h->dk_first.reserve(GE));
+    CUDA_TRY(h, h->dk_last.reserve(GE));
+    CUDA_TRY(h, h->dk_shift.reserve(GE));
+    CUDA_TRY(h, h->dk_meta.reserve(kDecayMetaLen));
+    CUDA_TRY(h, h->dk_off.reserve(static_cast<size_t>(E) + 1));
+    CUDA_TRY(h, h->dk_etot.reserve(static_cast<size_t>(E)));
+    CUDA_TRY(h, h->dk_etiles.reserve(static_cast<size_t>(std::max(offsets_num_tiles(E), 1))));
+    CUDA_TRY(h, h->dk_fail.reserve(1));
+
+    run->meta.assign(kDecayMetaLen, 0);
+    run->meta[kDecayMetaNIn] = n0;
+    CUDA_TRY(h, cudaMemcpyAsync(h->dk_meta.ptr, run->meta.data(), 8 * run->meta.size(), cudaMemcpyHostToDevice, s));
+    CUDA_TRY(h, cudaMemsetAsync(h->dk_fail.ptr, 0, sizeof(unsigned long long), s));
+
+    DecayBuffers& b = run->b;
+    b.ev = h->dk_ev.ptr;
+    b.pid = h->dk_pid.ptr;
+    b.chan = h->dk_chan.ptr;
+    b.cnt = h->dk_cnt.ptr;
+    b.off = h->dk_coff.ptr;
+    b.tiles = h->dk_tiles.ptr;
+    b.first = h->dk_first.ptr;
+    b.last = h->dk_last.ptr;
+    b.shift = h->dk_shift.ptr;
+    b.meta = h->dk_meta.ptr;
+    b.failures = h->dk_fail.ptr;
+    b.s_cap = run->s_cap;
+    b.u_cap = run->u_cap;
+    b.i_cap = run->i_cap;
+    b.g_max = static_cast<uint32_t>(G);
+    CUDA_TRY(h, launch_decay_inputs(c, h->d_species.ptr, h->d_pids.ptr, h->d_offsets.ptr,
+                                    from_records ? h->d_hadrons.ptr : nullptr, n0, b, h->num_sms, s));
+    // the first batch has as many generations as the last call had, so that a
+    // repeated workload waits once
+    run->g = 0;
+    const int batch = h->dk_gen_hint > 0 ? std::min(h->dk_gen_hint, kDecayBatch) : kDecayBatch;
+    for (int k = 0; k < batch && run->g < G; k++, run->g++)
+        CUDA_TRY(h, launch_decay_count_generation(c, run->t, static_cast<uint32_t>(run->g), b, E, h->num_sms, s));
+    return ISS_OK;
+}
+
+// Tables and first sizes, and the first batch: what the last call needed, else
+// gpu_decay_arena_factor (default 2.0) times the sampled hadrons for the final
+// lists, gpu_decay_next_factor (0.5) for one generation's records and the
+// sampled hadrons plus twice that for the inputs of all generations; too small
+// only costs a rerun of the count sweep
+iss_status decays_begin(iss_handle* h, DecayRun* run, int64_t n0, cudaStream_t s) {
+    iss_status st = decay_tables(h, &run->t);
+    if (st != ISS_OK) return st;
+    run->n0 = n0;
     h->dk_reruns = 0;
-    if (n0 <= 0 || E <= 0) {
-        *failures_out = 0;
-        return ISS_OK;
-    }
-    const int G = kDecayMaxGenerations;
-    // first sizes: what the last call needed, else gpu_decay_arena_factor
-    // (default 2.0) times the sampled hadrons for the final lists,
-    // gpu_decay_next_factor (0.5) for one generation's records and the
-    // sampled hadrons plus twice that for the inputs of all generations; too
-    // small only costs a rerun of the count sweep
+    if (n0 <= 0 || h->cfg.n_events <= 0) return ISS_OK;
     const double fa = h->params.get_or("gpu_decay_arena_factor", 2.0);
     const double fu = h->params.get_or("gpu_decay_next_factor", 0.5);
     if (!(fa > 0.0) || !(fu > 0.0))
         return fail(h, ISS_ERR_INVALID_ARG, "gpu_decay_arena_factor / gpu_decay_next_factor must be > 0");
-    int64_t s_cap = std::max<int64_t>(h->dk_scap_hint, static_cast<int64_t>(fa * static_cast<double>(n0)) + 64);
-    int64_t u_cap = std::max<int64_t>(h->dk_ucap_hint, static_cast<int64_t>(fu * static_cast<double>(n0)) + 64);
-    int64_t i_cap = std::max<int64_t>(h->dk_icap_hint, n0 + 2 * u_cap);
-    std::vector<int64_t> meta_h(kDecayMetaLen, 0);
-    // the scans add (stable << 32 | unstable) counts of at most 3 each: the
-    // unstable half stays below 2^32 while a generation has < 2^32 / 3 inputs
-    constexpr int64_t kMaxDecayInputs = (int64_t(1) << 32) / 3 - 1;
     if (n0 > kMaxDecayInputs)
         return fail(h, ISS_ERR_UNSUPPORTED, "resonance decays of more than %lld sampled hadrons",
                     static_cast<long long>(kMaxDecayInputs));
-    const size_t GE = static_cast<size_t>(G) * static_cast<size_t>(E);
+    run->s_cap = std::max<int64_t>(h->dk_scap_hint, static_cast<int64_t>(fa * static_cast<double>(n0)) + 64);
+    run->u_cap = std::max<int64_t>(h->dk_ucap_hint, static_cast<int64_t>(fu * static_cast<double>(n0)) + 64);
+    run->i_cap = std::max<int64_t>(h->dk_icap_hint, n0 + 2 * run->u_cap);
+    return decays_enqueue(h, run, false, s);
+}
+
+// The rest of the count sweep on s, with one wait (and a copy of the sizes) per
+// batch of generations, and the layout of the final lists, whose event offsets
+// go to eh->tail.
+iss_status decays_count(iss_handle* h, DecayRun* run, bool from_records, cudaStream_t s) {
+    DevConfig& c = h->cfg;
+    const int E = c.n_events, G = kDecayMaxGenerations;
+    std::vector<int64_t>& meta = run->meta;
     for (int attempt = 0;; attempt++) {
-        u_cap = std::min(u_cap, kMaxDecayInputs);
-        i_cap = std::max(i_cap, n0);
-        const int64_t gen_cap = std::max(n0, u_cap);
-        for (int k = 0; k < 2; k++) CUDA_TRY(h, h->dk_u[k].reserve(static_cast<size_t>(u_cap)));
-        CUDA_TRY(h, h->dk_final.reserve(static_cast<size_t>(s_cap)));
-        CUDA_TRY(h, h->dk_ev.reserve(static_cast<size_t>(i_cap)));
-        CUDA_TRY(h, h->dk_pid.reserve(static_cast<size_t>(i_cap)));
-        CUDA_TRY(h, h->dk_chan.reserve(static_cast<size_t>(i_cap)));
-        CUDA_TRY(h, h->dk_coff.reserve(static_cast<size_t>(i_cap) + G + 1));
-        CUDA_TRY(h, h->dk_cnt.reserve(static_cast<size_t>(gen_cap)));
-        CUDA_TRY(h, h->dk_tiles.reserve(static_cast<size_t>(gen_cap / 4096 + 1)));
-        CUDA_TRY(h, h->dk_first.reserve(GE));
-        CUDA_TRY(h, h->dk_last.reserve(GE));
-        CUDA_TRY(h, h->dk_scnt.reserve(GE));
-        CUDA_TRY(h, h->dk_shift.reserve(GE));
-        CUDA_TRY(h, h->dk_meta.reserve(kDecayMetaLen));
-        CUDA_TRY(h, h->dk_off.reserve(static_cast<size_t>(E) + 1));
-        CUDA_TRY(h, h->dk_evoff.reserve(static_cast<size_t>(E) + 1));
-        CUDA_TRY(h, h->dk_etot.reserve(static_cast<size_t>(E)));
-        CUDA_TRY(h, h->dk_etiles.reserve(static_cast<size_t>(std::max(offsets_num_tiles(E), 1))));
-        CUDA_TRY(h, h->dk_fail.reserve(1));
-
-        std::fill(meta_h.begin(), meta_h.end(), 0);
-        meta_h[kDecayMetaNIn] = n0;
-        CUDA_TRY(h, cudaMemcpyAsync(h->dk_meta.ptr, meta_h.data(), 8 * meta_h.size(),
-                                    cudaMemcpyHostToDevice, s));
-        CUDA_TRY(h, cudaMemsetAsync(h->dk_first.ptr, 0xFF, 8 * GE, s));
-        CUDA_TRY(h, cudaMemsetAsync(h->dk_last.ptr, 0xFF, 8 * GE, s));
-        CUDA_TRY(h, cudaMemsetAsync(h->dk_fail.ptr, 0, sizeof(unsigned long long), s));
-        CUDA_TRY(h, cudaMemcpyAsync(h->dk_evoff.ptr, h->event_offsets.data(), 8 * (static_cast<size_t>(E) + 1),
-                                    cudaMemcpyHostToDevice, s));
-
-        DecayBuffers b{};
-        b.rec0 = h->d_hadrons.ptr;
-        b.ev = h->dk_ev.ptr;
-        b.pid = h->dk_pid.ptr;
-        b.chan = h->dk_chan.ptr;
-        b.cnt = h->dk_cnt.ptr;
-        b.off = h->dk_coff.ptr;
-        b.tiles = h->dk_tiles.ptr;
-        b.first = h->dk_first.ptr;
-        b.last = h->dk_last.ptr;
-        b.scnt = h->dk_scnt.ptr;
-        b.shift = h->dk_shift.ptr;
-        b.meta = h->dk_meta.ptr;
-        b.failures = h->dk_fail.ptr;
-        b.s_cap = s_cap;
-        b.u_cap = u_cap;
-        b.i_cap = i_cap;
-        b.g_max = static_cast<uint32_t>(G);
-        CUDA_TRY(h, launch_decay_first_generation(h->dk_evoff.ptr, E, b, s));
-        // count sweep: batches of generations, one wait (and a copy of the
-        // sizes) per batch; the first batch has as many generations as the
-        // last call had, so that a repeated workload waits once
-        int g = 0;
-        int batch = h->dk_gen_hint > 0 ? std::min(h->dk_gen_hint, kDecayBatch) : kDecayBatch;
         for (;;) {
-            for (int k = 0; k < batch && g < G; k++, g++)
-                CUDA_TRY(h, launch_decay_count_generation(c, t, static_cast<uint32_t>(g), b, E, h->num_sms, s));
-            batch = kDecayBatch;
-            CUDA_TRY(h, cudaMemcpyAsync(meta_h.data(), h->dk_meta.ptr, 8 * meta_h.size(),
-                                        cudaMemcpyDeviceToHost, s));
+            CUDA_TRY(h, cudaMemcpyAsync(meta.data(), h->dk_meta.ptr, 8 * meta.size(), cudaMemcpyDeviceToHost, s));
             CUDA_TRY(h, cudaStreamSynchronize(s));
-            if (meta_h[kDecayMetaFlags] != 0 || meta_h[kDecayMetaNIn + g] == 0 || g >= G) break;
+            if (meta[kDecayMetaFlags] != 0 || meta[kDecayMetaNIn + run->g] == 0 || run->g >= G) break;
+            for (int k = 0; k < kDecayBatch && run->g < G; k++, run->g++)
+                CUDA_TRY(h, launch_decay_count_generation(c, run->t, static_cast<uint32_t>(run->g), run->b, E,
+                                                          h->num_sms, s));
         }
-        const int64_t flags = meta_h[kDecayMetaFlags];
+        const int64_t flags = meta[kDecayMetaFlags];
         if (flags & 4)
             return fail(h, ISS_ERR_SAMPLING, "decay chains longer than %d generations", G);
-        if (flags & 11) {
-            if (attempt >= 8) return fail(h, ISS_ERR_CUDA, "decay buffers did not settle");
-            h->dk_reruns++;
-            if (flags & 1) s_cap = std::max(s_cap * 2, meta_h[kDecayMetaNeedS] + meta_h[kDecayMetaNeedS] / 4);
-            if (flags & 2) u_cap = std::max(u_cap * 2, meta_h[kDecayMetaNeedU] + meta_h[kDecayMetaNeedU] / 4);
-            if (flags & 8) i_cap = std::max(i_cap * 2, meta_h[kDecayMetaNeedI] + meta_h[kDecayMetaNeedI] / 4);
-            continue;
-        }
-        // generations with inputs: 0 .. n_gen - 1
-        int n_gen = 0;
-        while (n_gen < g && meta_h[kDecayMetaNIn + n_gen] > 0) n_gen++;
-        const int64_t total = meta_h[kDecayMetaSBase + n_gen];
-        CUDA_TRY(h, launch_decay_layout(b, n_gen, E, h->dk_etot.ptr, h->dk_etiles.ptr, h->dk_off.ptr, s));
-        // write sweep
-        for (int k = 0; k < n_gen; k++) {
-            const HadronRec* in = k == 0 ? h->d_hadrons.ptr : h->dk_u[(k - 1) & 1].ptr;
-            CUDA_TRY(h, launch_decay_write_generation(c, t, static_cast<uint32_t>(k), meta_h[kDecayMetaNIn + k],
-                                                      meta_h[kDecayMetaIBase + k], in, h->dk_u[k & 1].ptr, b, E,
-                                                      h->num_sms, h->dk_final.ptr, s));
-        }
-        h->event_offsets.assign(static_cast<size_t>(E) + 1, 0);
-        unsigned long long nf = 0;
-        CUDA_TRY(h, cudaMemcpyAsync(h->event_offsets.data(), h->dk_off.ptr, 8 * (static_cast<size_t>(E) + 1),
-                                    cudaMemcpyDeviceToHost, s));
-        CUDA_TRY(h, cudaMemcpyAsync(&nf, h->dk_fail.ptr, sizeof(nf), cudaMemcpyDeviceToHost, s));
-        CUDA_TRY(h, cudaStreamSynchronize(s));
-        if (h->event_offsets[E] != total)
-            return fail(h, ISS_ERR_CUDA, "decay lists disagree (%lld vs %lld hadrons)",
-                        static_cast<long long>(h->event_offsets[E]), static_cast<long long>(total));
-        *failures_out = nf;
-        // sizes for the next call: what this one needed, with headroom
-        const int64_t inputs = meta_h[kDecayMetaIBase + n_gen];
-        h->dk_scap_hint = std::max(h->dk_scap_hint, total + total / 8 + 4096);
-        h->dk_ucap_hint = std::max(h->dk_ucap_hint, meta_h[kDecayMetaMaxU] + meta_h[kDecayMetaMaxU] / 8 + 4096);
-        h->dk_icap_hint = std::max(h->dk_icap_hint, inputs + inputs / 8 + 4096);
-        h->dk_gen_hint = n_gen;
-        std::swap(h->dk_final.ptr, h->d_hadrons.ptr);
-        std::swap(h->dk_final.cap, h->d_hadrons.cap);
-        h->n_hadrons = total;
-        return ISS_OK;
+        if (!(flags & 11)) break;
+        if (attempt >= 8) return fail(h, ISS_ERR_CUDA, "decay buffers did not settle");
+        h->dk_reruns++;
+        if (flags & 1) run->s_cap = std::max(run->s_cap * 2, meta[kDecayMetaNeedS] + meta[kDecayMetaNeedS] / 4);
+        if (flags & 2) run->u_cap = std::max(run->u_cap * 2, meta[kDecayMetaNeedU] + meta[kDecayMetaNeedU] / 4);
+        if (flags & 8) run->i_cap = std::max(run->i_cap * 2, meta[kDecayMetaNeedI] + meta[kDecayMetaNeedI] / 4);
+        const iss_status st = decays_enqueue(h, run, from_records, s);
+        if (st != ISS_OK) return st;
     }
+    // generations with inputs: 0 .. n_gen - 1
+    run->n_gen = 0;
+    while (run->n_gen < run->g && meta[kDecayMetaNIn + run->n_gen] > 0) run->n_gen++;
+    run->total = meta[kDecayMetaSBase + run->n_gen];
+    CUDA_TRY(h, launch_decay_layout(run->b, run->n_gen, E, h->dk_etot.ptr, h->dk_etiles.ptr, h->dk_off.ptr, s));
+    CUDA_TRY(h, cudaMemcpyAsync(h->eh->tail, h->dk_off.ptr, 8 * (static_cast<size_t>(E) + 1),
+                                cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(h, cudaEventRecord(h->ev_join, s));   // the layout, there and on the host
+    return ISS_OK;
+}
+
+// The write sweep of a counted run, and with a host destination that holds the
+// lists the copies to it.
+iss_status decays_write(iss_handle* h, const DecayRun& run, iss_hadron_t* host_out, int64_t capacity, bool* copied,
+                        unsigned long long* failures_out) {
+    DevConfig& c = h->cfg;
+    cudaStream_t s = h->stream;
+    const int E = c.n_events;
+    const int64_t n0 = run.n0, total = run.total;
+    CUDA_TRY(h, cudaStreamWaitEvent(s, h->ev_join, 0));
+    // write sweep: all events at once, or for a host destination in groups
+    // of events, each copied out while the next ones are written (the
+    // groups alternate between two streams)
+    const bool to_host = host_out != nullptr && total <= capacity && total > 0;
+    std::vector<int> edge{0};
+    const int64_t group = to_host ? std::max(kDecayGroupRecords, (n0 + kDecayGroups - 1) / kDecayGroups) : n0;
+    for (int e = 1; e < E; e++)
+        if (h->event_offsets[e] - h->event_offsets[edge.back()] >= group) edge.push_back(e);
+    edge.push_back(E);
+    const int n_groups = static_cast<int>(edge.size()) - 1;
+    if (to_host) {
+        const iss_status cst = ensure_copy_stream(h, n_groups);
+        if (cst != ISS_OK) return cst;
+    }
+    if (n_groups > 1) {
+        const iss_status sst = fork_sample_stream(h);
+        if (sst != ISS_OK) return sst;
+    }
+    for (int q = 0; q < n_groups; q++) {
+        cudaStream_t gs = (q & 1) ? h->sample_stream : s;
+        const double share = static_cast<double>(h->event_offsets[edge[q + 1]] - h->event_offsets[edge[q]]) /
+                             static_cast<double>(n0);
+        for (int k = 0; k < run.n_gen; k++) {
+            // generation k >= 1's records start where its inputs do, less
+            // the sampled ones
+            const int64_t ib = run.meta[kDecayMetaIBase + k], ib_next = run.meta[kDecayMetaIBase + k + 1];
+            const HadronRec* in = k == 0 ? h->d_hadrons.ptr : h->dk_u.ptr + (ib - n0);
+            const int64_t about = 1 + static_cast<int64_t>(share * static_cast<double>(run.meta[kDecayMetaNIn + k]));
+            CUDA_TRY(h, launch_decay_write_generation(c, run.t, static_cast<uint32_t>(k), edge[q], edge[q + 1], about,
+                                                      ib, in, h->dk_u.ptr + (ib_next - n0), run.b, E, h->num_sms,
+                                                      h->dk_final.ptr, gs));
+        }
+        if (to_host) CUDA_TRY(h, cudaEventRecord(h->chunk_ev[q], gs));
+    }
+    if (n_groups > 1) {
+        const iss_status jst = join_sample_stream(h);
+        if (jst != ISS_OK) return jst;
+    }
+    CUDA_TRY(h, cudaEventRecord(h->ev_decay[1], s));
+    unsigned long long nf = 0;
+    if (to_host) {
+        CUDA_TRY(h, cudaEventSynchronize(h->ev_join));
+        for (int q = 0; q < n_groups; q++) {
+            const int64_t b0 = h->eh->tail[edge[q]], n = h->eh->tail[edge[q + 1]] - b0;
+            CUDA_TRY(h, cudaStreamWaitEvent(h->copy_stream, h->chunk_ev[q], 0));
+            if (n > 0)
+                CUDA_TRY(h, cudaMemcpyAsync(host_out + b0, h->dk_final.ptr + b0,
+                                            sizeof(iss_hadron_t) * static_cast<size_t>(n),
+                                            cudaMemcpyDeviceToHost, h->copy_stream));
+        }
+    }
+    CUDA_TRY(h, cudaMemcpyAsync(&nf, h->dk_fail.ptr, sizeof(nf), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(h, cudaStreamSynchronize(s));
+    if (to_host) {
+        CUDA_TRY(h, cudaStreamSynchronize(h->copy_stream));
+        *copied = true;
+    }
+    h->event_offsets.assign(h->eh->tail, h->eh->tail + E + 1);
+    if (h->event_offsets[E] != total)
+        return fail(h, ISS_ERR_CUDA, "decay lists disagree (%lld vs %lld hadrons)",
+                    static_cast<long long>(h->event_offsets[E]), static_cast<long long>(total));
+    *failures_out = nf;
+    // sizes for the next call: what this one needed, with headroom
+    const int64_t inputs = run.meta[kDecayMetaIBase + run.n_gen], max_u = run.meta[kDecayMetaMaxU];
+    h->dk_scap_hint = std::max(h->dk_scap_hint, total + total / 8 + 4096);
+    h->dk_ucap_hint = std::max(h->dk_ucap_hint, max_u + max_u / 8 + 4096);
+    h->dk_icap_hint = std::max(h->dk_icap_hint, inputs + inputs / 8 + 4096);
+    h->dk_gen_hint = run.n_gen;
+    std::swap(h->dk_final.ptr, h->d_hadrons.ptr);
+    std::swap(h->dk_final.cap, h->d_hadrons.cap);
+    h->n_hadrons = total;
+    return ISS_OK;
 }
 
 // host_out != nullptr: iss_gpu_generate_into -- the sampler runs in chunks of
@@ -1510,13 +1627,8 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     // with decays the records change after sampling: no copies during it
     const bool to_host = host_out != nullptr && n_units <= capacity && n_units > 0 && !h->decays;
     if (to_host) {
-        if (!h->copy_stream)
-            CUDA_TRY(h, cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
-        while (static_cast<int>(h->chunk_ev.size()) < n_chunks) {
-            cudaEvent_t e;
-            CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            h->chunk_ev.push_back(e);
-        }
+        st = ensure_copy_stream(h, n_chunks);
+        if (st != ISS_OK) return st;
     }
     // streamed: the record buffer and cell_of hold two chunks (ring slots
     // ch & 1), the largest chunk sets their size
@@ -1527,13 +1639,8 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
             ring = std::max(ring, h->event_offsets[e1] - h->event_offsets[e0]);
         }
         ring = std::max<int64_t>(ring, 1);
-        if (!h->copy_stream)
-            CUDA_TRY(h, cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
-        while (static_cast<int>(h->chunk_ev.size()) < n_chunks) {
-            cudaEvent_t e;
-            CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            h->chunk_ev.push_back(e);
-        }
+        st = ensure_copy_stream(h, n_chunks);
+        if (st != ISS_OK) return st;
         while (static_cast<int>(h->copy_ev.size()) < n_chunks) {
             cudaEvent_t e;
             CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1608,12 +1715,8 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     const int64_t group_records =
         std::min(h->use_learned ? kLearnedGroupRecords : kGroupRecords, (n_units + 1) / 2);
     if (to_host && n_chunks > 1) {
-        if (!h->sample_stream) {
-            CUDA_TRY(h, cudaStreamCreateWithFlags(&h->sample_stream, cudaStreamNonBlocking));
-            for (auto& e : h->ev_sample2) CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        }
-        CUDA_TRY(h, cudaEventRecord(h->ev_sample2[0], s));
-        CUDA_TRY(h, cudaStreamWaitEvent(h->sample_stream, h->ev_sample2[0], 0));
+        st = fork_sample_stream(h);
+        if (st != ISS_OK) return st;
     }
     int n_groups = 0;
     for (int ch = 0; ch < n_chunks && !sink; n_groups++) {
@@ -1643,10 +1746,22 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
         }
     }
     if (n_groups > 1) {
-        CUDA_TRY(h, cudaEventRecord(h->ev_sample2[1], h->sample_stream));
-        CUDA_TRY(h, cudaStreamWaitEvent(s, h->ev_sample2[1], 0));
+        st = join_sample_stream(h);
+        if (st != ISS_OK) return st;
     }
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvSample], s));
+    // the count sweep of the decays needs the segments' offsets only: it runs
+    // beside the cell assignment and the sampler
+    const bool any_decays = h->decays && n_units > 0 && E > 0;
+    DecayRun decay;
+    if (h->decays) {
+        st = decays_begin(h, &decay, n_units, a);
+        if (st == ISS_OK && any_decays) st = decays_count(h, &decay, false, a);
+        if (st != ISS_OK) {
+            cudaStreamSynchronize(s);   // the sampler still runs
+            return st;
+        }
+    }
     CUDA_TRY(h, cudaMemcpyAsync(&h->eh->ctr, h->d_counters.ptr, sizeof(SampleCounters), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(h, cudaStreamSynchronize(s));
     const SampleCounters ctr = h->eh->ctr;
@@ -1661,21 +1776,22 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     const bool streamed = sink != nullptr;
     unsigned long long decay_failures = 0;
     float ms_decays = 0.f;
-    if (h->decays) {
+    if (any_decays) {
         for (auto& e : h->ev_decay)
             if (!e) CUDA_TRY(h, cudaEventCreate(&e));
         CUDA_TRY(h, cudaEventRecord(h->ev_decay[0], s));
-        const iss_status dst = run_decays(h, &decay_failures);
-        if (dst != ISS_OK) return dst;
-        CUDA_TRY(h, cudaEventRecord(h->ev_decay[1], s));
+        // abandoned hadrons have no particle id in their records: counted anew
+        if (ctr.failures > 0 || ctr.error_code != 0) {
+            st = decays_enqueue(h, &decay, true, s);
+            if (st == ISS_OK) st = decays_count(h, &decay, true, s);
+            if (st != ISS_OK) return st;
+        }
+        bool done = false;
+        st = decays_write(h, decay, host_out, capacity, &done, &decay_failures);
+        if (st != ISS_OK) return st;
+        if (done && copied) *copied = true;
         CUDA_TRY(h, cudaEventSynchronize(h->ev_decay[1]));
         cudaEventElapsedTime(&ms_decays, h->ev_decay[0], h->ev_decay[1]);
-        if (host_out && h->n_hadrons <= capacity && h->n_hadrons > 0) {
-            CUDA_TRY(h, cudaMemcpy(host_out, h->d_hadrons.ptr,
-                                   sizeof(iss_hadron_t) * static_cast<size_t>(h->n_hadrons),
-                                   cudaMemcpyDeviceToHost));
-            if (copied) *copied = true;
-        }
     }
 
     iss_timings_t& t = h->timings;

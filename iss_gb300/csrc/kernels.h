@@ -137,18 +137,21 @@ constexpr int kDecayMetaSBase = kDecayMetaNIn + kDecayMaxGenerations + 1;
 constexpr int kDecayMetaIBase = kDecayMetaSBase + kDecayMaxGenerations + 1;
 constexpr int kDecayMetaLen = kDecayMetaIBase + kDecayMaxGenerations + 1;
 
+constexpr int kDecayTile = 1024;
+// up to this many events the final lists are laid out by one block
+constexpr int kDecayLayoutEvents = 4096;
+
 struct DecayBuffers {
-    const HadronRec* rec0;      // the sampled records (generation 0's input), event-sorted
     int32_t* ev;                // [i_cap] event of every input, generations back to back
-    int32_t* pid;               // [i_cap] particle id of every input of generations >= 1
+    int32_t* pid;               // [i_cap] particle id of every input
     int32_t* chan;              // [i_cap] per input: (type << 16) | channel, or < 0
-    int64_t* cnt;               // [largest generation] (stable products << 32) | unstable ones
-    int64_t* off;               // [i_cap + g_max + 1] generation g's exclusive scan of cnt
+    uint8_t* cnt;               // [largest generation] stable products | unstable ones << 4
+    int64_t* off;               // [i_cap + g_max + 1] generation g's exclusive scan of
+                                // (stable << 32) | unstable products
                                 // (inputs + 1 entries) from IBase + g: both offsets at once
-    int64_t* tiles;             // one per scan tile of 4096 inputs
+    int64_t* tiles;             // one per scan tile of kDecayTile inputs
     int64_t* first;             // [g_max][n_events] input range of each event per generation
-    int64_t* last;              //   (-1: none)
-    int64_t* scnt;              // [g_max][n_events] stable products of each event per generation
+    int64_t* last;              //   ([first, last), empty ones included)
     int64_t* shift;             // [g_max][n_events] final place of the event's first stable
                                 //   product of the generation, less its stable scan offset
     int64_t* meta;              // DecayMeta
@@ -157,9 +160,12 @@ struct DecayBuffers {
     uint32_t g_max;
 };
 
-// event ids and input ranges of generation 0 from the sampled event offsets
-cudaError_t launch_decay_first_generation(const int64_t* evoff, int n_events, const DecayBuffers& b,
-                                          cudaStream_t s);
+// generation 0's events, particle ids and input ranges from the offsets of the
+// sampled (event, species) segments; records: take the ids of the n sampled
+// records instead
+cudaError_t launch_decay_inputs(const DevConfig& cfg, const SpeciesDev* species, const int32_t* pids,
+                                const int64_t* offsets, const HadronRec* records, int64_t n,
+                                const DecayBuffers& b, int num_sms, cudaStream_t s);
 // count sweep of one generation: channel cache, packed scan, sizes of the
 // next generation, its inputs' ids and events, per-event ranges
 cudaError_t launch_decay_count_generation(const DevConfig& cfg, const DecayTablesDev& t, uint32_t gen,
@@ -169,11 +175,12 @@ cudaError_t launch_decay_count_generation(const DevConfig& cfg, const DecayTable
 // (evoff, n_events + 1) and the per (generation, event) shifts
 cudaError_t launch_decay_layout(const DecayBuffers& b, int n_gen, int n_events, int32_t* ev_tot,
                                 int64_t* tiles, int64_t* evoff, cudaStream_t s);
-// write sweep of generation gen (n inputs from ib): stable products to out,
+// write sweep of generation gen (its inputs from ib) for the events [e0, e1)
+// (about n_about inputs, which sizes the launch): stable products to out,
 // unstable ones to out_u (the next generation's records)
-cudaError_t launch_decay_write_generation(const DevConfig& cfg, const DecayTablesDev& t, uint32_t gen,
-                                          int64_t n, int64_t ib, const HadronRec* in, HadronRec* out_u,
-                                          const DecayBuffers& b, int n_events, int num_sms,
+cudaError_t launch_decay_write_generation(const DevConfig& cfg, const DecayTablesDev& t, uint32_t gen, int e0,
+                                          int e1, int64_t n_about, int64_t ib, const HadronRec* in,
+                                          HadronRec* out_u, const DecayBuffers& b, int n_events, int num_sms,
                                           HadronRec* out, cudaStream_t s);
 
 // kernels_output.cu: OSCAR text (FSSW::combine_samples_to_OSCAR) of hadrons

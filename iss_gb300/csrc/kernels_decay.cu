@@ -142,48 +142,6 @@ __device__ __forceinline__ int64_t meta_ib(const int64_t* __restrict__ meta, uin
     return meta[kDecayMetaIBase + gen];
 }
 
-// Count kernel of generation gen: the channel cache and the packed counts of
-// every input.  The particle id comes from the sampled records (generation 0)
-// or from the ids the previous generation's scan wrote (later generations).
-__global__ void __launch_bounds__(kDecayThreads)
-decay_count_kernel(DevConfig cfg, DecayTablesDev t, uint32_t gen, const HadronRec* __restrict__ rec0,
-                   const int32_t* __restrict__ pid_all, const int32_t* __restrict__ ev_all,
-                   const int64_t* __restrict__ first, const int64_t* __restrict__ meta,
-                   int32_t* __restrict__ chan_all, int64_t* __restrict__ cnt) {
-    __shared__ int2 s_hash[kDecayHash];
-    const int64_t n = meta_n(meta, gen), ib = meta_ib(meta, gen);
-    // blocks without inputs leave before staging the table (late generations
-    // are small)
-    if (static_cast<int64_t>(blockIdx.x) * blockDim.x >= n) return;
-    for (int j = threadIdx.x; j < kDecayHash; j += blockDim.x) s_hash[j] = t.hash[j];
-    __syncthreads();
-    const int32_t* ev = ev_all + ib;
-    int32_t* chan = chan_all + ib;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int e = ev[i];
-        const int pid = gen == 0 ? rec0[i].pid : pid_all[ib + i];
-        const DecayPlan d = plan(t, s_hash, cfg, pid, static_cast<uint32_t>(i - first[e]),
-                                 cfg.event_offset + static_cast<uint32_t>(e), gen);
-        int s = 0, u = 0;
-        int32_t c;
-        if (d.channel < 0) {
-            s = d.n;   // stable (or no channel: nothing)
-            c = d.n == 1 ? kChanStable : kChanNone;
-        } else if (d.n == 0) {
-            c = kChanNone;
-        } else {
-            c = static_cast<int32_t>((static_cast<uint32_t>(d.type) << 16) |
-                                     static_cast<uint32_t>(d.channel));
-            for (int k = 0; k < d.n; k++) {
-                if (daughter_stable(t, t.channels[d.channel].daughter[k])) s++; else u++;
-            }
-        }
-        chan[i] = c;
-        cnt[i] = (static_cast<int64_t>(s) << 32) | static_cast<int64_t>(u);
-    }
-}
-
 // The mother's 4-velocity: gamma = E/m and u = p/m (computing gamma from
 // 1 - v^2 in FP32 would lose digits for fast mothers)
 struct Lorentz {
@@ -331,7 +289,8 @@ __device__ __noinline__ void decay_one(const DevConfig& cfg, const DecayTablesDe
     }
 }
 
-// The write pass of a generation.  Each warp walks its chunks of 32 inputs:
+// The write pass of a generation for the events [e0, e1), whose inputs are
+// consecutive.  Each warp walks its chunks of 32 inputs:
 // stable inputs are copied to their final places at once, decaying ones are
 // queued in shared memory, and whenever 32 are queued the whole warp decays
 // them together, so lanes that copy do not wait on lanes that decay.  Stable
@@ -341,9 +300,10 @@ __device__ __noinline__ void decay_one(const DevConfig& cfg, const DecayTablesDe
 constexpr int kDecayQueue = 64;
 
 __global__ void __launch_bounds__(kDecayThreads, 3)
-decay_write_kernel(DevConfig cfg, DecayTablesDev t, uint32_t gen, int64_t n,
+decay_write_kernel(DevConfig cfg, DecayTablesDev t, uint32_t gen, int e0, int e1,
                    const HadronRec* __restrict__ in, const int32_t* __restrict__ ev,
-                   const int64_t* __restrict__ first, const int32_t* __restrict__ chan,
+                   const int64_t* __restrict__ first, const int64_t* __restrict__ last,
+                   const int32_t* __restrict__ chan,
                    const int64_t* __restrict__ off, const int64_t* __restrict__ shift,
                    HadronRec* __restrict__ out, HadronRec* __restrict__ out_u,
                    unsigned long long* __restrict__ failures) {
@@ -360,7 +320,8 @@ decay_write_kernel(DevConfig cfg, DecayTablesDev t, uint32_t gen, int64_t n,
                   shift[e] + (o >> 32), o & 0xFFFFFFFFll, out, out_u, failures);
     };
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-    for (int64_t b0 = (static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + wid) * 32; b0 < n;
+    const int64_t n = last[e1 - 1];
+    for (int64_t b0 = first[e0] + (static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + wid) * 32; b0 < n;
          b0 += warps * 32) {
         const int64_t i = b0 + lane;
         const int32_t c = i < n ? chan[i] : kChanNone;
@@ -380,29 +341,47 @@ decay_write_kernel(DevConfig cfg, DecayTablesDev t, uint32_t gen, int64_t n,
     if (lane < qn) decay(q[lane]);
 }
 
-// event ids of the sampled records from the event offsets
-__global__ void event_ids_kernel(const int64_t* __restrict__ off, int n_events,
-                                 int32_t* __restrict__ ev) {
-    const int e = blockIdx.x;
-    if (e >= n_events) return;
-    for (int64_t i = off[e] + threadIdx.x; i < off[e + 1]; i += blockDim.x) ev[i] = e;
+// Generation 0's inputs, a warp per (event, species) segment of the sampled
+// records: the event and particle id of each (with charge pairs every second
+// record of a positive species is its antiparticle) and the events' input
+// ranges.  They follow from the segments' offsets alone, so the count sweep can
+// run beside the sampling.  blockIdx.y shares a segment's records.
+__global__ void __launch_bounds__(kDecayThreads)
+decay_inputs_kernel(const int64_t* __restrict__ offsets, const SpeciesDev* __restrict__ species,
+                    const int32_t* __restrict__ pids, int n_species, int n_events, int lcc,
+                    int32_t* __restrict__ ev, int32_t* __restrict__ pid, int64_t* __restrict__ first,
+                    int64_t* __restrict__ last) {
+    const int lane = threadIdx.x & 31;
+    const int64_t seg = static_cast<int64_t>(blockIdx.x) * (kDecayThreads / 32) + (threadIdx.x >> 5);
+    if (seg >= static_cast<int64_t>(n_events) * n_species) return;
+    const int e = static_cast<int>(seg / n_species), s = static_cast<int>(seg - static_cast<int64_t>(e) * n_species);
+    const int64_t b = offsets[seg], end = offsets[seg + 1];
+    if (blockIdx.y == 0 && lane == 0) {
+        if (s == 0) first[e] = b;
+        if (s == n_species - 1) last[e] = end;
+    }
+    const int p = pids[s];
+    const int second = lcc && species[s].charge > 0 ? -p : p;
+    for (int64_t i = b + blockIdx.y * 32 + lane; i < end; i += gridDim.y * 32) {
+        ev[i] = e;
+        pid[i] = ((i - b) & 1) ? second : p;
+    }
 }
 
-// generation 0's input range per event: the sampled records of the event
-__global__ void dk_first_gen_kernel(const int64_t* __restrict__ evoff, int n_events,
-                                    int64_t* __restrict__ first, int64_t* __restrict__ last) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_events) return;
-    const bool any = evoff[e + 1] > evoff[e];
-    first[e] = any ? evoff[e] : -1;
-    last[e] = any ? evoff[e + 1] : -1;
+// the ids as the sampler left them (an abandoned hadron has none)
+__global__ void __launch_bounds__(kDecayThreads)
+decay_record_ids_kernel(const HadronRec* __restrict__ rec, int64_t n, int32_t* __restrict__ pid) {
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+        pid[i] = rec[i].pid;
 }
 
 // ---- exclusive scans of the packed counts, input size on the device ----
 
 constexpr int kDkScanThreads = 256;
-constexpr int kDkScanPer = 16;
+constexpr int kDkScanPer = 4;
 constexpr int kDkTile = kDkScanThreads * kDkScanPer;
+static_assert(kDkTile == kDecayTile, "the host sizes the tile sums");
 
 __device__ __forceinline__ long long dk_warp_incl(long long v) {
     const int lane = threadIdx.x & 31;
@@ -434,22 +413,90 @@ __device__ long long dk_block_excl(long long v, long long* s_warp, long long* to
     return out;
 }
 
-// Exclusive scan of the packed counts (stable << 32 | unstable): one int64
-// scan gives both offsets, since no partial sum of the unstable half reaches
-// 2^32 (it is bounded by the next-input capacity).  Generation gen's scan
-// lands at off_all + meta_ib + gen (n + 1 entries, the last the total).
-// tile sums: tiles[t] for the tiles of 4096 inputs
+// stable and unstable products of an input in one byte (at most 3 each), and
+// packed for the scans
+__device__ __forceinline__ uint8_t dk_byte(int s, int u) { return static_cast<uint8_t>(s | u << 4); }
+__device__ __forceinline__ long long dk_packed(uint8_t c) {
+    return (static_cast<long long>(c & 15) << 32) | static_cast<long long>(c >> 4);
+}
+
+// Generation gen's scan (n + 1 entries, the last the total)
+__device__ __forceinline__ const int64_t* gen_off(const int64_t* off_all, const int64_t* meta, uint32_t gen) {
+    return off_all + meta_ib(meta, gen) + gen;
+}
+// where event e's inputs of generation gen + 1 start (end) given where those of
+// generation gen do: the unstable products before
+__device__ __forceinline__ int64_t next_bound(const int64_t* off_gen, int64_t bound) {
+    return off_gen[bound] & 0xFFFFFFFFll;
+}
+
+// Count kernel of generation gen, a block per tile: the channel cache and the
+// products of every input, and the tile's sum.  Generations after the first also write their events' input ranges,
+// [first, last), empty ones included; the blocks take their inputs' first from
+// the previous generation, whose ranges and scan are complete.
 __global__ void __launch_bounds__(kDkScanThreads)
-dk_tile_sum_kernel(const int64_t* __restrict__ c, const int64_t* __restrict__ meta, uint32_t gen,
-                   int64_t* __restrict__ tiles) {
+decay_count_kernel(DevConfig cfg, DecayTablesDev t, uint32_t gen, const int32_t* __restrict__ pid_all, const int32_t* __restrict__ ev_all,
+                   int64_t* __restrict__ first, int64_t* __restrict__ last, int n_events,
+                   const int64_t* __restrict__ off_all, const int64_t* __restrict__ meta,
+                   int32_t* __restrict__ chan_all, uint8_t* __restrict__ cnt, int64_t* __restrict__ tiles) {
+    __shared__ int2 s_hash[kDecayHash];
     __shared__ long long s_warp[33];
-    const int64_t n = meta_n(meta, gen);
+    const int64_t n = meta_n(meta, gen), ib = meta_ib(meta, gen);
+    const int64_t* off_prev = gen > 0 ? gen_off(off_all, meta, gen - 1) : nullptr;
+    const int64_t* first_prev = first + static_cast<int64_t>(gen > 0 ? gen - 1 : 0) * n_events;
+    if (gen > 0 && meta[kDecayMetaFlags] == 0) {   // (a chain that ended has no ranges to go on from)
+        const int64_t* last_prev = last + static_cast<int64_t>(gen - 1) * n_events;
+        const int64_t row = static_cast<int64_t>(gen) * n_events;
+        for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_events; e += gridDim.x * blockDim.x) {
+            first[row + e] = next_bound(off_prev, first_prev[e]);
+            last[row + e] = next_bound(off_prev, last_prev[e]);
+        }
+    }
     const int64_t nt = (n + kDkTile - 1) / kDkTile;
+    // blocks without inputs leave before staging the table (late generations
+    // are small)
+    if (blockIdx.x >= nt) return;
+    for (int j = threadIdx.x; j < kDecayHash; j += blockDim.x) s_hash[j] = t.hash[j];
+    __syncthreads();
+    const int32_t* ev = ev_all + ib;
+    int32_t* chan = chan_all + ib;
     for (int64_t tl = blockIdx.x; tl < nt; tl += gridDim.x) {
         long long acc = 0;
+        // the tile's ids and events are read at once, ahead of the chains of
+        // look-ups
+        int32_t e_k[kDkScanPer], pid_k[kDkScanPer];
+#pragma unroll
+        for (int k = 0; k < kDkScanPer; k++) {
+            const int64_t i = min(tl * kDkTile + k * kDkScanThreads + threadIdx.x, n - 1);
+            e_k[k] = ev[i];
+            pid_k[k] = pid_all[ib + i];
+        }
+#pragma unroll
         for (int k = 0; k < kDkScanPer; k++) {
             const int64_t i = tl * kDkTile + k * kDkScanThreads + threadIdx.x;
-            if (i < n) acc += c[i];
+            if (i >= n) break;
+            const int e = e_k[k], pid = pid_k[k];
+            const int64_t f = gen == 0 ? first_prev[e] : next_bound(off_prev, first_prev[e]);
+            const DecayPlan d = plan(t, s_hash, cfg, pid, static_cast<uint32_t>(i - f),
+                                     cfg.event_offset + static_cast<uint32_t>(e), gen);
+            int s = 0, u = 0;
+            int32_t c;
+            if (d.channel < 0) {
+                s = d.n;   // stable (or no channel: nothing)
+                c = d.n == 1 ? kChanStable : kChanNone;
+            } else if (d.n == 0) {
+                c = kChanNone;
+            } else {
+                c = static_cast<int32_t>((static_cast<uint32_t>(d.type) << 16) |
+                                         static_cast<uint32_t>(d.channel));
+                for (int j = 0; j < d.n; j++) {
+                    if (daughter_stable(t, t.channels[d.channel].daughter[j])) s++; else u++;
+                }
+            }
+            chan[i] = c;
+            const uint8_t b = dk_byte(s, u);
+            cnt[i] = b;
+            acc += dk_packed(b);
         }
         long long tot;
         dk_block_excl(acc, s_warp, &tot);
@@ -457,15 +504,57 @@ dk_tile_sum_kernel(const int64_t* __restrict__ c, const int64_t* __restrict__ me
     }
 }
 
-// one block: tile sums -> tile offsets (in place), the total to off[n]
-__global__ void __launch_bounds__(kDkScanThreads)
-dk_tile_offset_kernel(int64_t* __restrict__ tiles, const int64_t* __restrict__ meta, uint32_t gen,
-                      int64_t* __restrict__ off_all) {
+// Sizes of the next generation: its inputs (this generation's unstable
+// products) follow this generation's in the per-input arrays, and the stable
+// products so far give the final lists' length.  A generation that does not
+// fit (final lists, one generation's records, all inputs) or would exceed
+// g_max sets a flag, records what it needed and ends the chain.
+__device__ void dk_advance(int64_t* __restrict__ meta, uint32_t gen, int64_t tot, int64_t s_cap, int64_t u_cap,
+                           int64_t i_cap, uint32_t g_max) {
+    const int64_t n = meta[kDecayMetaNIn + gen];
+    const int64_t ib = meta[kDecayMetaIBase + gen];
+    const int64_t sb = meta[kDecayMetaSBase + gen];
+    const int64_t st = tot >> 32, ut = tot & 0xFFFFFFFFll;
+    int64_t next_n = ut;
+    const int64_t next_sb = sb + st, next_ib = ib + n;
+    int64_t flags = meta[kDecayMetaFlags];
+    if (flags == 0 && next_sb > s_cap) {
+        flags |= 1;
+        meta[kDecayMetaNeedS] = next_sb;
+    }
+    if (flags == 0 && ut > u_cap) {
+        flags |= 2;
+        meta[kDecayMetaNeedU] = ut;
+    }
+    if (flags == 0 && next_ib + ut > i_cap) {
+        flags |= 8;
+        meta[kDecayMetaNeedI] = next_ib + ut;
+    }
+    if (flags == 0 && gen + 1 >= g_max && ut > 0) flags |= 4;
+    meta[kDecayMetaFlags] = flags;
+    if (flags != 0) next_n = 0;
+    meta[kDecayMetaNIn + gen + 1] = next_n;
+    meta[kDecayMetaSBase + gen + 1] = next_sb;
+    meta[kDecayMetaIBase + gen + 1] = next_ib;
+    if (ut > meta[kDecayMetaMaxU]) meta[kDecayMetaMaxU] = ut;
+}
+
+// One block: tile sums -> tile offsets (in place), the total to off[n], the
+// sizes of the next generation.  The packed counts (stable << 32 | unstable)
+// give both offsets in one int64 scan, since no partial sum of the unstable
+// half reaches 2^32 (it is bounded by the next-input capacity).  Generation
+// gen's scan lands at off_all + meta_ib + gen.
+constexpr int kDkOffsetThreads = 1024;
+
+__global__ void __launch_bounds__(kDkOffsetThreads)
+dk_tile_offset_kernel(int64_t* __restrict__ tiles, int64_t* __restrict__ meta, uint32_t gen,
+                      int64_t* __restrict__ off_all, int64_t s_cap, int64_t u_cap, int64_t i_cap,
+                      uint32_t g_max) {
     __shared__ long long s_warp[33];
     const int64_t n = meta_n(meta, gen);
     const int64_t nt = (n + kDkTile - 1) / kDkTile;
     long long carry = 0;
-    for (int64_t b0 = 0; b0 < nt; b0 += kDkScanThreads) {
+    for (int64_t b0 = 0; b0 < nt; b0 += kDkOffsetThreads) {
         const int64_t i = b0 + threadIdx.x;
         const long long v = i < nt ? tiles[i] : 0;
         long long tot;
@@ -473,7 +562,10 @@ dk_tile_offset_kernel(int64_t* __restrict__ tiles, const int64_t* __restrict__ m
         if (i < nt) tiles[i] = carry + ex;
         carry += tot;
     }
-    if (threadIdx.x == 0) off_all[meta_ib(meta, gen) + gen + n] = carry;
+    if (threadIdx.x == 0) {
+        off_all[meta_ib(meta, gen) + gen + n] = carry;
+        dk_advance(meta, gen, carry, s_cap, u_cap, i_cap, g_max);
+    }
 }
 
 // the next generation's inputs made by input c (a decaying hadron of event
@@ -494,12 +586,12 @@ __device__ void write_daughters(const DecayTablesDev& t, int32_t c, int e, int64
     }
 }
 
-// The scan of each tile, and the next generation's inputs: a thread scans 16
+// The scan of each tile, and the next generation's inputs: a thread scans 4
 // consecutive inputs and writes the products of those with unstable ones
 // (whose inputs follow this generation's, at meta_ib + n); the offsets go
 // back through shared memory to coalesced stores.
 __global__ void __launch_bounds__(kDkScanThreads)
-dk_tile_scan_kernel(DecayTablesDev t, const int64_t* __restrict__ c, const int64_t* __restrict__ meta,
+dk_tile_scan_kernel(DecayTablesDev t, const uint8_t* __restrict__ c, const int64_t* __restrict__ meta,
                     uint32_t gen, const int64_t* __restrict__ tiles, const int32_t* __restrict__ chan_all,
                     int32_t* __restrict__ ev_all, int32_t* __restrict__ pid_all, int64_t i_cap,
                     int64_t* __restrict__ off_all) {
@@ -513,7 +605,7 @@ dk_tile_scan_kernel(DecayTablesDev t, const int64_t* __restrict__ c, const int64
         for (int k = 0; k < kDkScanPer; k++) {
             const int e = k * kDkScanThreads + threadIdx.x;
             const int64_t i = t0 + e;
-            s_in[(e / kDkScanPer) * (kDkScanPer + 1) + e % kDkScanPer] = i < n ? c[i] : 0;
+            s_in[(e / kDkScanPer) * (kDkScanPer + 1) + e % kDkScanPer] = i < n ? dk_packed(c[i]) : 0;
         }
         __syncthreads();
         long long* mine = s_in + threadIdx.x * (kDkScanPer + 1);
@@ -541,102 +633,87 @@ dk_tile_scan_kernel(DecayTablesDev t, const int64_t* __restrict__ c, const int64
     }
 }
 
-// Sizes of the next generation: its inputs (this generation's unstable
-// products) follow this generation's in the per-input arrays, and the stable
-// products so far give the final lists' length.  A generation that does not
-// fit (final lists, one generation's records, all inputs) or would exceed
-// g_max sets a flag, records what it needed and ends the chain.
-__global__ void dk_advance_kernel(int64_t* __restrict__ meta, uint32_t gen, const int64_t* __restrict__ off_all,
-                                  int64_t s_cap, int64_t u_cap, int64_t i_cap, uint32_t g_max) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int64_t n = meta[kDecayMetaNIn + gen];
-    const int64_t ib = meta[kDecayMetaIBase + gen];
-    const int64_t sb = meta[kDecayMetaSBase + gen];
-    const int64_t tot = off_all[ib + gen + n];
-    const int64_t st = tot >> 32, ut = tot & 0xFFFFFFFFll;
-    int64_t next_n = ut;
-    const int64_t next_sb = sb + st, next_ib = ib + n;
-    if (meta[kDecayMetaFlags] == 0 && next_sb > s_cap) {
-        meta[kDecayMetaFlags] |= 1;
-        meta[kDecayMetaNeedS] = next_sb;
-    }
-    if (meta[kDecayMetaFlags] == 0 && ut > u_cap) {
-        meta[kDecayMetaFlags] |= 2;
-        meta[kDecayMetaNeedU] = ut;
-    }
-    if (meta[kDecayMetaFlags] == 0 && next_ib + ut > i_cap) {
-        meta[kDecayMetaFlags] |= 8;
-        meta[kDecayMetaNeedI] = next_ib + ut;
-    }
-    if (meta[kDecayMetaFlags] == 0 && gen + 1 >= g_max && ut > 0) meta[kDecayMetaFlags] |= 4;
-    if (meta[kDecayMetaFlags] != 0) next_n = 0;
-    meta[kDecayMetaNIn + gen + 1] = next_n;
-    meta[kDecayMetaSBase + gen + 1] = next_sb;
-    meta[kDecayMetaIBase + gen + 1] = next_ib;
-    if (ut > meta[kDecayMetaMaxU]) meta[kDecayMetaMaxU] = ut;
-}
-
-// Per event: its stable products in this generation (scnt) and its input
-// range in the next one (the unstable products of its inputs, contiguous
-// because the inputs are grouped by event).
-__global__ void dk_next_bounds_kernel(const int64_t* __restrict__ meta, uint32_t gen,
-                                      const int64_t* __restrict__ off_all, int n_events, uint32_t g_max,
-                                      int64_t* __restrict__ first, int64_t* __restrict__ last,
-                                      int64_t* __restrict__ scnt) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_events || meta[kDecayMetaFlags] != 0) return;
-    const int64_t r = static_cast<int64_t>(gen) * n_events + e;
-    const int64_t f = first[r];
-    int64_t sc = 0;
-    if (f >= 0) {
-        const int64_t* off = off_all + meta_ib(meta, gen) + gen;
-        const int64_t a = off[f], b = off[last[r]];
-        sc = (b >> 32) - (a >> 32);
-        const int64_t ua = a & 0xFFFFFFFFll, ub = b & 0xFFFFFFFFll;
-        if (ub > ua && gen + 1 < g_max) {
-            first[r + n_events] = ua;
-            last[r + n_events] = ub;
-        }
-    }
-    scnt[r] = sc;
-}
-
 // ---- the final lists ----------------------------------------------------
 
-// per event: its stable products over generations g < n_gen
-__global__ void dk_event_totals_kernel(const int64_t* __restrict__ scnt, int n_gen, int n_events,
-                                       int32_t* __restrict__ tot) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_events) return;
-    int64_t k = 0;
-    for (int g = 0; g < n_gen; g++) k += scnt[static_cast<int64_t>(g) * n_events + e];
-    tot[e] = static_cast<int32_t>(k);
+// stable products of event e in generation g
+__device__ __forceinline__ int64_t event_stable(const int64_t* __restrict__ first, const int64_t* __restrict__ last,
+                                                const int64_t* __restrict__ off_all,
+                                                const int64_t* __restrict__ meta, int g, int n_events, int e) {
+    const int64_t r = static_cast<int64_t>(g) * n_events + e;
+    const int64_t* off = gen_off(off_all, meta, static_cast<uint32_t>(g));
+    return (off[last[r]] >> 32) - (off[first[r]] >> 32);
 }
 
 // shift[g][e] = final place of event e's first stable product of generation
-// g, less the stable scan offset of the event's first input in g
-__global__ void dk_shift_kernel(const int64_t* __restrict__ scnt, const int64_t* __restrict__ first,
+// g, less the stable scan offset of the event's first input in g; b: where the
+// event's final list starts
+__device__ __forceinline__ void event_shifts(const int64_t* __restrict__ first, const int64_t* __restrict__ last,
+                                             const int64_t* __restrict__ off_all,
+                                             const int64_t* __restrict__ meta, int n_gen, int n_events, int e,
+                                             int64_t b, int64_t* __restrict__ shift) {
+    for (int g = 0; g < n_gen; g++) {
+        const int64_t r = static_cast<int64_t>(g) * n_events + e;
+        shift[r] = b - (gen_off(off_all, meta, static_cast<uint32_t>(g))[first[r]] >> 32);
+        b += event_stable(first, last, off_all, meta, g, n_events, e);
+    }
+}
+
+// per event: its stable products over generations g < n_gen
+__global__ void dk_event_totals_kernel(const int64_t* __restrict__ first, const int64_t* __restrict__ last,
+                                       const int64_t* __restrict__ off_all, const int64_t* __restrict__ meta,
+                                       int n_gen, int n_events, int32_t* __restrict__ tot) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n_events) return;
+    int64_t k = 0;
+    for (int g = 0; g < n_gen; g++) k += event_stable(first, last, off_all, meta, g, n_events, e);
+    tot[e] = static_cast<int32_t>(k);
+}
+
+__global__ void dk_shift_kernel(const int64_t* __restrict__ first, const int64_t* __restrict__ last,
                                 const int64_t* __restrict__ off_all, const int64_t* __restrict__ meta,
                                 const int64_t* __restrict__ evoff, int n_gen, int n_events,
                                 int64_t* __restrict__ shift) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_events) return;
-    int64_t b = evoff[e];
-    for (int g = 0; g < n_gen; g++) {
-        const int64_t r = static_cast<int64_t>(g) * n_events + e;
-        const int64_t f = first[r];
-        if (f >= 0) shift[r] = b - (off_all[meta_ib(meta, static_cast<uint32_t>(g)) + g + f] >> 32);
-        b += scnt[r];
+    if (e < n_events) event_shifts(first, last, off_all, meta, n_gen, n_events, e, evoff[e], shift);
+}
+
+// both and the scan between them, in one block
+__global__ void __launch_bounds__(kDkOffsetThreads)
+dk_layout_kernel(const int64_t* __restrict__ first, const int64_t* __restrict__ last,
+                 const int64_t* __restrict__ off_all, const int64_t* __restrict__ meta, int n_gen, int n_events,
+                 int64_t* __restrict__ evoff, int64_t* __restrict__ shift) {
+    __shared__ long long s_warp[33];
+    long long carry = 0;
+    for (int b0 = 0; b0 < n_events; b0 += kDkOffsetThreads) {
+        const int e = b0 + threadIdx.x;
+        long long k = 0;
+        if (e < n_events)
+            for (int g = 0; g < n_gen; g++) k += event_stable(first, last, off_all, meta, g, n_events, e);
+        long long tot;
+        const long long at = carry + dk_block_excl(k, s_warp, &tot);
+        if (e < n_events) {
+            evoff[e] = at;
+            event_shifts(first, last, off_all, meta, n_gen, n_events, e, at, shift);
+        }
+        carry += tot;
     }
+    if (threadIdx.x == 0) evoff[n_events] = carry;
 }
 
 }  // namespace
 
-cudaError_t launch_decay_first_generation(const int64_t* evoff, int n_events, const DecayBuffers& b,
-                                          cudaStream_t s) {
-    if (n_events <= 0) return cudaSuccess;
-    event_ids_kernel<<<n_events, 128, 0, s>>>(evoff, n_events, b.ev);
-    dk_first_gen_kernel<<<(n_events + 255) / 256, 256, 0, s>>>(evoff, n_events, b.first, b.last);
+cudaError_t launch_decay_inputs(const DevConfig& cfg, const SpeciesDev* species, const int32_t* pids,
+                                const int64_t* offsets, const HadronRec* records, int64_t n,
+                                const DecayBuffers& b, int num_sms, cudaStream_t s) {
+    const int64_t nseg = static_cast<int64_t>(cfg.n_events) * cfg.n_species;
+    if (nseg <= 0) return cudaSuccess;
+    const unsigned blocks = static_cast<unsigned>((nseg + kDecayThreads / 32 - 1) / (kDecayThreads / 32));
+    // the segments of few events are shared by more warps
+    const unsigned share = std::max(1u, std::min(64u, 8u * static_cast<unsigned>(num_sms) / blocks));
+    decay_inputs_kernel<<<dim3(blocks, share), kDecayThreads, 0, s>>>(offsets, species, pids, cfg.n_species,
+                                                                     cfg.n_events, cfg.lcc, b.ev, b.pid, b.first,
+                                                                     b.last);
+    if (records) decay_record_ids_kernel<<<num_sms * 8, kDecayThreads, 0, s>>>(records, n, b.pid);
     return cudaGetLastError();
 }
 
@@ -646,41 +723,42 @@ cudaError_t launch_decay_count_generation(const DevConfig& cfg, const DecayTable
     // grid-stride kernels launched with what fits on the SMs at once (eight
     // blocks of 256)
     const int grid = num_sms * 8;
-    const int64_t* first = b.first + static_cast<int64_t>(gen) * n_events;
-    decay_count_kernel<<<grid, kDecayThreads, 0, s>>>(cfg, t, gen, b.rec0, b.pid, b.ev, first, b.meta,
-                                                      b.chan, b.cnt);
-    dk_tile_sum_kernel<<<grid, kDkScanThreads, 0, s>>>(b.cnt, b.meta, gen, b.tiles);
-    dk_tile_offset_kernel<<<1, kDkScanThreads, 0, s>>>(b.tiles, b.meta, gen, b.off);
+    decay_count_kernel<<<grid, kDkScanThreads, 0, s>>>(cfg, t, gen, b.pid, b.ev, b.first, b.last, n_events,
+                                                       b.off, b.meta, b.chan, b.cnt, b.tiles);
+    dk_tile_offset_kernel<<<1, kDkOffsetThreads, 0, s>>>(b.tiles, b.meta, gen, b.off, b.s_cap, b.u_cap, b.i_cap,
+                                                         b.g_max);
     dk_tile_scan_kernel<<<grid, kDkScanThreads, 0, s>>>(t, b.cnt, b.meta, gen, b.tiles, b.chan, b.ev, b.pid,
                                                         b.i_cap, b.off);
-    dk_advance_kernel<<<1, 32, 0, s>>>(b.meta, gen, b.off, b.s_cap, b.u_cap, b.i_cap, b.g_max);
-    dk_next_bounds_kernel<<<(n_events + 255) / 256, 256, 0, s>>>(b.meta, gen, b.off, n_events, b.g_max,
-                                                                 b.first, b.last, b.scnt);
     return cudaGetLastError();
 }
 
 cudaError_t launch_decay_layout(const DecayBuffers& b, int n_gen, int n_events, int32_t* ev_tot,
                                 int64_t* tiles, int64_t* evoff, cudaStream_t s) {
     if (n_events <= 0) return cudaSuccess;
+    if (n_events <= kDecayLayoutEvents) {
+        dk_layout_kernel<<<1, kDkOffsetThreads, 0, s>>>(b.first, b.last, b.off, b.meta, n_gen, n_events, evoff,
+                                                        b.shift);
+        return cudaGetLastError();
+    }
     const unsigned eb = static_cast<unsigned>((n_events + 255) / 256);
-    dk_event_totals_kernel<<<eb, 256, 0, s>>>(b.scnt, n_gen, n_events, ev_tot);
+    dk_event_totals_kernel<<<eb, 256, 0, s>>>(b.first, b.last, b.off, b.meta, n_gen, n_events, ev_tot);
     cudaError_t e = launch_offsets_scan(ev_tot, n_events, tiles, evoff, s);
     if (e != cudaSuccess) return e;
-    dk_shift_kernel<<<eb, 256, 0, s>>>(b.scnt, b.first, b.off, b.meta, evoff, n_gen, n_events, b.shift);
+    dk_shift_kernel<<<eb, 256, 0, s>>>(b.first, b.last, b.off, b.meta, evoff, n_gen, n_events, b.shift);
     return cudaGetLastError();
 }
 
-cudaError_t launch_decay_write_generation(const DevConfig& cfg, const DecayTablesDev& t, uint32_t gen,
-                                          int64_t n, int64_t ib, const HadronRec* in, HadronRec* out_u,
-                                          const DecayBuffers& b, int n_events, int num_sms,
+cudaError_t launch_decay_write_generation(const DevConfig& cfg, const DecayTablesDev& t, uint32_t gen, int e0,
+                                          int e1, int64_t n_about, int64_t ib, const HadronRec* in,
+                                          HadronRec* out_u, const DecayBuffers& b, int n_events, int num_sms,
                                           HadronRec* out, cudaStream_t s) {
-    if (n <= 0) return cudaSuccess;
+    if (n_about <= 0 || e0 >= e1) return cudaSuccess;
     // three blocks of 256 fit per SM at 80 registers; small generations get
     // one warp per 32 inputs at most
-    const int64_t want = (n + kDecayThreads - 1) / kDecayThreads;
+    const int64_t want = (n_about + kDecayThreads - 1) / kDecayThreads;
     const int grid = static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(num_sms) * 3));
     const int64_t r = static_cast<int64_t>(gen) * n_events;
-    decay_write_kernel<<<grid, kDecayThreads, 0, s>>>(cfg, t, gen, n, in, b.ev + ib, b.first + r,
+    decay_write_kernel<<<grid, kDecayThreads, 0, s>>>(cfg, t, gen, e0, e1, in, b.ev + ib, b.first + r, b.last + r,
                                                       b.chan + ib, b.off + ib + gen, b.shift + r, out,
                                                       out_u, b.failures);
     return cudaGetLastError();
