@@ -831,12 +831,6 @@ constexpr int kDecayBatch = 8;
 constexpr int64_t kGroupRecords = 256 << 10;
 constexpr int64_t kLearnedGroupRecords = 512 << 10;
 
-// iss_gpu_generate_into with decays: event groups of the write sweep, of at
-// least so many sampled hadrons (some 1.7 records each) and not more than so
-// many groups (run_decays)
-constexpr int64_t kDecayGroupRecords = 256 << 10;
-constexpr int64_t kDecayGroups = 8;
-
 // the copy stream and at least n chunk events
 iss_status ensure_copy_stream(iss_handle* h, int n) {
     if (!h->copy_stream) CUDA_TRY(h, cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
@@ -1066,35 +1060,22 @@ iss_status decays_count(iss_handle* h, DecayRun* run, bool from_records, cudaStr
     return ISS_OK;
 }
 
-// The write sweep of a counted run, and with a host destination that holds the
-// lists the copies to it.
-iss_status decays_write(iss_handle* h, const DecayRun& run, iss_hadron_t* host_out, int64_t capacity, bool* copied,
-                        unsigned long long* failures_out) {
+// The write sweep of a counted run on stream w, in the groups of events
+// [edge[q], edge[q + 1]): each after chunk_ev[q] (its records are sampled) where
+// after_sampling, and where host_out is given followed by its copy there, which
+// runs beside the next group's.
+iss_status decays_write(iss_handle* h, const DecayRun& run, const std::vector<int>& edge, bool after_sampling,
+                        iss_hadron_t* host_out, cudaStream_t w) {
     DevConfig& c = h->cfg;
-    cudaStream_t s = h->stream;
-    const int E = c.n_events;
-    const int64_t n0 = run.n0, total = run.total;
-    CUDA_TRY(h, cudaStreamWaitEvent(s, h->ev_join, 0));
-    // write sweep: all events at once, or for a host destination in groups
-    // of events, each copied out while the next ones are written (the
-    // groups alternate between two streams)
-    const bool to_host = host_out != nullptr && total <= capacity && total > 0;
-    std::vector<int> edge{0};
-    const int64_t group = to_host ? std::max(kDecayGroupRecords, (n0 + kDecayGroups - 1) / kDecayGroups) : n0;
-    for (int e = 1; e < E; e++)
-        if (h->event_offsets[e] - h->event_offsets[edge.back()] >= group) edge.push_back(e);
-    edge.push_back(E);
-    const int n_groups = static_cast<int>(edge.size()) - 1;
-    if (to_host) {
-        const iss_status cst = ensure_copy_stream(h, n_groups);
-        if (cst != ISS_OK) return cst;
-    }
-    if (n_groups > 1) {
-        const iss_status sst = fork_sample_stream(h);
-        if (sst != ISS_OK) return sst;
+    const int E = c.n_events, n_groups = static_cast<int>(edge.size()) - 1;
+    const int64_t n0 = run.n0;
+    if (host_out) {
+        const iss_status st = ensure_copy_stream(h, 2 * n_groups);
+        if (st != ISS_OK) return st;
+        CUDA_TRY(h, cudaEventSynchronize(h->ev_join));   // the lists' offsets are on the host
     }
     for (int q = 0; q < n_groups; q++) {
-        cudaStream_t gs = (q & 1) ? h->sample_stream : s;
+        if (after_sampling) CUDA_TRY(h, cudaStreamWaitEvent(w, h->chunk_ev[q], 0));
         const double share = static_cast<double>(h->event_offsets[edge[q + 1]] - h->event_offsets[edge[q]]) /
                              static_cast<double>(n0);
         for (int k = 0; k < run.n_gen; k++) {
@@ -1105,33 +1086,29 @@ iss_status decays_write(iss_handle* h, const DecayRun& run, iss_hadron_t* host_o
             const int64_t about = 1 + static_cast<int64_t>(share * static_cast<double>(run.meta[kDecayMetaNIn + k]));
             CUDA_TRY(h, launch_decay_write_generation(c, run.t, static_cast<uint32_t>(k), edge[q], edge[q + 1], about,
                                                       ib, in, h->dk_u.ptr + (ib_next - n0), run.b, E, h->num_sms,
-                                                      h->dk_final.ptr, gs));
+                                                      h->dk_final.ptr, w));
         }
-        if (to_host) CUDA_TRY(h, cudaEventRecord(h->chunk_ev[q], gs));
-    }
-    if (n_groups > 1) {
-        const iss_status jst = join_sample_stream(h);
-        if (jst != ISS_OK) return jst;
-    }
-    CUDA_TRY(h, cudaEventRecord(h->ev_decay[1], s));
-    unsigned long long nf = 0;
-    if (to_host) {
-        CUDA_TRY(h, cudaEventSynchronize(h->ev_join));
-        for (int q = 0; q < n_groups; q++) {
+        if (host_out) {
             const int64_t b0 = h->eh->tail[edge[q]], n = h->eh->tail[edge[q + 1]] - b0;
-            CUDA_TRY(h, cudaStreamWaitEvent(h->copy_stream, h->chunk_ev[q], 0));
+            CUDA_TRY(h, cudaEventRecord(h->chunk_ev[n_groups + q], w));
+            CUDA_TRY(h, cudaStreamWaitEvent(h->copy_stream, h->chunk_ev[n_groups + q], 0));
             if (n > 0)
                 CUDA_TRY(h, cudaMemcpyAsync(host_out + b0, h->dk_final.ptr + b0,
                                             sizeof(iss_hadron_t) * static_cast<size_t>(n),
                                             cudaMemcpyDeviceToHost, h->copy_stream));
         }
     }
-    CUDA_TRY(h, cudaMemcpyAsync(&nf, h->dk_fail.ptr, sizeof(nf), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(h, cudaStreamSynchronize(s));
-    if (to_host) {
-        CUDA_TRY(h, cudaStreamSynchronize(h->copy_stream));
-        *copied = true;
-    }
+    return ISS_OK;
+}
+
+// Waits for the written lists, which become the call's hadrons.
+iss_status decays_finish(iss_handle* h, const DecayRun& run, cudaStream_t w, unsigned long long* failures_out) {
+    const int E = h->cfg.n_events;
+    const int64_t total = run.total;
+    unsigned long long nf = 0;
+    CUDA_TRY(h, cudaMemcpyAsync(&nf, h->dk_fail.ptr, sizeof(nf), cudaMemcpyDeviceToHost, w));
+    CUDA_TRY(h, cudaStreamSynchronize(w));
+    if (h->copy_stream) CUDA_TRY(h, cudaStreamSynchronize(h->copy_stream));
     h->event_offsets.assign(h->eh->tail, h->eh->tail + E + 1);
     if (h->event_offsets[E] != total)
         return fail(h, ISS_ERR_CUDA, "decay lists disagree (%lld vs %lld hadrons)",
@@ -1537,7 +1514,7 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     CUDA_TRY(h, h->d_off_tiles.reserve(static_cast<size_t>(std::max(offsets_num_tiles(nseg), 1))));
     // sampling chunks: one without a host destination, else up to kMaxChunks
     const int E = c.n_events;
-    int n_chunks = (host_out && !h->decays) ? std::min(h->tune.copy_chunks, std::max(E, 1)) : 1;
+    int n_chunks = host_out ? std::min(h->tune.copy_chunks, std::max(E, 1)) : 1;
     c.chunk_events = std::max(1, (E + n_chunks - 1) / n_chunks);
     if (sink) c.chunk_events = std::max(1, std::min(sink->chunk_events, std::max(E, 1)));
     n_chunks = std::max(1, (E + c.chunk_events - 1) / c.chunk_events);
@@ -1624,9 +1601,11 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
         if (lst != ISS_OK) return lst;
     }
 
-    // with decays the records change after sampling: no copies during it
+    // with decays the final lists are copied, not the sampled records
+    const bool any_decays = h->decays && n_units > 0;
     const bool to_host = host_out != nullptr && n_units <= capacity && n_units > 0 && !h->decays;
-    if (to_host) {
+    const bool grouped = to_host || (any_decays && host_out != nullptr);
+    if (to_host || any_decays) {
         st = ensure_copy_stream(h, n_chunks);
         if (st != ISS_OK) return st;
     }
@@ -1657,6 +1636,19 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     }
     CUDA_TRY(h, h->d_hadrons.reserve(static_cast<size_t>(sink ? 2 * ring : headroom(n_units))));
     CUDA_TRY(h, h->d_cell_of.reserve(static_cast<size_t>(sink ? 2 * ring : headroom(n_units))));
+    // The count sweep of the decays needs the segments' offsets only: it runs on
+    // the second stream while the CDF scan ends, ahead of the sampler (beside it,
+    // each of the sweep's kernels waits for long blocks to end).  A group's lists
+    // are written there as soon as it is sampled, and copied out while the next
+    // ones are (2.2 M sampled hadrons on 100,000 cells: 1.49 ms a call, 1.63 with
+    // the writing after all sampling, 1.78 with the sweep there too).
+    DecayRun decay;
+    if (h->decays) {
+        st = decays_begin(h, &decay, n_units, a);
+        if (st != ISS_OK) return st;
+        CUDA_TRY(h, cudaEventRecord(h->ev_join, a));
+        CUDA_TRY(h, cudaStreamWaitEvent(s, h->ev_join, 0));
+    }
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvSampleStart], s));
     if (sink) n_launches += 2 * n_chunks;   // the cell assignment and the sampler
     // hands chunk ch's records (already copied to the host) to the sink
@@ -1714,11 +1706,12 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     // 0.77 ms.)
     const int64_t group_records =
         std::min(h->use_learned ? kLearnedGroupRecords : kGroupRecords, (n_units + 1) / 2);
-    if (to_host && n_chunks > 1) {
+    if (grouped && n_chunks > 1) {
         st = fork_sample_stream(h);
         if (st != ISS_OK) return st;
     }
     int n_groups = 0;
+    std::vector<int> edge{0};   // first event of every group, and the end
     for (int ch = 0; ch < n_chunks && !sink; n_groups++) {
         const int e0 = ch * c.chunk_events;
         const int ch0 = ch;
@@ -1726,7 +1719,8 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
         do {
             ch++;
             e1 = std::min(E, ch * c.chunk_events);
-        } while (ch < n_chunks && (!to_host || h->event_offsets[e1] - h->event_offsets[e0] < group_records));
+        } while (ch < n_chunks && (!grouped || h->event_offsets[e1] - h->event_offsets[e0] < group_records));
+        edge.push_back(e1);
         cudaStream_t gs = (n_groups & 1) ? h->sample_stream : s;
         CUDA_TRY(h, launch_sampler(c, cell_arrays(h), h->d_species.ptr, h->d_pids.ptr, cell_rows(h),
                                    h->d_offsets.ptr, h->d_item_off.ptr, h->d_item_seg.ptr,
@@ -1734,10 +1728,10 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
                                    h->d_hadrons.ptr, h->d_work.ptr + n_groups, h->d_counters.ptr,
                                    h->num_sms, gs));
         n_launches += 2;
+        if (to_host || any_decays) CUDA_TRY(h, cudaEventRecord(h->chunk_ev[n_groups], gs));
         if (to_host) {
             // records of events [e0, e1) are final: copy them while the next group runs
             const int64_t b = h->event_offsets[e0], n = h->event_offsets[e1] - b;
-            CUDA_TRY(h, cudaEventRecord(h->chunk_ev[n_groups], gs));
             CUDA_TRY(h, cudaStreamWaitEvent(h->copy_stream, h->chunk_ev[n_groups], 0));
             if (n > 0)
                 CUDA_TRY(h, cudaMemcpyAsync(host_out + b, h->d_hadrons.ptr + b,
@@ -1750,17 +1744,19 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
         if (st != ISS_OK) return st;
     }
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvSample], s));
-    // the count sweep of the decays needs the segments' offsets only: it runs
-    // beside the cell assignment and the sampler
-    const bool any_decays = h->decays && n_units > 0 && E > 0;
-    DecayRun decay;
+    const auto lists_out = [&] { return decay.total <= capacity && decay.total > 0 ? host_out : nullptr; };
     if (h->decays) {
-        st = decays_begin(h, &decay, n_units, a);
-        if (st == ISS_OK && any_decays) st = decays_count(h, &decay, false, a);
+        for (auto& e : h->ev_decay)
+            if (!e) CUDA_TRY(h, cudaEventCreate(&e));
+        CUDA_TRY(h, cudaEventRecord(h->ev_decay[0], s));
+        if (any_decays) st = decays_count(h, &decay, false, a);
+        if (st == ISS_OK && any_decays) st = decays_write(h, decay, edge, true, lists_out(), a);
         if (st != ISS_OK) {
             cudaStreamSynchronize(s);   // the sampler still runs
+            cudaStreamSynchronize(a);
             return st;
         }
+        CUDA_TRY(h, cudaEventRecord(h->ev_decay[1], a));
     }
     CUDA_TRY(h, cudaMemcpyAsync(&h->eh->ctr, h->d_counters.ptr, sizeof(SampleCounters), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(h, cudaStreamSynchronize(s));
@@ -1777,20 +1773,19 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     unsigned long long decay_failures = 0;
     float ms_decays = 0.f;
     if (any_decays) {
-        for (auto& e : h->ev_decay)
-            if (!e) CUDA_TRY(h, cudaEventCreate(&e));
-        CUDA_TRY(h, cudaEventRecord(h->ev_decay[0], s));
         // abandoned hadrons have no particle id in their records: counted anew
         if (ctr.failures > 0 || ctr.error_code != 0) {
-            st = decays_enqueue(h, &decay, true, s);
-            if (st == ISS_OK) st = decays_count(h, &decay, true, s);
+            CUDA_TRY(h, cudaStreamSynchronize(a));
+            if (h->copy_stream) CUDA_TRY(h, cudaStreamSynchronize(h->copy_stream));
+            st = decays_enqueue(h, &decay, true, a);
+            if (st == ISS_OK) st = decays_count(h, &decay, true, a);
+            if (st == ISS_OK) st = decays_write(h, decay, {0, E}, false, lists_out(), a);
             if (st != ISS_OK) return st;
+            CUDA_TRY(h, cudaEventRecord(h->ev_decay[1], a));
         }
-        bool done = false;
-        st = decays_write(h, decay, host_out, capacity, &done, &decay_failures);
+        st = decays_finish(h, decay, a, &decay_failures);
         if (st != ISS_OK) return st;
-        if (done && copied) *copied = true;
-        CUDA_TRY(h, cudaEventSynchronize(h->ev_decay[1]));
+        if (lists_out() && copied) *copied = true;
         cudaEventElapsedTime(&ms_decays, h->ev_decay[0], h->ev_decay[1]);
     }
 
