@@ -119,17 +119,38 @@ __device__ double qmu_coeff(const double* tb, double T, double muB) {
 // division in the 14-moment lookup, the sums that round to float after each term
 // without the steps that cannot change that float (ff_add_f_float), the products
 // that several components share taken once, and the 128-byte records written
-// only where a kernel reads them: 200,000 cells 108 -> 65 us (69 with the FP64 1/T
-// of the yields, which costs them more), 100,000 cells of a
-// baryon-rich surface 68 -> 50 us.  Unrolling the sums' outer loops as well costs
-// more in instruction fetch than it saves; 4 to 8 blocks per SM measure the same
-// at one wave, and 8 are 10 % faster over several (16 surfaces, 75 -> 68 us).
-__global__ void __launch_bounds__(kPrologueThreads, 8)
+// only where a kernel reads them, and the records read 16 bytes at a time, all
+// in flight at once: 200,000 cells 108 -> 58 us (with the FP64 1/T of the yields,
+// which costs them more), 100,000 cells of a baryon-rich surface 68 -> 43 us.
+// Unrolling the sums' outer loops costs more in instruction fetch than it saves;
+// rolling the rest up around shared memory, a third of the code, measures the
+// same.  6 blocks per SM; 8 spill (63 us) and 4 leave warps out (73 us).
+__global__ void __launch_bounds__(kPrologueThreads, 6)
 cell_prologue_kernel(DevConfig cfg, const float* __restrict__ fo34, int64_t n, CellArrays cells) {
-    __shared__ float s_rec[kPrologueThreads * 34];
+    __shared__ __align__(16) float s_rec[kPrologueThreads * 34];
     const int64_t base = static_cast<int64_t>(blockIdx.x) * kPrologueThreads;
     const int64_t nrec = min(static_cast<int64_t>(kPrologueThreads), n - base);
-    for (int k = threadIdx.x; k < nrec * 34; k += kPrologueThreads) s_rec[k] = fo34[base * 34 + k];
+    {
+        // the block's records, which start on a 16-byte boundary: all of a
+        // thread's reads in flight at once (four bytes each in a loop cost nine
+        // round trips to memory)
+        static_assert(kPrologueThreads * 34 % 4 == 0, "blocks start on a float4");
+        constexpr int kRounds = (kPrologueThreads * 34 / 4 + kPrologueThreads - 1) / kPrologueThreads;
+        const int floats = static_cast<int>(nrec) * 34, quads = floats / 4;
+        const float4* src = reinterpret_cast<const float4*>(fo34 + base * 34);
+        float4 v[kRounds];
+#pragma unroll
+        for (int k = 0; k < kRounds; k++) {
+            const int i = k * kPrologueThreads + threadIdx.x;
+            if (i < quads) v[k] = __ldg(src + i);
+        }
+        for (int i = quads * 4 + threadIdx.x; i < floats; i += kPrologueThreads) s_rec[i] = fo34[base * 34 + i];
+#pragma unroll
+        for (int k = 0; k < kRounds; k++) {
+            const int i = k * kPrologueThreads + threadIdx.x;
+            if (i < quads) reinterpret_cast<float4*>(s_rec)[i] = v[k];
+        }
+    }
     __syncthreads();
     if (threadIdx.x >= nrec) return;
     const int64_t l = base + threadIdx.x;
