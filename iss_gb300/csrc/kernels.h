@@ -37,13 +37,14 @@ struct CdfBuffers {
 // allow_sparse and n_tiles >= kSparseTiles), the scan writes the CDF rows and
 // guide tables of the dense rows.  surf is a device array.
 //
-// A CDF row costs about 4.5 ps per cell to write, a draw on a sparse row some
-// 30 ps more than on a dense one: at 8 cells per draw both calls with few and
-// with many events gain (200,000 cells: 1 event CDF 365 -> 119 us, 300 events
-// 371 -> 185 us; 4, 16 and 32 cells per draw were no better).  Below 2048
-// tiles (13,000 cells of 319 species) the rows are written in a wave or two
-// of blocks, less than the longer search takes.
-constexpr int kSparseDraws = 8;
+// A CDF row costs about 2 ps per cell to write, a draw on a sparse row some
+// 30 ps more than on a dense one: at 16 cells per draw both calls with few and
+// with many events gain (200,000 cells, CDF and sampling together: 1 event 402 ->
+// 124 us, 300 events 1177 -> 1081, 1,000 events 2701 -> 2751 for 475 us less
+// before them; at 8 cells per draw 300 events take 1083 us and 1,000 2794, at 32
+// 1083 and 2762).  Below 2048 tiles (13,000 cells of 319 species) the rows are
+// written in a wave or two of blocks, less than the longer search takes.
+constexpr int kSparseDraws = 16;
 constexpr int64_t kSparseTiles = 2048;
 cudaError_t launch_cdf_head(const float* yields, int64_t N, const SurfSeg* surf, int n_surf,
                             int64_t n_tiles, int S, const uint32_t* ymax, double ymult, bool allow_sparse,

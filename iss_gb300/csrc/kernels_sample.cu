@@ -231,6 +231,12 @@ constexpr int kAssignSpan = 3;
 // where a warp takes several work items, the draws of items of up to this many
 // are dealt out to its lanes (cell_assign_kernel)
 constexpr int kDealtDraws = 16;
+// work items that a warp takes at a time, at most: the warps that run together
+// then stay on neighbouring species, whose rows the L2 holds (200,000 cells and
+// 1,000 events: cell assignment 528 us with single items, 791 with groups of up
+// to 32, which spread the warps over all species and read the rows twice from
+// memory; 300 events, cell assignment and sampler 930 us with 8, 942 with 2)
+constexpr int kAssignGroup = 8;
 
 // Work items are ordered by event chunk (cfg.chunk_events consecutive events),
 // then species, then event: warps that run at the same time mostly sample one
@@ -599,7 +605,7 @@ __device__ __forceinline__ int last_le(const unsigned long long* __restrict__ a,
 // prefix sums C holds v, so the cell is the one a search of the full row finds.
 // Some six rounds of reads and 32 quantised yields: dear per draw, but the row
 // itself need not be written.
-__device__ __noinline__ int sparse_cell(const CellRows& rows, const SurfSeg* __restrict__ surf, int b, int s,
+__device__ __forceinline__ int sparse_cell(const CellRows& rows, const SurfSeg* __restrict__ surf, int b, int s,
                                         unsigned long long v) {
     const SurfSeg sg = surf[b];
     const int64_t tile0 = sg.tile_base + static_cast<int64_t>(s) * sg.nt;
@@ -640,7 +646,7 @@ __device__ __noinline__ int sparse_cell(const CellRows& rows, const SurfSeg* __r
 // (cdf_quantize) -- the reference's binarySearch (src/arsenal.cpp:644-678) on
 // integer sums.  On a dense row the guide bucket j = r >> (64 - g) brackets the
 // cell by guide[j] <= i <= guide[j+1]; when both agree no CDF entry is read.
-__device__ __noinline__ int cell_search(const CellRows& rows, const SurfSeg* __restrict__ surf, int b, int s,
+__device__ __forceinline__ int cell_search_in(const CellRows& rows, const SurfSeg* __restrict__ surf, int b, int s,
                                         unsigned long long r) {
     const SurfSeg& sg = surf[b];
     const int q = b * rows.n_species + s;
@@ -657,6 +663,12 @@ __device__ __noinline__ int cell_search(const CellRows& rows, const SurfSeg* __r
         if (__ldg(row + mid) <= v) lo = mid; else hi = mid - 1;
     }
     return lo;
+}
+
+// as a call, for the kernels that it leaves without spills
+__device__ __noinline__ int cell_search(const CellRows& rows, const SurfSeg* __restrict__ surf, int b, int s,
+                                        unsigned long long r) {
+    return cell_search_in(rows, surf, b, s, r);
 }
 
 // returns false when m/T - mu/T is outside the reference's momentum tables.
@@ -1618,7 +1630,7 @@ cell_assign_kernel(DevConfig cfg_in, const __grid_constant__ CellRows rows, cons
     const int lane = threadIdx.x & 31;
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    const int group = static_cast<int>(min(static_cast<int64_t>(32), max(static_cast<int64_t>(1),
+    const int group = static_cast<int>(min(static_cast<int64_t>(kAssignGroup), max(static_cast<int64_t>(1),
                                                                         (k_end - k_begin) / n_warps)));
     for (int64_t k0 = k_begin + warp * group; k0 < k_end; k0 += n_warps * group) {
         // this lane's item
@@ -1887,7 +1899,10 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
                     const unsigned long long r = (static_cast<unsigned long long>(w.x) << 32) |
                                                  static_cast<unsigned long long>(w.y);
                     const int b = cfg.ev_surf[u.eg - cfg.event_offset];
-                    l = static_cast<int>(cfg.surf[b].c0) + cell_search(rows, cfg.surf, b, u.s, r);
+                    // (inlined where that leaves the kernel without spills: the
+                    // call cost the plain one 16 bytes in its loop, 8 % of its time)
+                    l = static_cast<int>(cfg.surf[b].c0) + (kLearned || kLcc ? cell_search(rows, cfg.surf, b, u.s, r)
+                                                                             : cell_search_in(rows, cfg.surf, b, u.s, r));
                 }
                 u.cell = l;
                 u.tries_cell = 0;
