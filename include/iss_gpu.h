@@ -73,7 +73,8 @@ typedef struct iss_timings {
     int64_t n_cell_redraws;  /* cells redrawn after the try cap (src/FSSW.cpp:1017-1021) */
     int64_t n_failures;   /* hadrons abandoned after the redraw cap (never expected)  */
     int32_t kernel_launches; /* kernels launched by the last iss_gpu_generate (without decays) */
-    double ms_decays;     /* resonance decays (perform_decays = 1), not in ms_total   */
+    double ms_decays;     /* resonance decays after the sampling (perform_decays = 1), not
+                             in ms_total; their count sweep runs before and beside it */
     int32_t decay_reruns; /* decay passes rerun because a buffer was too small (the
                              sizes are then kept for later calls; results unchanged) */
     int64_t n_sampled;    /* hadrons the sampler wrote (before resonance decays)      */
@@ -158,9 +159,12 @@ iss_status iss_gpu_generate(iss_handle* h);
 
 /* iSS::generate_samples followed by reading every event's hadron list
  * (get_hadron_list_iev for iev = 0 .. n_events-1, src/iSS.h:85-91) in one call.
- *   - The sampler runs in up to 16 chunks of consecutive events.
- *   - Each chunk's records are copied into out[0 .. n_total) while the next
- *     chunk is sampled.
+ *   - The events are numbered in up to 16 chunks (iss_tuning_t), and one
+ *     sampler launch takes consecutive chunks until it holds 256k hadrons
+ *     (512k with the learned proposal) or half of them all.
+ *   - A launch's records are copied into out[0 .. n_total) while the next
+ *     ones are sampled; with decays its events' final lists are, as soon as
+ *     they are written.
  *   - `out` should be page-locked (cudaHostAlloc or cudaHostRegister). Then
  *     the copies run beside the sampling.
  *   - The hadrons and their order are those of iss_gpu_generate followed by
@@ -290,7 +294,7 @@ const char* iss_gpu_status_string(int status);
  * for bit.  It changes only the time. */
 typedef struct iss_tuning {
     int32_t item_size;      /* draws per sampler work item: 32, 64, ..., 1024 (default 64) */
-    int32_t yield_groups;   /* species groups per cell in the yields kernel: 1..32 (4)     */
+    int32_t yield_groups;   /* least species groups per 128 cells in the yields kernel: 1..32 (4) */
     int32_t sampler_ctas;   /* sampler blocks of 256 threads per SM: 1..3 (3)               */
     int32_t assign_blocks;  /* cell-assignment blocks per SM: 1..32 (8)                     */
     int32_t copy_chunks;    /* event chunks copied out by iss_gpu_generate_into: 1..64 (16) */

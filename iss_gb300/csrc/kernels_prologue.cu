@@ -114,8 +114,8 @@ __device__ double qmu_coeff(const double* tb, double T, double muB) {
 }
 
 // Bound by the FP64 pipe (two lanes per SM and clock: at 200,000 cells 975,000
-// warp instructions of cosh, sinh and the coefficient lookups took 50 of 108 us)
-// and by the serial float-float sums.  Hence one expm1 for cosh and sinh, one
+// warp instructions of cosh, sinh and five divisions in the coefficient lookups
+// took 50 of 89 us) and by the serial float-float sums.  Hence one expm1 for cosh and sinh, one
 // division in the 14-moment lookup, the sums that round to float after each term
 // without the steps that cannot change that float (ff_add_f_float), the products
 // that several components share taken once, and the 128-byte records written
