@@ -95,9 +95,9 @@ struct iss_handle {
     DevBuf<int2> d_dhash;                 // pid -> particle index (kDecayHash slots)
     int n_decay_particles = 0;
     cudaEvent_t ev_decay[2] = {nullptr, nullptr};
-    // decay work buffers (grow-only): one generation's records (ping-pong),
-    // the per-input arrays of all generations, per-(generation, event) tables
-    // and the final lists
+    // decay work buffers (grow-only): the records of the generations after the
+    // sampled one, the per-input arrays of all generations, per-(generation,
+    // event) tables and the final lists
     DevBuf<HadronRec> dk_u, dk_final;
     DevBuf<int32_t> dk_ev, dk_pid, dk_chan, dk_etot;
     DevBuf<uint8_t> dk_cnt;
@@ -402,9 +402,9 @@ cudaError_t upload_changed(DevBuf<T>& d, std::vector<T>& last, const std::vector
     if (now.empty() || (d.ptr == before && last.size() == now.size() &&
                         std::memcmp(last.data(), now.data(), sizeof(T) * now.size()) == 0))
         return cudaSuccess;
-    last.clear();
-    e = cudaMemcpyAsync(d.ptr, now.data(), sizeof(T) * now.size(), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) last = now;
+    last = now;
+    e = cudaMemcpyAsync(d.ptr, last.data(), sizeof(T) * last.size(), cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) last.clear();
     return e;
 }
 
@@ -820,8 +820,8 @@ float elapsed(iss_handle* h, int a, int b) {
 // all events (kernels_decay.cu); replaces d_hadrons and the event offsets
 // with the final-state lists.  The count sweep runs on the device in batches
 // of kDecayBatch generations with one host wait per batch (the sizes stay on
-// the device); the layout and the write sweep follow, then one wait for the
-// event offsets.  A generation whose products do not fit a buffer ends the
+// the device), ahead of the sampler; the layout follows, and the write sweep
+// group by group as the sampler's groups of events end.  A generation whose products do not fit a buffer ends the
 // count sweep with a flag; the call then reruns the sweep with buffers sized
 // from what it needed (same results).  The work buffers stay allocated in the
 // handle for later calls.
@@ -1125,10 +1125,6 @@ iss_status decays_finish(iss_handle* h, const DecayRun& run, cudaStream_t w, uns
     h->n_hadrons = total;
     return ISS_OK;
 }
-
-// host_out != nullptr: iss_gpu_generate_into -- the sampler runs in chunks of
-// consecutive events and each chunk's records are copied to host_out on a
-// second stream while the next chunk is sampled.
 
 // Learned proposal of one generate: the species whose expected hadrons per
 // cell (over all events) reach gpu_learned_min_hadrons_per_cell, the network
@@ -1449,6 +1445,9 @@ struct StreamSink {
     void* user;
 };
 
+// host_out != nullptr: iss_gpu_generate_into -- the sampler runs in groups of
+// consecutive events, and each group's records (with decays its final lists)
+// are copied to host_out on another stream while the next groups are sampled.
 iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t capacity = 0,
                         bool* copied = nullptr, const StreamSink* sink = nullptr) {
     if (copied) *copied = false;
@@ -1512,7 +1511,7 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     CUDA_TRY(h, h->d_offsets.reserve(static_cast<size_t>(nseg + 1)));
     CUDA_TRY(h, h->d_item_off.reserve(static_cast<size_t>(nseg + 1)));
     CUDA_TRY(h, h->d_off_tiles.reserve(static_cast<size_t>(std::max(offsets_num_tiles(nseg), 1))));
-    // sampling chunks: one without a host destination, else up to kMaxChunks
+    // sampling chunks: one without a host destination, else up to copy_chunks
     const int E = c.n_events;
     int n_chunks = host_out ? std::min(h->tune.copy_chunks, std::max(E, 1)) : 1;
     c.chunk_events = std::max(1, (E + n_chunks - 1) / n_chunks);
