@@ -50,3 +50,16 @@ def test_yields_do_not_depend_on_the_cells_per_thread(n, kind):
     cut = n // 2 + 3
     both = yields(None, kind, [np.ascontiguousarray(fo[:cut]), np.ascontiguousarray(fo[cut:])])
     assert both.tobytes() == whole.tobytes()
+
+
+@pytest.mark.parametrize("kind", ["none", "ce", "14"])
+@pytest.mark.parametrize("T", [(0.1, 0.6), (0.0005, 0.2)])
+def test_arguments_off_the_tables(T, kind):
+    """Pions above 0.27 GeV and every species in very cold cells leave the
+    special-function tables; they are evaluated by a kernel of their own."""
+    n = 3000
+    fo = S.viscous_3d(n, seed=7).fo_surf().copy()
+    fo[:, 13] = np.linspace(*T, n).astype(np.float32)
+    whole = yields(fo, kind)
+    pieces = np.concatenate([yields(np.ascontiguousarray(fo[a:a + 1000]), kind) for a in range(0, n, 1000)], axis=1)
+    assert whole.max() > 0 and whole.tobytes() == np.ascontiguousarray(pieces).tobytes()
