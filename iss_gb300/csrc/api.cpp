@@ -1278,7 +1278,7 @@ cudaError_t enqueue_generate(iss_handle* h, const DevConfig& c) {
     GTRY(cudaStreamWaitEvent(a, h->ev_fork, 0));
     GTRY(cudaMemsetAsync(h->d_error.ptr, 0, sizeof(int), a));
     GTRY(launch_counts(c, h->d_species.ptr, h->d_totals.ptr, h->d_pois.ptr, h->d_counts.ptr,
-                       h->d_items.ptr, h->d_error.ptr, a));
+                       h->d_items.ptr, h->d_error.ptr, nullptr, a));
     GTRY(launch_offsets_scan(h->d_counts.ptr, nseg, h->d_off_tiles.ptr, h->d_offsets.ptr, a));
     GTRY(launch_offsets_scan(h->d_items.ptr, nseg, h->d_off_tiles.ptr, h->d_item_off.ptr, a));
     GTRY(launch_graph_limits(h->d_offsets.ptr, h->d_item_off.ptr, nseg, h->graph_cap_units,
@@ -1545,9 +1545,9 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     CUDA_TRY(h, cudaMemsetAsync(h->d_counters.ptr, 0, sizeof(SampleCounters), a));
     CUDA_TRY(h, cudaMemsetAsync(h->d_error.ptr, 0, sizeof(int), a));
     CUDA_TRY(h, cudaStreamWaitEvent(a, h->ev_fork, 0));
+    int n_launches = 6;   // prologue, yields (2), CDF (3)
     CUDA_TRY(h, launch_counts(c, h->d_species.ptr, h->d_totals.ptr, h->d_pois.ptr, h->d_counts.ptr,
-                              h->d_items.ptr, h->d_error.ptr, a));
-    int n_launches = 6 + (nseg > 0 ? 2 : 0);   // prologue, yields (2), CDF (3); counts (2)
+                              h->d_items.ptr, h->d_error.ptr, &n_launches, a));
     bool mapped = false;
     const CountReport rep{h->eh->sizes, &h->eh->count_err, h->eh->tail, h->eh->tail + E + 1, c.chunk_events, n_chunks};
     CUDA_TRY(h, launch_count_scans(h->d_counts.ptr, h->d_items.ptr, nseg, S, E, h->d_off_tiles.ptr,

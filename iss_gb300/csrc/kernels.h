@@ -56,10 +56,12 @@ cudaError_t launch_cdf_scan(const float* yields, int64_t N, const SurfSeg* surf,
 // kernels_sample.cu
 // two launches: Poisson constants and inversion tables of every (surface,
 // species) row (pois, (kPoissonConsts + kInvTable + 1) doubles per row), then
-// one count per (event, species); totals has n_surfaces * S rows
+// one count per (event, species); totals has n_surfaces * S rows.  With launches
+// (which is raised by their number; null: always the two) one launch for the few
+// events of a single surface.
 cudaError_t launch_counts(const DevConfig& cfg, const SpeciesDev* species, const double* totals,
                           double* pois, int32_t* counts, int32_t* items, int* error,
-                          cudaStream_t stream);
+                          int* launches, cudaStream_t stream);
 // draws per work item of the lab-frame sampler (even: the cell assignment
 // pairs draws)
 constexpr int kEfaItem = 4;

@@ -283,34 +283,19 @@ count_consts_kernel(DevConfig cfg, const double* __restrict__ totals, PoissonC* 
     poisson_inv_table(c, inv[s], threadIdx.x);
 }
 
-// (blocks of 64: one event's 319 draws share the FP64 pipes of five SMs, not two)
-constexpr int kCountThreads = 64;
-
-__global__ void __launch_bounds__(kCountThreads)
-counts_kernel(DevConfig cfg_in, const SpeciesDev* __restrict__ species,
-                              const double* __restrict__ totals,
-                              const PoissonC* __restrict__ pois,
-                              const PoissonInv* __restrict__ inv, int32_t* __restrict__ counts,
-                              int32_t* __restrict__ items, int* __restrict__ error) {
-    const DevConfig cfg = with_run_keys(cfg_in);
-    const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t total = static_cast<int64_t>(cfg.n_events) * cfg.n_species;
-    if (idx >= total) return;
-    // species-major threads: a warp draws one species in consecutive events,
-    // so its lanes take the same branch (inversion table or PTRS) and read
-    // the same constants; every draw is keyed by (event, species)
-    const int s = static_cast<int>(idx / cfg.n_events);
-    const int e = static_cast<int>(idx % cfg.n_events);
+// Count of species s in event e (mean dN; pc0 and inv: the Poisson constants and
+// inversion table of that mean), its records and work items
+__device__ __forceinline__ void draw_count(const DevConfig& cfg, const SpeciesDev& sp, int s, int e, double dN,
+                                           const PoissonC& pc0, const PoissonInv* inv,
+                                           int32_t* __restrict__ counts, int32_t* __restrict__ items,
+                                           int* __restrict__ error) {
     const int64_t seg = static_cast<int64_t>(e) * cfg.n_species + s;
     const uint32_t c2 = cfg.event_offset + static_cast<uint32_t>(e);
     const uint32_t c3 = static_cast<uint32_t>(s) | (kTagCount << 16);
-    const int row = cfg.ev_surf[e] * cfg.n_species + s;    // (surface, species)
-    const double dN = __dmul_rn(totals[row], cfg.ymult);
     const int64_t dN_int = static_cast<int64_t>(dN);
     const double frac = __dadd_rn(dN, -static_cast<double>(dN_int));
     const double para1 = cfg.sampling_para1;
     int64_t nsamp = 0;
-    const SpeciesDev sp = species[s];
     if (cfg.lcc && sp.charge < 0) {
         nsamp = 0;   // sampled as partners of the positive species
     } else if (dN < 0) {
@@ -325,20 +310,63 @@ counts_kernel(DevConfig cfg_in, const SpeciesDev* __restrict__ species,
             nsamp = dN_int;
         } else {
             const double g = gamma_draw(c2, c3, cfg.key0, cfg.key1, 0u, kk);
-            const PoissonC pc = poisson_consts(__dmul_rn(g, __dadd_rn(1.0, -p)) / p);
-            const int64_t nb = poisson_draw(c2, c3, cfg.key0, cfg.key1, 1u << 20, pc, cfg.tab.logfact);
+            const PoissonC pg = poisson_consts(__dmul_rn(g, __dadd_rn(1.0, -p)) / p);
+            const int64_t nb = poisson_draw(c2, c3, cfg.key0, cfg.key1, 1u << 20, pg, cfg.tab.logfact);
             nsamp = (cfg.sampling_model == 10) ? dN_int + nb : nb;
             if (g < 0.0 || nb < 0) atomicCAS(error, 0, 3);
         }
     } else {
         nsamp = (dN < 1e-15) ? 0
-                             : poisson_draw(c2, c3, cfg.key0, cfg.key1, 0u, pois[row],
-                                            cfg.tab.logfact, inv + row);
+                             : poisson_draw(c2, c3, cfg.key0, cfg.key1, 0u, pc0,
+                                            cfg.tab.logfact, inv);
         if (nsamp < 0) atomicCAS(error, 0, 3);
     }
     const int32_t c = static_cast<int32_t>(nsamp < 0 ? 0 : nsamp);
     counts[seg] = c * records_per_draw(cfg, sp);       // records of the segment
     items[item_index(cfg, e, s)] = (c + cfg.item_size - 1) / cfg.item_size;
+}
+
+// (blocks of 64: one event's 319 draws share the FP64 pipes of five SMs, not two)
+constexpr int kCountThreads = 64;
+
+__global__ void __launch_bounds__(kCountThreads)
+counts_kernel(DevConfig cfg_in, const SpeciesDev* __restrict__ species,
+              const double* __restrict__ totals, const PoissonC* __restrict__ pois,
+              const PoissonInv* __restrict__ inv, int32_t* __restrict__ counts,
+              int32_t* __restrict__ items, int* __restrict__ error) {
+    const DevConfig cfg = with_run_keys(cfg_in);
+    const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t total = static_cast<int64_t>(cfg.n_events) * cfg.n_species;
+    if (idx >= total) return;
+    // species-major threads: a warp draws one species in consecutive events,
+    // so its lanes take the same branch (inversion table or PTRS) and read
+    // the same constants; every draw is keyed by (event, species)
+    const int s = static_cast<int>(idx / cfg.n_events);
+    const int e = static_cast<int>(idx % cfg.n_events);
+    const int row = cfg.ev_surf[e] * cfg.n_species + s;    // (surface, species)
+    draw_count(cfg, species[s], s, e, __dmul_rn(totals[row], cfg.ymult), pois[row], inv + row, counts, items, error);
+}
+
+// Constants, table and counts of one surface's few events in one launch, a warp
+// and a block per species: the FP64 chains of both kernels are latency, which
+// this takes once, and one event's draws spread over 319 blocks instead of five
+// (a call of one event on 1,245 cells 177 -> 165 us, on 200,000 cells 592 -> 572).
+// Up to an event per lane: CDF and counts of 5,000 cells take 50, 56, 93 and
+// 110 us so with 1, 8, 32 and 64 events, 71, 73, 106 and 105 us in two launches.
+constexpr int kFewEvents = 32;
+
+__global__ void __launch_bounds__(32)
+counts_few_kernel(DevConfig cfg, const SpeciesDev* __restrict__ species, const double* __restrict__ totals,
+                  int32_t* __restrict__ counts, int32_t* __restrict__ items, int* __restrict__ error) {
+    __shared__ PoissonInv s_inv;
+    const int s = blockIdx.x;
+    const double dN = __dmul_rn(totals[s], cfg.ymult);
+    const PoissonC c = poisson_consts(dN);
+    poisson_inv_table(c, s_inv, threadIdx.x);
+    __syncwarp();
+    const SpeciesDev sp = species[s];
+    for (int e = threadIdx.x; e < cfg.n_events; e += 32)
+        draw_count(cfg, sp, s, e, dN, c, &s_inv, counts, items, error);
 }
 
 // item -> segment map: item_seg[item_off[q] + k] = q for k < items[q], q the
@@ -2365,9 +2393,15 @@ __global__ void learned_train_rows_kernel(DevConfig cfg, CellArrays cells,
 
 cudaError_t launch_counts(const DevConfig& cfg, const SpeciesDev* species, const double* totals,
                           double* pois, int32_t* counts, int32_t* items, int* error,
-                          cudaStream_t stream) {
+                          int* launches, cudaStream_t stream) {
     const int64_t total = static_cast<int64_t>(cfg.n_events) * cfg.n_species;
     if (total <= 0) return cudaSuccess;
+    if (launches && cfg.n_surfaces == 1 && cfg.n_events <= kFewEvents) {
+        counts_few_kernel<<<cfg.n_species, 32, 0, stream>>>(cfg, species, totals, counts, items, error);
+        *launches += 1;
+        return cudaGetLastError();
+    }
+    if (launches) *launches += 2;
     const int rows = cfg.n_surfaces * cfg.n_species;
     PoissonC* pc = reinterpret_cast<PoissonC*>(pois);
     PoissonInv* inv = reinterpret_cast<PoissonInv*>(pc + rows);
