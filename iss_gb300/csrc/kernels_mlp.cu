@@ -327,14 +327,19 @@ mlp_loss_kernel(const float* __restrict__ out, const float4* __restrict__ target
                      vy * tg.z + vz * tg.w;
     const float cmax = row_max(lc);
     const float L = cmax + logf(row_sum(expf(lc - cmax)));
-    if (on) {
-        const float r = live ? expf(lc - L) : 0.0f;
-        const float w = live ? expf(zk - lse_w) : 0.0f;
+    float* g = dout + row * kOut;
+    if (on && !live) {
+        // stored zeros, not products with zero: the direction of such a row may
+        // be anything, a NaN too
+#pragma unroll
+        for (int j = 0; j < kOut; j += 8) g[j + k] = 0.0f;
+    } else if (on) {
+        const float r = expf(lc - L);
+        const float w = expf(zk - lse_w);
         const float gk = langevin_over_kappa(kap);
-        float* g = dout + row * kOut;
         g[k] = (w - r) * inv_n;
         g[8 + k] = -r * d * is2 * inv_n;
-        g[16 + k] = (live && sraw > kLogSigMin && sraw < kLogSigMax) ? -r * (d * d * is2 - 1.0f) * inv_n : 0.0f;
+        g[16 + k] = (sraw > kLogSigMin && sraw < kLogSigMax) ? -r * (d * d * is2 - 1.0f) * inv_n : 0.0f;
         g[24 + 3 * k] = -r * (tg.y - gk * vx) * inv_n;
         g[25 + 3 * k] = -r * (tg.z - gk * vy) * inv_n;
         g[26 + 3 * k] = -r * (tg.w - gk * vz) * inv_n;
