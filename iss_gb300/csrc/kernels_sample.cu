@@ -2093,14 +2093,16 @@ efa_sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restr
             const auto propose = [&](const PropEfa& p, int l, int limit, int phase) {
                 const float bound = efa_bin_bound(cfg, p, lane);
                 int queued = 0;
-                for (int b0 = 0; b0 < limit; b0 += 32 * kEfaUnroll) {
+                // counted down: the cap is a user's, up to 2^31 - 1, and counting up
+                // in steps of 128 would run past it
+                uint32_t t0 = t + static_cast<uint32_t>(lane);
+                for (int left = limit; left > 0; left -= 32 * kEfaUnroll, t0 += 32u * kEfaUnroll) {
                     uint32_t x[kEfaUnroll], w[kEfaUnroll];
-                    const uint32_t t0 = t + static_cast<uint32_t>(b0 + lane);
                     efa_words(stream, t0, c3, cfg.key0, cfg.key1, x, w);
 #pragma unroll
                     for (int j = 0; j < kEfaUnroll; j++) {
                         const float bnd = __shfl_sync(FULL, bound, static_cast<int>(x[j] >> 27));
-                        const bool keep = b0 + 32 * j + lane < limit && !(u01f(w[j]) >= bnd);
+                        const bool keep = 32 * j + lane < left && !(u01f(w[j]) >= bnd);
                         const unsigned kept = __ballot_sync(FULL, keep);
                         if (keep) queue[queued + __popc(kept & ((1u << lane) - 1u))] = t0 + 32u * j;
                         queued += __popc(kept);
@@ -2108,7 +2110,7 @@ efa_sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restr
                     __syncwarp();
                     // evaluate the queue when it is worth a warp's while, at the end
                     // all of it (a hadron found late has cost proposals too many)
-                    const int enough = b0 + 32 * kEfaUnroll < limit ? kEfaBatch : 1;
+                    const int enough = left > 32 * kEfaUnroll ? kEfaBatch : 1;
                     int head = 0;
                     for (; queued - head >= enough; head += 32) {
                         float4 pl;
