@@ -108,6 +108,24 @@ __device__ __forceinline__ double log_factorial(const double* __restrict__ table
                      __dmul_rn(r, t));
 }
 
+// by a thread, or (below) by a warp
+__device__ void poisson_inv_table(const PoissonC& c, PoissonInv& t) {
+    t.len = 0;
+    if (!(c.mu < 12.0)) return;
+    double p = c.emu, cdf = p;
+    t.icdf[0] = floor_2p53(cdf);
+    for (int k = 1; k < kInvTable; k++) {
+        p = __dmul_rn(p, c.mu / static_cast<double>(k));
+        const double next = __dadd_rn(cdf, p);
+        if (next == cdf && static_cast<double>(k) > c.mu) {
+            t.len = k;
+            return;
+        }
+        cdf = next;
+        t.icdf[k] = floor_2p53(cdf);
+    }
+}
+
 // by a warp: the quotients mu / k, four per lane, in parallel; then every lane
 // forms the sums in the loop's own order and keeps the entries k = lane + 32 j
 __device__ void poisson_inv_table(const PoissonC& c, PoissonInv& t, int lane) {
@@ -269,10 +287,18 @@ __device__ __forceinline__ void item_decode(const DevConfig& cfg, int q, int& e,
     e = e0 + (r - s * ne);
 }
 
-// Poisson constants and inversion table of the model-30 draws (same mu in every
-// event), a warp and a block per (surface, species) row: the FP64 chains are
-// bound by latency, and a block each spreads them over the SMs' narrow FP64
-// pipes (319 rows: 32 us with a thread per row, 4 us so)
+// Poisson constants and inversion tables of the model-30 draws (same mu in every
+// event), one per (surface, species) row, in one of two forms.
+//
+// Up to kWarpRows rows a warp and a block take a row: the FP64 chain of one row is
+// latency, which the parallel quotients shorten, and a block each spreads the rows
+// over the SMs' narrow FP64 pipes.  Its 32 lanes repeat the chain, though, so with
+// more rows the pipes are full of repeated work and a thread takes a row, in
+// blocks of a warp.  Rows of 319 species, a warp against a thread per row: 319
+// rows 12 and 33 us, 1,914 20 and 33, 3,828 31 and 33, 5,104 40 and 33, 20,416
+// 138 and 35, 81,664 517 and 57 us.
+constexpr int kWarpRows = 4096;
+
 __global__ void __launch_bounds__(32)
 count_consts_kernel(DevConfig cfg, const double* __restrict__ totals, PoissonC* __restrict__ pois,
                     PoissonInv* __restrict__ inv) {
@@ -281,6 +307,17 @@ count_consts_kernel(DevConfig cfg, const double* __restrict__ totals, PoissonC* 
     const PoissonC c = poisson_consts(dN);
     if (threadIdx.x == 0) pois[s] = c;
     poisson_inv_table(c, inv[s], threadIdx.x);
+}
+
+__global__ void __launch_bounds__(32)
+count_consts_rows_kernel(DevConfig cfg, const double* __restrict__ totals, PoissonC* __restrict__ pois,
+                         PoissonInv* __restrict__ inv) {
+    const int s = blockIdx.x * 32 + threadIdx.x;
+    if (s >= cfg.n_surfaces * cfg.n_species) return;
+    const double dN = __dmul_rn(totals[s], cfg.ymult);
+    const PoissonC c = poisson_consts(dN);
+    pois[s] = c;
+    poisson_inv_table(c, inv[s]);
 }
 
 // Count of species s in event e (mean dN; pc0 and inv: the Poisson constants and
@@ -2407,7 +2444,10 @@ cudaError_t launch_counts(const DevConfig& cfg, const SpeciesDev* species, const
     const int rows = cfg.n_surfaces * cfg.n_species;
     PoissonC* pc = reinterpret_cast<PoissonC*>(pois);
     PoissonInv* inv = reinterpret_cast<PoissonInv*>(pc + rows);
-    count_consts_kernel<<<rows, 32, 0, stream>>>(cfg, totals, pc, inv);
+    if (rows <= kWarpRows)
+        count_consts_kernel<<<rows, 32, 0, stream>>>(cfg, totals, pc, inv);
+    else
+        count_consts_rows_kernel<<<(rows + 31) / 32, 32, 0, stream>>>(cfg, totals, pc, inv);
     const unsigned blocks = static_cast<unsigned>((total + kCountThreads - 1) / kCountThreads);
     counts_kernel<<<blocks, kCountThreads, 0, stream>>>(cfg, species, totals, pc, inv, counts, items, error);
     return cudaGetLastError();
