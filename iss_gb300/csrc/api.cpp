@@ -299,11 +299,16 @@ iss_status fail(iss_handle* h, iss_status st, const char* fmt, ...) {
     return st;
 }
 
+// (the runtime keeps a failed call's error for the thread's next
+// cudaGetLastError, where the launches of a later call, on this handle or
+// another, would take it for their own: it is cleared here)
 #define CUDA_TRY(h, call)                                                                   \
     do {                                                                                    \
         cudaError_t _e = (call);                                                            \
-        if (_e != cudaSuccess)                                                              \
+        if (_e != cudaSuccess) {                                                            \
+            cudaGetLastError();                                                             \
             return fail((h), ISS_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(_e)); \
+        }                                                                                   \
     } while (0)
 
 // The species list of the yields kernel (YieldGroup, device_common.cuh).  The
