@@ -2621,24 +2621,33 @@ iss_status iss_gpu_learned_train(iss_handle* h, const iss_learned_train_t* opt, 
         return fail(h, ISS_ERR_UNSUPPORTED, "training rows with local_charge_conservation");
     if (!h->batch_cells.empty())
         return fail(h, ISS_ERR_UNSUPPORTED, "training rows from a batch of surfaces");
-    // the plain sampler draws the training momenta; the caller's settings come back afterwards
-    const char* keys[] = {"gpu_sampler", "perform_decays", "number_of_repeated_sampling",
-                          "sample_upto_desired_particle_number", "gpu_event_offset"};
-    double saved[5];
-    bool had[5];
-    for (int i = 0; i < 5; i++) had[i] = h->params.get(keys[i], &saved[i]);
-    const int64_t saved_seed = h->seed;
-    const bool saved_seed_set = h->seed_set;
-    auto restore = [&]() {
-        for (int i = 0; i < 5; i++) {
-            if (had[i]) h->params.set(keys[i], saved[i]);
-            else h->params.erase(keys[i]);
+    // the plain sampler draws the training momenta; the caller's settings come
+    // back afterwards, on every way out
+    struct CallerSettings {
+        iss_handle* h;
+        const char* keys[5] = {"gpu_sampler", "perform_decays", "number_of_repeated_sampling",
+                               "sample_upto_desired_particle_number", "gpu_event_offset"};
+        double saved[5];
+        bool had[5];
+        int64_t seed;
+        bool seed_set, kept = true;
+        explicit CallerSettings(iss_handle* handle) : h(handle), seed(handle->seed), seed_set(handle->seed_set) {
+            for (int i = 0; i < 5; i++) had[i] = h->params.get(keys[i], &saved[i]);
         }
-        h->seed = saved_seed;
-        h->seed_set = saved_seed_set;
-        h->samples_valid = false;
-        h->want_records = false;
-    };
+        ~CallerSettings() { restore(); }
+        void restore() {
+            if (!kept) return;
+            kept = false;
+            for (int i = 0; i < 5; i++) {
+                if (had[i]) h->params.set(keys[i], saved[i]);
+                else h->params.erase(keys[i]);
+            }
+            h->seed = seed;
+            h->seed_set = seed_set;
+            h->samples_valid = false;
+            h->want_records = false;
+        }
+    } caller(h);
     h->want_records = true;
     h->params.set("gpu_sampler", 0);
     h->params.set("perform_decays", 0);
@@ -2649,20 +2658,14 @@ iss_status iss_gpu_learned_train(iss_handle* h, const iss_learned_train_t* opt, 
     h->params.set("number_of_repeated_sampling", 1);
     h->seed = opt->first_seed;
     st = run_generate(h);
-    if (st != ISS_OK) {
-        restore();
-        return st;
-    }
+    if (st != ISS_OK) return st;
     double per_event = 0.0;
     {
         std::vector<double> tot(h->species.size());
         CUDA_TRY(h, cudaMemcpy(tot.data(), h->d_totals.ptr, 8 * tot.size(), cudaMemcpyDeviceToHost));
         for (double v : tot) per_event += v * h->cfg.ymult;
     }
-    if (!(per_event > 0.0)) {
-        restore();
-        return fail(h, ISS_ERR_SAMPLING, "the surface emits no hadrons");
-    }
+    if (!(per_event > 0.0)) return fail(h, ISS_ERR_SAMPLING, "the surface emits no hadrons");
     const int64_t per_seed = (opt->n_momenta + opt->n_seeds - 1) / opt->n_seeds;
     const int ev = static_cast<int>(std::min<double>(1e7, std::ceil(1.02 * per_seed / per_event) + 1));
     // sorted PDG ids -> species index
@@ -2689,10 +2692,7 @@ iss_status iss_gpu_learned_train(iss_handle* h, const iss_learned_train_t* opt, 
         h->params.set("number_of_repeated_sampling", ev);
         h->seed = static_cast<int64_t>(opt->first_seed) + k;
         st = run_generate(h);
-        if (st != ISS_OK) {
-            restore();
-            return st;
-        }
+        if (st != ISS_OK) return st;
         const int64_t take = std::min<int64_t>({h->n_hadrons, per_seed, opt->n_momenta - filled});
         CUDA_TRY(h, launch_learned_train_rows(h->cfg, cell_arrays(h), h->d_species.ptr, h->d_spid.ptr,
                                               h->d_spid.ptr + S, S, h->d_hadrons.ptr, h->d_cell_of.ptr,
@@ -2704,7 +2704,7 @@ iss_status iss_gpu_learned_train(iss_handle* h, const iss_learned_train_t* opt, 
     CUDA_TRY(h, cudaMemcpyAsync(&nll_plain, L.loss.ptr, sizeof(double), cudaMemcpyDeviceToHost,
                                 h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    restore();
+    caller.restore();
     L.n_data = filled;
     h->lstats.train_nll_plain = filled > 0 ? nll_plain / static_cast<double>(filled) : 0.0;
     h->lstats.n_train_rows = filled;
