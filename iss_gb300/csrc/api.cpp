@@ -2683,6 +2683,9 @@ iss_status iss_gpu_learned_train(iss_handle* h, const iss_learned_train_t* opt, 
         CUDA_TRY(h, cudaMemcpy(h->d_spid.ptr, tab.data(), 4 * tab.size(), cudaMemcpyHostToDevice));
     }
     const int S = static_cast<int>(h->species.size());
+    // no rows are held until the new ones are all there: a buffer that grows
+    // gives the old ones up first, also where it then finds no memory
+    L.n_data = 0;
     CUDA_TRY(h, L.data_x.reserve(static_cast<size_t>(opt->n_momenta) * mlp::kIn0));
     CUDA_TRY(h, L.data_t.reserve(static_cast<size_t>(opt->n_momenta)));
     CUDA_TRY(h, L.loss.reserve(std::max<size_t>(static_cast<size_t>(opt->n_steps), 1)));

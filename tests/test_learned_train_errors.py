@@ -38,3 +38,23 @@ def test_failed_training_leaves_the_handle_alone():
     had, o = sample(s)
     assert np.array_equal(o, off) and had.tobytes() == ref.tobytes()
     s.close()
+
+
+def test_failed_training_holds_no_rows():
+    """The rows held before went with their buffer: more steps on them, and
+    reading them, are refused."""
+    s = handle()
+    s.set_params(perform_decays=0)
+    s.learned_train(n_momenta=4000, n_seeds=1, n_steps=2, batch=256)
+    rows, _ = s.learned_rows(0, 4000)
+    assert np.abs(rows).max() > 0
+    with pytest.raises(IssError):
+        s.learned_train(n_momenta=1 << 44, n_seeds=1, n_steps=1)
+    with pytest.raises(IssError, match="needs training rows"):
+        s.learned_train(n_momenta=0, n_seeds=1, n_steps=1)
+    with pytest.raises(IssError, match="0 training rows held"):
+        s.learned_rows(0, 1)
+    s.learned_train(n_momenta=4000, n_seeds=1, n_steps=2, batch=256)
+    again, _ = s.learned_rows(0, 4000)
+    assert np.array_equal(again, rows)
+    s.close()
