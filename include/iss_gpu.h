@@ -293,9 +293,11 @@ const char* iss_gpu_status_string(int status);
  * (draw, hadron, event, species), so any shape gives the same hadrons bit
  * for bit.  It changes only the time. */
 typedef struct iss_tuning {
-    int32_t item_size;      /* draws per sampler work item: 32, 64, ..., 1024 (default 64) */
+    int32_t item_size;      /* draws per sampler work item: 32, 64, ..., 1024 (default 64);
+                               without effect for MC_sampling = 2, whose items are 4 draws */
     int32_t yield_groups;   /* least species groups per 128 cells in the yields kernel: 1..32 (4) */
-    int32_t sampler_ctas;   /* sampler blocks of 256 threads per SM: 1..3 (3)               */
+    int32_t sampler_ctas;   /* sampler blocks of 256 threads per SM: 1..3 (3); the learned
+                               sampler takes 2 at most, that of MC_sampling = 2 always 4    */
     int32_t assign_blocks;  /* cell-assignment blocks per SM: 1..32 (8)                     */
     int32_t copy_chunks;    /* event chunks copied out by iss_gpu_generate_into: 1..64 (16) */
 } iss_tuning_t;
@@ -305,9 +307,11 @@ iss_status iss_gpu_set_tuning(iss_handle* h, const iss_tuning_t* tuning);
  * candidate launch shapes and keeps the fastest: species groups per cell by
  * the yields phase, then draws per work item, sampler blocks per SM and
  * cell-assignment blocks per SM by the sample phase (coordinate descent, two
- * generates per candidate, a 2 % margin to switch).  The result is cached per
- * workload shape (cells, surfaces, events, species, local charge
- * conservation, sampler, hydro mode) for every handle of the process; with
+ * generates per candidate, a 2 % margin to switch).  What the call's sampler
+ * does not take is left as it is.  The result is cached per workload shape and
+ * kernels (cells, surfaces, events, species, local charge conservation,
+ * sampler, MC_sampling, gpu_compat_fermion_cdf2, diffusion, bulk form, hydro
+ * mode) for every handle of the process; with
  * gpu_autotune = 1 the first generate of a new shape tunes or takes the
  * cached shape.  Leaves the samples of its last trial; ms_before / ms_after
  * (optional) are the device times of one generate. */

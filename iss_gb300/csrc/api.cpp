@@ -1841,8 +1841,9 @@ bool tuning_valid(const iss_tuning_t& t) {
            t.assign_blocks <= 32 && t.copy_chunks >= 1 && t.copy_chunks <= 64;
 }
 
-// Tuning results per workload shape, shared by the handles of the process.
-using TuneKey = std::tuple<int64_t, int64_t, int, int, int, int, int>;
+// Tuning results per workload shape and kernels (the sampler's and the yields'
+// instantiations), shared by the handles of the process.
+using TuneKey = std::tuple<int64_t, int64_t, int, int, int, int, int, int, int, int, int>;
 std::mutex g_tune_mutex;
 std::map<TuneKey, iss_tuning_t> g_tune_cache;
 
@@ -1852,7 +1853,12 @@ TuneKey tune_key(iss_handle* h) {
                    static_cast<int>(h->species.size()),
                    static_cast<int>(h->params.get_or("local_charge_conservation", 0)),
                    static_cast<int>(h->params.get_or("gpu_sampler", 0)),
-                   static_cast<int>(h->params.get_or("hydro_mode", 2))};
+                   static_cast<int>(h->params.get_or("hydro_mode", 2)),
+                   static_cast<int>(h->params.get_or("MC_sampling", 4)),
+                   static_cast<int>(h->params.get_or("gpu_compat_fermion_cdf2", 0)),
+                   static_cast<int>(h->params.get_or("include_deltaf_diffusion", 0)),
+                   h->params.get_or("include_deltaf_bulk", 0) == 1
+                       ? static_cast<int>(h->params.get_or("bulk_deltaf_kind", 1)) : -1};
 }
 
 // Coordinate descent over the launch shape on the handle's own workload:
@@ -1860,6 +1866,8 @@ TuneKey tune_key(iss_handle* h) {
 // item, sampler CTAs per SM and cell-assignment blocks per SM (objective: the
 // sample phase).  Each candidate runs two generates and keeps the faster
 // device time; a candidate replaces the incumbent only when it is 2 % faster.
+// What the call's sampler does not take is not measured: the lab-frame sampler
+// has its own work items and blocks, the learned one two blocks per SM at most.
 iss_status autotune(iss_handle* h, double* ms_before, double* ms_after) {
     auto measure = [&](const iss_tuning_t& t, double* y, double* smp, double* tot) -> iss_status {
         h->tune = t;
@@ -1893,8 +1901,9 @@ iss_status autotune(iss_handle* h, double* ms_before, double* ms_after) {
     // the sample phase: re-measure the incumbent with the chosen groups
     if ((st = measure(best, &by, &bs, &bt)) != ISS_OK) return st;
     const int items[] = {32, 64, 128, 256, 512};
+    const bool lab_frame = h->cfg.mc_sampling == 2;
     for (int it : items) {
-        if (it == best.item_size) continue;
+        if (lab_frame || it == best.item_size) continue;
         iss_tuning_t t = best;
         t.item_size = it;
         double y, smp, tot;
@@ -1905,8 +1914,9 @@ iss_status autotune(iss_handle* h, double* ms_before, double* ms_after) {
         }
     }
     const int ctas[] = {2, 3};
+    const int most = h->use_learned ? 2 : 3;
     for (int c : ctas) {
-        if (c == best.sampler_ctas) continue;
+        if (lab_frame || std::min(c, most) == std::min<int>(best.sampler_ctas, most)) continue;
         iss_tuning_t t = best;
         t.sampler_ctas = c;
         double y, smp, tot;
