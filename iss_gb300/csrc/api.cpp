@@ -150,8 +150,8 @@ struct iss_handle {
     DevBuf<int32_t> d_counts, d_items, d_item_seg, d_guide, d_cell_of, d_ev_surf;
     DevBuf<SurfSeg> d_surf;
     // what the small inputs above hold (upload_changed), and the yield list of
-    // up_species
-    std::vector<SpeciesDev> up_species;
+    // ylist_species
+    std::vector<SpeciesDev> up_species, ylist_species;
     std::vector<int32_t> up_pids, up_ev_surf;
     std::vector<float4> up_ylist, ylist;
     std::vector<SurfSeg> up_segs;
@@ -706,9 +706,13 @@ iss_status prepare(iss_handle* h) {
     // (same float-float mass, statistics and number of terms) form one group
     // of the yields kernel; the series runs once per group and cell whenever
     // the members' chemical potentials agree in that cell
-    if (h->ylist.empty() || h->up_species.size() != sd.size() ||
-        std::memcmp(h->up_species.data(), sd.data(), sizeof(SpeciesDev) * sd.size()) != 0)
+    // (kept while the species it was made from are these: what is on the device
+    // says less, since an empty species list uploads nothing)
+    if (h->ylist.empty() || h->ylist_species.size() != sd.size() ||
+        (!sd.empty() && std::memcmp(h->ylist_species.data(), sd.data(), sizeof(SpeciesDev) * sd.size()) != 0)) {
         h->ylist = yield_list(sd, &h->n_ygroups, &h->n_yruns);
+        h->ylist_species = sd;
+    }
     c.n_ygroups = h->n_ygroups;
     c.n_yruns = h->n_yruns;
     CUDA_TRY(h, upload_changed(h->d_species, h->up_species, sd, h->stream));
