@@ -1334,6 +1334,9 @@ iss_status capture_graph(iss_handle* h, int64_t n_items) {
                                    sizeof(GraphHost) + sizeof(int64_t) * static_cast<size_t>(E + 1)));
         h->gh_events = static_cast<size_t>(E);
     }
+    // (replays copy the offsets there, without a species none: every event is
+    // empty then, whatever an earlier graph left)
+    std::fill(h->gh->event_offsets, h->gh->event_offsets + E + 1, 0);
     h->graph_cap_units = static_cast<int64_t>(h->d_hadrons.cap);
     h->graph_cap_items = static_cast<int64_t>(h->d_item_seg.cap);
     if (h->graph_cap_items < n_items) return ISS_OK;

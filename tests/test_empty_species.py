@@ -1,6 +1,7 @@
 """A species list that becomes empty and comes back: a user's table folder whose
 list for one afterburner names no particle samples no hadron there, and the
-handle's next call with the full list is that of a fresh handle, bit for bit."""
+handle's next call with the full list is that of a fresh handle, bit for bit, also
+with replayed graphs."""
 import shutil
 
 import numpy as np
@@ -23,7 +24,7 @@ def sample(s, afterburner, fo):
     return had.copy(), np.asarray(off).copy(), s.species_yields()
 
 
-@pytest.mark.parametrize("graph", [0])
+@pytest.mark.parametrize("graph", [0, 1])
 def test_the_full_list_after_an_empty_one(tmp_path, graph):
     tables = tmp_path / "iSS_tables"
     shutil.copytree(S.TABLE_DIR, tables)
