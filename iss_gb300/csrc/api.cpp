@@ -782,7 +782,7 @@ iss_status run_cells(iss_handle* h) {
     CUDA_TRY(h, h->d_totals.reserve(rows));
     CUDA_TRY(h, h->d_sparse.reserve(rows));
     CUDA_TRY(h, h->d_qtot.reserve(rows));
-    CUDA_TRY(h, h->d_ymax.reserve(rows + 1));   // and launch_yields' flag
+    CUDA_TRY(h, h->d_ymax.reserve(rows + kYieldFlags));
     CUDA_TRY(h, h->d_guide.reserve(static_cast<size_t>(std::max<int64_t>(h->guide_len, 1))));
     const CellArrays cells = cell_arrays(h);
     CUDA_TRY(h, cudaEventRecord(h->ev[kEvStart], st));

@@ -11,10 +11,12 @@ namespace iss {
 // kernels_cells.cu
 cudaError_t launch_cell_prologue(const DevConfig& cfg, const float* fo34, int64_t n,
                                  const CellArrays& cells, cudaStream_t stream);
-// per-cell yields [species][cell] and, in ymax (n_surf * S rows and one flag
-// behind them, zeroed here first), the largest yield of every (surface,
+// per-cell yields [species][cell] and, in ymax (n_surf * S rows and kYieldFlags
+// words behind them, zeroed here first), the largest yield of every (surface,
 // species) row as float bits; two launches, the second of which leaves at once
 // unless an argument was off the special-function tables
+constexpr int kOffRows = 16;
+constexpr int kYieldFlags = 1 + kOffRows;
 cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, float* yields, uint32_t* ymax,
                           int num_sms, cudaStream_t stream);
 int cdf_num_tiles(int64_t n);

@@ -553,30 +553,56 @@ yields_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yields, uint3
     }
 }
 
+// Whether a term of the group's series has an argument off the special-function
+// tables in this cell (thermal_series: n x_1 grows with n, so the first and the
+// last term tell) and the direct evaluation gives other than the zero that
+// yields_kernel left (K_n is zero above 700, in every term above x_1)
+__device__ __forceinline__ bool off_series(const CellYieldIn& c, const YieldGroup& gr) {
+    const float x1 = __fmul_rn(gr.m_hi, c.b_hi);
+    const float xn = __fmul_rn(gr.light && c.warm ? 10.0f : 1.0f, x1);
+    return !(x1 >= 0.5f && xn <= 399.95f) && !(x1 > 701.0f);
+}
+
 // The yields that yields_kernel left out, where it left out any: the series
-// with an argument off the tables, evaluated directly.  A thread per cell and
-// gridDim.y rows of groups.
+// with an argument off the tables, evaluated directly.  Row y of the grid takes
+// every kOffRows-th group; its warps fetch 32 cells at a time, since 32 hot cells
+// cost a thousand times what others do: in a grid over the cells whose blocks
+// took one turn or two, all waited for those with two.  Bound by the FP64 pipe.
+// Calls of 50,000 cells at 0.3 GeV 15.6 -> 11.3 ms (11.6 with the evaluation
+// inlined in the yields kernel), at 5 MeV 2.13 -> 1.41 (1.46; 1.59 in 8 rows
+// instead of 16), 20,000 at 0.5 MeV, where all is zero, 0.37 -> 0.15 (0.28).
 template <int kBulk, bool kDiff>
 __global__ void __launch_bounds__(kYieldThreads)
 yields_off_table_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yields, uint32_t* __restrict__ ymax,
-                        const uint32_t* __restrict__ off_table) {
+                        uint32_t* __restrict__ off_table) {
     if (*off_table == 0u) return;
+    extern __shared__ float4 s_dyn[];
+    constexpr unsigned FULL = 0xffffffffu;
     const int nsp = cfg.n_species;
     const int G = cfg.n_ygroups;
-    const YieldGroup* groups = reinterpret_cast<const YieldGroup*>(cfg.ylist);
-    const float4* list = cfg.ylist + G + cfg.n_yruns;
+    const int words4 = yield_list_float4(nsp, G, cfg.n_yruns);
+    for (int k = threadIdx.x; k < words4; k += kYieldThreads) s_dyn[k] = cfg.ylist[k];
+    __syncthreads();
+    const YieldGroup* groups = reinterpret_cast<const YieldGroup*>(s_dyn);
+    const float4* list = s_dyn + G + cfg.n_yruns;
     const int32_t* gst = reinterpret_cast<const int32_t*>(list + nsp);
     const int32_t* rst = gst + G + 1;
     const int32_t* mem = rst + cfg.n_yruns + 1;
     const int64_t n = cfg.n_cells;
-    for (int64_t l = static_cast<int64_t>(blockIdx.x) * kYieldThreads + threadIdx.x; l < n;
-         l += static_cast<int64_t>(gridDim.x) * kYieldThreads) {
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        uint32_t turn = 0;
+        if (lane == 0) turn = atomicAdd(off_table + 1 + blockIdx.y, 1u);
+        const int64_t l0 = static_cast<int64_t>(__shfl_sync(FULL, turn, 0)) * 32;
+        if (l0 >= n) break;
+        const int64_t l = min(l0 + lane, n - 1);
         const float4 da = cells.da[l];
-        if (da.x < 0.0f) continue;
+        const bool live = l0 + lane < n && !(da.x < 0.0f);
         const CellYieldIn c = cell_yield_in<kBulk, kDiff>(cfg, cells, l, da);
         const int64_t row0 = static_cast<int64_t>(surface_of(cfg.surf, cfg.n_surfaces, l)) * nsp;
         for (int g = blockIdx.y; g < G; g += gridDim.y) {
             const YieldGroup gr = groups[g];
+            if (!(live && off_series(c, gr))) continue;
             float2 xy = make_float2(0.0f, 0.0f);
             float mu_of = __int_as_float(0x7fc00000);
             bool off = false;
@@ -594,6 +620,7 @@ yields_off_table_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yie
                 if (yv > 0.0f) atomicMax(ymax + row0 + mem[t], __float_as_uint(yv));
             }
         }
+        __syncwarp();
     }
 }
 
@@ -926,10 +953,11 @@ cdf_tile_scan_kernel(const float* __restrict__ yields, int64_t N, const SurfSeg*
 
 cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, float* yields, uint32_t* ymax,
                           int num_sms, cudaStream_t stream) {
-    // ymax and, behind it, the flag of arguments off the tables
+    // ymax and, behind it, the flag of arguments off the tables and the turns of
+    // the kernel that evaluates them
     const size_t rows = static_cast<size_t>(cfg.n_surfaces) * cfg.n_species;
     uint32_t* off_table = ymax + rows;
-    cudaError_t e0 = cudaMemsetAsync(ymax, 0, sizeof(uint32_t) * (rows + 1), stream);
+    cudaError_t e0 = cudaMemsetAsync(ymax, 0, sizeof(uint32_t) * (rows + kYieldFlags), stream);
     if (e0 != cudaSuccess) return e0;
     if (cfg.n_cells <= 0) return cudaSuccess;
     // two cells per thread once a row of blocks is more than the groups can
@@ -948,15 +976,18 @@ cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, float* 
         {yields_kernel<kNoBulk, false, 1>, yields_kernel<kNoBulk, false, 2>, yields_kernel<kNoBulk, true, 1>},
         {yields_kernel<kBulkCe, false, 1>, yields_kernel<kBulkCe, false, 2>, yields_kernel<kBulkCe, true, 1>},
         {yields_kernel<kBulk14, false, 1>, yields_kernel<kBulk14, false, 2>, yields_kernel<kBulk14, true, 1>}};
-    using OffKernel = void (*)(DevConfig, CellArrays, float*, uint32_t*, const uint32_t*);
+    using OffKernel = void (*)(DevConfig, CellArrays, float*, uint32_t*, uint32_t*);
     const OffKernel off_kernels[3][2] = {
         {yields_off_table_kernel<kNoBulk, false>, yields_off_table_kernel<kNoBulk, true>},
         {yields_off_table_kernel<kBulkCe, false>, yields_off_table_kernel<kBulkCe, true>},
         {yields_off_table_kernel<kBulk14, false>, yields_off_table_kernel<kBulk14, true>}};
     const Kernel kernel = kernels[bulk][cfg.include_diff ? 2 : per_thread - 1];
+    const OffKernel off_kernel = off_kernels[bulk][cfg.include_diff ? 1 : 0];
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(off_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
     }
     // rows of species groups: as tuned (per 128 cells), more where that leaves
@@ -968,7 +999,8 @@ cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, float* 
     want = std::max(want, static_cast<int>((static_cast<int64_t>(num_sms) * (per_thread == 2 ? 16 : 21) + blocks - 1) / blocks));
     const unsigned groups = static_cast<unsigned>(std::max(1, std::min(want, cfg.n_ygroups)));
     kernel<<<dim3(blocks, groups), kYieldThreads, smem, stream>>>(cfg, cells, yields, ymax, off_table);
-    off_kernels[bulk][cfg.include_diff ? 1 : 0]<<<dim3(std::min(blocks, 2u * static_cast<unsigned>(num_sms)), 4), kYieldThreads, 0, stream>>>(
+    const unsigned turns = static_cast<unsigned>((cfg.n_cells + kYieldThreads - 1) / kYieldThreads);
+    off_kernel<<<dim3(std::min(turns, static_cast<unsigned>(num_sms)), kOffRows), kYieldThreads, smem, stream>>>(
         cfg, cells, yields, ymax, off_table);
     return cudaGetLastError();
 }
