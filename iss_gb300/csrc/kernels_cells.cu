@@ -212,7 +212,7 @@ __device__ __forceinline__ void series_term(const DevConfig& cfg, const CellYiel
         }
         const float arg = xh;
         const float em = expf(-xh) * (1.0f - xl);
-        float I = em / arg * (2.0f / (arg * arg) + 2.0f / arg - 0.5f) + 0.375f * En[0];
+        float I = fmaf(0.375f, En[0], __fmul_rn(em / arg, 2.0f / __fmul_rn(arg, arg) + 2.0f / arg - 0.5f));
         // 3 (2k-5)!! / (2^k k!) for k = 3..10
         const float ck[8] = {0.0625f, 0.0234375f, 0.01171875f, 0.0068359375f,
                              0.00439453125f, 0.0030212402343750f,
@@ -277,14 +277,15 @@ __device__ __forceinline__ float2 yield_coefs(const CellYieldIn& c, const YieldG
         x = fmaf(c.bulkPi, fmaf(__fmul_rn(r1, m2), cf.x, __fmul_rn(r3, cf.z)), x);
         y = __fmul_rn(__fmul_rn(c.bulkPi, r2), cf.y);
     }
-    x *= c.da0;
-    y *= c.da0;
     if (kDiff) {
-        const float r4 = m2 * T * T * ss.q1;
-        const float r5 = (T * T * T / 3.0f) * ss.q2;
-        const float dq = c.dsq * c.inv_kappa;
-        x -= dq * c.pref_q * r4;
-        y -= dq * r5;
+        const float r4 = __fmul_rn(m2 * T * T, ss.q1);
+        const float r5 = __fmul_rn(T * T * T / 3.0f, ss.q2);
+        const float dq = __fmul_rn(c.dsq, c.inv_kappa);
+        x = fmaf(x, c.da0, -__fmul_rn(__fmul_rn(dq, c.pref_q), r4));
+        y = fmaf(y, c.da0, -__fmul_rn(dq, r5));
+    } else {
+        x = __fmul_rn(x, c.da0);
+        y = __fmul_rn(y, c.da0);
     }
     return make_float2(c.unit_pref * x, c.unit_pref * y);
 }
@@ -317,7 +318,7 @@ __device__ __forceinline__ CellYieldIn cell_yield_in(const DevConfig& cfg, const
     c.dsq = c.pref_q = c.inv_kappa = 0.0f;
     if (kDiff) {
         const float4 p2 = cells.pi2[l];
-        c.dsq = p2.y * da.y + p2.z * da.z + p2.w * da.w;
+        c.dsq = fmaf(p2.w, da.w, fmaf(p2.y, da.y, __fmul_rn(p2.z, da.z)));
         c.pref_q = c.th2.z / (c.th2.x + c.th2.y);
         c.inv_kappa = 1.0f / c.cf.w;
     }
