@@ -1288,12 +1288,13 @@ __device__ __forceinline__ bool try_efa(const DevConfig& cfg, const PropEfa& p, 
 // rejected whatever its phi and y are.  About one in twenty survives.  The
 // margins (epsilons of 2e-6 of the largest terms, 1 % on the whole) are far above
 // the rounding of try_efa's own sums; where the bound does not hold (no
-// restrict_deltaf, energies at the peak or below a boson's mu) it is infinite,
-// and a NaN rejects nothing.
+// restrict_deltaf, energies at the peak or below a boson's mu, the negative
+// maximum of a boson with a mu above its mass) it is infinite, and a NaN rejects
+// nothing.
 constexpr int kEfaBins = 32;
 __device__ float efa_bin_bound(const DevConfig& cfg, const PropEfa& p, int bin) {
     const float inf = __int_as_float(0x7f800000);
-    if (!cfg.restrict_df) return inf;
+    if (!cfg.restrict_df || !(p.bmax > 0.0f)) return inf;
     const float pa = cfg.pt_max * sqrtf(bin * (1.0f / kEfaBins));
     const float pb = cfg.pt_max * sqrtf((bin + 1) * (1.0f / kEfaBins));
     const float uT2 = p.u1 * p.u1 + p.u2 * p.u2;
