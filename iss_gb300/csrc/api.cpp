@@ -311,6 +311,8 @@ iss_status fail(iss_handle* h, iss_status st, const char* fmt, ...) {
         }                                                                                   \
     } while (0)
 
+constexpr char kTooManyHadrons[] = "more hadrons of one species in one event than an int32 counts";
+
 // The species list of the yields kernel (YieldGroup, device_common.cuh).  The
 // thermal series of calculate_dN_analytic (src/FSSW.cpp:719-848) depends on a
 // species only through its mass, statistics, number of terms and chemical
@@ -1409,6 +1411,7 @@ iss_status replay_graph(iss_handle* h, bool* done) {
     CUDA_TRY(h, cudaStreamSynchronize(s));
     h->yields_valid = true;
     if (g->count_err == 2) return fail(h, ISS_ERR_OUT_OF_RANGE, "negative particle yield (dN < 0)");
+    if (g->count_err == 4) return fail(h, ISS_ERR_OUT_OF_RANGE, "%s", kTooManyHadrons);
     if (g->count_err != 0) return fail(h, ISS_ERR_SAMPLING, "count draw did not converge");
     if (g->limits[1] != 0) {
         // more draws than the captured buffers hold: nothing was sampled
@@ -1585,6 +1588,7 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
     std::vector<int64_t> chunk_item(h->eh->tail + E + 1, h->eh->tail + E + 1 + n_chunks);
     chunk_item.push_back(n_items);
     if (count_err == 2) return fail(h, ISS_ERR_OUT_OF_RANGE, "negative particle yield (dN < 0)");
+    if (count_err == 4) return fail(h, ISS_ERR_OUT_OF_RANGE, "%s", kTooManyHadrons);
     if (count_err != 0) return fail(h, ISS_ERR_SAMPLING, "count draw did not converge");
     const bool graph_mode = graph_eligible(h, host_out, sink != nullptr);
     // a call that will be captured gets 15 % headroom in the buffers whose

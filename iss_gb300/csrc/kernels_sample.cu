@@ -320,6 +320,12 @@ count_consts_rows_kernel(DevConfig cfg, const double* __restrict__ totals, Poiss
     poisson_inv_table(c, inv[s]);
 }
 
+// records of a segment at most: a count is an int32, and rounding it up to work
+// items adds up to an item's draws.  A mean above it comes of a surface that is
+// not one (a space-time rapidity of 25, whose boost cancels in float); the
+// count would wrap and the segments' offsets with it.
+constexpr int64_t kMaxCount = 0x7FFFFFFF - 1024;
+
 // Count of species s in event e (mean dN; pc0 and inv: the Poisson constants and
 // inversion table of that mean), its records and work items
 __device__ __forceinline__ void draw_count(const DevConfig& cfg, const SpeciesDev& sp, int s, int e, double dN,
@@ -337,6 +343,8 @@ __device__ __forceinline__ void draw_count(const DevConfig& cfg, const SpeciesDe
         nsamp = 0;   // sampled as partners of the positive species
     } else if (dN < 0) {
         atomicCAS(error, 0, 2);
+    } else if (dN > kMaxCount) {
+        nsamp = kMaxCount + 1;
     } else if (cfg.sampling_model == 1) {
         const uint4 w = block(0u, 0u, c2, c3, cfg.key0, cfg.key1);
         nsamp = dN_int + (u53(w.x, w.y) < frac ? 1 : 0);
@@ -358,8 +366,13 @@ __device__ __forceinline__ void draw_count(const DevConfig& cfg, const SpeciesDe
                                             cfg.tab.logfact, inv);
         if (nsamp < 0) atomicCAS(error, 0, 3);
     }
+    const int mult = records_per_draw(cfg, sp);
+    if (nsamp > kMaxCount / mult) {
+        atomicCAS(error, 0, 4);
+        nsamp = 0;
+    }
     const int32_t c = static_cast<int32_t>(nsamp < 0 ? 0 : nsamp);
-    counts[seg] = c * records_per_draw(cfg, sp);       // records of the segment
+    counts[seg] = c * mult;       // records of the segment
     items[item_index(cfg, e, s)] = (c + cfg.item_size - 1) / cfg.item_size;
 }
 
