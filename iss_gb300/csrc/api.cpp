@@ -1709,16 +1709,19 @@ iss_status run_generate(iss_handle* h, iss_hadron_t* host_out = nullptr, int64_t
         if (dst != ISS_OK) return dst;
     }
     // iss_gpu_generate_into: consecutive chunks are sampled by one launch until
-    // it holds kGroupRecords hadrons (or half of them all).  A launch ends with
-    // a tail of some 50 us (its longest work items), in which the link copies
-    // 256k records, so smaller launches only add tails; larger ones leave the
-    // link idle for longer before the first copy (512k, 1M and 4M records: 300
-    // events of 200,000 cells 3.81, 3.86 and 4.07 ms, 3.80 so).  The learned
+    // it holds kGroupRecords hadrons, or half of them all.  A launch ends with a
+    // tail of some 50 us (its longest work items), in which the link copies 256k
+    // records, so smaller launches only add tails; larger ones leave the link
+    // idle for longer before the first copy (200,000 cells, calls of 2.7 and 13.3 M
+    // hadrons: 1.23 and 3.59 ms with 128k and 256k records, 1.24 and 3.59 with
+    // 512k, 1.29 and 3.63 with 1M, 1.32 and 3.82 with 4M).  Half of a small call's
+    // records: its first half is copied while the second is sampled (20,000 cells,
+    // calls of 48,000, 97,000, 199,000 and 398,000 hadrons: 205, 229, 287 and 360
+    // us with two launches, 203, 232, 293 and 366 with one).  The learned
     // sampler, slower than the link, takes twice as many (1.77 -> 1.65 ms on
-    // 50,000 cells and 200 events).  The launches alternate
-    // between two streams, so that one's tail runs beside the next one.
-    // (37,211 cells, 37 events, 146,000 hadrons: 13 launches in a row took
-    // 0.77 ms.)
+    // 50,000 cells and 200 events).  The launches alternate between two streams,
+    // so that one's tail runs beside the next one.  (37,211 cells, 37 events,
+    // 146,000 hadrons: 13 launches in a row took 0.77 ms.)
     const int64_t group_records =
         std::min(h->use_learned ? kLearnedGroupRecords : kGroupRecords, (n_units + 1) / 2);
     if (grouped && n_chunks > 1) {
@@ -1991,8 +1994,9 @@ iss_status ensure_host_copy(iss_handle* h) {
 // and written, one chunk being formatted and copied while another is written.
 // The chunks' buffers (kOscarBuffers x kOscarChunk on either side) stay with
 // the handle: allocating and pinning them for each call took longer than the
-// write itself (222,078 hadrons, 57 MB to a RAM disk: 8.3 ms, now 4.6, of which
-// the write is 4.5).  Chunks of 8 MB start the write after some 60 us.
+// write itself (222,385 hadrons, 57 MB to a RAM disk: 8.1 ms, now 4.6; writing
+// the same bytes from ordinary memory takes 3.3).  Chunks of 8 MB start the write
+// after some 60 us.
 constexpr int64_t kOscarChunk = int64_t(8) << 20;
 constexpr int kOscarBuffers = 2;
 

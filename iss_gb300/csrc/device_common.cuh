@@ -71,7 +71,7 @@ struct DevConfig {
     // 0: the pilot envelope alone, whose ratios above 1 are counted
     int lexact;
     // launch shape (results do not depend on it; the autotuner picks it)
-    int item_size;       // draws per sampler work item (multiple of 32, <= 1024)
+    int item_size;       // draws per sampler work item (even, <= 1024)
     int yield_groups;    // species groups per cell in the yields kernel (grid y)
     // yields kernel: the yield list (YieldGroup) of n_ygroups groups and
     // n_yruns runs

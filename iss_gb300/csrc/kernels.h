@@ -40,12 +40,16 @@ struct CdfBuffers {
 // guide tables of the dense rows.  surf is a device array.
 //
 // A CDF row costs about 2 ps per cell to write, a draw on a sparse row some
-// 30 ps more than on a dense one: at 16 cells per draw both calls with few and
-// with many events gain (200,000 cells, CDF and sampling together: 1 event 402 ->
-// 124 us, 300 events 1177 -> 1081, 1,000 events 2701 -> 2751 for 475 us less
-// before them; at 8 cells per draw 300 events take 1083 us and 1,000 2794, at 32
-// 1083 and 2762).  Below 2048 tiles (13,000 cells of 319 species) the rows are
-// written in a wave or two of blocks, less than the longer search takes.
+// 30 ps more than on a dense one.  200,000 cells, CDF and counts + sampling, us:
+//   events    all rows written   16 cells per draw    8               32
+//        1         384 +    35         113 +   44     113 +   45      113 +   45
+//       30         390 +   125         150 +  165     148 +  164      153 +  163
+//      300         409 +   780         238 +  884     231 +  918      279 +  813
+//    1,000         503 + 2,420         434 + 2,465    350 + 2,617     480 + 2,430
+// so calls with few events gain most, and with many the longer sampling stays
+// below what the rows cost (the sample phase by itself gets 2 % longer).  Below
+// 2048 tiles (13,000 cells of 319 species) the rows are written in a wave or two
+// of blocks, less than the longer search takes.
 constexpr int kSparseDraws = 16;
 constexpr int64_t kSparseTiles = 2048;
 cudaError_t launch_cdf_head(const float* yields, int64_t N, const SurfSeg* surf, int n_surf,
@@ -64,9 +68,10 @@ cudaError_t launch_cdf_scan(const float* yields, int64_t N, const SurfSeg* surf,
 cudaError_t launch_counts(const DevConfig& cfg, const SpeciesDev* species, const double* totals,
                           double* pois, int32_t* counts, int32_t* items, int* error,
                           int* launches, cudaStream_t stream);
-// draws per work item of the lab-frame sampler (even: the cell assignment
-// pairs draws)
+// draws per work item of the lab-frame sampler (even, as every item size: the
+// cell assignment pairs draws 2k and 2k + 1 on a Philox block)
 constexpr int kEfaItem = 4;
+static_assert(kEfaItem % 2 == 0, "an item starts at an even draw");
 int offsets_num_tiles(int64_t n);
 cudaError_t launch_offsets_scan(const int32_t* counts, int64_t n, int64_t* tile_sum,
                                 int64_t* offsets, cudaStream_t stream);

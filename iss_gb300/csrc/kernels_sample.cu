@@ -1782,7 +1782,7 @@ cell_assign_kernel(DevConfig cfg_in, const __grid_constant__ CellRows rows, cons
         const uint32_t c3 = static_cast<uint32_t>(s) | (kTagCell << 16);
         // 64 draws at a time: each lane takes the pair (2k, 2k + 1), whose
         // 64-bit uniforms are the two halves of one Philox block with counter
-        // k (d_begin is even: item sizes are multiples of 32), and issues both
+        // k (d_begin is even: item sizes are), and issues both
         // guide lookups before either search, so their latencies overlap
         for (int64_t d_sub = d_begin; d_sub < d_end; d_sub += kAssignSub) {
         const int64_t d0 = d_sub + 2 * lane, d1 = d0 + 1;
@@ -2088,10 +2088,12 @@ sampler_kernel(DevConfig cfg_in, CellArrays cells, const SpeciesDev* __restrict_
 
 // The lab-frame sampler (MC_sampling = 2).  A hadron takes about 1,900
 // proposals on average and up to max_tries x (max_redraws + 1), so one hadron
-// belongs to a whole warp: the 32 lanes make proposals t .. t + 31, those that
-// the bound of their pT bin does not reject are queued, and whenever 32 are
-// queued the warp evaluates them; the first accepted one (lowest counter) is
-// the hadron, which is the draw a single lane would have made one by one.  A
+// belongs to a whole warp: in a step the 32 lanes make four proposals each
+// (kEfaUnroll), those that the bound of their pT bin does not reject are queued
+// in the order of their counters, and whenever a step leaves 24 (kEfaBatch) or
+// more in the queue the warp evaluates them, up to 32 at a time; the first
+// accepted one (lowest counter) is the hadron, which is the draw a single lane
+// would have made one by one.  A
 // lane per hadron, as the FSSW kernel has it, left the chip waiting for the few
 // lanes with the longest chains: 50,000 cells, 40 events, 213,000 hadrons took
 // 194 ms; 2.84 ms with every proposal evaluated, 1.87 so.  The kernel is bound
