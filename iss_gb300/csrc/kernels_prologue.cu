@@ -84,9 +84,10 @@ __device__ void ce_neos_coeff(const double* tb, double Edec, double nB, double* 
     const int Ne1 = idx_e * 200, Ne2 = (idx_e + 1) * 200;
     const double e_frac = (Edec - tb[5 * Ne1]) / de;
     const double dnB1 = tb[5 * (Ne1 + 1) + 1], dnB2 = tb[5 * (Ne2 + 1) + 1];
-    // the reference clamps these indices from above only
-    const int i1 = min(198, static_cast<int>(nB / dnB1));
-    const int i2 = min(198, static_cast<int>(nB / dnB2));
+    // the reference clamps these indices from above only: a negative density
+    // reads the rows of lower energy densities, here not past the table's start
+    const int i1 = max(-Ne1, min(198, static_cast<int>(nB / dnB1)));
+    const int i2 = max(-Ne2, min(198, static_cast<int>(nB / dnB2)));
     const double f1 = fmin(1., (nB - tb[5 * (Ne1 + i1) + 1]) / dnB1);
     const double f2 = fmin(1., (nB - tb[5 * (Ne2 + i2) + 1]) / dnB2);
     double c[3];
