@@ -15,8 +15,7 @@ cudaError_t launch_cell_prologue(const DevConfig& cfg, const float* fo34, int64_
 // words behind them, zeroed here first), the largest yield of every (surface,
 // species) row as float bits; two launches, the second of which leaves at once
 // unless an argument was off the special-function tables
-constexpr int kOffRows = 16;
-constexpr int kYieldFlags = 1 + kOffRows;
+constexpr int kYieldFlags = 2;   // an argument was off the tables; turns taken of those
 cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, float* yields, uint32_t* ymax,
                           int num_sms, cudaStream_t stream);
 int cdf_num_tiles(int64_t n);

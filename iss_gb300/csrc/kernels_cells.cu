@@ -565,15 +565,25 @@ __device__ __forceinline__ bool off_series(const CellYieldIn& c, const YieldGrou
 }
 
 // The yields that yields_kernel left out, where it left out any: the series
-// with an argument off the tables, evaluated directly.  Row y of the grid takes
-// every kOffRows-th group; its warps fetch 32 cells at a time, since 32 hot cells
-// cost a thousand times what others do: in a grid over the cells whose blocks
-// took one turn or two, all waited for those with two.  Bound by the FP64 pipe.
-// Calls of 50,000 cells at 0.3 GeV 15.6 -> 11.3 ms (11.6 with the evaluation
-// inlined in the yields kernel), at 5 MeV 2.13 -> 1.41 (1.46; 1.59 in 8 rows
-// instead of 16), 20,000 at 0.5 MeV, where all is zero, 0.37 -> 0.15 (0.28).
+// with an argument off the tables, evaluated directly, by blocks of a warp in
+// turns of 32 cells and every kOffRows-th group.  32 hot cells cost a thousand
+// times what others do and the FP64 pipe of their SM bounds them, so what counts
+// is that the dear turns (those of the first rows: the groups come in decreasing
+// order of work) are spread over the SMs: the first turn goes by the place of the
+// block, the next ones to the warps that come free.  (A grid over the cells, whose
+// blocks take one turn or two, waits for those with two; first turns by arrival
+// leave SMs without; 4, 5, 6 and 8 blocks per SM: 20,000 cells at 0.3 GeV 6.0, 5.0,
+// 5.0 and 5.8 ms, with diffusion 4.5, 2.9, 3.2 and 4.2.)
+// Calls of one event, ms, with the evaluation inlined in the yields kernel, in a
+// grid of 304 blocks over the cells and so: 1,000 cells at 0.3 GeV 2.24, 2.17, 1.97;
+// 20,000 5.88, 7.77, 5.03; 50,000 11.55, 15.59, 11.07; 100,000, one in 40 of them hot
+// 19.2, 18.4, 15.6; 20,000 with diffusion 4.41, 4.43, 2.87; 50,000 at 5 MeV 1.46, 2.13,
+// 1.26; 20,000 at 0.5 MeV, where all is zero, 0.28, 0.37, 0.15.
+constexpr int kOffRows = 16;
+constexpr int kOffBlocks = 5;   // per SM
+
 template <int kBulk, bool kDiff>
-__global__ void __launch_bounds__(kYieldThreads)
+__global__ void __launch_bounds__(32)
 yields_off_table_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yields, uint32_t* __restrict__ ymax,
                         uint32_t* __restrict__ off_table) {
     if (*off_table == 0u) return;
@@ -582,26 +592,28 @@ yields_off_table_kernel(DevConfig cfg, CellArrays cells, float* __restrict__ yie
     const int nsp = cfg.n_species;
     const int G = cfg.n_ygroups;
     const int words4 = yield_list_float4(nsp, G, cfg.n_yruns);
-    for (int k = threadIdx.x; k < words4; k += kYieldThreads) s_dyn[k] = cfg.ylist[k];
-    __syncthreads();
+    for (int k = threadIdx.x; k < words4; k += 32) s_dyn[k] = cfg.ylist[k];
+    __syncwarp();
     const YieldGroup* groups = reinterpret_cast<const YieldGroup*>(s_dyn);
     const float4* list = s_dyn + G + cfg.n_yruns;
     const int32_t* gst = reinterpret_cast<const int32_t*>(list + nsp);
     const int32_t* rst = gst + G + 1;
     const int32_t* mem = rst + cfg.n_yruns + 1;
     const int64_t n = cfg.n_cells;
-    const int lane = threadIdx.x & 31;
-    for (;;) {
-        uint32_t turn = 0;
-        if (lane == 0) turn = atomicAdd(off_table + 1 + blockIdx.y, 1u);
-        const int64_t l0 = static_cast<int64_t>(__shfl_sync(FULL, turn, 0)) * 32;
-        if (l0 >= n) break;
+    const int lane = threadIdx.x;
+    // the first turns by the place of the block, which spreads the dear ones over
+    // the SMs, the others as warps come free
+    const int64_t chunks = (n + 31) / 32;
+    for (int64_t turn = blockIdx.x; turn < chunks * kOffRows;
+         turn = gridDim.x + static_cast<int64_t>(__shfl_sync(FULL, lane == 0 ? atomicAdd(off_table + 1, 1u) : 0u, 0))) {
+        const int row = static_cast<int>(turn / chunks);
+        const int64_t l0 = (turn - row * chunks) * 32;
         const int64_t l = min(l0 + lane, n - 1);
         const float4 da = cells.da[l];
         const bool live = l0 + lane < n && !(da.x < 0.0f);
         const CellYieldIn c = cell_yield_in<kBulk, kDiff>(cfg, cells, l, da);
         const int64_t row0 = static_cast<int64_t>(surface_of(cfg.surf, cfg.n_surfaces, l)) * nsp;
-        for (int g = blockIdx.y; g < G; g += gridDim.y) {
+        for (int g = row; g < G; g += kOffRows) {
             const YieldGroup gr = groups[g];
             if (!(live && off_series(c, gr))) continue;
             float2 xy = make_float2(0.0f, 0.0f);
@@ -1000,9 +1012,9 @@ cudaError_t launch_yields(const DevConfig& cfg, const CellArrays& cells, float* 
     want = std::max(want, static_cast<int>((static_cast<int64_t>(num_sms) * (per_thread == 2 ? 16 : 21) + blocks - 1) / blocks));
     const unsigned groups = static_cast<unsigned>(std::max(1, std::min(want, cfg.n_ygroups)));
     kernel<<<dim3(blocks, groups), kYieldThreads, smem, stream>>>(cfg, cells, yields, ymax, off_table);
-    const unsigned turns = static_cast<unsigned>((cfg.n_cells + kYieldThreads - 1) / kYieldThreads);
-    off_kernel<<<dim3(std::min(turns, static_cast<unsigned>(num_sms)), kOffRows), kYieldThreads, smem, stream>>>(
-        cfg, cells, yields, ymax, off_table);
+    const int64_t turns = (cfg.n_cells + 31) / 32 * kOffRows;
+    const unsigned off_blocks = static_cast<unsigned>(std::min<int64_t>(turns, static_cast<int64_t>(num_sms) * kOffBlocks));
+    off_kernel<<<off_blocks, 32, smem, stream>>>(cfg, cells, yields, ymax, off_table);
     return cudaGetLastError();
 }
 
